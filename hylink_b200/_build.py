@@ -10,7 +10,7 @@ Produces, under ``hylink_b200/lib/``:
   on a machine without a GPU.
 * ``libhylink_nccl.so`` — the drop-in ``nccl*`` symbol layer; ``libhylink_cudashim.so`` — opt-in
   interposers of host-blocking CUDA runtime calls.
-* ``_hylink_c10d.so`` — the ``torch.distributed`` backend extension.
+* ``_hylink_c10d.so`` — the ``torch.distributed`` backend extension; ``_hylink_ops.so`` — the training-step operators.
 
 and ``hylink_b200/bin/hl_perf``, the stand-alone test executable.
 
@@ -33,7 +33,7 @@ CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
-CORE_DIRS = ["core", "ctrl", "hal", "ir", "host", "pcie", "nvl", "orch", "api"]
+CORE_DIRS = ["core", "ctrl", "hal", "ir", "host", "pcie", "nvl", "orch", "api", "train"]
 SEPARATE = {"nccl_shim.cpp", "cuda_block_shim.cpp"}  # built into libhylink_nccl.so
 
 
@@ -122,7 +122,14 @@ def build_nccl_shim(verbose: bool = False) -> Path | None:
 
 
 def build_torch_ext(verbose: bool = False) -> Path | None:
-    src = CSRC / "torch" / "backend.cpp"
+    """The two torch extensions: the process-group backend and the training-step operators."""
+    with cf.ThreadPoolExecutor(max_workers=2) as ex:
+        built = list(ex.map(lambda n: _torch_ext(*n, verbose), [("backend.cpp", "_hylink_c10d"), ("ops.cpp", "_hylink_ops")]))
+    return built[0]
+
+
+def _torch_ext(src_name: str, module: str, verbose: bool) -> Path | None:
+    src = CSRC / "torch" / src_name
     if not src.exists():
         return None
     import sysconfig
@@ -130,14 +137,14 @@ def build_torch_ext(verbose: bool = False) -> Path | None:
     import torch
     from torch.utils import cpp_extension as ce
 
-    target = LIB / "_hylink_c10d.so"
+    target = LIB / f"{module}.so"
     hdr = _newest_header()
     if target.exists() and target.stat().st_mtime > max(src.stat().st_mtime, hdr):
         return target
     tlib = Path(torch.__file__).parent / "lib"
     inc = [f"-I{p}" for p in ce.include_paths()] + [f"-I{sysconfig.get_paths()['include']}",
                                                      f"-I{CSRC}", f"-I{CSRC / 'include'}", f"-I{CUDA_HOME / 'include'}"]
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-pthread", "-DTORCH_EXTENSION_NAME=_hylink_c10d",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-pthread", f"-DTORCH_EXTENSION_NAME={module}",
            "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
            "-Wno-interference-size", *inc, str(src), "-o", str(target), f"-L{tlib}", "-ltorch", "-ltorch_cpu", "-lc10",
            "-ltorch_python", "-ltorch_cuda", "-lc10_cuda", f"-L{LIB}", "-lhylink_b200",

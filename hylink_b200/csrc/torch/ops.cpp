@@ -1,0 +1,271 @@
+// Autograd functions of the training step over the kernels of csrc/train: what surrounds the GEMMs and the attention
+// of a transformer block, and the language-model head with its loss. The GEMMs are torch's own (cuBLAS), the
+// attention between the two halves of a block is whatever torch's scaled_dot_product_attention picks.
+//
+// A block is cut in two around the attention:
+//   blockPre:   x1 = x + y; h = layer norm(x1); q, k, v = h Wqkv^T + b     (y: the branch of the block before)
+//   blockPost:  x2 = x1 + a Wproj^T + b; h = layer norm(x2); y2 = gelu(h Wfc^T + b) Wout^T + b;  returns x2, y2
+// The add of y2 is left to the next block's (or the final) layer norm, which reads x2 anyway.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/python.h>
+
+#include "train/train_kernels.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+namespace train = hl::train;
+
+void ok(hlResult_t r, const char* what) {
+  if (r != hlSuccess) TORCH_CHECK(false, "hylink ", what, ": ", hlGetErrorString(r), " (", hlGetLastError(), ")");
+}
+int code(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kHalf: return hlFloat16;
+    case at::kBFloat16: return hlBfloat16;
+    default: TORCH_CHECK(false, "hylink: training kernels take fp16 and bf16 tensors");
+  }
+}
+cudaStream_t streamOf(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+Tensor floats(const Tensor& like, at::IntArrayRef sizes) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+// Rows of a [..., width] tensor as one matrix.
+Tensor rowsOf(const Tensor& t) { return t.is_contiguous() ? t.view({-1, t.size(-1)}) : t.reshape({-1, t.size(-1)}); }
+Tensor dense(const Tensor& t) { return t.contiguous(); }
+
+// The gradients below are computed by kernels that autograd does not see into.
+void onceOnly() { TORCH_CHECK(!at::GradMode::is_enabled(), "hylink: the fused training step is differentiable once"); }
+
+// Column-sum partials collected over a backward pass and added up in one launch.
+class Columns {
+ public:
+  explicit Columns(const Tensor& like) : like_(like) {}
+  Tensor add(const float* src, int rows, int64_t width) {
+    Tensor out = at::empty({width}, like_.options());
+    segs_[n_++] = {src, out.data_ptr(), rows, (int)width};
+    return out;
+  }
+  void finish() { ok(train::finishColumns(code(like_), segs_, n_, streamOf(like_)), "column sums"); }
+
+ private:
+  Tensor like_;
+  train::ColSegment segs_[train::kMaxColSegments];
+  int n_ = 0;
+};
+
+struct Normed {
+  Tensor sum, out, mean, rstd;
+};
+// Layer norm of x + y (y may be undefined). Forward stays with torch's kernels: their results are what the layers above
+// see, and a 24-layer model turns a last-bit difference in one mean into rounding noise everywhere.
+Normed normForward(const Tensor& x, const Tensor& y, const Tensor& gamma, const Tensor& beta, double eps) {
+  Normed r;
+  r.sum = y.defined() ? at::add(x, y) : x;
+  std::tie(r.out, r.mean, r.rstd) = at::native_layer_norm(r.sum, {x.size(-1)}, gamma, beta, eps);
+  return r;
+}
+// Returns dx; `partials` becomes [3][parts][width].
+Tensor normBackward(const Tensor& dh, const Tensor& x, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, const Tensor& residual,
+                    Tensor* partials, int* parts) {
+  const int64_t width = x.size(-1), rows = x.numel() / width;
+  *parts = train::layerNormPartials(rows);
+  *partials = floats(x, {3, *parts, width});
+  Tensor dx = at::empty_like(x);
+  ok(train::layerNormBackward(code(x), dh.data_ptr(), x.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr(),
+                              residual.defined() ? residual.data_ptr() : nullptr, dx.data_ptr(), partials->data_ptr<float>(), rows, (int)width,
+                              streamOf(x)),
+     "layer norm backward");
+  return dx;
+}
+
+class AddNorm : public torch::autograd::Function<AddNorm> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& x_, const std::optional<Variable>& y_, const Variable& gamma, const Variable& beta, double eps) {
+    c10::cuda::CUDAGuard dg(x_.device());
+    const Tensor x = dense(x_), y = y_ ? dense(*y_) : Tensor();
+    Normed n = normForward(x, y, gamma, beta, eps);
+    ctx->save_for_backward({n.sum, n.mean, n.rstd, gamma});
+    ctx->saved_data["y"] = y.defined();
+    return n.out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    c10::cuda::CUDAGuard dg(s[0].device());
+    Tensor parts;
+    int np;
+    const int64_t w = s[0].size(-1);
+    Tensor dx = normBackward(dense(g[0]), s[0], s[1], s[2], s[3], Tensor(), &parts, &np);
+    Columns cols(s[3]);
+    const float* p = parts.data_ptr<float>();
+    Tensor dgamma = cols.add(p, np, w), dbeta = cols.add(p + np * w, np, w);
+    cols.finish();
+    return {dx, ctx->saved_data["y"].toBool() ? dx : Tensor(), dgamma, dbeta, Tensor()};
+  }
+};
+
+class BlockPre : public torch::autograd::Function<BlockPre> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const Variable& x_, const std::optional<Variable>& y_, const Variable& gamma, const Variable& beta,
+                               const Variable& w, const Variable& b, int64_t heads, double eps) {
+    c10::cuda::CUDAGuard dg(x_.device());
+    const Tensor x = dense(x_), y = y_ ? dense(*y_) : Tensor();
+    const int64_t batch = x.size(0), seq = x.size(1), width = x.size(2), hd = w.size(0) / 3 / heads;
+    Normed n = normForward(x, y, gamma, beta, eps);
+    const Tensor h = n.out.view({-1, width});
+    const Tensor qkv = at::addmm(b, h, w.t()).view({batch, seq, 3, heads, hd}).permute({2, 0, 3, 1, 4});
+    ctx->save_for_backward({n.sum, n.mean, n.rstd, gamma, h, w});
+    ctx->saved_data["y"] = y.defined();
+    return {n.sum, qkv[0], qkv[1], qkv[2]};   // without y the sum is the input itself
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &gamma = s[3], &h = s[4], &w = s[5];
+    c10::cuda::CUDAGuard dg(x.device());
+    const int64_t batch = x.size(0), seq = x.size(1), width = x.size(2);
+    const int64_t heads = g[1].size(1), hd = g[1].size(3), rows = batch * seq, n3 = 3 * heads * hd;
+    Tensor dqkv = at::empty({rows, n3}, x.options());
+    const int sp = train::stripPartials(rows);
+    Tensor bias_parts = floats(x, {sp, n3});
+    train::Strided4 gs[3];
+    Tensor keep[3];
+    for (int i = 0; i < 3; ++i) {
+      Tensor t = g[1 + i];
+      if (t.stride(3) != 1 || t.stride(0) % 8 || t.stride(1) % 8 || t.stride(2) % 8 || ((uintptr_t)t.data_ptr() & 15)) t = t.contiguous();
+      keep[i] = t;
+      gs[i] = {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)};
+    }
+    ok(train::packQkvGradient(code(x), gs, dqkv.data_ptr(), bias_parts.data_ptr<float>(), batch, seq, (int)heads, (int)hd, streamOf(x)),
+       "attention gradient");
+    Tensor dw = at::mm(dqkv.t(), h);
+    Tensor dh = at::mm(dqkv, w);
+    Tensor parts;
+    int np;
+    Tensor dx = normBackward(dh, x, s[1], s[2], gamma, g[0].defined() ? dense(g[0]) : Tensor(), &parts, &np);
+    Columns cols(gamma);
+    const float* p = parts.data_ptr<float>();
+    Tensor dgamma = cols.add(p, np, width), dbeta = cols.add(p + np * width, np, width);
+    Tensor db = cols.add(bias_parts.data_ptr<float>(), sp, n3);
+    cols.finish();
+    return {dx, ctx->saved_data["y"].toBool() ? dx : Tensor(), dgamma, dbeta, dw, db, Tensor(), Tensor()};
+  }
+};
+
+class BlockPost : public torch::autograd::Function<BlockPost> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const Variable& x_, const Variable& a_, const Variable& wp, const Variable& bp,
+                               const Variable& gamma, const Variable& beta, const Variable& wf, const Variable& bf, const Variable& wo,
+                               const Variable& bo, double eps) {
+    c10::cuda::CUDAGuard dg(x_.device());
+    const Tensor x = dense(x_), a = rowsOf(a_);
+    const int64_t width = x.size(-1);
+    const Tensor p = at::addmm(bp, a, wp.t());
+    Normed n = normForward(x, p.view(x.sizes()), gamma, beta, eps);
+    const Tensor h = n.out.view({-1, width});
+    const Tensor u = at::addmm(bf, h, wf.t());
+    Tensor act = at::empty_like(u);
+    ok(train::geluForward(code(u), u.data_ptr(), act.data_ptr(), u.numel(), streamOf(u)), "gelu");
+    const Tensor y = at::addmm(bo, act, wo.t()).view(x.sizes());
+    ctx->save_for_backward({a, wp, n.sum, n.mean, n.rstd, gamma, h, wf, u, act, wo});
+    ctx->saved_data["a"] = a_.sizes().vec();
+    return {n.sum, y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &a = s[0], &wp = s[1], &x2 = s[2], &gamma = s[5], &h = s[6], &wf = s[7], &u = s[8], &act = s[9], &wo = s[10];
+    c10::cuda::CUDAGuard dg(x2.device());
+    const int64_t width = x2.size(-1), rows = x2.numel() / width, hidden = u.size(1);
+    const int dt = code(x2), sp = train::stripPartials(rows);
+    cudaStream_t st = streamOf(x2);
+    TORCH_CHECK(g[1].defined(), "hylink: the block's branch has no gradient");
+    const Tensor gy = rowsOf(g[1]);
+    Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {sp, hidden});
+    ok(train::columnSums(dt, gy.data_ptr(), out_parts.data_ptr<float>(), rows, (int)width, st), "bias gradient");
+    Tensor dact = at::mm(gy, wo);
+    Tensor dwo = at::mm(gy.t(), act);
+    Tensor du = at::empty_like(u);
+    ok(train::geluBackward(dt, dact.data_ptr(), u.data_ptr(), du.data_ptr(), fc_parts.data_ptr<float>(), rows, (int)hidden, st), "gelu backward");
+    Tensor dwf = at::mm(du.t(), h);
+    Tensor dh = at::mm(du, wf);
+    Tensor parts;
+    int np;
+    Tensor dx = normBackward(dh, x2, s[3], s[4], gamma, g[0].defined() ? dense(g[0]) : Tensor(), &parts, &np);
+    const Tensor dxr = dx.view({rows, width});
+    Tensor dwp = at::mm(dxr.t(), a);
+    Tensor da = at::mm(dxr, wp).view(ctx->saved_data["a"].toIntVector());
+    Columns cols(gamma);
+    const float* p = parts.data_ptr<float>();
+    Tensor dgamma = cols.add(p, np, width), dbeta = cols.add(p + np * width, np, width), dbp = cols.add(p + 2 * np * width, np, width);
+    Tensor dbf = cols.add(fc_parts.data_ptr<float>(), sp, hidden), dbo = cols.add(out_parts.data_ptr<float>(), sp, width);
+    cols.finish();
+    return {dx, da, dwp, dbp, dgamma, dbeta, dwf, dbf, dwo, dbo, Tensor()};
+  }
+};
+
+// logits = h W^T and their mean cross entropy. The vocabulary is padded to a multiple of 64: an odd leading dimension
+// keeps cuBLAS off the tensor-memory kernels (8192 x 50257 x 1024 in bf16 on B200: 7.43 ms against 0.60 for the logits,
+// 4.71 against 0.55 for the weight gradient); padding the weight is a copy of 0.04 ms.
+// The input gradient sums over the vocabulary, unpadded (5.6 ms): padded it takes 0.55 ms, but there the products of
+// 50257 tiny probabilities and one large entry are added up with another rounding, the same way for every token, and
+// the gradients of a 24-layer model move by 1.4 % where run-to-run noise is 0.5 %.
+class HeadLoss : public torch::autograd::Function<HeadLoss> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& h_, const Variable& w, const Variable& targets_) {
+    c10::cuda::CUDAGuard dg(h_.device());
+    const Tensor h = rowsOf(h_), targets = targets_.reshape({-1}).contiguous();
+    const int64_t vocab = w.size(0), padded = (vocab + 63) / 64 * 64, rows = h.size(0);
+    Tensor wpad = w;
+    if (padded != vocab || !w.is_contiguous()) {
+      wpad = at::empty({padded, w.size(1)}, w.options());
+      wpad.narrow(0, 0, vocab).copy_(w);
+      if (padded != vocab) wpad.narrow(0, vocab, padded - vocab).zero_();
+    }
+    Tensor logits = at::mm(h, wpad.t());
+    Tensor lse = floats(h, {rows}), row_loss = floats(h, {rows}), loss = floats(h, {2});
+    ok(train::crossEntropyForward(code(h), logits.data_ptr(), padded, targets.data_ptr<int64_t>(), rows, (int)vocab, -100, lse.data_ptr<float>(),
+                                  row_loss.data_ptr<float>(), loss.data_ptr<float>(), streamOf(h)),
+       "cross entropy");
+    ctx->save_for_backward({h, w, targets, logits, lse, loss});
+    ctx->saved_data["h"] = h_.sizes().vec();
+    return loss.select(0, 0).clone();
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &h = s[0], &w = s[1], &targets = s[2], &logits = s[3], &lse = s[4], &loss = s[5];
+    c10::cuda::CUDAGuard dg(h.device());
+    const int64_t vocab = w.size(0);
+    const Tensor grad = g[0].to(at::kFloat).contiguous();
+    Tensor dlogits = at::empty_like(logits);
+    ok(train::crossEntropyBackward(code(h), logits.data_ptr(), logits.size(1), targets.data_ptr<int64_t>(), h.size(0), (int)vocab, -100,
+                                   lse.data_ptr<float>(), loss.data_ptr<float>(), grad.data_ptr<float>(), dlogits.data_ptr(), streamOf(h)),
+       "cross entropy backward");
+    const Tensor d = dlogits.narrow(1, 0, vocab);
+    Tensor dw = at::mm(d.t(), h);
+    Tensor dh = at::mm(d, w).view(ctx->saved_data["h"].toIntVector());
+    return {dh, dw, Tensor()};
+  }
+};
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.attr("max_norm_width") = train::kMaxNormWidth;
+  m.def("add_norm", [](const Tensor& x, const std::optional<Tensor>& y, const Tensor& gamma, const Tensor& beta, double eps) {
+    return AddNorm::apply(x, y, gamma, beta, eps);
+  });
+  m.def("block_pre", [](const Tensor& x, const std::optional<Tensor>& y, const Tensor& gamma, const Tensor& beta, const Tensor& w, const Tensor& b,
+                        int64_t heads, double eps) { return BlockPre::apply(x, y, gamma, beta, w, b, heads, eps); });
+  m.def("block_post", [](const Tensor& x, const Tensor& a, const Tensor& wp, const Tensor& bp, const Tensor& gamma, const Tensor& beta,
+                         const Tensor& wf, const Tensor& bf, const Tensor& wo, const Tensor& bo, double eps) {
+    return BlockPost::apply(x, a, wp, bp, gamma, beta, wf, bf, wo, bo, eps);
+  });
+  m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });
+}

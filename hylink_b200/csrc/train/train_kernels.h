@@ -1,0 +1,56 @@
+// Launch interface of the training-step kernels: what surrounds the GEMMs and the attention of a transformer block,
+// the language-model loss, and the optimizer. 16-bit element types only unless noted; every accumulation is fp32.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "core/core.h"
+
+namespace hl {
+namespace train {
+
+constexpr int kMaxNormWidth = 1024;   // a warp holds a whole row and three column sums in registers
+
+// Column sums end in two steps: the kernels that walk the rows write one fp32 partial per CTA and column, one later
+// launch adds up the partials of several of them. `src` is [rows][width], `dst` has the element type of the call.
+struct ColSegment {
+  const float* src;
+  void* dst;
+  int rows, width;
+};
+constexpr int kMaxColSegments = 8;
+
+// dx = residual + gradient of the layer norm at x for the output gradient dh (residual may be null).
+// partials: [3][layerNormPartials(rows)][width]: dgamma, dbeta, and the column sums of dx as stored.
+int layerNormPartials(int64_t rows);
+hlResult_t layerNormBackward(int dt, const void* dh, const void* x, const float* mean, const float* rstd, const void* gamma,
+                             const void* residual, void* dx, float* partials, int64_t rows, int width, cudaStream_t s);
+
+// out = gelu(u), tanh form.
+hlResult_t geluForward(int dt, const void* u, void* out, int64_t count, cudaStream_t s);
+// Rows a strip kernel gives to one CTA: its partials are [stripPartials(rows)][width].
+int stripPartials(int64_t rows);
+// du = dg * gelu'(u), and column-sum partials of du. width a multiple of 8.
+hlResult_t geluBackward(int dt, const void* dg, const void* u, void* du, float* partials, int64_t rows, int width, cudaStream_t s);
+// Column-sum partials of a [rows][width] matrix.
+hlResult_t columnSums(int dt, const void* src, float* partials, int64_t rows, int width, cudaStream_t s);
+// The gradients of the three attention operands, each [batch, heads, seq, head_dim] by strides (head_dim contiguous),
+// written side by side as [batch * seq][3 * heads * head_dim], with column-sum partials.
+struct Strided4 {
+  const void* p;
+  int64_t sb, sh, st;
+};
+hlResult_t packQkvGradient(int dt, const Strided4 grads[3], void* dqkv, float* partials, int64_t batch, int64_t seq, int heads, int head_dim,
+                           cudaStream_t s);
+hlResult_t finishColumns(int dt, const ColSegment* segs, int n, cudaStream_t s);
+
+// Cross entropy over the rows of `logits` ([rows] of `vocab` elements, `stride` apart, stride a multiple of 8):
+// lse[row]; loss[0] = mean over the rows whose target is not ignore_index, loss[1] = how many those are.
+// scratch: 2 floats per row.
+hlResult_t crossEntropyForward(int dt, const void* logits, int64_t stride, const int64_t* targets, int64_t rows, int vocab, int64_t ignore_index,
+                               float* lse, float* row_loss, float* loss, cudaStream_t s);
+// dlogits (same layout; the padding behind `vocab` becomes zero) for the gradient *grad of the mean loss.
+hlResult_t crossEntropyBackward(int dt, const void* logits, int64_t stride, const int64_t* targets, int64_t rows, int vocab, int64_t ignore_index,
+                                const float* lse, const float* loss, const float* grad, void* dlogits, cudaStream_t s);
+
+}  // namespace train
+}  // namespace hl

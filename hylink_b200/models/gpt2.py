@@ -16,6 +16,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops.extension import ops
+
 
 @dataclass
 class GPT2Config:
@@ -38,6 +40,10 @@ class GPT2Config:
     def by_name(name: str) -> "GPT2Config":
         return {"gpt2-medium": GPT2Config.medium, "medium": GPT2Config.medium, "tiny": GPT2Config.tiny,
                 "gpt2-small": lambda: GPT2Config(n_layer=12, n_head=12, d_model=768)}[name]()
+
+
+def _hooked(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
 
 
 class Block(nn.Module):
@@ -83,6 +89,8 @@ class GPT2(nn.Module):
         b, t = idx.shape
         pos = torch.arange(t, device=idx.device)
         x = self.wte(idx) + self.wpe(pos)
+        if targets is not None and self._fusable(x, targets):
+            return self._fused_loss(x, targets)
         for blk in self.blocks:
             x = blk(x)
         x = self.ln_f(x)
@@ -90,6 +98,38 @@ class GPT2(nn.Module):
         if targets is None:
             return logits
         return F.cross_entropy(logits.float().view(-1, logits.size(-1)), targets.reshape(-1))
+
+    def _fusable(self, x: torch.Tensor, targets: torch.Tensor) -> bool:
+        """Whether the loss can go through the fused operators: a 16-bit model on a GPU, made of the plain modules
+        above (no hooks, nothing replaced), at widths whose rows a warp can hold."""
+        c = self.config
+        if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.numel() and targets.is_cuda and targets.dtype == torch.int64):
+            return False
+        if c.d_model > ops().max_norm_width or c.d_model % 8 or (c.d_model // c.n_head) % 8 or torch.is_autocast_enabled("cuda"):
+            return False
+        mods = [self.ln_f, self.wte]
+        for blk in self.blocks:
+            if type(blk) is not Block or _hooked(blk):
+                return False
+            mods += (blk.ln1, blk.qkv, blk.proj, blk.ln2, blk.fc, blk.out)
+        for m in mods:
+            if type(m) not in (nn.LayerNorm, nn.Linear, nn.Embedding) or _hooked(m) or m.weight.dtype != x.dtype:
+                return False
+            if type(m) is not nn.Embedding and m.bias is None:
+                return False
+        return True
+
+    def _fused_loss(self, x: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        f = ops()
+        b, t, d = x.shape
+        branch = None      # what the block before adds to the residual stream: the next layer norm reads both
+        for blk in self.blocks:
+            x, q, k, v = f.block_pre(x, branch, blk.ln1.weight, blk.ln1.bias, blk.qkv.weight, blk.qkv.bias, blk.n_head, blk.ln1.eps)
+            a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
+            x, branch = f.block_post(x, a.transpose(1, 2).reshape(b, t, d), blk.proj.weight, blk.proj.bias, blk.ln2.weight, blk.ln2.bias,
+                                     blk.fc.weight, blk.fc.bias, blk.out.weight, blk.out.bias, blk.ln2.eps)
+        h = f.add_norm(x, branch, self.ln_f.weight, self.ln_f.bias, self.ln_f.eps)
+        return f.head_loss(h, self.wte.weight, targets)
 
     def num_params(self) -> int:
         return sum(p.numel() for p in self.parameters())
