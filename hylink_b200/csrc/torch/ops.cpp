@@ -1,5 +1,5 @@
 // Autograd functions of the training step over the kernels of csrc/train: what surrounds the GEMMs and the attention
-// of a transformer block, and the language-model head with its loss. The GEMMs are torch's own (cuBLAS), the
+// of a transformer block, the language-model head with its loss, and the sharded optimizer. The GEMMs are torch's own (cuBLAS), the
 // attention between the two halves of a block is whatever torch's scaled_dot_product_attention picks.
 //
 // A block is cut in two around the attention:
@@ -254,6 +254,20 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
   }
 };
 
+void shardedAdamW(const Tensor& grad, const Tensor& weight, const std::optional<Tensor>& master, const Tensor& m, const Tensor& v, int64_t ranks,
+                  double keep, double beta1, double beta2, double step, double correction2, double eps) {
+  c10::cuda::CUDAGuard dg(weight.device());
+  const int64_t n = weight.numel();
+  TORCH_CHECK(grad.is_contiguous() && weight.is_contiguous() && m.is_contiguous() && v.is_contiguous() && grad.numel() == n && m.numel() == n &&
+                  v.numel() == n && (!master || (master->is_contiguous() && master->numel() == n)),
+              "hylink: sharded AdamW needs contiguous tensors of one size");
+  const train::AdamWArgs a = {(float)ranks, (float)keep, (float)beta1, (float)(1 - beta1), (float)beta2, (float)(1 - beta2), (float)step, (float)correction2, (float)eps};
+  const int dt = weight.scalar_type() == at::kFloat ? (int)hlFloat32 : code(weight);
+  ok(train::shardedAdamW(dt, grad.data_ptr(), weight.data_ptr(), master ? master->data_ptr<float>() : nullptr, m.data_ptr<float>(),
+                         v.data_ptr<float>(), n, a, streamOf(weight)),
+     "sharded AdamW");
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -267,5 +281,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                          const Tensor& wf, const Tensor& bf, const Tensor& wo, const Tensor& bo, double eps) {
     return BlockPost::apply(x, a, wp, bp, gamma, beta, wf, bf, wo, bo, eps);
   });
+  m.def("sharded_adamw", &shardedAdamW);
   m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });
 }

@@ -29,7 +29,7 @@ hlResult_t layerNormBackward(int dt, const void* dh, const void* x, const float*
 hlResult_t geluForward(int dt, const void* u, void* out, int64_t count, cudaStream_t s);
 // Rows a strip kernel gives to one CTA: its partials are [stripPartials(rows)][width].
 int stripPartials(int64_t rows);
-// du = dg * gelu'(u), and column-sum partials of du. width a multiple of 8.
+// du = dg * gelu'(u), and column-sum partials of du (unless null). width a multiple of 8.
 hlResult_t geluBackward(int dt, const void* dg, const void* u, void* du, float* partials, int64_t rows, int width, cudaStream_t s);
 // Column-sum partials of a [rows][width] matrix.
 hlResult_t columnSums(int dt, const void* src, float* partials, int64_t rows, int width, cudaStream_t s);
@@ -51,6 +51,15 @@ hlResult_t crossEntropyForward(int dt, const void* logits, int64_t stride, const
 // dlogits (same layout; the padding behind `vocab` becomes zero) for the gradient *grad of the mean loss.
 hlResult_t crossEntropyBackward(int dt, const void* logits, int64_t stride, const int64_t* targets, int64_t rows, int vocab, int64_t ignore_index,
                                 const float* lse, const float* loss, const float* grad, void* dlogits, cudaStream_t s);
+
+// One AdamW update of `count` elements (a multiple of 8). The gradient is a sum over `ranks`; `keep` = 1 - lr * decay,
+// `rest1` = 1 - beta1 and `rest2` = 1 - beta2 (not to be taken in fp32: 1 - 0.999f is 5e-5 off), `step` =
+// lr / (1 - beta1^t), `correction2` = 1 - beta2^t. master: fp32 copy of 16-bit weights, or null.
+struct AdamWArgs {
+  float ranks, keep, beta1, rest1, beta2, rest2, step, correction2, eps;
+};
+hlResult_t shardedAdamW(int dt, const void* grad, void* weight, float* master, float* m, float* v, int64_t count, const AdamWArgs& a,
+                        cudaStream_t s);
 
 }  // namespace train
 }  // namespace hl

@@ -15,6 +15,8 @@ from __future__ import annotations
 import torch
 import torch.distributed as dist
 
+from ..ops.extension import ops
+
 
 class ShardedAdamW:
     """AdamW whose moments (and, optionally, fp32 master weights) exist only for this rank's 1/n of the parameters."""
@@ -44,7 +46,8 @@ class ShardedAdamW:
         self.master = mine.float().clone() if (master_fp32 and dt != torch.float32) else None
         self.m = torch.zeros(self.shard, dtype=torch.float32, device=dev)
         self.v = torch.zeros(self.shard, dtype=torch.float32, device=dev)
-        self.grad_shard = torch.empty(self.shard, dtype=dt, device=dev)
+        # one rank owns every gradient already: its shard is the flat buffer itself and the reduce-scatter moves nothing
+        self.grad_shard = self.flat_grad if self.n == 1 else torch.empty(self.shard, dtype=dt, device=dev)
         self.lr, self.betas, self.eps, self.wd = lr, betas, eps, weight_decay
         self.t = 0
 
@@ -55,19 +58,21 @@ class ShardedAdamW:
     def step(self) -> None:
         """Mean-reduce gradients to their owners, update the owned shard, gather the new parameters."""
         dist.reduce_scatter_tensor(self.grad_shard, self.flat_grad, op=dist.ReduceOp.SUM, group=self.group)
-        g = self.grad_shard.float().div_(self.n)
         self.t += 1
         b1, b2 = self.betas
+        keep, step, correction2 = 1 - self.lr * self.wd, self.lr / (1 - b1 ** self.t), 1 - b2 ** self.t
         mine = self.flat[self.r * self.shard:(self.r + 1) * self.shard]
-        w = self.master if self.master is not None else mine.float()
-        w.mul_(1 - self.lr * self.wd)
-        self.m.mul_(b1).add_(g, alpha=1 - b1)
-        self.v.mul_(b2).addcmul_(g, g, value=1 - b2)
-        step = self.lr / (1 - b1 ** self.t)
-        denom = (self.v / (1 - b2 ** self.t)).sqrt_().add_(self.eps)
-        w.addcdiv_(self.m, denom, value=-step)
-        mine.copy_(w)
-        dist.all_gather_into_tensor(self.flat, mine.clone(), group=self.group)
+        if mine.is_cuda and mine.dtype in (torch.bfloat16, torch.float16, torch.float32):
+            ops().sharded_adamw(self.grad_shard, mine, self.master, self.m, self.v, self.n, keep, b1, b2, step, correction2, self.eps)
+        else:
+            g = self.grad_shard.float() / self.n
+            w = self.master if self.master is not None else mine.float()
+            w.mul_(keep)
+            self.m.mul_(b1).add_(g, alpha=1 - b1)
+            self.v.mul_(b2).addcmul_(g, g, value=1 - b2)
+            w.addcdiv_(self.m, (self.v / correction2).sqrt_().add_(self.eps), value=-step)
+            mine.copy_(w)
+        dist.all_gather_into_tensor(self.flat, mine, group=self.group)   # in place: the shard lies in its own segment
 
     def state_bytes_per_rank(self) -> int:
         return (self.m.numel() + self.v.numel() + (self.master.numel() if self.master is not None else 0)) * 4
