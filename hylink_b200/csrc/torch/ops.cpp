@@ -1,5 +1,5 @@
 // Autograd functions of the training step over the kernels of csrc/train: what surrounds the GEMMs and the attention
-// of a transformer block, the language-model head with its loss, and the sharded optimizer. The GEMMs are torch's own (cuBLAS), the
+// of a transformer block, the language-model head with its loss, the mixture-of-experts layer; and the sharded optimizer. The GEMMs are torch's own (cuBLAS), the
 // attention between the two halves of a block is whatever torch's scaled_dot_product_attention picks.
 //
 // A block is cut in two around the attention:
@@ -254,6 +254,103 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
   }
 };
 
+// Routing and dispatch of a top-1 mixture of experts. Returns x again (the residual path: its gradient then joins the
+// others in one pass), the dispatch buffer, the gates, and the maps token -> row and row -> token.
+class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const Variable& x_, const Variable& router, int64_t capacity) {
+    c10::cuda::CUDAGuard dg(x_.device());
+    const Tensor x = dense(x_);
+    const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
+    const auto ints = x.options().dtype(at::kInt);
+    const Tensor logits = at::mm(x, router.t());
+    Tensor expert = at::empty({tokens}, ints), row_of = at::empty({tokens}, ints), token_of = at::empty({experts * capacity}, ints);
+    Tensor gate = floats(x, {tokens}), send = at::empty({experts * capacity, width}, x.options());
+    ok(train::moeRoute(code(x), logits.data_ptr(), (int)tokens, (int)experts, (int)capacity, expert.data_ptr<int>(), gate.data_ptr<float>(),
+                       row_of.data_ptr<int>(), token_of.data_ptr<int>(), streamOf(x)),
+       "MoE routing");
+    ok(train::moeGather(x.data_ptr(), token_of.data_ptr<int>(), send.data_ptr(), (int)(experts * capacity), (int)width, streamOf(x)), "MoE dispatch");
+    ctx->save_for_backward({x, router, logits, gate, row_of});
+    ctx->saved_data["rows"] = experts * capacity;
+    ctx->mark_non_differentiable({row_of, token_of});
+    ctx->set_materialize_grads(false);
+    return {x, send, gate, row_of, token_of};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &router = s[1], &logits = s[2], &gate = s[3], &row_of = s[4];
+    c10::cuda::CUDAGuard dg(x.device());
+    const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
+    const Tensor dres = g[0].defined() ? dense(g[0]) : Tensor();
+    const Tensor dsend = g[1].defined() ? dense(g[1]) : at::zeros({ctx->saved_data["rows"].toInt(), width}, x.options());
+    const Tensor dgate = g[2].defined() ? dense(g[2]) : at::zeros_like(gate);
+    Tensor dx = at::empty_like(x), dlogits = at::empty_like(logits);
+    ok(train::moeTokenGradient(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
+                               gate.data_ptr<float>(), dgate.data_ptr<float>(), router.data_ptr(), dx.data_ptr(), dlogits.data_ptr(), (int)tokens,
+                               (int)width, (int)experts, streamOf(x)),
+       "MoE token gradient");
+    if (!train::moeRouterFits((int)experts, (int)width)) dx.addmm_(dlogits, router);
+    return {dx, at::mm(dlogits.t(), x), Tensor()};
+  }
+};
+
+// out = gelu(h W1) W2, per expert.
+class MoeExperts : public torch::autograd::Function<MoeExperts> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& h, const Variable& w1, const Variable& w2) {
+    c10::cuda::CUDAGuard dg(h.device());
+    const Tensor u = at::bmm(h, w1);
+    Tensor act = at::empty_like(u);
+    ok(train::geluForward(code(u), u.data_ptr(), act.data_ptr(), u.numel(), streamOf(u)), "gelu");
+    ctx->save_for_backward({h, w1, w2, u, act});
+    return at::bmm(act, w2);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &h = s[0], &w1 = s[1], &w2 = s[2], &u = s[3], &act = s[4];
+    c10::cuda::CUDAGuard dg(h.device());
+    const Tensor dout = dense(g[0]);
+    Tensor dact = at::bmm(dout, w2.transpose(1, 2));
+    Tensor dw2 = at::bmm(act.transpose(1, 2), dout);
+    Tensor du = at::empty_like(u);
+    ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
+       "gelu backward");
+    Tensor dw1 = at::bmm(h.transpose(1, 2), du);
+    Tensor dh = at::bmm(du, w1.transpose(1, 2));
+    return {dh, dw1, dw2};
+  }
+};
+
+// y = x + gate * rows[row_of] for the tokens that have a row.
+class MoeCombine : public torch::autograd::Function<MoeCombine> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& x, const Variable& gate, const Variable& rows_, const Variable& row_of,
+                          const Variable& token_of) {
+    c10::cuda::CUDAGuard dg(x.device());
+    const Tensor rows = dense(rows_);
+    Tensor y = at::empty_like(x);
+    ok(train::moeCombine(code(x), x.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), row_of.data_ptr<int>(), y.data_ptr(), (int)x.size(0),
+                         (int)x.size(1), streamOf(x)),
+       "MoE combine");
+    ctx->save_for_backward({gate, rows, token_of});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &gate = s[0], &rows = s[1], &token_of = s[2];
+    c10::cuda::CUDAGuard dg(rows.device());
+    const Tensor dy = dense(g[0]);
+    Tensor drows = at::empty_like(rows), dgate = at::empty_like(gate);   // dgate: only tokens with a row are written, and read
+    ok(train::moeRowGradient(code(rows), dy.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), token_of.data_ptr<int>(), drows.data_ptr(),
+                             dgate.data_ptr<float>(), (int)rows.size(0), (int)rows.size(1), streamOf(rows)),
+       "MoE row gradient");
+    return {dy, dgate, drows, Tensor(), Tensor()};
+  }
+};
+
 void shardedAdamW(const Tensor& grad, const Tensor& weight, const std::optional<Tensor>& master, const Tensor& m, const Tensor& v, int64_t ranks,
                   double keep, double beta1, double beta2, double step, double correction2, double eps) {
   c10::cuda::CUDAGuard dg(weight.device());
@@ -280,6 +377,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("block_post", [](const Tensor& x, const Tensor& a, const Tensor& wp, const Tensor& bp, const Tensor& gamma, const Tensor& beta,
                          const Tensor& wf, const Tensor& bf, const Tensor& wo, const Tensor& bo, double eps) {
     return BlockPost::apply(x, a, wp, bp, gamma, beta, wf, bf, wo, bo, eps);
+  });
+  m.def("moe_dispatch", [](const Tensor& x, const Tensor& router, int64_t capacity) { return MoeDispatch::apply(x, router, capacity); });
+  m.def("moe_experts", [](const Tensor& h, const Tensor& w1, const Tensor& w2) { return MoeExperts::apply(h, w1, w2); });
+  m.def("moe_combine", [](const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of, const Tensor& token_of) {
+    return MoeCombine::apply(x, gate, rows, row_of, token_of);
   });
   m.def("sharded_adamw", &shardedAdamW);
   m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });

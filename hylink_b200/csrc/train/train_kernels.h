@@ -61,5 +61,17 @@ struct AdamWArgs {
 hlResult_t shardedAdamW(int dt, const void* grad, void* weight, float* master, float* m, float* v, int64_t count, const AdamWArgs& a,
                         cudaStream_t s);
 
+// Mixture of experts (moe.cu). row_of: [tokens], row of the dispatch buffer or -1; token_of: [experts * capacity].
+hlResult_t moeRoute(int dt, const void* logits, int tokens, int experts, int capacity, int* expert, float* gate, int* row_of, int* token_of,
+                    cudaStream_t s);
+hlResult_t moeGather(const void* src, const int* index, void* dst, int rows, int width, cudaStream_t s);
+hlResult_t moeCombine(int dt, const void* x, const float* gate, const void* rows, const int* row_of, void* y, int tokens, int width, cudaStream_t s);
+hlResult_t moeRowGradient(int dt, const void* dy, const float* gate, const void* rows, const int* token_of, void* drows, float* dgate, int n_rows,
+                          int width, cudaStream_t s);
+// Whether moeTokenGradient adds the router's share to dx itself (else the caller adds dlogits * router). dy may be null.
+bool moeRouterFits(int experts, int width);
+hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const float* gate, const float* dgate,
+                            const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s);
+
 }  // namespace train
 }  // namespace hl

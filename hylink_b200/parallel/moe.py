@@ -17,6 +17,8 @@ import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops.extension import ops
+
 
 class _AllToAll(torch.autograd.Function):
     """Equal-split all-to-all over dimension 0; its own transpose in backward."""
@@ -58,6 +60,8 @@ class ExpertParallelMLP(nn.Module):
     def forward(self, x):
         """x: [tokens, d_model] (this rank's tokens). Returns the same shape."""
         t, d = x.shape
+        if self._fusable(x):
+            return self._fused(x)
         probs = F.softmax(self.router(x).float(), dim=-1)
         gate, expert = probs.max(dim=-1)                                   # top-1
         # position of every token in its expert's queue on THIS rank (arrival order), capacity cut
@@ -76,6 +80,25 @@ class ExpertParallelMLP(nn.Module):
         y = x.clone()
         y[keep] = x[keep] + gate[keep, None].to(x.dtype) * got[slot[keep]]
         return y
+
+    def _fusable(self, x) -> bool:
+        """16-bit tokens on a GPU, a plain router of the same type, rows of whole 16-byte packets that a CTA can hold."""
+        r = self.router
+        return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.shape[0] > 0 and x.shape[1] % 8 == 0 and x.shape[1] <= 2048
+                and self.w1.shape[2] % 8 == 0 and type(r) is nn.Linear and r.bias is None and r.weight.dtype == x.dtype
+                and not (r._forward_hooks or r._forward_pre_hooks or r._backward_hooks or r._backward_pre_hooks)
+                and not torch.is_autocast_enabled("cuda"))
+
+    def _fused(self, x):
+        f, d = ops(), x.shape[1]
+        x, send, gate, row_of, token_of = f.moe_dispatch(x, self.router.weight, self.cap)
+        # rows are ordered (destination rank, local expert, slot); with one rank they are where they belong
+        recv = all_to_all(send, self.group) if self.n > 1 else send
+        h = recv.view(self.n, self.epr, self.cap, d).transpose(0, 1).reshape(self.epr, self.n * self.cap, d)
+        h = f.moe_experts(h, self.w1.to(h.dtype), self.w2.to(h.dtype))
+        back = h.view(self.epr, self.n, self.cap, d).transpose(0, 1).reshape(self.n_experts * self.cap, d)
+        got = all_to_all(back, self.group) if self.n > 1 else back
+        return f.moe_combine(x, gate, got, row_of, token_of)
 
     def dense_reference(self, x, all_w1, all_w2):
         """The same layer computed without communication from all experts' weights (for tests)."""

@@ -45,3 +45,46 @@ def test_sharded_adamw_matches_adamw(count, dtype, master):
     torch.testing.assert_close(opt.m[:count].double(), st["exp_avg"], rtol=1e-5, atol=1e-8)
     torch.testing.assert_close(opt.v[:count].double(), st["exp_avg_sq"], rtol=1e-5, atol=1e-12)
     assert not opt.flat[count:].any() and not opt.m[count:].any()
+
+
+# one token; tokens that fill no warp; overflowing experts; more than a CTA of tokens; experts in and beyond registers
+@pytest.mark.parametrize("tokens,width,experts,capacity", [(1, 8, 1, 1), (37, 64, 4, 5), (1500, 264, 8, 200), (2100, 1024, 16, 256), (515, 2048, 24, 30)])
+def test_moe_matches_the_dense_layer(tokens, width, experts, capacity):
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+
+    torch.manual_seed(tokens)
+    layer = ExpertParallelMLP(width, 4 * width, experts_per_rank=experts, capacity=capacity).cuda().to(torch.bfloat16)
+    with torch.no_grad():
+        layer.router.weight.mul_(2)
+    ref = ExpertParallelMLP(width, 4 * width, experts_per_rank=experts, capacity=capacity).cuda()
+    ref.load_state_dict({k: v.float() for k, v in layer.state_dict().items()})
+    # the choice of expert is a step function: both layers have to start from the same 16-bit logits
+    class Rounded(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, z):
+            return z.to(torch.bfloat16).float()
+
+        @staticmethod
+        def backward(ctx, g):
+            return g
+
+    plain = ref.router.forward
+    ref.router.forward = lambda z: Rounded.apply(plain(z))
+    x = torch.randn(tokens, width, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    with torch.no_grad():
+        close = (layer.router(x).float() - ref.router(x.float())).abs().amax(1) > 0     # rounded another way: leave those tokens out
+        x[close] = x[~close][0] if bool((~close).any()) else x[close]
+    xr = x.detach().float().requires_grad_(True)
+    assert layer._fusable(x)
+    y, yr = layer(x), ref(xr)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    yr.backward(dy.float())
+
+    def rel(a, b):
+        return float((a.float() - b).norm() / b.norm().clamp_min(1e-12))
+
+    assert rel(y, yr) < 5e-3 and rel(x.grad, xr.grad) < 1e-2
+    for (n, p), q in zip(layer.named_parameters(), ref.parameters()):
+        if float(q.grad.norm()) > 1e-6:
+            assert rel(p.grad, q.grad) < 2e-2, n
