@@ -1,12 +1,11 @@
 // Landing reduce, doorbell and warm-up kernels of the PCIe path (sm_100a).
 //
 // reduceLanding: dst = scale * op(src_0 .. src_{k-1}) (optionally with dst as
-// an extra first operand). 16-byte vector accesses, four packets in flight per
-// thread and per source, fp32 accumulation for fp16/bf16 with one rounding,
-// up to eight sources reduced in ONE pass so that a batch of landed chunks is
-// folded with a single read of each. A source may be pinned host memory: the
-// kernel then reads the staging buffer over PCIe itself, fusing the H2D copy
-// with the reduction.
+// an extra first operand). 16-byte vector accesses, fp32 accumulation for
+// fp16/bf16 with one rounding, up to eight sources reduced in ONE pass so that
+// a batch of landed chunks is folded with a single read of each. A source may
+// be pinned host memory: the kernel then reads the staging buffer over PCIe
+// itself, fusing the H2D copy with the reduction.
 //
 // Parity: replaces D2DReduceTypedKernel<T>, D2DReduceHalfRawKernel and
 // D2DReduceBfloat16RawKernel (pcie-ccl-cuda/kernels/wait_kernel.cu:255-360),
@@ -15,6 +14,8 @@
 // wait_kernel.cu:13-109 with one kernel whose spin is bounded.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "nvl/nvl_device.cuh"
 #include "nvl/nvl_launch.h"
 
@@ -22,93 +23,67 @@ namespace hl {
 namespace dev {
 
 constexpr int kRlThreads = 256;
-constexpr int kRlUnroll = 4;
 
-template <typename T>
-__global__ void __launch_bounds__(kRlThreads) kReduceLanding(const __grid_constant__ nvl::ReduceLandingArgs a) {
+// Bound by memory. A thread folds one packet: it has the loads of all its operands in flight at once (the operand
+// count is compiled in, in classes), adds in a fixed order and stores. The grid covers the message; CTAs that retire
+// and start keep more loads in flight than a resident grid whose threads alternate between loading and storing
+// (4 x 32 MiB of bf16 into one on B200: 26.8 us = 6.3 TB/s against 28.7; before, with the sources in a run-time loop
+// four packets deep and the operator chosen per element, 38.9). A caller's own block count makes it loop.
+// kSum: the operator is known to be an addition; otherwise it is looked up per element.
+template <typename T, int MR, bool kSum>
+__global__ void __launch_bounds__(kRlThreads) kReduceLanding(const __grid_constant__ nvl::ReduceLandingArgs a, const void* const first, int n) {
   constexpr int N = Packet<T>::N;
   using Acc = typename Wire<T>::Acc;
-  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t tid = (uint64_t)blockIdx.x * kRlThreads + threadIdx.x;
+  const uint64_t nthreads = (uint64_t)gridDim.x * kRlThreads;
+  // operand 0 is `first` (dst itself when accumulating), operand q > 0 is source q - accumulate
+  auto operand = [&](int q) { return q == 0 ? first : a.src[q - (a.accumulate ? 1 : 0)]; };
   bool vec = aligned16(a.dst);
-  for (int s = 0; s < a.nsrc; ++s) vec = vec && aligned16(a.src[s]);
+#pragma unroll
+  for (int q = 0; q < MR; ++q)
+    if (q < n) vec = vec && aligned16(operand(q));
   const uint64_t np = vec ? a.count / N : 0;  // whole packets handled by the vector loop
   T* dst = reinterpret_cast<T*>(a.dst);
-  for (uint64_t i = tid; i < np; i += nthreads * kRlUnroll) {
-    Acc acc[kRlUnroll][N];
-    bool have[kRlUnroll];
+  for (uint64_t i = tid; i < np; i += nthreads) {
+    uint4 v[MR];
 #pragma unroll
-    for (int u = 0; u < kRlUnroll; ++u) {
-      const uint64_t j = i + (uint64_t)u * nthreads;
-      have[u] = j < np;
-      if (have[u] && a.accumulate) Packet<T>::unpack(reinterpret_cast<const uint4*>(dst)[j], acc[u]);
-    }
-    for (int s = 0; s < a.nsrc; ++s) {
-      uint4 v[kRlUnroll];
-      const uint4* src = reinterpret_cast<const uint4*>(a.src[s]);
+    for (int q = 0; q < MR; ++q)
+      if (q < n) v[q] = reinterpret_cast<const uint4*>(operand(q))[i];
+    Acc acc[N], b[N];
+    Packet<T>::unpack(v[0], acc);
 #pragma unroll
-      for (int u = 0; u < kRlUnroll; ++u) {
-        const uint64_t j = i + (uint64_t)u * nthreads;
-        if (have[u]) v[u] = src[j];
+    for (int q = 1; q < MR; ++q)
+      if (q < n) {
+        Packet<T>::unpack(v[q], b);
+#pragma unroll
+        for (int e = 0; e < N; ++e) acc[e] = kSum ? (Acc)(acc[e] + b[e]) : applyOp(a.op, acc[e], b[e]);
       }
-#pragma unroll
-      for (int u = 0; u < kRlUnroll; ++u) {
-        if (!have[u]) continue;
-        if (s == 0 && !a.accumulate) {
-          Packet<T>::unpack(v[u], acc[u]);
-        } else {
-          Acc b[N];
-          Packet<T>::unpack(v[u], b);
-#pragma unroll
-          for (int e = 0; e < N; ++e) acc[u][e] = applyOp(a.op, acc[u][e], b[e]);
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kRlUnroll; ++u) {
-      const uint64_t j = i + (uint64_t)u * nthreads;
-      if (!have[u]) continue;
-      finish<T>(acc[u], a.scale, 0);
-      reinterpret_cast<uint4*>(dst)[j] = Packet<T>::pack(acc[u]);
-    }
+    finish<T>(acc, a.scale, 0);
+    reinterpret_cast<uint4*>(dst)[i] = Packet<T>::pack(acc);
   }
   // ragged tail, or everything when some pointer is not 16-byte aligned
   for (uint64_t e = np * N + tid; e < a.count; e += nthreads) {
-    Acc acc;
-    int first = 0;
-    if (a.accumulate) acc = Wire<T>::up(dst[e]);
-    else { acc = Wire<T>::up(reinterpret_cast<const T*>(a.src[0])[e]); first = 1; }
-    for (int s = first; s < a.nsrc; ++s) acc = applyOp(a.op, acc, Wire<T>::up(reinterpret_cast<const T*>(a.src[s])[e]));
+    Acc acc = Wire<T>::up(reinterpret_cast<const T*>(first)[e]);
+    for (int q = 1; q < n; ++q) acc = applyOp(a.op, acc, Wire<T>::up(reinterpret_cast<const T*>(operand(q))[e]));
     if constexpr (Wire<T>::kFloat) { if (a.scale != 1.0f) acc = (Acc)(acc * (Acc)a.scale); }
     dst[e] = Wire<T>::down(acc);
   }
 }
 
-// Plain device-to-device copy of whole 16-byte packets (the one-rank form of every collective). Eight packets per
-// thread in flight; with kStream (HYLINK_COPY_STREAM_HINTS=1) the loads and stores carry the streaming cache hints,
-// which keep a one-touch copy from displacing the L2 working set of the kernels around it but cost 5 % of the rate.
-constexpr int kCopyThreads = 512;
-constexpr int kCopyUnroll = 8;
-template <bool kStream>
+// Plain device-to-device copy of whole 16-byte packets (the one-rank form of every collective). Like the fold, the
+// grid covers the message: 128 MiB in 43.1 us (6.2 TB/s) against 46.6 with a resident grid. U packets per thread:
+// one while the message leaves SMs idle, four above, where fewer CTAs do.
+constexpr int kCopyThreads = 256;
+template <int U>
 __global__ void __launch_bounds__(kCopyThreads) kCopyPackets(uint4* __restrict__ dst, const uint4* __restrict__ src, uint64_t packets) {
-  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = tid; i < packets; i += nthreads * kCopyUnroll) {
-    uint4 v[kCopyUnroll];
+  const uint64_t i0 = (uint64_t)blockIdx.x * (kCopyThreads * U) + threadIdx.x;
+  uint4 v[U];
 #pragma unroll
-    for (int u = 0; u < kCopyUnroll; ++u) {
-      const uint64_t j = i + (uint64_t)u * nthreads;
-      if (j < packets) v[u] = kStream ? __ldcs(src + j) : src[j];
-    }
+  for (int u = 0; u < U; ++u)
+    if (i0 + u * kCopyThreads < packets) v[u] = src[i0 + u * kCopyThreads];
 #pragma unroll
-    for (int u = 0; u < kCopyUnroll; ++u) {
-      const uint64_t j = i + (uint64_t)u * nthreads;
-      if (j < packets) {
-        if (kStream) __stcs(dst + j, v[u]);
-        else dst[j] = v[u];
-      }
-    }
-  }
+  for (int u = 0; u < U; ++u)
+    if (i0 + u * kCopyThreads < packets) dst[i0 + u * kCopyThreads] = v[u];
 }
 
 __global__ void kWarmup(int* sink) {
@@ -145,37 +120,42 @@ __global__ void kDoorbell(volatile uint64_t* ready, uint64_t ready_value, volati
 
 namespace nvl {
 
-static const void* reduceLandingFn(int dt) {
+// Operand classes: 2 (one source into an accumulator), 4, 9; operators other than the sum share the widest.
+template <typename T>
+static const void* reduceLandingFor(int operands, bool sum) {
   using namespace dev;
+  if (!sum) return (const void*)kReduceLanding<T, 9, false>;
+  if (operands <= 2) return (const void*)kReduceLanding<T, 2, true>;
+  if (operands <= 4) return (const void*)kReduceLanding<T, 4, true>;
+  return (const void*)kReduceLanding<T, 9, true>;
+}
+static const void* reduceLandingFn(int dt, int operands, bool sum) {
   switch (dt) {
-    case hlInt8: return (const void*)kReduceLanding<int8_t>;
-    case hlUint8: return (const void*)kReduceLanding<uint8_t>;
-    case hlInt32: return (const void*)kReduceLanding<int32_t>;
-    case hlUint32: return (const void*)kReduceLanding<uint32_t>;
-    case hlInt64: return (const void*)kReduceLanding<long long>;
-    case hlUint64: return (const void*)kReduceLanding<unsigned long long>;
-    case hlFloat16: return (const void*)kReduceLanding<__half>;
-    case hlFloat32: return (const void*)kReduceLanding<float>;
-    case hlFloat64: return (const void*)kReduceLanding<double>;
-    case hlBfloat16: return (const void*)kReduceLanding<__nv_bfloat16>;
+    case hlInt8: return reduceLandingFor<int8_t>(operands, sum);
+    case hlUint8: return reduceLandingFor<uint8_t>(operands, sum);
+    case hlInt32: return reduceLandingFor<int32_t>(operands, sum);
+    case hlUint32: return reduceLandingFor<uint32_t>(operands, sum);
+    case hlInt64: return reduceLandingFor<long long>(operands, sum);
+    case hlUint64: return reduceLandingFor<unsigned long long>(operands, sum);
+    case hlFloat16: return reduceLandingFor<__half>(operands, sum);
+    case hlFloat32: return reduceLandingFor<float>(operands, sum);
+    case hlFloat64: return reduceLandingFor<double>(operands, sum);
+    case hlBfloat16: return reduceLandingFor<__nv_bfloat16>(operands, sum);
     default: return nullptr;
   }
 }
 
 hlResult_t launchReduceLanding(const ReduceLandingArgs& a, int blocks, cudaStream_t stream) {
-  const void* fn = reduceLandingFn(a.dtype);
-  if (!fn) return fail(hlUnsupported, "reduce landing: unsupported dtype %d", a.dtype);
   if (a.nsrc < 1 || a.nsrc > 8) return fail(hlInvalidArgument, "reduce landing: nsrc %d out of [1,8]", a.nsrc);
+  int operands = a.nsrc + (a.accumulate ? 1 : 0);
+  const void* fn = reduceLandingFn(a.dtype, operands, a.op == hlSum || a.op == hlAvg);
+  if (!fn) return fail(hlUnsupported, "reduce landing: unsupported dtype %d", a.dtype);
   if (a.count == 0) return hlSuccess;
   const size_t es = hlTypeSize((hlDataType_t)a.dtype);
   const uint64_t packets = (a.count * es + 15) / 16;
-  if (blocks <= 0) {
-    // one packet-quad per thread up to four CTAs per SM of a 148-SM part
-    uint64_t want = (packets + (uint64_t)dev::kRlThreads * dev::kRlUnroll - 1) / ((uint64_t)dev::kRlThreads * dev::kRlUnroll);
-    blocks = (int)(want < 1 ? 1 : (want > 148 * 4 ? 148 * 4 : want));
-  }
-  ReduceLandingArgs copy = a;
-  void* args[1] = {(void*)&copy};
+  if (blocks <= 0) blocks = (int)std::min<uint64_t>((packets + dev::kRlThreads - 1) / dev::kRlThreads, 1u << 30);
+  const void* first = a.accumulate ? a.dst : a.src[0];
+  void* args[3] = {(void*)&a, (void*)&first, (void*)&operands};
   cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(dev::kRlThreads), args, 0, stream);
   if (e != cudaSuccess) return fail(hlDeviceError, "reduce landing launch: %s", cudaGetErrorString(e));
   return hlSuccess;
@@ -185,30 +165,27 @@ hlResult_t launchReduceLanding(const ReduceLandingArgs& a, int blocks, cudaStrea
 hlResult_t launchCopy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
   const uint64_t packets = bytes / 16;
   if (!packets) return hlSuccess;
-  static const int forced_blocks = (int)envInt({"HYLINK_COPY_BLOCKS"}, 0);
-  static const bool stream_hints = envBool({"HYLINK_COPY_STREAM_HINTS"}, false);
-  const uint64_t per_block = (uint64_t)dev::kCopyThreads * dev::kCopyUnroll;
-  uint64_t want = (packets + per_block - 1) / per_block;
-  // measured on B200 (1 GiB, copy rate): 2.91 TB/s with 4 CTAs per SM and streaming hints, 3.05-3.08 with 8 CTAs per
-  // SM or without the hints (cudaMemcpyAsync: 3.21)
-  const uint64_t cap = forced_blocks > 0 ? (uint64_t)forced_blocks : 148 * 8;
-  const unsigned blocks = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
-  if (stream_hints) dev::kCopyPackets<true><<<blocks, dev::kCopyThreads, 0, stream>>>((uint4*)dst, (const uint4*)src, packets);
-  else dev::kCopyPackets<false><<<blocks, dev::kCopyThreads, 0, stream>>>((uint4*)dst, (const uint4*)src, packets);
+  const int unroll = packets >= (uint64_t)148 * 8 * dev::kCopyThreads * 4 ? 4 : 1;   // from 19 MiB: four packets still fill every SM
+  const uint64_t per_block = (uint64_t)dev::kCopyThreads * unroll;
+  const unsigned blocks = (unsigned)((packets + per_block - 1) / per_block);
+  if (unroll == 4) dev::kCopyPackets<4><<<blocks, dev::kCopyThreads, 0, stream>>>((uint4*)dst, (const uint4*)src, packets);
+  else dev::kCopyPackets<1><<<blocks, dev::kCopyThreads, 0, stream>>>((uint4*)dst, (const uint4*)src, packets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(hlDeviceError, "copy launch: %s", cudaGetErrorString(e));
   return hlSuccess;
 }
 
 hlResult_t prepareReduceLanding() {
-  for (int dt = 0; dt < hlNumTypes; ++dt) {
-    cudaFuncAttributes at;
-    cudaError_t e = cudaFuncGetAttributes(&at, reduceLandingFn(dt));
-    if (e != cudaSuccess) return fail(hlDeviceError, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
-  }
+  for (int dt = 0; dt < hlNumTypes; ++dt)
+    for (int operands : {2, 4, 9})
+      for (bool sum : {false, true}) {
+        cudaFuncAttributes at;
+        cudaError_t e = cudaFuncGetAttributes(&at, reduceLandingFn(dt, operands, sum));
+        if (e != cudaSuccess) return fail(hlDeviceError, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
+      }
   cudaFuncAttributes at;
-  cudaFuncGetAttributes(&at, (const void*)dev::kCopyPackets<true>);
-  cudaFuncGetAttributes(&at, (const void*)dev::kCopyPackets<false>);
+  cudaFuncGetAttributes(&at, (const void*)dev::kCopyPackets<1>);
+  cudaFuncGetAttributes(&at, (const void*)dev::kCopyPackets<4>);
   cudaFuncGetAttributes(&at, (const void*)dev::kDoorbell);
   cudaFuncGetAttributes(&at, (const void*)dev::kWarmup);
   return hlSuccess;
