@@ -60,6 +60,7 @@ hlResult_t setUp(int device, unsigned char** base_out) {
         c.rank = (int)r;
         c.nranks = (int)n;
         c.max_blocks = kMaxBlocks;
+        c.one_device = 1;
         for (size_t q = 0; q < n; ++q) {
           c.stage[q] = ptr + kStageOff + q * kStagePerRank;
           c.flags[q] = reinterpret_cast<uint64_t*>(ptr + kFlagsOff + q * kFlagsPerRank);

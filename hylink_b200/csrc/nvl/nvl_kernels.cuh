@@ -32,6 +32,7 @@
 // all-reduce, :355-374 all-gather, :537-554 reduce-scatter, :740-757
 // all-to-all) and packs/merges segment prefixes with extra D2D copies
 // (virtual_collective.h:162-183).
+#pragma once
 #include <cuda_runtime.h>
 
 #include "nvl/nvl_device.cuh"
@@ -106,13 +107,22 @@ __device__ __forceinline__ uint4 reducePackets(const uint4* v, int n, int op, fl
   constexpr int N = Packet<W>::N;
   typename Wire<W>::Acc acc[N], b[N];
   Packet<W>::unpack(v[0], acc);
+  if (op == hlSum || op == hlAvg) {   // one branch per packet instead of a choice of operator per element
 #pragma unroll
-  for (int q = 1; q < MR; ++q) {
-    if (q < n) {
-      Packet<W>::unpack(v[q], b);
+    for (int q = 1; q < MR; ++q)
+      if (q < n) {
+        Packet<W>::unpack(v[q], b);
 #pragma unroll
-      for (int i = 0; i < N; ++i) acc[i] = applyOp(op, acc[i], b[i]);
-    }
+        for (int i = 0; i < N; ++i) acc[i] = (typename Wire<W>::Acc)(acc[i] + b[i]);
+      }
+  } else {
+#pragma unroll
+    for (int q = 1; q < MR; ++q)
+      if (q < n) {
+        Packet<W>::unpack(v[q], b);
+#pragma unroll
+        for (int i = 0; i < N; ++i) acc[i] = applyOp(op, acc[i], b[i]);
+      }
   }
   finish<W>(acc, scale, int_div);
   return Packet<W>::pack(acc);
@@ -151,15 +161,6 @@ __device__ __forceinline__ uint64_t segElems(uint64_t count, uint64_t first, uin
   return left < span ? left : span;
 }
 
-// ------------------------------------------------------------------ barrier
-__global__ void __launch_bounds__(HL_NVL_THREADS) kBarrier(const HlCommDev* comms, HlEmuCalls calls) {
-  const HlCommDev& c = comms[blockIdx.y];
-  HlCallArgs a = calls.c[blockIdx.y];
-  if (!entryOk(c, a)) return;
-  blockBarrier(c, a.seq + 1, 1);
-  callDone(c, 0);
-}
-
 // ------------------------------------------------------------------ all-reduce, one-shot
 // copy-in | barrier | every rank reduces all n copies of the whole message
 // straight into its output | barrier (peers done reading).
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllReduceOneShot(const HlComm
   const Ctx x = makeCtx();
   const uint64_t np = (a.count + N - 1) / N;
   copyInAny<W>(reinterpret_cast<uint4*>(c.stage[c.rank]), a.in, a.in_dt, 0, a.count, x);
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
+  if (!blockBarrier(c, a, 1, 1)) return;
   const bool vec = aligned16(a.out);
   for (uint64_t i = x.g0; i < np; i += x.gstride) {
     uint4 v[HL_MAX_RANKS];
@@ -183,8 +184,8 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllReduceOneShot(const HlComm
     const uint4 r = reducePackets<W>(v, n, a.op, a.scale, a.int_div);
     HL_USER_TYPE_SWITCH(W, a.out_dt, D, storeUserPacket<W, D>(reinterpret_cast<D*>(a.out), i * N, a.count, vec, r));
   }
-  blockBarrier(c, a.seq + 2, 2);
-  callDone(c, 0);
+  blockBarrier(c, a, 2, 2);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ all-reduce, two-shot over P2P
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllReduceTwoShot(const HlComm
   uint4* mine = reinterpret_cast<uint4*>(c.stage[r]);
   for (int s = 0; s < n; ++s)
     copyInAny<W>(mine + s * sp, a.in, a.in_dt, s * sp * N, segElems(a.count, s * sp * N, sp * N), x);
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
+  if (!blockBarrier(c, a, 1, 1)) return;
   {
     const uint64_t first = (uint64_t)r * sp;
     const uint64_t shard_np = first >= np ? 0 : (np - first < sp ? np - first : sp);
@@ -221,14 +222,14 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllReduceTwoShot(const HlComm
       if (j < shard_np) mine[first + j] = reducePackets<W>(v1, n, a.op, a.scale, a.int_div);
     }
   }
-  if (!blockBarrier(c, a.seq + 2, 2)) return;
+  if (!blockBarrier(c, a, 2, 2)) return;
   for (int k = 0; k < n; ++k) {
     const int s = (r + k) % n;  // start at the local shard, then walk the peers
     copyOutAny<W>(a.out, a.out_dt, s * sp * N, reinterpret_cast<const uint4*>(c.stage[s]) + s * sp,
                   segElems(a.count, s * sp * N, sp * N), x);
   }
-  blockBarrier(c, a.seq + 3, 3);
-  callDone(c, 0);
+  blockBarrier(c, a, 3, 3);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ all-reduce through NVSwitch (NVLS)
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllReduceNvls(const HlCommDev
   uint4* mine = reinterpret_cast<uint4*>(c.stage[r]);
   for (int s = 0; s < n; ++s)
     copyInAny<W>(mine + s * sp, a.in, a.in_dt, s * sp * N, segElems(a.count, s * sp * N, sp * N), x);
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
+  if (!blockBarrier(c, a, 1, 1)) return;
   {
     const uint64_t first = (uint64_t)r * sp;
     const uint64_t shard_np = first >= np ? 0 : (np - first < sp ? np - first : sp);
@@ -275,11 +276,11 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllReduceNvls(const HlCommDev
       }
     }
   }
-  if (!blockBarrier(c, a.seq + 2, 2)) return;
+  if (!blockBarrier(c, a, 2, 2)) return;
   for (int s = 0; s < n; ++s)
     copyOutAny<W>(a.out, a.out_dt, s * sp * N, mine + s * sp, segElems(a.count, s * sp * N, sp * N), x);
-  blockBarrier(c, a.seq + 3, 3);   // rule A: a peer's next call may store into this staging
-  callDone(c, 0);
+  blockBarrier(c, a, 3, 3);   // rule A: a peer's next call may store into this staging
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ pipelined all-reduce / reduce-scatter
@@ -307,7 +308,7 @@ __device__ __forceinline__ void groupSync(int id, int threads) {
 // the CTA triple (or pair) when they are CTAs of their own.
 __device__ __forceinline__ void tileSignal(const HlCommDev& c, int kind, uint64_t value, int gtid, unsigned lane) {
   if (gtid < c.nranks) {
-    stReleaseSys(c.flags[gtid] + ((size_t)kind * HL_MAX_BLOCKS + lane) * HL_MAX_RANKS + c.rank, value);
+    stRelease(c.one_device != 0, c.flags[gtid] + ((size_t)kind * HL_MAX_BLOCKS + lane) * HL_MAX_RANKS + c.rank, value);
   }
 }
 
@@ -318,7 +319,7 @@ __device__ __forceinline__ void tileWait(const HlCommDev& c, int kind, uint64_t 
     const uint64_t* mine = c.flags[c.rank] + ((size_t)kind * HL_MAX_BLOCKS + lane) * HL_MAX_RANKS + gtid;
     uint64_t t0 = 0;
     uint32_t spins = 0;
-    while (ldAcquireSys(mine) < value) {
+    while (ldAcquire(c.one_device != 0, mine) < value) {
       if ((++spins & 31u) == 0) {
         const uint64_t now = globalTimerNs();
         if (t0 == 0) t0 = now;
@@ -419,16 +420,16 @@ template <typename W, bool kNvls, bool kAllReduce>
 __global__ void __launch_bounds__(kPipeThreads) kPipelined(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
-  if (!entryOk(c, a)) return;
-  __shared__ int s_abort;
-  if (threadIdx.x == 0) s_abort = 0;
-  __syncthreads();
   constexpr int N = Packet<W>::N;
   const int n = c.nranks, r = c.rank;
   const uint64_t np = (a.count + N - 1) / N;
   const uint64_t sp = kAllReduce ? (np + n - 1) / n : np;   // packets per shard (all-reduce) or per segment (reduce-scatter)
   const uint64_t tps = a.tile_packets;
   const uint64_t tiles = (sp + tps - 1) / tps;
+  if (!entryOk(c, a, (tiles + gridDim.x - 1) / gridDim.x)) return;
+  __shared__ int s_abort;
+  if (threadIdx.x == 0) s_abort = 0;
+  __syncthreads();
   const uint64_t in_stride = kAllReduce ? sp * N : a.in_seg_stride;   // elements between shards / segments in the input
   const uint64_t seg_elems = a.count;                                 // reduce-scatter: valid elements per segment
   const int warp = threadIdx.x >> 5;
@@ -543,8 +544,8 @@ __global__ void __launch_bounds__(kPipeThreads) kPipelined(const HlCommDev* comm
   }
   // rule A. Reduce-scatter: peers pull from this rank's staging in their exchange stage. All-reduce: the copy-out
   // stage reads this rank's own staging, which a peer's next call may store into.
-  blockBarrier(c, a.seq + 1, 3);
-  callDone(c, (tiles + gridDim.x - 1) / gridDim.x);
+  blockBarrier(c, a, 1, 3);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ pipelined push all-reduce / reduce-scatter, one CTA per stage
@@ -594,14 +595,6 @@ template <typename W, bool kAllReduce, int MR>
 __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
-  if (!entryOk(c, a)) return;
-  __shared__ int s_abort;
-  __shared__ unsigned long long s_stop_at;   // tile (ordinal within this lane) at which the workers gave up
-  if (threadIdx.x == 0) {
-    s_abort = 0;
-    s_stop_at = ~0ull;
-  }
-  __syncthreads();
   constexpr int N = Packet<W>::N;
   // CTAs per lane. All-reduce: push, fold (which pushes the result on), copy-out. Reduce-scatter: one pusher and
   // three folders that each take a third of the tile — 16 to 37 CTAs of posted stores fill the link, while the
@@ -615,6 +608,15 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* c
   const uint64_t tiles = (sp + tps - 1) / tps;
   const uint64_t in_stride = kAllReduce ? sp * N : a.in_seg_stride;
   const uint64_t res_off = sp * (uint64_t)n;                // results live behind the n slots
+  const unsigned lanes_all = gridDim.x / kRoles;
+  if (!entryOk(c, a, lanes_all ? (tiles + lanes_all - 1) / lanes_all : 0)) return;
+  __shared__ int s_abort;
+  __shared__ unsigned long long s_stop_at;   // tile (ordinal within this lane) at which the workers gave up
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    s_stop_at = ~0ull;
+  }
+  __syncthreads();
   const unsigned member = blockIdx.x % kRoles, lane = blockIdx.x / kRoles, lanes = gridDim.x / kRoles;
   const unsigned role = kAllReduce ? member : (member == 0 ? 0u : 1u);   // 0 push, 1 fold, 2 copy-out
   const unsigned part = kAllReduce ? 0u : (member == 0 ? 0u : member - 1);
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* c
   }
   // rule A: a pusher of the next call may overwrite slots that a slower peer is still folding (or, all-reduce,
   // result areas that it is still copying out): nobody leaves before every peer's CTA of the same index is through
-  blockBarrier(c, a.seq + 1, 3);
+  blockBarrier(c, a, 1, 3);
   if (timed && blockIdx.x < HL_TL_BLOCKS) {
     lap(t_work);
     // slots 1..3 hold entry + duration, so that "time since entry" reads as the three sums; slot 4 carries the
@@ -709,69 +711,228 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* c
     st[3] = e + t_work;
     st[4] = e + (uint64_t)role * 1000000ull;
   }
-  callDone(c, lanes ? (tiles + lanes - 1) / lanes : 0);
+  callDone(c, a);
 }
 
-// ------------------------------------------------------------------ push all-reduce / reduce-scatter over peer pointers
-// Every NVLink access is a posted store and every load is local:
-//   1. push: each rank streams, straight from the caller's buffer, shard s of
-//      its input into slot `rank` of shard s's owner (nothing is staged locally);
-//   barrier
-//   2. fold: the owner adds its own shard (read from the caller's buffer) and
-//      the n-1 landed slots in ascending rank order, writes its part of the
-//      result to the caller's output and (all-reduce) pushes it into every
-//      peer's result area;
-//   barrier
-//   3. (all-reduce) copy the other owners' results from the local result area
-//      to the caller's output.
-// All 512 threads of every CTA work in every phase, so each phase has the
-// whole grid's loads and stores in flight. The caller's element type is the
-// wire type (converting calls use the staged kernels).
-template <typename W, bool kAllReduce>
+// ------------------------------------------------------------------ push kernels over peer pointers
+// Every access to a peer is a posted store and every load is local:
+//   all-reduce      stream shard s of the input straight from the caller's buffer into slot `rank` of its owner | barrier |
+//                   fold the own shard (read from the caller's buffer) and the landed slots in ascending rank order,
+//                   store the result to the caller's output and into every peer's result area | barrier | copy the
+//                   peers' results out of the local result area | barrier
+//   reduce-scatter  push the peers' segments | barrier | fold | barrier
+//   all-gather      store the own segment into every peer's slot and into the own output | barrier | copy out | barrier
+//   all-to-all      push the peers' segments, copy the own one | barrier | copy out | barrier
+// All 512 threads of every CTA work in every phase, so each phase has the whole grid's loads and stores in flight. The
+// caller's element type is the wire type (converting calls use the staged kernels).
+// Copies go peer by peer, eight packets of one stream per thread; the fold takes a packet of all sources at once. (8
+// ranks x 16 MiB of fp32 emulated on one GPU: pushing to seven peers packet by packet takes 70 us instead of 36, since
+// every thread then walks seven distant streams; a fold that also had the choices "own or landed", "vector or ragged"
+// and the operator inside its loop took 82 us instead of 40. At 6.4 to 7 TB/s the phases are bound by L2 and HBM:
+// cutting the message into slices whose staging stays in L2 gained nothing.)
+
+// Parts of a user buffer, `stride` elements apart. Part q ends after `count` elements, or, where the parts are cut from
+// one buffer whose last part may be short, with the buffer (`total` elements, else 0).
+template <typename W>
+struct Parts {
+  static constexpr int N = Packet<W>::N;
+  W* base;
+  uint64_t stride, count, total;
+  __device__ __forceinline__ Parts(const void* p, uint64_t stride_, uint64_t count_, uint64_t total_)
+      : base(reinterpret_cast<W*>(const_cast<void*>(p))), stride(stride_), count(count_), total(total_) {}
+  __device__ __forceinline__ W* at(int q) const { return base + (uint64_t)q * stride; }
+  __device__ __forceinline__ uint64_t elems(int q) const {
+    if (!total) return count;
+    return segElems(total, (uint64_t)q * stride, stride);
+  }
+};
+
+// The k-th peer of rank r, k = 1 .. n - 1: every rank starts with its successor, so that the owners are loaded evenly.
+__device__ __forceinline__ int peerOf(int r, int k, int n) { return r + k < n ? r + k : r + k - n; }
+
+// Whole packets at the front of `cnt` elements that two (or one) user buffers hold as 16-byte vectors.
+template <typename W>
+__device__ __forceinline__ uint32_t wholePackets(uint64_t cnt, const void* p, const void* q) {
+  return aligned16(p) && aligned16(q) ? (uint32_t)(cnt / Packet<W>::N) : 0;
+}
+// The first packet behind `whole` that this thread handles.
+__device__ __forceinline__ uint64_t restFrom(uint32_t whole, const Ctx& x) {
+  return whole <= x.g0 ? x.g0 : x.g0 + (whole - x.g0 + x.gstride - 1) / x.gstride * x.gstride;
+}
+// Packets of 16 bytes between aligned places, U per thread in flight.
+template <int U = kPushUnroll>
+__device__ __forceinline__ void copyWhole(uint4* dst, const uint4* src, uint32_t packets, const Ctx& x) {
+  const uint32_t g = (uint32_t)x.gstride;
+  for (uint32_t i = (uint32_t)x.g0; i < packets; i += g * U) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * g < packets) v[u] = src[i + u * g];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * g < packets) dst[i + u * g] = v[u];
+  }
+}
+// User buffer -> staging slot, staging slot -> user buffer: vectors, then the ragged rest element by element.
+template <typename W>
+__device__ __forceinline__ void pushPart(uint4* slot, const W* src, uint64_t cnt, const Ctx& x) {
+  constexpr int N = Packet<W>::N;
+  const uint32_t whole = wholePackets<W>(cnt, src, src);
+  copyWhole(slot, reinterpret_cast<const uint4*>(src), whole, x);
+  for (uint64_t i = restFrom(whole, x); i * N < cnt; i += x.gstride) slot[i] = loadUserPacket<W, W>(src, i * N, cnt, false);
+}
+template <typename W>
+__device__ __forceinline__ void pullPart(W* dst, const uint4* slot, uint64_t cnt, const Ctx& x) {
+  constexpr int N = Packet<W>::N;
+  const uint32_t whole = wholePackets<W>(cnt, dst, dst);
+  copyWhole(reinterpret_cast<uint4*>(dst), slot, whole, x);
+  for (uint64_t i = restFrom(whole, x); i * N < cnt; i += x.gstride) storeUserPacket<W, W>(dst, i * N, cnt, false, slot[i]);
+}
+
+template <typename W, bool kAllReduce, int MR>
 __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, HlEmuCalls calls) {
+  const HlCommDev& c = comms[blockIdx.y];
+  HlCallArgs a = calls.c[blockIdx.y];
+  if (!entryOk(c, a)) return;
+  constexpr int N = Packet<W>::N;
+  constexpr int U = MR <= 2 ? 4 : (MR <= 4 ? 2 : 1);   // fold: about eight loads in flight per thread
+  const int n = c.nranks, r = c.rank;
+  const Ctx x = makeCtx();
+  const uint64_t np = (a.count + N - 1) / N;
+  const uint64_t sp = kAllReduce ? (np + n - 1) / n : np;
+  const Parts<W> in(a.in, kAllReduce ? sp * N : a.in_seg_stride, a.count, kAllReduce ? a.count : 0);
+  const Parts<W> out(a.out, sp * N, a.count, kAllReduce ? a.count : 0);   // reduce-scatter: part 0 alone
+  const uint64_t res_off = sp * (uint64_t)n;                              // results live behind the slots
+  for (int k = 1; k < n; ++k) {
+    const int q = peerOf(r, k, n);
+    pushPart<W>(reinterpret_cast<uint4*>(c.stage[q]) + (uint64_t)r * sp, in.at(q), in.elems(q), x);
+  }
+  if (!blockBarrier(c, a, 1, 1)) return;
+  {
+    const uint64_t cnt = in.elems(r);
+    const W* own = in.at(r);
+    W* res = out.at(kAllReduce ? r : 0);
+    const uint32_t whole = wholePackets<W>(cnt, own, res), g = (uint32_t)x.gstride;
+    const uint4* src[MR];   // ascending rank order: the sum order
+    uint4* dst[MR];
+#pragma unroll
+    for (int q = 0; q < MR; ++q)
+      if (q < n) src[q] = q == r ? reinterpret_cast<const uint4*>(own) : reinterpret_cast<const uint4*>(c.stage[r]) + (uint64_t)q * sp;
+    if constexpr (kAllReduce) {
+#pragma unroll
+      for (int k = 1; k < MR; ++k)
+        if (k < n) dst[k] = reinterpret_cast<uint4*>(c.stage[peerOf(r, k, n)]) + res_off + (uint64_t)r * sp;
+    }
+    for (uint32_t i = (uint32_t)x.g0; i < whole; i += g * U) {
+      uint4 v[U][MR];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < MR; ++q)
+          if (q < n && i + u * g < whole) v[u][q] = src[q][i + u * g];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i + u * g < whole) {
+          const uint4 red = reducePackets<W, MR>(v[u], n, a.op, a.scale, a.int_div);
+          reinterpret_cast<uint4*>(res)[i + u * g] = red;
+          if constexpr (kAllReduce) {
+#pragma unroll
+            for (int k = 1; k < MR; ++k)
+              if (k < n) dst[k][i + u * g] = red;
+          }
+        }
+    }
+    for (uint64_t i = restFrom(whole, x); i * N < cnt; i += g) {
+      uint4 v[MR];
+#pragma unroll
+      for (int q = 0; q < MR; ++q)
+        if (q < n && q != r) v[q] = src[q][i];
+      const uint4 mine = loadUserPacket<W, W>(own, i * N, cnt, false);
+#pragma unroll
+      for (int q = 0; q < MR; ++q)
+        if (q == r) v[q] = mine;
+      const uint4 red = reducePackets<W, MR>(v, n, a.op, a.scale, a.int_div);
+      storeUserPacket<W, W>(res, i * N, cnt, false, red);
+      if constexpr (kAllReduce) {
+#pragma unroll
+        for (int k = 1; k < MR; ++k)
+          if (k < n) dst[k][i] = red;
+      }
+    }
+  }
+  if (!blockBarrier(c, a, 2, 2)) return;
+  if constexpr (kAllReduce) {
+    for (int k = 1; k < n; ++k) {
+      const int q = peerOf(r, k, n);
+      pullPart<W>(out.at(q), reinterpret_cast<const uint4*>(c.stage[r]) + res_off + (uint64_t)q * sp, out.elems(q), x);
+    }
+    // rule A: the result areas just read are where a peer's next (larger) call pushes its slots
+    blockBarrier(c, a, 3, 3);
+  }
+  callDone(c, a);
+}
+
+// All-gather and all-to-all: nothing to fold, a segment goes from the sender's buffer through the receiver's slot into
+// the receiver's output.
+template <typename W, bool kGather>
+__global__ void __launch_bounds__(HL_NVL_THREADS) kExchangePush(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
   if (!entryOk(c, a)) return;
   constexpr int N = Packet<W>::N;
   const int n = c.nranks, r = c.rank;
   const Ctx x = makeCtx();
-  const uint64_t np = (a.count + N - 1) / N;
-  const uint64_t sp = kAllReduce ? (np + n - 1) / n : np;
-  const uint64_t in_stride = kAllReduce ? sp * N : a.in_seg_stride;
-  const uint64_t res_off = sp * (uint64_t)n;
-  const W* in = reinterpret_cast<const W*>(a.in);
-  W* out = reinterpret_cast<W*>(a.out);
-  auto shardElems = [&](int s) -> uint64_t {
-    if constexpr (kAllReduce) return segElems(a.count, (uint64_t)s * sp * N, sp * N);
-    else return a.count;
-  };
-  for (int k = 1; k < n; ++k) {
-    const int s = (r + k) % n;
-    pushTile<W, W, kPushUnroll>(reinterpret_cast<uint4*>(c.stage[s]) + (uint64_t)r * sp, in + (uint64_t)s * in_stride, shardElems(s), x);
-  }
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
-  {
-    const uint64_t cnt = shardElems(r);
-    const uint64_t first = kAllReduce ? (uint64_t)r * sp * N : 0;
-    // about a dozen landed packets per thread in flight whatever the rank count (more spills registers)
-    if (n <= 2)
-      foldTile<W, W, W, kAllReduce, 6, 2>(c, a, in + (uint64_t)r * in_stride, cnt, out + first, cnt, sp, 0, (cnt + N - 1) / N, res_off, x);
-    else if (n <= 4)
-      foldTile<W, W, W, kAllReduce, 3, 4>(c, a, in + (uint64_t)r * in_stride, cnt, out + first, cnt, sp, 0, (cnt + N - 1) / N, res_off, x);
-    else
-      foldTile<W, W, W, kAllReduce, 2, HL_MAX_RANKS>(c, a, in + (uint64_t)r * in_stride, cnt, out + first, cnt, sp, 0, (cnt + N - 1) / N, res_off, x);
-  }
-  if (!blockBarrier(c, a.seq + 2, 2)) return;
-  if constexpr (kAllReduce) {
-    const uint4* mine = reinterpret_cast<const uint4*>(c.stage[r]);
-    for (int k = 1; k < n; ++k) {
-      const int s = (r + k) % n;
-      segCopyOut<W, W, kPushUnroll>(out + (uint64_t)s * sp * N, mine + res_off + (uint64_t)s * sp, shardElems(s), x);
+  const uint64_t sp = (a.count + N - 1) / N;
+  const Parts<W> in(a.in, kGather ? 0 : a.in_seg_stride, a.count, 0), out(a.out, a.out_seg_stride, a.count, 0);
+  W* mine = out.at(r);
+  const W* from = in.at(r);
+  if constexpr (kGather) {
+    // a packet is loaded once and stored n times
+    constexpr int U = kPushUnroll;
+    const bool own = from != mine;   // in place: the input already lies in its segment of the output
+    const uint32_t whole = wholePackets<W>(a.count, from, own ? mine : from), g = (uint32_t)x.gstride;
+    for (uint32_t i = (uint32_t)x.g0; i < whole; i += g * U) {
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i + u * g < whole) v[u] = reinterpret_cast<const uint4*>(from)[i + u * g];
+      for (int k = 1; k < n; ++k) {
+        uint4* slot = reinterpret_cast<uint4*>(c.stage[peerOf(r, k, n)]) + (uint64_t)r * sp;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i + u * g < whole) slot[i + u * g] = v[u];
+      }
+      if (own) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i + u * g < whole) reinterpret_cast<uint4*>(mine)[i + u * g] = v[u];
+      }
     }
-    // rule A: the result areas just read are where a peer's next (larger) call pushes its slots
-    blockBarrier(c, a.seq + 3, 3);
+    for (uint64_t i = restFrom(whole, x); i < sp; i += g) {
+      const uint4 v = loadUserPacket<W, W>(from, i * N, a.count, false);
+      for (int k = 1; k < n; ++k) (reinterpret_cast<uint4*>(c.stage[peerOf(r, k, n)]) + (uint64_t)r * sp)[i] = v;
+      if (own) storeUserPacket<W, W>(mine, i * N, a.count, false, v);
+    }
+  } else {
+    for (int k = 1; k < n; ++k) {
+      const int q = peerOf(r, k, n);
+      pushPart<W>(reinterpret_cast<uint4*>(c.stage[q]) + (uint64_t)r * sp, in.at(q), a.count, x);
+    }
+    if (from != mine) {
+      const uint32_t whole = wholePackets<W>(a.count, from, mine);
+      copyWhole(reinterpret_cast<uint4*>(mine), reinterpret_cast<const uint4*>(from), whole, x);
+      for (uint64_t i = restFrom(whole, x); i < sp; i += x.gstride)
+        storeUserPacket<W, W>(mine, i * N, a.count, false, loadUserPacket<W, W>(from, i * N, a.count, false));
+    }
   }
-  callDone(c, 0);
+  if (!blockBarrier(c, a, 1, 1)) return;
+  for (int k = 1; k < n; ++k) {
+    const int q = peerOf(r, k, n);
+    pullPart<W>(out.at(q), reinterpret_cast<const uint4*>(c.stage[r]) + (uint64_t)q * sp, a.count, x);
+  }
+  // the peers' next pushes may land in these slots: nobody leaves before every peer has copied out
+  blockBarrier(c, a, 2, 2);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ reduce-scatter
@@ -789,7 +950,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kReduceScatter(const HlCommDev
   const uint64_t sp = (a.count + N - 1) / N;
   uint4* mine = reinterpret_cast<uint4*>(c.stage[r]);
   for (int s = 0; s < n; ++s) copyInAny<W>(mine + s * sp, a.in, a.in_dt, s * a.in_seg_stride, a.count, x);
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
+  if (!blockBarrier(c, a, 1, 1)) return;
   const bool vec = aligned16(a.out);
   const uint64_t first = (uint64_t)r * sp;
   if constexpr (kNvls) {
@@ -834,8 +995,8 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kReduceScatter(const HlCommDev
       }
     }
   }
-  blockBarrier(c, a.seq + 2, 2);
-  callDone(c, 0);
+  blockBarrier(c, a, 2, 2);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ all-gather
@@ -855,69 +1016,22 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllGather(const HlCommDev* co
   const uint64_t sp = (a.count + N - 1) / N;
   uint4* mine = reinterpret_cast<uint4*>(c.stage[r]);
   if constexpr (kNvls) {
-    if (!blockBarrier(c, a.seq + 1, 1)) return;
+    if (!blockBarrier(c, a, 1, 1)) return;
     uint4* mc = reinterpret_cast<uint4*>(c.mc_stage) + (uint64_t)r * sp;
     copyInAny<W, true>(mc, a.in, a.in_dt, 0, a.count, x);
-    if (!blockBarrier(c, a.seq + 2, 2)) return;
+    if (!blockBarrier(c, a, 2, 2)) return;
     for (int q = 0; q < n; ++q) copyOutAny<W>(a.out, a.out_dt, q * a.out_seg_stride, mine + q * sp, a.count, x);
-    blockBarrier(c, a.seq + 3, 3);   // rule A
+    blockBarrier(c, a, 3, 3);   // rule A
   } else {
     copyInAny<W>(mine, a.in, a.in_dt, 0, a.count, x);
-    if (!blockBarrier(c, a.seq + 1, 1)) return;
+    if (!blockBarrier(c, a, 1, 1)) return;
     for (int k = 0; k < n; ++k) {
       const int q = (r + k) % n;
       copyOutAny<W>(a.out, a.out_dt, q * a.out_seg_stride, reinterpret_cast<const uint4*>(c.stage[q]), a.count, x);
     }
-    blockBarrier(c, a.seq + 2, 2);
+    blockBarrier(c, a, 2, 2);
   }
-  callDone(c, 0);
-}
-
-// Stores-only all-gather over peer pointers: every rank pushes its prefix straight from the caller's buffer into
-// slot `rank` of every peer's staging (no local staging copy, and posted stores run ~7 % above loads from a peer on
-// this link), copies its own prefix to its place in the output while the peers' data is on its way, and after the
-// barrier copies the landed slots out locally. The caller's element type is the wire type.
-template <typename W>
-__global__ void __launch_bounds__(HL_NVL_THREADS) kAllGatherPush(const HlCommDev* comms, HlEmuCalls calls) {
-  const HlCommDev& c = comms[blockIdx.y];
-  HlCallArgs a = calls.c[blockIdx.y];
-  if (!entryOk(c, a)) return;
-  constexpr int N = Packet<W>::N;
-  const int n = c.nranks, r = c.rank;
-  const Ctx x = makeCtx();
-  const uint64_t sp = (a.count + N - 1) / N;
-  const W* in = reinterpret_cast<const W*>(a.in);
-  W* out = reinterpret_cast<W*>(a.out);
-  for (int k = 1; k < n; ++k) {
-    const int s = (r + k) % n;
-    pushTile<W, W, kPushUnroll>(reinterpret_cast<uint4*>(c.stage[s]) + (uint64_t)r * sp, in, a.count, x);
-  }
-  W* own = out + (uint64_t)r * a.out_seg_stride;
-  if (own != in) {  // in place (the input already sits in its segment of the output): nothing to copy
-    const bool vin = aligned16(in), vout = aligned16(own);
-    for (uint64_t i = x.g0; i < sp; i += x.gstride * kPipeCopyUnroll) {
-      uint4 v[kPipeCopyUnroll];
-#pragma unroll
-      for (int u = 0; u < kPipeCopyUnroll; ++u) {
-        const uint64_t j = i + (uint64_t)u * x.gstride;
-        if (j < sp) v[u] = loadUserPacket<W, W>(in, j * N, a.count, vin);
-      }
-#pragma unroll
-      for (int u = 0; u < kPipeCopyUnroll; ++u) {
-        const uint64_t j = i + (uint64_t)u * x.gstride;
-        if (j < sp) storeUserPacket<W, W>(own, j * N, a.count, vout, v[u]);
-      }
-    }
-  }
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
-  const uint4* mine = reinterpret_cast<const uint4*>(c.stage[r]);
-  for (int k = 1; k < n; ++k) {
-    const int s = (r + k) % n;
-    segCopyOut<W, W, kPushUnroll>(out + (uint64_t)s * a.out_seg_stride, mine + (uint64_t)s * sp, a.count, x);
-  }
-  // the peers' next pushes may land in these slots: nobody leaves before every peer has copied out
-  blockBarrier(c, a.seq + 2, 2);
-  callDone(c, 0);
+  callDone(c, a);
 }
 
 // The stores-only all-gather cut into tiles, with the link stage and the HBM stage on CTAs of their own (see
@@ -928,10 +1042,6 @@ template <typename W>
 __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kAllGatherLanes(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
-  if (!entryOk(c, a)) return;
-  __shared__ int s_abort;
-  if (threadIdx.x == 0) s_abort = 0;
-  __syncthreads();
   constexpr int N = Packet<W>::N;
   const unsigned kParts = (unsigned)(a.lane_parts >= 1 && a.lane_parts <= 7 ? a.lane_parts : 3);
   const unsigned kMembers = 1 + kParts;
@@ -939,6 +1049,11 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kAllGatherLanes(const HlCom
   const uint64_t sp = (a.count + N - 1) / N;
   const uint64_t tps = a.tile_packets;
   const uint64_t tiles = (sp + tps - 1) / tps;
+  const unsigned lanes_all = gridDim.x / kMembers;
+  if (!entryOk(c, a, lanes_all ? (tiles + lanes_all - 1) / lanes_all : 0)) return;
+  __shared__ int s_abort;
+  if (threadIdx.x == 0) s_abort = 0;
+  __syncthreads();
   const unsigned member = blockIdx.x % kMembers, lane = blockIdx.x / kMembers, lanes = gridDim.x / kMembers;
   const bool pusher = member == 0;
   const int workers = pusher ? (int)blockDim.x - 32 : (int)blockDim.x;
@@ -1004,8 +1119,8 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kAllGatherLanes(const HlCom
     }
   }
   // the peers' next pushes may land in these slots: nobody leaves before every peer's CTA of the same index is through
-  blockBarrier(c, a.seq + 1, 3);
-  callDone(c, lanes ? (tiles + lanes - 1) / lanes : 0);
+  blockBarrier(c, a, 1, 3);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ broadcast
@@ -1019,22 +1134,22 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kBroadcast(const HlCommDev* co
   const Ctx x = makeCtx();
   uint4* mine = reinterpret_cast<uint4*>(c.stage[r]);
   if constexpr (kNvls) {
-    if (!blockBarrier(c, a.seq + 1, 1)) return;
+    if (!blockBarrier(c, a, 1, 1)) return;
     if (r == a.root) {
       uint4* mc = reinterpret_cast<uint4*>(c.mc_stage);
       copyInAny<W, true>(mc, a.in, a.in_dt, 0, a.count, x);
     }
-    if (!blockBarrier(c, a.seq + 2, 2)) return;
+    if (!blockBarrier(c, a, 2, 2)) return;
     if (r != a.root || a.out != a.in) copyOutAny<W>(a.out, a.out_dt, 0, mine, a.count, x);
-    blockBarrier(c, a.seq + 3, 3);   // rule A
+    blockBarrier(c, a, 3, 3);   // rule A
   } else {
     if (r == a.root) copyInAny<W>(mine, a.in, a.in_dt, 0, a.count, x);
-    if (!blockBarrier(c, a.seq + 1, 1)) return;
+    if (!blockBarrier(c, a, 1, 1)) return;
     if (r != a.root || a.out != a.in)
       copyOutAny<W>(a.out, a.out_dt, 0, reinterpret_cast<const uint4*>(c.stage[a.root]), a.count, x);
-    blockBarrier(c, a.seq + 2, 2);
+    blockBarrier(c, a, 2, 2);
   }
-  callDone(c, 0);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ all-to-all
@@ -1050,14 +1165,14 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kAllToAll(const HlCommDev* com
   const uint64_t sp = (a.count + N - 1) / N;
   uint4* mine = reinterpret_cast<uint4*>(c.stage[r]);
   for (int s = 0; s < n; ++s) copyInAny<W>(mine + s * sp, a.in, a.in_dt, s * a.in_seg_stride, a.count, x);
-  if (!blockBarrier(c, a.seq + 1, 1)) return;
+  if (!blockBarrier(c, a, 1, 1)) return;
   for (int k = 0; k < n; ++k) {
     const int q = (r + k) % n;
     copyOutAny<W>(a.out, a.out_dt, q * a.out_seg_stride, reinterpret_cast<const uint4*>(c.stage[q]) + (uint64_t)r * sp,
                   a.count, x);
   }
-  blockBarrier(c, a.seq + 2, 2);
-  callDone(c, 0);
+  blockBarrier(c, a, 2, 2);
+  callDone(c, a);
 }
 
 // ------------------------------------------------------------------ zero-copy kernels on registered memory
@@ -1087,7 +1202,7 @@ __device__ __forceinline__ bool zcHandshake(const HlCommDev& c, const HlCallArgs
     slot[0] = a.zc_in_off;
     slot[1] = a.zc_out_off;
   }
-  if (!blockBarrier(c, a.seq + 1, 1)) return false;
+  if (!blockBarrier(c, a, 1, 1)) return false;
   __shared__ int s_sym;
   if (t == 0) s_sym = 1;
   __syncthreads();
@@ -1165,7 +1280,17 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kZeroCopy(const HlCommDev* com
         }
       }
     } else {
-      constexpr int U = MR <= 2 ? 6 : (MR <= 4 ? 3 : 2);
+      // about eight packets per thread in flight; more of them means fewer warps or longer stalls between loading and
+      // storing (4 x 25 MiB emulated on one GPU: 37 us with eight, 39 with twelve)
+      constexpr int U = MR <= 2 ? 4 : (MR <= 4 ? 2 : 1);
+      const uint4* pi[MR];
+      uint4* po[MR];
+#pragma unroll
+      for (int q = 0; q < MR; ++q)
+        if (q < n) {
+          pi[q] = reinterpret_cast<const uint4*>(c.heap[q] + a.zc_in_off) + first;
+          po[q] = reinterpret_cast<uint4*>(c.heap[(r + q) % n] + a.zc_out_off) + first;
+        }
       for (uint64_t i = x.g0; i < cnt; i += x.gstride * U) {
         uint4 v[U][MR];
 #pragma unroll
@@ -1174,7 +1299,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kZeroCopy(const HlCommDev* com
           if (j < cnt) {
 #pragma unroll
             for (int q = 0; q < MR; ++q)
-              if (q < n) v[u][q] = (reinterpret_cast<const uint4*>(c.heap[q] + a.zc_in_off) + first)[j];
+              if (q < n) v[u][q] = pi[q][j];
           }
         }
 #pragma unroll
@@ -1185,7 +1310,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kZeroCopy(const HlCommDev* com
             if constexpr (kColl == kZcAllReduce) {
 #pragma unroll
               for (int q = 0; q < MR; ++q)
-                if (q < n) (reinterpret_cast<uint4*>(c.heap[(r + q) % n] + a.zc_out_off) + first)[j] = red;
+                if (q < n) po[q][j] = red;
             } else {
               out_local[j] = red;
             }
@@ -1227,17 +1352,17 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kZeroCopy(const HlCommDev* com
       }
     }
   }
-  blockBarrier(c, a.seq + 2, 2);
-  callDone(c, 0);
+  blockBarrier(c, a, 2, 2);
+  callDone(c, a);
 }
 
 }  // namespace dev
 
-// ====================================================================== host
 namespace nvl {
 
+// The kernel of a wire type; every type is instantiated in one of the nvl_kernels_*.cu files (they compile side by side).
 template <typename W>
-static const void* pickKernelT(int kind, int nranks) {
+const void* pickKernelT(int kind, int nranks) {
   using namespace dev;
   switch (kind) {
     case kNvlAllReduceOneShot: return (const void*)kAllReduceOneShot<W>;
@@ -1248,9 +1373,13 @@ static const void* pickKernelT(int kind, int nranks) {
     case kNvlAllToAll: return (const void*)kAllToAll<W>;
     case kNvlAllGatherNvls: return (const void*)kAllGather<W, true>;
     case kNvlBroadcastNvls: return (const void*)kBroadcast<W, true>;
-    case kNvlAllReducePush: return (const void*)kPush<W, true>;
-    case kNvlReduceScatterPush: return (const void*)kPush<W, false>;
-    case kNvlAllGatherPush: return (const void*)kAllGatherPush<W>;
+    // one variant per rank-count class (the sources a fold has in flight)
+    case kNvlAllReducePush:
+      return nranks <= 2 ? (const void*)kPush<W, true, 2> : (nranks <= 4 ? (const void*)kPush<W, true, 4> : (const void*)kPush<W, true, HL_MAX_RANKS>);
+    case kNvlReduceScatterPush:
+      return nranks <= 2 ? (const void*)kPush<W, false, 2> : (nranks <= 4 ? (const void*)kPush<W, false, 4> : (const void*)kPush<W, false, HL_MAX_RANKS>);
+    case kNvlAllGatherPush: return (const void*)kExchangePush<W, true>;
+    case kNvlAllToAllPush: return (const void*)kExchangePush<W, false>;
     case kNvlAllGatherLanes: return (const void*)kAllGatherLanes<W>;
     case kNvlAllReducePipeP2p:   // one variant per rank-count class (the unrolled source loop of the fold)
       return nranks <= 2 ? (const void*)kPipeCta<W, true, 2> : (nranks <= 4 ? (const void*)kPipeCta<W, true, 4> : (const void*)kPipeCta<W, true, HL_MAX_RANKS>);
@@ -1278,110 +1407,6 @@ static const void* pickKernelT(int kind, int nranks) {
     }
   }
   return nullptr;
-}
-
-const void* kernelFor(int kind, int wire_dt, int nranks) {
-  if (kind == kNvlBarrier) return (const void*)dev::kBarrier;
-  if (kind == kNvlLlAllReduce || kind == kNvlLlReduceScatter || kind == kNvlLlAllGather || kind == kNvlLlAllToAll) return lowLatencyKernelFor(kind, wire_dt);
-  switch (wire_dt) {
-    case hlInt8: return pickKernelT<int8_t>(kind, nranks);
-    case hlUint8: return pickKernelT<uint8_t>(kind, nranks);
-    case hlInt32: return pickKernelT<int32_t>(kind, nranks);
-    case hlUint32: return pickKernelT<uint32_t>(kind, nranks);
-    case hlInt64: return pickKernelT<long long>(kind, nranks);
-    case hlUint64: return pickKernelT<unsigned long long>(kind, nranks);
-    case hlFloat16: return pickKernelT<__half>(kind, nranks);
-    case hlFloat32: return pickKernelT<float>(kind, nranks);
-    case hlFloat64: return pickKernelT<double>(kind, nranks);
-    case hlBfloat16: return pickKernelT<__nv_bfloat16>(kind, nranks);
-    default: return nullptr;
-  }
-}
-
-const char* kernelName(int kind) {
-  switch (kind) {
-    case kNvlBarrier: return "barrier";
-    case kNvlAllReduceOneShot: return "allreduce_oneshot";
-    case kNvlAllReduceTwoShot: return "allreduce_twoshot_p2p";
-    case kNvlAllReduceNvls: return "allreduce_nvls";
-    case kNvlReduceScatter: return "reducescatter_p2p";
-    case kNvlReduceScatterNvls: return "reducescatter_nvls";
-    case kNvlAllGather: return "allgather_p2p";
-    case kNvlBroadcast: return "broadcast_p2p";
-    case kNvlAllToAll: return "alltoall_p2p";
-    case kNvlAllGatherNvls: return "allgather_nvls";
-    case kNvlBroadcastNvls: return "broadcast_nvls";
-    case kNvlAllReducePush: return "allreduce_push";
-    case kNvlReduceScatterPush: return "reducescatter_push";
-    case kNvlAllGatherPush: return "allgather_push";
-    case kNvlAllGatherLanes: return "allgather_lanes";
-    case kNvlAllReducePipeP2p: return "allreduce_pipelined_p2p";
-    case kNvlAllReducePipeNvls: return "allreduce_pipelined_nvls";
-    case kNvlReduceScatterPipeP2p: return "reducescatter_pipelined_p2p";
-    case kNvlReduceScatterPipeNvls: return "reducescatter_pipelined_nvls";
-    case kNvlZcAllReduceNvls: return "allreduce_zerocopy_nvls";
-    case kNvlZcAllReduceP2p: return "allreduce_zerocopy_p2p";
-    case kNvlZcReduceScatterNvls: return "reducescatter_zerocopy_nvls";
-    case kNvlZcReduceScatterP2p: return "reducescatter_zerocopy_p2p";
-    case kNvlZcAllGatherNvls: return "allgather_zerocopy_nvls";
-    case kNvlZcAllGatherP2p: return "allgather_zerocopy_p2p";
-    case kNvlZcBroadcastNvls: return "broadcast_zerocopy_nvls";
-    case kNvlZcBroadcastP2p: return "broadcast_zerocopy_p2p";
-    case kNvlLlAllReduce: return "allreduce_lowlatency";
-    case kNvlLlReduceScatter: return "reducescatter_lowlatency";
-    case kNvlLlAllGather: return "allgather_lowlatency";
-    case kNvlLlAllToAll: return "alltoall_lowlatency";
-    default: return "?";
-  }
-}
-
-hlResult_t launch(int kind, int wire_dt, const HlCommDev* dcomms, const HlEmuCalls& calls, int emu_ranks, int blocks,
-                  cudaStream_t stream, int nranks) {
-  const void* fn = kernelFor(kind, wire_dt, nranks);
-  if (!fn) return fail(hlUnsupported, "no %s kernel for wire type %d", kernelName(kind), wire_dt);
-  if (blocks < 1) blocks = 1;
-  if (blocks > HL_MAX_BLOCKS) blocks = HL_MAX_BLOCKS;
-  dim3 grid((unsigned)blocks, (unsigned)(emu_ranks > 1 ? emu_ranks : 1), 1);
-  const bool pipe = kind == kNvlAllReducePipeNvls || kind == kNvlReduceScatterPipeNvls;  // warp-group stages: 384 threads
-  dim3 block(pipe ? dev::kPipeThreads : HL_NVL_THREADS, 1, 1);
-  void* args[2] = {(void*)&dcomms, (void*)&calls};
-  cudaError_t e;
-  if (emu_ranks > 1) {
-    // The emulated ranks wait on one another: all their blocks must be
-    // co-resident, which only a cooperative launch guarantees (it fails
-    // cleanly instead of deadlocking when they would not fit).
-    e = cudaLaunchCooperativeKernel(fn, grid, block, args, 0, stream);
-  } else {
-    e = cudaLaunchKernel(fn, grid, block, args, 0, stream);
-  }
-  if (e != cudaSuccess) return fail(hlDeviceError, "launch of %s failed: %s", kernelName(kind), cudaGetErrorString(e));
-  return hlSuccess;
-}
-
-hlResult_t prepareKernels() {
-  // Resolve every variant once on the init thread: lazy module loading plus
-  // concurrent first launches from several threads can deadlock in the driver
-  // (same cure as pcie-ccl-cuda/kernels/wait_kernel.cu:216-234,400-432).
-  static const int kinds[] = {kNvlBarrier, kNvlAllReduceOneShot, kNvlAllReduceTwoShot, kNvlAllReduceNvls,
-                              kNvlReduceScatter, kNvlReduceScatterNvls, kNvlAllGather, kNvlBroadcast,
-                              kNvlAllToAll, kNvlAllGatherNvls, kNvlBroadcastNvls, kNvlAllReducePipeP2p,
-                              kNvlAllReducePipeNvls, kNvlReduceScatterPipeP2p, kNvlReduceScatterPipeNvls, kNvlAllReducePush,
-                              kNvlReduceScatterPush, kNvlAllGatherPush, kNvlAllGatherLanes, kNvlZcAllReduceNvls,
-                              kNvlZcAllReduceP2p, kNvlZcReduceScatterNvls, kNvlZcReduceScatterP2p, kNvlZcAllGatherNvls,
-                              kNvlZcAllGatherP2p, kNvlZcBroadcastNvls, kNvlZcBroadcastP2p, kNvlLlAllReduce,
-                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll};
-  for (int k : kinds)
-    for (int dt = 0; dt < hlNumTypes; ++dt) {
-      for (int nr : {2, 4, HL_MAX_RANKS}) {   // rank-count classes (only the pipelined push kernels differ by it)
-        const void* fn = kernelFor(k, dt, nr);
-        if (!fn) continue;
-        cudaFuncAttributes at;
-        cudaError_t e = cudaFuncGetAttributes(&at, fn);
-        if (e != cudaSuccess) return fail(hlDeviceError, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
-      }
-      if (k == kNvlBarrier) break;
-    }
-  return hlSuccess;
 }
 
 }  // namespace nvl

@@ -14,9 +14,9 @@ const void* kernelFor(int kind, int wire_dt, int nranks = HL_MAX_RANKS);
 const char* kernelName(int kind);
 // The barrier-free small-message kernels live in a file of their own (nvl_ll_kernels.cu).
 const void* lowLatencyKernelFor(int kind, int wire_dt);
-// emu_ranks > 1: cooperative launch with one grid row per emulated rank.
+// emu_ranks > 1: cooperative launch with one grid row per emulated rank. threads: of a CTA (0: what the kernel is made for).
 hlResult_t launch(int kind, int wire_dt, const HlCommDev* dcomms, const HlEmuCalls& calls, int emu_ranks, int blocks,
-                  cudaStream_t stream, int nranks = HL_MAX_RANKS);
+                  cudaStream_t stream, int nranks = HL_MAX_RANKS, int threads = 0);
 hlResult_t prepareKernels();
 // Bare copy between this rank's staging and `peer`'s (see link_probe.cu); mode 0 push, 1 pull, 2 local, 3 stores
 // only, 4 loads only; `packets` 16-byte packets from offset 0 to offset dst_off.
@@ -40,7 +40,7 @@ struct ReduceLandingArgs {
 hlResult_t launchLinkProbeBulk(const HlCommDev* dcomm, int to_peer, int blocks, uint32_t tile_bytes, uint64_t bytes, uint64_t dst_off_bytes,
                                int peer, cudaStream_t stream);
 hlResult_t launchReduceLanding(const ReduceLandingArgs& a, int blocks, cudaStream_t stream);
-// Device-to-device copy of whole 16-byte packets between 16-byte aligned buffers (streaming cache hints).
+// Device-to-device copy of whole 16-byte packets between 16-byte aligned buffers.
 hlResult_t launchCopy(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 hlResult_t prepareReduceLanding();
 

@@ -64,6 +64,7 @@ hlResult_t NvlPath::finishInit(int timeout_ms) {
     c.rank = emu_ ? i : rank_;
     c.nranks = nranks_;
     c.max_blocks = HL_MAX_BLOCKS;
+    c.one_device = emu_ ? 1 : 0;
     for (int q = 0; q < nranks_; ++q) {
       uint8_t* base = (uint8_t*)(emu_ ? emu_mem_[q] : region_.ptr[q]);
       c.stage[q] = base;
@@ -634,13 +635,17 @@ hlResult_t NvlPath::launchLowLatency(int kind, const NvlBufs& b, const NvlCall& 
     a.kind = kind;
   }
   // one thread per packet it sends to (and receives from) every peer; at most one CTA per SM, so that the CTAs
-  // with the same index are resident on every rank at the same time (they wait for one another's packets)
+  // with the same index are resident on every rank at the same time (they wait for one another's packets). Small
+  // messages spread over more and smaller CTAs: a packet is 2 (n - 1) stores and as many polls of its thread, and an
+  // SM issues them one after the other.
   int cap = c.max_blocks > 0 ? std::min(c.max_blocks, 148) : 148;
   if (Config::get().nvl_max_blocks > 0) cap = std::min(cap, Config::get().nvl_max_blocks);
   if (emu_) cap = std::min(cap, std::max(1, 148 / nranks_));
-  const uint64_t want = std::max<uint64_t>(1, (packets + HL_NVL_THREADS - 1) / HL_NVL_THREADS);
+  int threads = 64;
+  while (threads < HL_LL_THREADS && packets > (uint64_t)cap * threads) threads *= 2;
+  const uint64_t want = std::max<uint64_t>(1, (packets + threads - 1) / threads);
   const int blocks = (int)std::min<uint64_t>(want, (uint64_t)cap);
-  HL_CHECK(nvl::launch(kind, c.wire_dt, dcomm_, calls, emu_ ? emu_active_ : 1, blocks, s, nranks_));
+  HL_CHECK(nvl::launch(kind, c.wire_dt, dcomm_, calls, emu_ ? emu_active_ : 1, blocks, s, nranks_, threads));
   ++launches_;
   return hlSuccess;
 }
@@ -716,7 +721,8 @@ hlResult_t NvlPath::reduceScatter(const NvlBufs& b, const NvlCall& c, cudaStream
   } else if (same && c.algo != hlAlgoTwoShotP2p && c.algo != hlAlgoOneShot) {
     // Peer pointers: the phased stores-only kernel, and from 128 MiB the lane kernel that folds while it pushes
     // (2 GPUs, bf16: 513 against 449 GB/s at 256 MiB, 580 against 485 GB/s at 1 GiB; 347 against 359 at 64 MiB).
-    const bool lanes = c.algo == hlAlgoPipelined || (c.algo == hlAlgoAuto && wire_bytes >= lanesMinBytes());
+    // Ranks of one GPU have no link to keep busy while others fold: the phases with the whole grid are faster.
+    const bool lanes = c.algo == hlAlgoPipelined || (c.algo == hlAlgoAuto && !emu_ && wire_bytes >= lanesMinBytes());
     kind = lanes ? kNvlReduceScatterPipeP2p : kNvlReduceScatterPush;
   }
   return launchSliced(kind, b, c, true, s);
@@ -771,7 +777,10 @@ hlResult_t NvlPath::allToAll(const NvlBufs& b, const NvlCall& c, cudaStream_t s)
     if (ll < 0) return fail(hlUnsupported, "all-to-all: the low-latency kernel converts no types and needs a message that fits its slots");
     if (ll > 0) return launchLowLatency(kNvlLlAllToAll, b, c, (seg_wire + 15) / 16, s);
   }
-  return launchSliced(kNvlAllToAll, b, c, true, s);
+  // stores straight from the caller's buffer into the peers' staging, unless the call converts types or asks for the
+  // pull kernel by name; the own segment never touches the staging
+  const bool push = c.in_dt == c.wire_dt && c.out_dt == c.wire_dt && c.algo != hlAlgoTwoShotP2p;
+  return launchSliced(push ? kNvlAllToAllPush : kNvlAllToAll, b, c, true, s);
 }
 
 hlResult_t NvlPath::barrier(cudaStream_t s) {

@@ -6,6 +6,7 @@
 #define HL_MAX_RANKS 8        // one NVSwitch domain of an HGX B200 board
 #define HL_MAX_BLOCKS 592     // 148 SMs x 4 resident CTAs
 #define HL_NVL_THREADS 512
+#define HL_LL_THREADS 256       // low-latency kernels: at most
 #define HL_SEQ_STRIDE 4       // flag values consumed per collective call
 #define HL_FLAG_KINDS 3       // 0: block barriers; 1, 2: tile hand-offs of the pipelined kernels
 // Kernel timeline (off unless the communicator was created with it): a ring of the last HL_TL_CALLS launches, for
@@ -30,14 +31,14 @@ struct HlCommDev {
   int rank;
   int nranks;
   int max_blocks;
-  int pad0;
+  int one_device;                  // all ranks share this GPU: flags are exchanged at GPU scope
   uint8_t* stage[HL_MAX_RANKS];    // symmetric staging region
   uint64_t* flags[HL_MAX_RANKS];   // [HL_FLAG_KINDS][HL_MAX_BLOCKS][HL_MAX_RANKS] monotonically increasing words
   uint8_t* mc_stage;               // NVSwitch multicast alias of stage (null without NVLS)
   uint64_t* status;                // host-visible: [0] code, [1] detail (step<<32 | peer), [2] block
   uint32_t* abort_word;            // device word: non-zero poisons the communicator
   uint64_t* seq_words;             // device words: [0] flag base of the next call, [1] tile base of the next pipelined
-                                   // call, [2] CTAs of the running call that have finished
+                                   // call, [2] CTAs of the running call that have read both
   uint64_t stage_bytes;
   uint64_t timeout_ns;
   uint64_t* timeline;              // device ring of HL_TL_WORDS words, null when the timeline is off
@@ -119,5 +120,6 @@ enum HlNvlKernel {
   kNvlLlReduceScatter = 28,
   kNvlLlAllGather = 29,
   kNvlLlAllToAll = 30,
+  kNvlAllToAllPush = 31,
 };
 #define HL_DEV_ASYMMETRIC 4   // zero-copy call whose buffers do not sit at the same heap offset on every rank
