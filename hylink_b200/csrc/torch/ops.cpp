@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/python.h>
 
+#include "hylink/hylink_ext.h"
 #include "train/train_kernels.h"
 
 namespace {
@@ -365,6 +366,51 @@ void shardedAdamW(const Tensor& grad, const Tensor& weight, const std::optional<
      "sharded AdamW");
 }
 
+// ---- calls whose cost on the host is most of a small one: argument lists are taken apart here, not in Python
+int typeCode(at::ScalarType t) {
+  switch (t) {
+    case at::kChar: return hlInt8;
+    case at::kByte: return hlUint8;
+    case at::kInt: return hlInt32;
+    case at::kLong: return hlInt64;
+    case at::kHalf: return hlFloat16;
+    case at::kFloat: return hlFloat32;
+    case at::kDouble: return hlFloat64;
+    case at::kBFloat16: return hlBfloat16;
+    default: TORCH_CHECK(false, "hylink: unsupported dtype ", t);
+  }
+}
+using TensorList = std::vector<std::optional<Tensor>>;
+
+// One collective of an emulated group on the current stream; returns the library's result code.
+int emuRun(uintptr_t group, int nranks, int kind, const std::optional<TensorList>& ins, const std::optional<TensorList>& outs, size_t count,
+           size_t in_stride, size_t out_stride, const std::optional<at::ScalarType>& wire, int op, double scale, int root, int algo, int max_blocks) {
+  const void* in[8] = {nullptr};
+  void* out[8] = {nullptr};
+  TORCH_CHECK(nranks <= 8 && (!ins || (int)ins->size() <= nranks) && (!outs || (int)outs->size() <= nranks), "hylink: more buffers than ranks");
+  for (size_t i = 0; ins && i < ins->size(); ++i)
+    if ((*ins)[i]) in[i] = (*ins)[i]->data_ptr();
+  for (size_t i = 0; outs && i < outs->size(); ++i)
+    if ((*outs)[i]) out[i] = (*outs)[i]->data_ptr();
+  const int in_dt = ins ? typeCode((*ins)[0]->scalar_type()) : (int)hlFloat32;
+  const int out_dt = outs ? typeCode((*outs)[0]->scalar_type()) : in_dt;
+  return (int)hlEmuCollective(reinterpret_cast<hlEmu_t>(group), kind, in, out, count, in_stride, out_stride, in_dt, out_dt,
+                              wire ? typeCode(*wire) : in_dt, op, (float)scale, root, algo, max_blocks, c10::cuda::getCurrentCUDAStream().stream());
+}
+
+int reduceLanding(const Tensor& dst, const std::vector<Tensor>& srcs, int op, double scale, bool accumulate, int blocks) {
+  TORCH_CHECK_VALUE(dst.is_cuda(), "reduce_landing needs a CUDA destination");
+  std::vector<const void*> p;
+  p.reserve(srcs.size());
+  for (const Tensor& s : srcs) {
+    TORCH_CHECK_VALUE(s.numel() == dst.numel() && s.scalar_type() == dst.scalar_type(), "sources must match the destination's size and dtype");
+    TORCH_CHECK_VALUE(s.is_cuda() || s.is_pinned(), "host sources must be pinned");
+    p.push_back(s.data_ptr());
+  }
+  return (int)hlReduceLanding(dst.data_ptr(), p.data(), (int)p.size(), accumulate, (size_t)dst.numel(), (hlDataType_t)typeCode(dst.scalar_type()),
+                              (hlRedOp_t)op, (float)scale, blocks, c10::cuda::getCurrentCUDAStream().stream());
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -384,5 +430,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return MoeCombine::apply(x, gate, rows, row_of, token_of);
   });
   m.def("sharded_adamw", &shardedAdamW);
+  m.def("emu_run", [](uintptr_t group, int nranks, int kind, const std::optional<TensorList>& ins, const std::optional<TensorList>& outs, size_t count,
+                      size_t in_stride, size_t out_stride, const py::object& wire, int op, double scale, int root, int algo, int max_blocks) {
+    return emuRun(group, nranks, kind, ins, outs, count, in_stride, out_stride,
+                  wire.is_none() ? std::nullopt : std::make_optional(torch::python::detail::py_object_to_dtype(wire)), op, scale, root, algo, max_blocks);
+  });
+  m.def("reduce_landing", &reduceLanding);
   m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });
 }

@@ -14,7 +14,8 @@ from typing import Sequence
 
 import torch
 
-from .._native import OPS, check, lib, torch_dtype_code
+from .._native import OPS, check, lib
+from .extension import ops
 
 KINDS = {"all_reduce": 0, "reduce_scatter": 1, "all_gather": 2, "broadcast": 3, "all_to_all": 4, "barrier": 5}
 ALGOS = {"auto": 0, "oneshot": 1, "twoshot": 2, "nvls": 3, "pipelined": 4, "push": 5, "zerocopy": 6, "zerocopy_nvls": 7,
@@ -38,23 +39,13 @@ class EmuGroup:
         except Exception:
             pass
 
-    def _ptrs(self, ts: Sequence[torch.Tensor] | None):
-        arr = (C.c_void_p * self.nranks)()
-        if ts is not None:
-            for i, t in enumerate(ts):
-                arr[i] = t.data_ptr() if t is not None else None
-        return arr
-
     def run(self, kind: str, ins, outs, count: int, *, in_seg_stride: int = 0, out_seg_stride: int = 0,
             wire_dtype=None, op: str = "sum", scale: float = 1.0, root: int = 0, algo: str = "auto",
             max_blocks: int = 0):
-        in_dt = torch_dtype_code(ins[0].dtype) if ins is not None else 7
-        out_dt = torch_dtype_code(outs[0].dtype) if outs is not None else in_dt
-        wire_dt = torch_dtype_code(wire_dtype) if wire_dtype is not None else in_dt
-        stream = torch.cuda.current_stream().cuda_stream
-        check(lib.hlEmuCollective(self._h, KINDS[kind], self._ptrs(ins), self._ptrs(outs), count, in_seg_stride,
-                                  out_seg_stride, in_dt, out_dt, wire_dt, OPS[op], scale, root, ALGOS[algo],
-                                  max_blocks, C.c_void_p(stream)), f"emu {kind}")
+        code = ops().emu_run(self._h.value or 0, self.nranks, KINDS[kind], ins, outs, count, in_seg_stride, out_seg_stride, wire_dtype, OPS[op],
+                             scale, root, ALGOS[algo], max_blocks)
+        if code:
+            check(code, f"emu {kind}")
 
     def alloc_registered(self, numel: int, dtype=torch.float32):
         """One tensor per emulated rank in registered memory (the same heap offset on every rank)."""
