@@ -20,21 +20,29 @@ namespace nvl {
 
 template <typename W>
 const void* pickKernelT(int kind, int nranks);   // nvl_kernels_*.cu
+template <typename W>
+const void* pickStreamT(int kind, int nranks);   // nvl_stream_*.cu
+
+static bool streamed(int kind) { return kind == kNvlStreamReduceScatter || kind == kNvlStreamAllGather || kind == kNvlStreamAllToAll; }
+template <typename W>
+static const void* pick(int kind, int nranks) {
+  return streamed(kind) ? pickStreamT<W>(kind, nranks) : pickKernelT<W>(kind, nranks);
+}
 
 const void* kernelFor(int kind, int wire_dt, int nranks) {
   if (kind == kNvlBarrier) return (const void*)dev::kBarrier;
   if (kind == kNvlLlAllReduce || kind == kNvlLlReduceScatter || kind == kNvlLlAllGather || kind == kNvlLlAllToAll) return lowLatencyKernelFor(kind, wire_dt);
   switch (wire_dt) {
-    case hlInt8: return pickKernelT<int8_t>(kind, nranks);
-    case hlUint8: return pickKernelT<uint8_t>(kind, nranks);
-    case hlInt32: return pickKernelT<int32_t>(kind, nranks);
-    case hlUint32: return pickKernelT<uint32_t>(kind, nranks);
-    case hlInt64: return pickKernelT<long long>(kind, nranks);
-    case hlUint64: return pickKernelT<unsigned long long>(kind, nranks);
-    case hlFloat16: return pickKernelT<__half>(kind, nranks);
-    case hlFloat32: return pickKernelT<float>(kind, nranks);
-    case hlFloat64: return pickKernelT<double>(kind, nranks);
-    case hlBfloat16: return pickKernelT<__nv_bfloat16>(kind, nranks);
+    case hlInt8: return pick<int8_t>(kind, nranks);
+    case hlUint8: return pick<uint8_t>(kind, nranks);
+    case hlInt32: return pick<int32_t>(kind, nranks);
+    case hlUint32: return pick<uint32_t>(kind, nranks);
+    case hlInt64: return pick<long long>(kind, nranks);
+    case hlUint64: return pick<unsigned long long>(kind, nranks);
+    case hlFloat16: return pick<__half>(kind, nranks);
+    case hlFloat32: return pick<float>(kind, nranks);
+    case hlFloat64: return pick<double>(kind, nranks);
+    case hlBfloat16: return pick<__nv_bfloat16>(kind, nranks);
     default: return nullptr;
   }
 }
@@ -73,6 +81,9 @@ const char* kernelName(int kind) {
     case kNvlLlAllGather: return "allgather_lowlatency";
     case kNvlLlAllToAll: return "alltoall_lowlatency";
     case kNvlAllToAllPush: return "alltoall_push";
+    case kNvlStreamReduceScatter: return "reducescatter_streamed";
+    case kNvlStreamAllGather: return "allgather_streamed";
+    case kNvlStreamAllToAll: return "alltoall_streamed";
     default: return "?";
   }
 }
@@ -85,6 +96,7 @@ hlResult_t launch(int kind, int wire_dt, const HlCommDev* dcomms, const HlEmuCal
   if (blocks > HL_MAX_BLOCKS) blocks = HL_MAX_BLOCKS;
   dim3 grid((unsigned)blocks, (unsigned)(emu_ranks > 1 ? emu_ranks : 1), 1);
   const bool pipe = kind == kNvlAllReducePipeNvls || kind == kNvlReduceScatterPipeNvls;  // warp-group stages: 384 threads
+  if (streamed(kind)) threads = HL_STREAM_WORKERS + 64;
   dim3 block((unsigned)(threads > 0 ? threads : (pipe ? dev::kPipeWarpGroupThreads : HL_NVL_THREADS)), 1, 1);
   void* args[2] = {(void*)&dcomms, (void*)&calls};
   cudaError_t e;
@@ -111,7 +123,8 @@ hlResult_t prepareKernels() {
                               kNvlReduceScatterPush, kNvlAllGatherPush, kNvlAllGatherLanes, kNvlZcAllReduceNvls,
                               kNvlZcAllReduceP2p, kNvlZcReduceScatterNvls, kNvlZcReduceScatterP2p, kNvlZcAllGatherNvls,
                               kNvlZcAllGatherP2p, kNvlZcBroadcastNvls, kNvlZcBroadcastP2p, kNvlLlAllReduce,
-                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlAllToAllPush};
+                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlAllToAllPush,
+                              kNvlStreamReduceScatter, kNvlStreamAllGather, kNvlStreamAllToAll};
   for (int k : kinds)
     for (int dt = 0; dt < hlNumTypes; ++dt) {
       for (int nr : {2, 4, HL_MAX_RANKS}) {   // rank-count classes (only the pipelined push kernels differ by it)

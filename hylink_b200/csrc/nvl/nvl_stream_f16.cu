@@ -1,0 +1,7 @@
+#include "nvl/nvl_stream_kernels.cuh"
+
+namespace hl {
+namespace nvl {
+template const void* pickStreamT<__half>(int kind, int nranks);
+}  // namespace nvl
+}  // namespace hl

@@ -7,6 +7,8 @@
 #define HL_MAX_BLOCKS 592     // 148 SMs x 4 resident CTAs
 #define HL_NVL_THREADS 512
 #define HL_LL_THREADS 256       // low-latency kernels: at most
+#define HL_STREAM_WORKERS 448    // streamed kernels: threads that move data (two more warps poll and signal)
+#define HL_STREAM_LAG 3          // iterations that data and flags have to travel (the ring holds twice as many pieces)
 #define HL_SEQ_STRIDE 4       // flag values consumed per collective call
 #define HL_FLAG_KINDS 3       // 0: block barriers; 1, 2: tile hand-offs of the pipelined kernels
 // Kernel timeline (off unless the communicator was created with it): a ring of the last HL_TL_CALLS launches, for
@@ -121,5 +123,9 @@ enum HlNvlKernel {
   kNvlLlAllGather = 29,
   kNvlLlAllToAll = 30,
   kNvlAllToAllPush = 31,
+  // large messages between ranks of one GPU: the push scheme through a ring of pieces that stays in L2
+  kNvlStreamReduceScatter = 32,
+  kNvlStreamAllGather = 33,
+  kNvlStreamAllToAll = 34,
 };
 #define HL_DEV_ASYMMETRIC 4   // zero-copy call whose buffers do not sit at the same heap offset on every rank

@@ -1,0 +1,96 @@
+"""Streamed push kernels (large messages between ranks of one GPU: a ring of pieces instead of staging of the message's
+size) against PyTorch, bit for bit: ascending rank order, fp32 accumulation, one rounding."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(count, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    if dtype.is_floating_point:
+        return torch.randn(count, generator=g, device="cuda").to(dtype)
+    return torch.randint(-50, 50, (count,), generator=g, device="cuda").to(dtype)
+
+
+def _sum(ts, dtype):
+    acc = ts[0].float() if dtype.is_floating_point else ts[0].clone()
+    for t in ts[1:]:
+        acc = acc + (t.float() if dtype.is_floating_point else t)
+    return acc.to(dtype)
+
+
+# whole pieces, ragged ends, every rank-count class and counts between the classes, a strided prefix of wider segments,
+# segments that start inside a packet (these keep the plain kernels)
+@pytest.mark.parametrize("n,seg,dtype,offset", [(2, (9 << 20) + 4, torch.float32, 0), (3, 3 * 1000003 + 1, torch.float32, 0),
+                                                (4, 3 << 20, torch.bfloat16, 0), (8, 448 * 8 * 200 + 5, torch.bfloat16, 0),
+                                                (8, (1 << 19) + 3, torch.int32, 0), (5, 1500001, torch.bfloat16, 1)])
+def test_streamed_collectives(n, seg, dtype, offset, monkeypatch):
+    from hylink_b200.ops import EmuGroup
+
+    monkeypatch.setenv("HYLINK_KERNEL_TIMELINE", "1")
+    g = EmuGroup(n)
+    kinds = lambda: {launch["kind"] for launch in g.kernel_timeline()}  # noqa: E731
+    pad = 16
+
+    def outs(elems):
+        return [torch.full((offset + elems + pad,), 7, dtype=dtype, device="cuda") for _ in range(n)]
+
+    def body(bufs, elems):
+        return [b[offset:offset + elems] for b in bufs]
+
+    stride = (seg + 31) // 8 * 8
+    wide = [_rand(offset + n * stride, dtype, 900 + r)[offset:] for r in range(n)]
+    sums = [_sum([w[r * stride:r * stride + seg] for w in wide], dtype) for r in range(n)]
+    for _ in range(2):                                # back to back: the ring and its flags carry over
+        o = outs(seg)
+        g.run("reduce_scatter", wide, body(o, seg), seg, in_seg_stride=stride)
+        for b, want in zip(o, sums):
+            assert torch.equal(b[offset:offset + seg], want) and bool((b[offset + seg:] == 7).all())
+    o = outs(n * stride)
+    g.run("all_gather", [w[:seg] for w in wide], body(o, n * stride), seg, out_seg_stride=stride)
+    for b in o:
+        for q in range(n):
+            at = offset + q * stride
+            assert torch.equal(b[at:at + seg], wide[q][:seg]) and bool((b[at + seg:at + stride] == 7).all())
+    o = outs(n * stride)
+    g.run("all_to_all", wide, body(o, n * stride), seg, in_seg_stride=stride, out_seg_stride=stride)
+    for r, b in enumerate(o):
+        for q in range(n):
+            at = offset + q * stride
+            assert torch.equal(b[at:at + seg], wide[q][r * stride:r * stride + seg]) and bool((b[at + seg:at + stride] == 7).all())
+    want = {"allgather_streamed", "alltoall_streamed"} | ({"reducescatter_streamed"} if n <= 4 else set())
+    assert {k for k in kinds() if k.endswith("streamed")} == (want if offset == 0 else set())
+    # in place: the result into the own segment of the input, the input out of the own segment of the output, one buffer
+    work = [w.clone() for w in wide]
+    g.run("reduce_scatter", work, [w[r * stride:r * stride + seg] for r, w in enumerate(work)], seg, in_seg_stride=stride)
+    assert all(torch.equal(w[r * stride:r * stride + seg], sums[r]) for r, w in enumerate(work))
+    work = [w.clone() for w in wide]
+    g.run("all_gather", [w[r * stride:r * stride + seg] for r, w in enumerate(work)], work, seg, out_seg_stride=stride)
+    assert all(torch.equal(w[q * stride:q * stride + seg], wide[q][q * stride:q * stride + seg]) for w in work for q in range(n))
+    work = [w.clone() for w in wide]
+    g.run("all_to_all", work, work, seg, in_seg_stride=stride, out_seg_stride=stride)
+    assert all(torch.equal(w[q * stride:q * stride + seg], wide[q][r * stride:r * stride + seg]) for r, w in enumerate(work) for q in range(n))
+    assert g.status(0)[0] == 0
+    g.close()
+
+
+def test_streamed_wait_is_bounded():
+    from hylink_b200.ops import EmuGroup
+
+    n, seg = 4, 2 << 20
+    g = EmuGroup(n, timeout_ms=200)
+    ins = [_rand(n * seg, torch.float32, r) for r in range(n)]
+    outs = [torch.zeros(seg, device="cuda") for _ in range(n)]
+    g.set_active_ranks(n - 1)
+    g.run("reduce_scatter", ins, outs, seg, in_seg_stride=seg)
+    torch.cuda.synchronize()                          # returns: the wait was bounded
+    code, _, peer, _ = g.status(0)
+    assert code == 1 and peer == n - 1
+    g.set_active_ranks(n)
+    g.reset()
+    g.run("reduce_scatter", ins, outs, seg, in_seg_stride=seg)
+    torch.cuda.synchronize()
+    assert g.status(0)[0] == 0
+    assert all(torch.equal(o, _sum([t[r * seg:(r + 1) * seg] for t in ins], torch.float32)) for r, o in enumerate(outs))
+    g.close()
