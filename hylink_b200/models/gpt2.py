@@ -46,6 +46,12 @@ def _hooked(m: nn.Module) -> bool:
     return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
 
 
+def _any_global_hook() -> bool:
+    from torch.nn.modules import module as g
+
+    return bool(g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)
+
+
 class Block(nn.Module):
     def __init__(self, c: GPT2Config):
         super().__init__()
@@ -107,6 +113,8 @@ class GPT2(nn.Module):
             return False
         if c.d_model > ops().max_norm_width or c.d_model % 8 or (c.d_model // c.n_head) % 8 or torch.is_autocast_enabled("cuda"):
             return False
+        if _any_global_hook():
+            return False
         mods = [self.ln_f, self.wte]
         for blk in self.blocks:
             if type(blk) is not Block or _hooked(blk):
@@ -118,6 +126,21 @@ class GPT2(nn.Module):
             if type(m) is not nn.Embedding and m.bias is None:
                 return False
         return True
+
+    def step_signature(self, idx: torch.Tensor, targets: torch.Tensor):
+        """What a recorded training step depends on besides its inputs' values: equal signatures may share a recording.
+        None when a step has effects that a recording would not repeat (hooks) or does not take the fused operators."""
+        if not self._fusable(self.wte.weight, targets) or _hooked(self) or not torch.is_grad_enabled():
+            return None
+        ps = list(self.parameters())
+        if any(p._backward_hooks or p._post_accumulate_grad_hooks for p in ps):
+            return None
+        cuda = torch.backends.cuda
+        flags = (torch.are_deterministic_algorithms_enabled(), cuda.flash_sdp_enabled(), cuda.mem_efficient_sdp_enabled(), cuda.cudnn_sdp_enabled(),
+                 cuda.math_sdp_enabled(), cuda.matmul.allow_bf16_reduced_precision_reduction, cuda.matmul.allow_fp16_reduced_precision_reduction)
+        eps = tuple(m.eps for blk in self.blocks for m in (blk.ln1, blk.ln2)) + (self.ln_f.eps,)
+        heads = tuple(blk.n_head for blk in self.blocks)
+        return tuple((p.data_ptr(), p.requires_grad, p.shape) for p in ps), eps, heads, flags
 
     def _fused_loss(self, x: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
         f = ops()

@@ -6,6 +6,14 @@ the model in ``DistributedDataParallel`` over this library's process group
 ``step(tokens)`` which takes a pinned host batch, copies it to the device,
 runs forward / backward (gradient all-reduces overlap the backward pass on the
 backend's own stream) / optimizer, and returns the loss as a Python float.
+
+A job of one rank has no gradient to reduce: the model is not wrapped then (the
+buckets would only cost a copy of every gradient), and models that can say when
+a step may be replayed (``step_signature``, as :class:`~hylink_b200.models.gpt2.GPT2`
+does) run forward and backward from a CUDA graph once a batch shape has come
+three times in a row. Issuing the thousand launches of a step takes the host
+longer than the GPU needs for a small batch. The graph holds the memory of one
+step; ``HYLINK_TRAIN_GRAPH=0`` or :meth:`DDPTrainer.close` gives it back.
 """
 from __future__ import annotations
 
@@ -32,6 +40,38 @@ def init_distributed(backend: str = "hylink"):
     if not dist.is_initialized():
         dist.init_process_group(backend, rank=rank, world_size=world, device_id=dev)
     return rank, world, dev
+
+
+class _StepGraph:
+    """Forward and backward of one batch shape as a CUDA graph. Inputs are copied into place, the loss and the
+    gradients are where the capture put them."""
+
+    def __init__(self, model: torch.nn.Module, params: list, idx: torch.Tensor, targets: torch.Tensor):
+        self.idx, self.targets = idx.clone(), targets.clone()
+        self.params = params
+        old = [p.grad for p in params]
+        try:
+            for p in params:
+                p.grad = None
+            self.graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(self.graph):
+                loss = model(self.idx, self.targets)
+                loss.backward()
+                self.loss = loss.detach()
+            self.grads = [p.grad for p in params]
+        except BaseException:
+            for p, g in zip(params, old):
+                p.grad = g
+            raise
+
+    def run(self, idx: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        self.idx.copy_(idx)
+        self.targets.copy_(targets)
+        self.graph.replay()
+        for p, g in zip(self.params, self.grads):
+            if p.grad is not g:
+                p.grad = g
+        return self.loss.clone()
 
 
 class DDPTrainer:
@@ -61,21 +101,54 @@ class DDPTrainer:
                 pool = registered_mem_pool()
             except Exception as ex:  # noqa: BLE001 - an older PyTorch without pluggable pools: buckets are staged
                 print(f"hylink: gradient buckets stay unregistered ({type(ex).__name__}: {ex})", flush=True)
+        self._ddp = None
+        self._bucket_cap_mb = bucket_cap_mb
+        self._graph, self._graph_key, self._key_seen = None, None, 0
+        self._use_graph = os.environ.get("HYLINK_TRAIN_GRAPH", "1") != "0"
         if pool is not None:
             with torch.cuda.use_mem_pool(pool):
-                self.ddp = DDP(self.model, device_ids=[device.index], bucket_cap_mb=bucket_cap_mb, gradient_as_bucket_view=True,
-                               static_graph=False)
+                self.ddp  # noqa: B018 - wrapped here, under the registered pool
             self.registered_buckets = True
             self._pool = pool
-        else:
-            self.ddp = DDP(self.model, device_ids=[device.index], bucket_cap_mb=bucket_cap_mb, gradient_as_bucket_view=True,
-                           static_graph=False)
-        self.opt = torch.optim.AdamW(self.ddp.parameters(), lr=lr, betas=(0.9, 0.95), weight_decay=0.1, fused=True)
+        elif dist.get_world_size() > 1:
+            self.ddp  # noqa: B018
+        self._params = list(self.model.parameters())
+        self.opt = torch.optim.AdamW(self._params, lr=lr, betas=(0.9, 0.95), weight_decay=0.1, fused=True)
         self._loss_host = torch.zeros(1, dtype=torch.float32).pin_memory()
         self._dev_batch = None
 
+    @property
+    def ddp(self) -> DDP:
+        """The ``DistributedDataParallel`` wrapper. A one-rank job makes it when it is asked for, and uses it from then on."""
+        if self._ddp is None:
+            self._graph = None
+            self._ddp = DDP(self.model, device_ids=[self.device.index], bucket_cap_mb=self._bucket_cap_mb, gradient_as_bucket_view=True,
+                            static_graph=False)
+        return self._ddp
+
+    def _replayable(self, idx: torch.Tensor, targets: torch.Tensor) -> bool:
+        """Whether this step runs from the graph; captures it when the same step has been run twice before."""
+        signature = getattr(self.model, "step_signature", None)
+        if not self._use_graph or signature is None or not (idx.is_cuda and targets.is_cuda) or torch.is_anomaly_enabled():
+            return False
+        sig = signature(idx, targets)
+        key = None if sig is None else (sig, idx.shape, idx.dtype, targets.shape, targets.dtype)
+        if key != self._graph_key:
+            self._graph, self._graph_key, self._key_seen = None, key, 0
+        if key is None:
+            return False
+        self._key_seen += 1
+        if self._graph is None and self._key_seen == 3:   # the two eager steps have loaded and sized everything
+            try:
+                self._graph = _StepGraph(self.model, self._params, idx, targets)
+            except (RuntimeError, torch.OutOfMemoryError) as ex:
+                print(f"hylink: training steps are not replayed from a graph ({type(ex).__name__}: {ex})", flush=True)
+                self._use_graph = False
+        return self._graph is not None
+
     def close(self) -> None:
-        """Gives the process group its previous CTA budget back."""
+        """Gives the process group its previous CTA budget back, and the memory of the step graph."""
+        self._graph, self._graph_key = None, None
         if self._old_budget is not None:
             from .backend import set_cta_budget
 
@@ -88,10 +161,17 @@ class DDPTrainer:
             # DDP re-buckets its gradients once, before the second forward pass, in the order they became ready:
             # do that here, under the registered pool, so that the new buckets are registered too.
             with torch.cuda.use_mem_pool(self._pool):
-                if self.ddp.reducer._rebuild_buckets():
-                    self.ddp._has_rebuilt_buckets = True
+                if self._ddp.reducer._rebuild_buckets():
+                    self._ddp._has_rebuilt_buckets = True
         self._steps += 1
-        loss = self.ddp(idx, targets)
+        if self._ddp is not None:
+            loss = self._ddp(idx, targets)
+        elif self._replayable(idx, targets):
+            loss = self._graph.run(idx, targets)
+            self.opt.step()
+            return loss
+        else:
+            loss = self.model(idx.to(self.device), targets.to(self.device))
         self.opt.zero_grad(set_to_none=True)
         loss.backward()
         self.opt.step()

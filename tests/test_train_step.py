@@ -51,3 +51,49 @@ def test_out_of_range_target_gives_nan_and_large_logits_stay_finite():
     torch.testing.assert_close(ops().head_loss(h, w, t), want, rtol=1e-4, atol=1e-4)
     t[1] = 33
     assert bool(ops().head_loss(h, w, t).isnan())
+
+
+@pytest.mark.parametrize("name,batch,seq", [("tiny", 3, 64), ("gpt2-small", 2, 100)])
+def test_replayed_steps_train_like_eager_ones(name, batch, seq, monkeypatch):
+    """Forward and backward from a graph from the third step on, against the same steps run eagerly: with a learning rate
+    that changes, gradients that the caller drops, another batch shape in between, and a hook that has to be called."""
+    import torch.distributed as dist
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.parallel.trainer import DDPTrainer, init_distributed
+
+    fresh = not dist.is_initialized()
+    if fresh:
+        init_distributed("hylink")
+    cfg = GPT2Config.by_name(name)
+    torch.manual_seed(3)
+    first = GPT2(cfg)
+    g = torch.Generator().manual_seed(5)
+    tokens = [torch.randint(0, cfg.vocab_size, (batch, (seq if i != 6 else seq // 2) + 1), generator=g).pin_memory() for i in range(12)]
+
+    def train(replay):
+        monkeypatch.setenv("HYLINK_TRAIN_GRAPH", "1" if replay else "0")
+        model = copy.deepcopy(first)
+        t = DDPTrainer(model, torch.device("cuda", 0))
+        losses, replayed, seen = [], [], []
+        for i, tok in enumerate(tokens):
+            t.opt.param_groups[0]["lr"] = 1e-3 / (1 + i)
+            if i == 5:
+                t.opt.zero_grad(set_to_none=True)
+            if i == 10:
+                model.ln_f.register_forward_hook(lambda *a: seen.append(1))
+            losses.append(t.step(tok))
+            replayed.append(t._graph is not None)
+        assert len(seen) == 2
+        out = torch.cat([p.detach().float().reshape(-1) for p in model.parameters()]), [p.grad.float() for p in model.parameters()]
+        t.close()
+        return losses, replayed, out
+
+    losses, replayed, (weights, grads) = train(True)
+    want_losses, never, (want, want_grads) = train(False)
+    # steps 2 to 5 replay; a batch of another shape; two eager steps of the old one before it is recorded again; hooked
+    assert replayed == [False] * 2 + [True] * 4 + [False] * 3 + [True] + [False] * 2 and not any(never)
+    torch.testing.assert_close(torch.tensor(losses), torch.tensor(want_losses), rtol=5e-3, atol=0)
+    assert float((weights - want).norm() / want.norm()) < 1e-2
+    if fresh:
+        dist.destroy_process_group()
