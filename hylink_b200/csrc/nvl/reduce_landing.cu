@@ -24,13 +24,15 @@ namespace dev {
 
 constexpr int kRlThreads = 256;
 
-// Bound by memory. A thread folds one packet: it has the loads of all its operands in flight at once (the operand
+// Bound by memory. A thread folds U packets: it has the loads of all their operands in flight at once (the operand
 // count is compiled in, in classes), adds in a fixed order and stores. The grid covers the message; CTAs that retire
 // and start keep more loads in flight than a resident grid whose threads alternate between loading and storing
 // (4 x 32 MiB of bf16 into one on B200: 26.8 us = 6.3 TB/s against 28.7; before, with the sources in a run-time loop
-// four packets deep and the operator chosen per element, 38.9). A caller's own block count makes it loop.
+// four packets deep and the operator chosen per element, 38.9). With one or two operands a thread that folds a single
+// packet is gone before its CTA has cost less than it moved: U is four there, while the CTAs still fill the SMs (28 MB
+// copied: 16.3 us with one packet, 12.3 with four). A caller's own block count makes it loop.
 // kSum: the operator is known to be an addition; otherwise it is looked up per element.
-template <typename T, int MR, bool kSum>
+template <typename T, int MR, int U, bool kSum>
 __global__ void __launch_bounds__(kRlThreads) kReduceLanding(const __grid_constant__ nvl::ReduceLandingArgs a, const void* const first, int n) {
   constexpr int N = Packet<T>::N;
   using Acc = typename Wire<T>::Acc;
@@ -44,22 +46,28 @@ __global__ void __launch_bounds__(kRlThreads) kReduceLanding(const __grid_consta
     if (q < n) vec = vec && aligned16(operand(q));
   const uint64_t np = vec ? a.count / N : 0;  // whole packets handled by the vector loop
   T* dst = reinterpret_cast<T*>(a.dst);
-  for (uint64_t i = tid; i < np; i += nthreads) {
-    uint4 v[MR];
+  for (uint64_t i0 = (uint64_t)blockIdx.x * (kRlThreads * U) + threadIdx.x; i0 < np; i0 += nthreads * U) {
+    uint4 v[U][MR];
 #pragma unroll
-    for (int q = 0; q < MR; ++q)
-      if (q < n) v[q] = reinterpret_cast<const uint4*>(operand(q))[i];
-    Acc acc[N], b[N];
-    Packet<T>::unpack(v[0], acc);
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-    for (int q = 1; q < MR; ++q)
-      if (q < n) {
-        Packet<T>::unpack(v[q], b);
+      for (int q = 0; q < MR; ++q)
+        if (q < n && i0 + u * kRlThreads < np) v[u][q] = reinterpret_cast<const uint4*>(operand(q))[i0 + u * kRlThreads];
 #pragma unroll
-        for (int e = 0; e < N; ++e) acc[e] = kSum ? (Acc)(acc[e] + b[e]) : applyOp(a.op, acc[e], b[e]);
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * kRlThreads < np) {
+        Acc acc[N], b[N];
+        Packet<T>::unpack(v[u][0], acc);
+#pragma unroll
+        for (int q = 1; q < MR; ++q)
+          if (q < n) {
+            Packet<T>::unpack(v[u][q], b);
+#pragma unroll
+            for (int e = 0; e < N; ++e) acc[e] = kSum ? (Acc)(acc[e] + b[e]) : applyOp(a.op, acc[e], b[e]);
+          }
+        finish<T>(acc, a.scale, 0);
+        reinterpret_cast<uint4*>(dst)[i0 + u * kRlThreads] = Packet<T>::pack(acc);
       }
-    finish<T>(acc, a.scale, 0);
-    reinterpret_cast<uint4*>(dst)[i] = Packet<T>::pack(acc);
   }
   // ragged tail, or everything when some pointer is not 16-byte aligned
   for (uint64_t e = np * N + tid; e < a.count; e += nthreads) {
@@ -120,27 +128,29 @@ __global__ void kDoorbell(volatile uint64_t* ready, uint64_t ready_value, volati
 
 namespace nvl {
 
-// Operand classes: 2 (one source into an accumulator), 4, 9; operators other than the sum share the widest.
+// Operand classes: 2 (one source into an accumulator), 4, 9; operators other than the sum share the widest. `packets`
+// of a thread: 1, or what reduceLandingUnroll says.
+static int reduceLandingUnroll(int operands, bool sum) { return !sum || operands > 2 ? 1 : 4; }
 template <typename T>
-static const void* reduceLandingFor(int operands, bool sum) {
+static const void* reduceLandingFor(int operands, bool sum, int packets) {
   using namespace dev;
-  if (!sum) return (const void*)kReduceLanding<T, 9, false>;
-  if (operands <= 2) return (const void*)kReduceLanding<T, 2, true>;
-  if (operands <= 4) return (const void*)kReduceLanding<T, 4, true>;
-  return (const void*)kReduceLanding<T, 9, true>;
+  if (!sum) return (const void*)kReduceLanding<T, 9, 1, false>;
+  if (operands <= 2) return packets == 1 ? (const void*)kReduceLanding<T, 2, 1, true> : (const void*)kReduceLanding<T, 2, 4, true>;
+  if (operands <= 4) return (const void*)kReduceLanding<T, 4, 1, true>;
+  return (const void*)kReduceLanding<T, 9, 1, true>;
 }
-static const void* reduceLandingFn(int dt, int operands, bool sum) {
+static const void* reduceLandingFn(int dt, int operands, bool sum, int packets) {
   switch (dt) {
-    case hlInt8: return reduceLandingFor<int8_t>(operands, sum);
-    case hlUint8: return reduceLandingFor<uint8_t>(operands, sum);
-    case hlInt32: return reduceLandingFor<int32_t>(operands, sum);
-    case hlUint32: return reduceLandingFor<uint32_t>(operands, sum);
-    case hlInt64: return reduceLandingFor<long long>(operands, sum);
-    case hlUint64: return reduceLandingFor<unsigned long long>(operands, sum);
-    case hlFloat16: return reduceLandingFor<__half>(operands, sum);
-    case hlFloat32: return reduceLandingFor<float>(operands, sum);
-    case hlFloat64: return reduceLandingFor<double>(operands, sum);
-    case hlBfloat16: return reduceLandingFor<__nv_bfloat16>(operands, sum);
+    case hlInt8: return reduceLandingFor<int8_t>(operands, sum, packets);
+    case hlUint8: return reduceLandingFor<uint8_t>(operands, sum, packets);
+    case hlInt32: return reduceLandingFor<int32_t>(operands, sum, packets);
+    case hlUint32: return reduceLandingFor<uint32_t>(operands, sum, packets);
+    case hlInt64: return reduceLandingFor<long long>(operands, sum, packets);
+    case hlUint64: return reduceLandingFor<unsigned long long>(operands, sum, packets);
+    case hlFloat16: return reduceLandingFor<__half>(operands, sum, packets);
+    case hlFloat32: return reduceLandingFor<float>(operands, sum, packets);
+    case hlFloat64: return reduceLandingFor<double>(operands, sum, packets);
+    case hlBfloat16: return reduceLandingFor<__nv_bfloat16>(operands, sum, packets);
     default: return nullptr;
   }
 }
@@ -148,12 +158,15 @@ static const void* reduceLandingFn(int dt, int operands, bool sum) {
 hlResult_t launchReduceLanding(const ReduceLandingArgs& a, int blocks, cudaStream_t stream) {
   if (a.nsrc < 1 || a.nsrc > 8) return fail(hlInvalidArgument, "reduce landing: nsrc %d out of [1,8]", a.nsrc);
   int operands = a.nsrc + (a.accumulate ? 1 : 0);
-  const void* fn = reduceLandingFn(a.dtype, operands, a.op == hlSum || a.op == hlAvg);
+  const bool sum = a.op == hlSum || a.op == hlAvg;
+  const uint64_t packets = (a.count * hlTypeSize((hlDataType_t)a.dtype) + 15) / 16;
+  int unroll = reduceLandingUnroll(operands, sum);
+  if (packets < (uint64_t)148 * 8 * dev::kRlThreads * unroll) unroll = 1;   // fewer than eight CTAs per SM
+  const void* fn = reduceLandingFn(a.dtype, operands, sum, unroll);
   if (!fn) return fail(hlUnsupported, "reduce landing: unsupported dtype %d", a.dtype);
   if (a.count == 0) return hlSuccess;
-  const size_t es = hlTypeSize((hlDataType_t)a.dtype);
-  const uint64_t packets = (a.count * es + 15) / 16;
-  if (blocks <= 0) blocks = (int)std::min<uint64_t>((packets + dev::kRlThreads - 1) / dev::kRlThreads, 1u << 30);
+  const uint64_t per_block = (uint64_t)dev::kRlThreads * unroll;
+  if (blocks <= 0) blocks = (int)std::min<uint64_t>((packets + per_block - 1) / per_block, 1u << 30);
   const void* first = a.accumulate ? a.dst : a.src[0];
   void* args[3] = {(void*)&a, (void*)&first, (void*)&operands};
   cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(dev::kRlThreads), args, 0, stream);
@@ -178,11 +191,12 @@ hlResult_t launchCopy(void* dst, const void* src, size_t bytes, cudaStream_t str
 hlResult_t prepareReduceLanding() {
   for (int dt = 0; dt < hlNumTypes; ++dt)
     for (int operands : {2, 4, 9})
-      for (bool sum : {false, true}) {
-        cudaFuncAttributes at;
-        cudaError_t e = cudaFuncGetAttributes(&at, reduceLandingFn(dt, operands, sum));
-        if (e != cudaSuccess) return fail(hlDeviceError, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
-      }
+      for (bool sum : {false, true})
+        for (int packets : {1, reduceLandingUnroll(operands, sum)}) {
+          cudaFuncAttributes at;
+          cudaError_t e = cudaFuncGetAttributes(&at, reduceLandingFn(dt, operands, sum, packets));
+          if (e != cudaSuccess) return fail(hlDeviceError, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
+        }
   cudaFuncAttributes at;
   cudaFuncGetAttributes(&at, (const void*)dev::kCopyPackets<1>);
   cudaFuncGetAttributes(&at, (const void*)dev::kCopyPackets<4>);
