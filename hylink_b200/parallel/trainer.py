@@ -10,13 +10,14 @@ backend's own stream) / optimizer, and returns the loss as a Python float.
 A job of one rank has no gradient to reduce: the model is not wrapped then (the
 buckets would only cost a copy of every gradient), and models that can say when
 a step may be replayed (``step_signature``, as :class:`~hylink_b200.models.gpt2.GPT2`
-does) run forward and backward from a CUDA graph once a batch shape has come
-three times in a row. Issuing the thousand launches of a step takes the host
+does) run forward and backward from a CUDA graph from the second step of a
+batch shape on. Issuing the thousand launches of a step takes the host
 longer than the GPU needs for a small batch. The graph holds the memory of one
 step; ``HYLINK_TRAIN_GRAPH=0`` or :meth:`DDPTrainer.close` gives it back.
 """
 from __future__ import annotations
 
+import gc
 import os
 
 import torch
@@ -53,21 +54,38 @@ class _StepGraph:
         try:
             for p in params:
                 p.grad = None
-            self.graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self.graph):
-                loss = model(self.idx, self.targets)
-                loss.backward()
-                self.loss = loss.detach()
-            self.grads = [p.grad for p in params]
+            self._capture(model)
         except BaseException:
             for p, g in zip(params, old):
                 p.grad = g
             raise
 
+    def _capture(self, model: torch.nn.Module) -> None:
+        self.graph, self.replays = torch.cuda.CUDAGraph(), 0
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        collecting = gc.isenabled()
+        gc.disable()                      # whatever a collection would free must not be freed inside the capture
+        try:
+            with torch.cuda.stream(side):
+                # other threads may go on calling CUDA; the memory of earlier steps stays in the allocator's cache
+                self.graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    loss = model(self.idx, self.targets)
+                    loss.backward()
+                    self.loss = loss.detach()
+                finally:
+                    self.graph.capture_end()
+        finally:
+            if collecting:
+                gc.enable()
+        self.grads = [p.grad for p in self.params]
+
     def run(self, idx: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
         self.idx.copy_(idx)
         self.targets.copy_(targets)
         self.graph.replay()
+        self.replays += 1
         for p, g in zip(self.params, self.grads):
             if p.grad is not g:
                 p.grad = g
@@ -103,7 +121,7 @@ class DDPTrainer:
                 print(f"hylink: gradient buckets stay unregistered ({type(ex).__name__}: {ex})", flush=True)
         self._ddp = None
         self._bucket_cap_mb = bucket_cap_mb
-        self._graph, self._graph_key, self._key_seen = None, None, 0
+        self._graph, self._graph_key, self._key_seen, self._patience = None, None, 0, 2
         self._use_graph = os.environ.get("HYLINK_TRAIN_GRAPH", "1") != "0"
         if pool is not None:
             with torch.cuda.use_mem_pool(pool):
@@ -127,23 +145,26 @@ class DDPTrainer:
         return self._ddp
 
     def _replayable(self, idx: torch.Tensor, targets: torch.Tensor) -> bool:
-        """Whether this step runs from the graph; captures it when the same step has been run twice before."""
+        """Whether this step runs from the graph; captures it when the same step has been run before."""
         signature = getattr(self.model, "step_signature", None)
         if not self._use_graph or signature is None or not (idx.is_cuda and targets.is_cuda) or torch.is_anomaly_enabled():
             return False
         sig = signature(idx, targets)
         key = None if sig is None else (sig, idx.shape, idx.dtype, targets.shape, targets.dtype)
         if key != self._graph_key:
+            if self._graph is not None and self._graph.replays < 16:   # a capture costs a few steps: shapes that keep changing
+                self._patience = min(2 * self._patience, 1 << 20)      # have to prove themselves for longer and longer
             self._graph, self._graph_key, self._key_seen = None, key, 0
         if key is None:
             return False
         self._key_seen += 1
-        if self._graph is None and self._key_seen == 3:   # the two eager steps have loaded and sized everything
+        if self._graph is None and self._key_seen >= self._patience:   # an eager step has loaded and sized everything
             try:
                 self._graph = _StepGraph(self.model, self._params, idx, targets)
-            except (RuntimeError, torch.OutOfMemoryError) as ex:
+            except RuntimeError as ex:   # out of memory among them
                 print(f"hylink: training steps are not replayed from a graph ({type(ex).__name__}: {ex})", flush=True)
                 self._use_graph = False
+                torch.cuda.empty_cache()
         return self._graph is not None
 
     def close(self) -> None:
