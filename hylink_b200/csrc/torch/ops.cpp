@@ -213,9 +213,35 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
 // logits = h W^T and their mean cross entropy. The vocabulary is padded to a multiple of 64: an odd leading dimension
 // keeps cuBLAS off the tensor-memory kernels (8192 x 50257 x 1024 in bf16 on B200: 7.43 ms against 0.60 for the logits,
 // 4.71 against 0.55 for the weight gradient); padding the weight is a copy of 0.04 ms.
-// The input gradient sums over the vocabulary, unpadded (5.6 ms): padded it takes 0.55 ms, but there the products of
-// 50257 tiny probabilities and one large entry are added up with another rounding, the same way for every token, and
-// the gradients of a 24-layer model move by 1.4 % where run-to-run noise is 0.5 %.
+// The input gradient sums over the vocabulary. Given the odd size cuBLAS takes a kernel that cuts the sum into parts and
+// carries it from part to part in 16 bits, as long as torch allows reduced-precision reductions, which is its default.
+// That shows: behind a token's target entry the tiny probabilities of the rest are lost, the same way for every token.
+// The number of parts is 5 from 192 tiles of 256 x 128 on (6144 rows of 1024, 8192 of 768), and 6 to 24 in no simple
+// order below. From there on the parts are computed here as products over the padded size on the fast kernels, into
+// fp32, and the carried sum is kept as it was, so that a training run goes on as it would have: 99.6 % of the elements
+// are the same bits. (In one pass, or in another number of parts, the gradients of a 24-layer model move by 2 to 3 % in
+// the second step, where the noise between two runs is 0.6 %.) 8192 x 50257 x 1024: 5.6 ms -> 0.7.
+// With reduced-precision reductions switched off the sum is one pass in fp32.
+constexpr int64_t kHeadParts = 5, kHeadPartTiles = 192;
+bool reducedPrecisionSums(at::ScalarType t) {
+  const auto& ctx = at::globalContext();
+  return (t == at::kBFloat16 ? ctx.allowBF16ReductionCuBLAS() : ctx.allowFP16ReductionCuBLAS()) == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK;
+}
+// d [rows][padded], zero behind `vocab`; w [padded][width].
+Tensor headInputGradient(const Tensor& d, const Tensor& w, int64_t vocab) {
+  const int64_t padded = d.size(1), tiles = (d.size(0) + 255) / 256 * ((w.size(1) + 127) / 128);
+  if (vocab % 8 == 0 || !reducedPrecisionSums(d.scalar_type())) return at::mm(d, w);
+  if (tiles < kHeadPartTiles) return at::mm(d.narrow(1, 0, vocab), w.narrow(0, 0, vocab));
+  const int64_t part = ((vocab + kHeadParts - 1) / kHeadParts + 7) / 8 * 8;
+  Tensor out = at::mm(d.narrow(1, 0, std::min(part, padded)), w.narrow(0, 0, std::min(part, padded)));
+  for (int64_t at = part; at < vocab; at += part) {
+    const int64_t k = std::min(part, padded - at);
+    const Tensor sum = at::mm(d.narrow(1, at, k), w.narrow(0, at, k), at::kFloat);
+    ok(train::carrySum(code(out), sum.data_ptr<float>(), out.data_ptr(), out.numel(), streamOf(out)), "head gradient");
+  }
+  return out;
+}
+
 class HeadLoss : public torch::autograd::Function<HeadLoss> {
  public:
   static Variable forward(AutogradContext* ctx, const Variable& h_, const Variable& w, const Variable& targets_) {
@@ -233,24 +259,24 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
     ok(train::crossEntropyForward(code(h), logits.data_ptr(), padded, targets.data_ptr<int64_t>(), rows, (int)vocab, -100, lse.data_ptr<float>(),
                                   row_loss.data_ptr<float>(), loss.data_ptr<float>(), streamOf(h)),
        "cross entropy");
-    ctx->save_for_backward({h, w, targets, logits, lse, loss});
+    ctx->save_for_backward({h, wpad, targets, logits, lse, loss});
+    ctx->saved_data["vocab"] = vocab;
     ctx->saved_data["h"] = h_.sizes().vec();
     return loss.select(0, 0).clone();
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &h = s[0], &w = s[1], &targets = s[2], &logits = s[3], &lse = s[4], &loss = s[5];
+    const Tensor &h = s[0], &wpad = s[1], &targets = s[2], &logits = s[3], &lse = s[4], &loss = s[5];
     c10::cuda::CUDAGuard dg(h.device());
-    const int64_t vocab = w.size(0);
+    const int64_t vocab = ctx->saved_data["vocab"].toInt();
     const Tensor grad = g[0].to(at::kFloat).contiguous();
     Tensor dlogits = at::empty_like(logits);
     ok(train::crossEntropyBackward(code(h), logits.data_ptr(), logits.size(1), targets.data_ptr<int64_t>(), h.size(0), (int)vocab, -100,
                                    lse.data_ptr<float>(), loss.data_ptr<float>(), grad.data_ptr<float>(), dlogits.data_ptr(), streamOf(h)),
        "cross entropy backward");
-    const Tensor d = dlogits.narrow(1, 0, vocab);
-    Tensor dw = at::mm(d.t(), h);
-    Tensor dh = at::mm(d, w).view(ctx->saved_data["h"].toIntVector());
+    Tensor dw = at::mm(dlogits.narrow(1, 0, vocab).t(), h);
+    Tensor dh = headInputGradient(dlogits, wpad, vocab).view(ctx->saved_data["h"].toIntVector());
     return {dh, dw, Tensor()};
   }
 };
