@@ -72,13 +72,13 @@ Normed normForward(const Tensor& x, const Tensor& y, const Tensor& gamma, const 
 }
 // Returns dx; `partials` becomes [3][parts][width].
 Tensor normBackward(const Tensor& dh, const Tensor& x, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, const Tensor& residual,
-                    Tensor* partials, int* parts) {
+                    bool dx_sums, Tensor* partials, int* parts) {
   const int64_t width = x.size(-1), rows = x.numel() / width;
   *parts = train::layerNormPartials(rows);
   *partials = floats(x, {3, *parts, width});
   Tensor dx = at::empty_like(x);
   ok(train::layerNormBackward(code(x), dh.data_ptr(), x.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr(),
-                              residual.defined() ? residual.data_ptr() : nullptr, dx.data_ptr(), partials->data_ptr<float>(), rows, (int)width,
+                              residual.defined() ? residual.data_ptr() : nullptr, dx.data_ptr(), dx_sums, partials->data_ptr<float>(), rows, (int)width,
                               streamOf(x)),
      "layer norm backward");
   return dx;
@@ -101,7 +101,7 @@ class AddNorm : public torch::autograd::Function<AddNorm> {
     Tensor parts;
     int np;
     const int64_t w = s[0].size(-1);
-    Tensor dx = normBackward(dense(g[0]), s[0], s[1], s[2], s[3], Tensor(), &parts, &np);
+    Tensor dx = normBackward(dense(g[0]), s[0], s[1], s[2], s[3], Tensor(), false, &parts, &np);
     Columns cols(s[3]);
     const float* p = parts.data_ptr<float>();
     Tensor dgamma = cols.add(p, np, w), dbeta = cols.add(p + np * w, np, w);
@@ -148,7 +148,7 @@ class BlockPre : public torch::autograd::Function<BlockPre> {
     Tensor dh = at::mm(dqkv, w);
     Tensor parts;
     int np;
-    Tensor dx = normBackward(dh, x, s[1], s[2], gamma, g[0].defined() ? dense(g[0]) : Tensor(), &parts, &np);
+    Tensor dx = normBackward(dh, x, s[1], s[2], gamma, dense(g[0]), false, &parts, &np);
     Columns cols(gamma);
     const float* p = parts.data_ptr<float>();
     Tensor dgamma = cols.add(p, np, width), dbeta = cols.add(p + np * width, np, width);
@@ -197,7 +197,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     Tensor dh = at::mm(du, wf);
     Tensor parts;
     int np;
-    Tensor dx = normBackward(dh, x2, s[3], s[4], gamma, g[0].defined() ? dense(g[0]) : Tensor(), &parts, &np);
+    Tensor dx = normBackward(dh, x2, s[3], s[4], gamma, dense(g[0]), true, &parts, &np);
     const Tensor dxr = dx.view({rows, width});
     Tensor dwp = at::mm(dxr.t(), a);
     Tensor da = at::mm(dxr, wp).view(ctx->saved_data["a"].toIntVector());

@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(256) kFinishColumns(const __grid_constant__ Se
   if (blockIdx.x * 32 >= g.width) return;
   float t = 0.f;
   if (col < g.width)
+#pragma unroll 8
     for (int r = warp; r < g.rows; r += 8) t += g.src[(int64_t)r * g.width + col];
   s_sum[warp][lane] = t;
   __syncthreads();

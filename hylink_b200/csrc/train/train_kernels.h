@@ -20,10 +20,10 @@ struct ColSegment {
 constexpr int kMaxColSegments = 8;
 
 // dx = residual + gradient of the layer norm at x for the output gradient dh (residual may be null).
-// partials: [3][layerNormPartials(rows)][width]: dgamma, dbeta, and the column sums of dx as stored.
+// partials: [3][layerNormPartials(rows)][width]: dgamma, dbeta, and (dx_sums) the column sums of dx as stored.
 int layerNormPartials(int64_t rows);
 hlResult_t layerNormBackward(int dt, const void* dh, const void* x, const float* mean, const float* rstd, const void* gamma,
-                             const void* residual, void* dx, float* partials, int64_t rows, int width, cudaStream_t s);
+                             const void* residual, void* dx, bool dx_sums, float* partials, int64_t rows, int width, cudaStream_t s);
 
 // out = gelu(u), tanh form.
 hlResult_t geluForward(int dt, const void* u, void* out, int64_t count, cudaStream_t s);
