@@ -281,44 +281,126 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
   }
 };
 
-// Routing and dispatch of a top-1 mixture of experts. Returns x again (the residual path: its gradient then joins the
-// others in one pass), the dispatch buffer, the gates, and the maps token -> row and row -> token.
+// ---- top-1 mixture of experts
+struct Routed {
+  Tensor logits, expert, gate, row_of, token_of, send;
+};
+Routed moeRouted(const Tensor& x, const Tensor& router, int64_t capacity) {
+  const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
+  const auto ints = x.options().dtype(at::kInt);
+  Routed r;
+  r.logits = at::mm(x, router.t());
+  r.expert = at::empty({tokens}, ints);
+  r.row_of = at::empty({tokens}, ints);
+  r.token_of = at::empty({experts * capacity}, ints);
+  r.gate = floats(x, {tokens});
+  r.send = at::empty({experts * capacity, width}, x.options());
+  ok(train::moeRoute(code(x), r.logits.data_ptr(), (int)tokens, (int)experts, (int)capacity, r.expert.data_ptr<int>(), r.gate.data_ptr<float>(),
+                     r.row_of.data_ptr<int>(), r.token_of.data_ptr<int>(), streamOf(x)),
+     "MoE routing");
+  ok(train::moeGather(x.data_ptr(), r.token_of.data_ptr<int>(), r.send.data_ptr(), (int)(experts * capacity), (int)width, streamOf(x)), "MoE dispatch");
+  return r;
+}
+// {dx, drouter}; dres may be undefined.
+std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& router, const Tensor& logits, const Tensor& expert, const Tensor& gate,
+                                            const Tensor& row_of, const Tensor& dres, const Tensor& dsend, const Tensor& dgate) {
+  const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
+  Tensor dx = at::empty_like(x), dlogits = at::empty_like(logits);
+  ok(train::moeTokenGradient(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
+                             expert.data_ptr<int>(), gate.data_ptr<float>(), dgate.data_ptr<float>(), router.data_ptr(), dx.data_ptr(),
+                             dlogits.data_ptr(), (int)tokens, (int)width, (int)experts, streamOf(x)),
+     "MoE token gradient");
+  if (!train::moeRouterFits((int)experts)) dx.addmm_(dlogits, router);
+  return {dx, at::mm(dlogits.t(), x)};
+}
+struct Expert {
+  Tensor u, act, out;
+};
+Expert moeExpert(const Tensor& h, const Tensor& w1, const Tensor& w2) {
+  Expert e;
+  e.u = at::bmm(h, w1);
+  e.act = at::empty_like(e.u);
+  ok(train::geluForward(code(e.u), e.u.data_ptr(), e.act.data_ptr(), e.u.numel(), streamOf(e.u)), "gelu");
+  e.out = at::bmm(e.act, w2);
+  return e;
+}
+// {dh, dw1, dw2}
+variable_list moeExpertBackward(const Tensor& h, const Tensor& w1, const Tensor& w2, const Tensor& u, const Tensor& act, const Tensor& dout) {
+  Tensor dact = at::bmm(dout, w2.transpose(1, 2));
+  Tensor dw2 = at::bmm(act.transpose(1, 2), dout);
+  Tensor du = at::empty_like(u);
+  ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
+     "gelu backward");
+  Tensor dw1 = at::bmm(h.transpose(1, 2), du);
+  return {at::bmm(du, w1.transpose(1, 2)), dw1, dw2};
+}
+Tensor moeCombined(const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of) {
+  Tensor y = at::empty_like(x);
+  ok(train::moeCombine(code(x), x.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), row_of.data_ptr<int>(), y.data_ptr(), (int)x.size(0),
+                       (int)x.size(1), streamOf(x)),
+     "MoE combine");
+  return y;
+}
+// {drows, dgate}; dgate: only tokens with a row are written, and read
+std::pair<Tensor, Tensor> moeCombinedBackward(const Tensor& dy, const Tensor& gate, const Tensor& rows, const Tensor& token_of) {
+  Tensor drows = at::empty_like(rows), dgate = at::empty_like(gate);
+  const int width = (int)rows.size(-1);
+  ok(train::moeRowGradient(code(rows), dy.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), token_of.data_ptr<int>(), drows.data_ptr(),
+                           dgate.data_ptr<float>(), (int)(rows.numel() / width), width, streamOf(rows)),
+     "MoE row gradient");
+  return {drows, dgate};
+}
+
+// The whole layer where the experts are all here: one node instead of a dozen. (Host time of a layer of 1072 tokens,
+// forward and backward: 300 us in pieces, 210 in one.)
+class MoeLayer : public torch::autograd::Function<MoeLayer> {
+ public:
+  static Variable forward(AutogradContext* ctx, const Variable& x_, const Variable& router, const Variable& w1, const Variable& w2, int64_t capacity) {
+    c10::cuda::CUDAGuard dg(x_.device());
+    const Tensor x = dense(x_);
+    const Routed r = moeRouted(x, router, capacity);
+    const Tensor h = r.send.view({router.size(0), capacity, x.size(1)});
+    const Expert e = moeExpert(h, w1, w2);
+    ctx->save_for_backward({x, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out});
+    return moeCombined(x, r.gate, e.out, r.row_of);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    onceOnly();
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &router = s[1], &w1 = s[2], &w2 = s[3], &h = s[9], &rows = s[12];
+    c10::cuda::CUDAGuard dg(x.device());
+    const Tensor dy = dense(g[0]);
+    const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8]);
+    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows);
+    const auto [dx, drouter] = moeRoutedBackward(x, router, s[4], s[5], s[6], s[7], dy, e[0], dgate);
+    return {dx, drouter, e[1], e[2], Tensor()};
+  }
+};
+
+// In pieces, with the tokens travelling between ranks in between. Dispatch returns x again (the residual path: its
+// gradient then joins the others in one pass), the dispatch buffer, the gates, and the maps token -> row and row -> token.
 class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
  public:
   static variable_list forward(AutogradContext* ctx, const Variable& x_, const Variable& router, int64_t capacity) {
     c10::cuda::CUDAGuard dg(x_.device());
     const Tensor x = dense(x_);
-    const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
-    const auto ints = x.options().dtype(at::kInt);
-    const Tensor logits = at::mm(x, router.t());
-    Tensor expert = at::empty({tokens}, ints), row_of = at::empty({tokens}, ints), token_of = at::empty({experts * capacity}, ints);
-    Tensor gate = floats(x, {tokens}), send = at::empty({experts * capacity, width}, x.options());
-    ok(train::moeRoute(code(x), logits.data_ptr(), (int)tokens, (int)experts, (int)capacity, expert.data_ptr<int>(), gate.data_ptr<float>(),
-                       row_of.data_ptr<int>(), token_of.data_ptr<int>(), streamOf(x)),
-       "MoE routing");
-    ok(train::moeGather(x.data_ptr(), token_of.data_ptr<int>(), send.data_ptr(), (int)(experts * capacity), (int)width, streamOf(x)), "MoE dispatch");
-    ctx->save_for_backward({x, router, logits, gate, row_of});
-    ctx->saved_data["rows"] = experts * capacity;
-    ctx->mark_non_differentiable({row_of, token_of});
+    const Routed r = moeRouted(x, router, capacity);
+    ctx->save_for_backward({x, router, r.logits, r.expert, r.gate, r.row_of});
+    ctx->saved_data["rows"] = router.size(0) * capacity;
+    ctx->mark_non_differentiable({r.row_of, r.token_of});
     ctx->set_materialize_grads(false);
-    return {x, send, gate, row_of, token_of};
+    return {x, r.send, r.gate, r.row_of, r.token_of};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &x = s[0], &router = s[1], &logits = s[2], &gate = s[3], &row_of = s[4];
+    const Tensor &x = s[0], &gate = s[4];
     c10::cuda::CUDAGuard dg(x.device());
-    const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
     const Tensor dres = g[0].defined() ? dense(g[0]) : Tensor();
-    const Tensor dsend = g[1].defined() ? dense(g[1]) : at::zeros({ctx->saved_data["rows"].toInt(), width}, x.options());
+    const Tensor dsend = g[1].defined() ? dense(g[1]) : at::zeros({ctx->saved_data["rows"].toInt(), x.size(1)}, x.options());
     const Tensor dgate = g[2].defined() ? dense(g[2]) : at::zeros_like(gate);
-    Tensor dx = at::empty_like(x), dlogits = at::empty_like(logits);
-    ok(train::moeTokenGradient(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
-                               gate.data_ptr<float>(), dgate.data_ptr<float>(), router.data_ptr(), dx.data_ptr(), dlogits.data_ptr(), (int)tokens,
-                               (int)width, (int)experts, streamOf(x)),
-       "MoE token gradient");
-    if (!train::moeRouterFits((int)experts, (int)width)) dx.addmm_(dlogits, router);
-    return {dx, at::mm(dlogits.t(), x), Tensor()};
+    const auto [dx, drouter] = moeRoutedBackward(x, s[1], s[2], s[3], gate, s[5], dres, dsend, dgate);
+    return {dx, drouter, Tensor()};
   }
 };
 
@@ -327,26 +409,15 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
  public:
   static Variable forward(AutogradContext* ctx, const Variable& h, const Variable& w1, const Variable& w2) {
     c10::cuda::CUDAGuard dg(h.device());
-    const Tensor u = at::bmm(h, w1);
-    Tensor act = at::empty_like(u);
-    ok(train::geluForward(code(u), u.data_ptr(), act.data_ptr(), u.numel(), streamOf(u)), "gelu");
-    ctx->save_for_backward({h, w1, w2, u, act});
-    return at::bmm(act, w2);
+    const Expert e = moeExpert(h, w1, w2);
+    ctx->save_for_backward({h, w1, w2, e.u, e.act});
+    return e.out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &h = s[0], &w1 = s[1], &w2 = s[2], &u = s[3], &act = s[4];
-    c10::cuda::CUDAGuard dg(h.device());
-    const Tensor dout = dense(g[0]);
-    Tensor dact = at::bmm(dout, w2.transpose(1, 2));
-    Tensor dw2 = at::bmm(act.transpose(1, 2), dout);
-    Tensor du = at::empty_like(u);
-    ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
-       "gelu backward");
-    Tensor dw1 = at::bmm(h.transpose(1, 2), du);
-    Tensor dh = at::bmm(du, w1.transpose(1, 2));
-    return {dh, dw1, dw2};
+    c10::cuda::CUDAGuard dg(s[0].device());
+    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]));
   }
 };
 
@@ -357,23 +428,15 @@ class MoeCombine : public torch::autograd::Function<MoeCombine> {
                           const Variable& token_of) {
     c10::cuda::CUDAGuard dg(x.device());
     const Tensor rows = dense(rows_);
-    Tensor y = at::empty_like(x);
-    ok(train::moeCombine(code(x), x.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), row_of.data_ptr<int>(), y.data_ptr(), (int)x.size(0),
-                         (int)x.size(1), streamOf(x)),
-       "MoE combine");
     ctx->save_for_backward({gate, rows, token_of});
-    return y;
+    return moeCombined(x, gate, rows, row_of);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &gate = s[0], &rows = s[1], &token_of = s[2];
-    c10::cuda::CUDAGuard dg(rows.device());
+    c10::cuda::CUDAGuard dg(s[1].device());
     const Tensor dy = dense(g[0]);
-    Tensor drows = at::empty_like(rows), dgate = at::empty_like(gate);   // dgate: only tokens with a row are written, and read
-    ok(train::moeRowGradient(code(rows), dy.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), token_of.data_ptr<int>(), drows.data_ptr(),
-                             dgate.data_ptr<float>(), (int)rows.size(0), (int)rows.size(1), streamOf(rows)),
-       "MoE row gradient");
+    const auto [drows, dgate] = moeCombinedBackward(dy, s[0], s[1], s[2]);
     return {dy, dgate, drows, Tensor(), Tensor()};
   }
 };
@@ -464,3 +527,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("reduce_landing", &reduceLanding);
   m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });
 }
+  m.def("moe_layer", [](const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w2, int64_t capacity) {
+    return MoeLayer::apply(x, router, w1, w2, capacity);
+  });

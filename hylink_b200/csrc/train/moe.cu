@@ -7,7 +7,7 @@
 // moeGather      rows of the dispatch buffer from the tokens
 // moeCombine     y = x + gate * row
 // moeRowGradient d row = gate * dy; d gate = <dy, row>
-// moeTokenGradient  dx = dy + d row + d logits * router; d logits of the gate's softmax
+// moeTokenGradient  d logits of the gate's softmax; dx = dy + d row + d logits * router
 // All of them are bound by memory (16-byte packets, a warp or more per row). As tensor operations the same layer took
 // a one-hot matrix, a scan of it along the tokens in 64-bit integers (1.7 ms for 8192 tokens), sorted index updates
 // and eleven host round trips for the sizes of boolean selections.
@@ -176,72 +176,69 @@ __global__ void __launch_bounds__(256) kMoeRowGradient(const T* __restrict__ dy,
   if (lane == 0) dgate[t] = dot;
 }
 
-// A CTA covers all columns (a thread eight of them) and walks tokens. The router's rows lie in shared memory (in
-// registers they cost the occupancy that hides the chain row -> packet: 31 us instead of 25 for 8192 x 1024, eight
-// experts). E bounds the experts this variant is compiled for; with kRouter false the router's share is left to a GEMM.
-template <typename T, int E, bool kRouter>
-__global__ void __launch_bounds__(256) kMoeTokenGradient(const T* __restrict__ dy, const T* __restrict__ drows, const int* __restrict__ row_of,
-                                                         const T* __restrict__ logits, const float* __restrict__ gate,
-                                                         const float* __restrict__ dgate, const T* __restrict__ router, T* __restrict__ dx,
-                                                         T* __restrict__ dlogits, int tokens, int width, int experts) {
-  extern __shared__ uint4 s_router[];          // [experts][width / 8]
-  const int cols = width / 8;                  // threads of one token
-  const int per = blockDim.x / cols;           // tokens side by side
-  const int sub = threadIdx.x / cols, col = threadIdx.x - sub * cols, c = col * 8;
-  if (kRouter) {
-    for (int i = threadIdx.x; i < experts * cols; i += blockDim.x) s_router[i] = reinterpret_cast<const uint4*>(router)[i];
-    __syncthreads();
+// A thread per token. gate = p_top: d logit_e = d gate * p_top * ([e is top] - p_e), with p_e = exp(l_e - l_top) * p_top.
+// No gradient for a token whose gate was not used.
+template <typename T>
+__global__ void __launch_bounds__(128) kMoeLogitGradient(const int* __restrict__ row_of, const T* __restrict__ logits, const int* __restrict__ expert,
+                                                         const float* __restrict__ gate, const float* __restrict__ dgate, T* __restrict__ dlogits,
+                                                         int tokens, int experts) {
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t >= tokens) return;
+  const T* l = logits + (int64_t)t * experts;
+  const int at = expert[t];
+  const float g = gate[t], dg = row_of[t] >= 0 ? dgate[t] * g : 0.f, top = (float)l[at];
+  for (int e = 0; e < experts; ++e) dlogits[(int64_t)t * experts + e] = (T)(dg * ((e == at ? 1.f : 0.f) - __expf((float)l[e] - top) * g));
+}
+
+// dx = dy + d row + d logits * router. A warp takes two tokens, whose gradients of the logits it holds in registers (E
+// bounds the experts), so that a packet of the router is loaded once for both. 8192 x 1024, eight experts: 21.6 us, plus
+// 3.1 for the logits' gradients above; with four tokens 21.5, with one kernel that walked tokens with the router in
+// shared memory 25, and that one was limited to rows of 2048. E = 0: the router's share is left to a GEMM.
+constexpr int kTokensPerWarp = 2;
+template <typename T, int E>
+__global__ void __launch_bounds__(256, 4) kMoeTokenGradient(const T* __restrict__ dy, const T* __restrict__ drows, const int* __restrict__ row_of,
+                                                            const T* __restrict__ router, const T* __restrict__ dlogits, T* __restrict__ dx,
+                                                            int tokens, int width, int experts) {
+  constexpr int K = kTokensPerWarp;
+  const int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * K, lane = threadIdx.x & 31;
+  if (t0 >= tokens) return;
+  int row[K];
+  T dl[K][E > 0 ? E : 1];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    row[k] = t0 + k < tokens ? row_of[t0 + k] : -1;
+#pragma unroll
+    for (int e = 0; e < E; ++e) dl[k][e] = e < experts && t0 + k < tokens ? dlogits[(int64_t)(t0 + k) * experts + e] : (T)0.f;
   }
-  if (sub >= per) return;
-  for (int t = blockIdx.x * per + sub; t < tokens; t += gridDim.x * per) {
-    const int row = row_of[t];
-    const uint4 a = dy ? *reinterpret_cast<const uint4*>(dy + (int64_t)t * width + c) : make_uint4(0u, 0u, 0u, 0u);
-    float f[8];
-    unpack8<T>(a, f);
-    if (row >= 0) {
+  for (int c = lane * 8; c < width; c += 256) {
+    uint4 a[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      a[k] = dy && t0 + k < tokens ? *reinterpret_cast<const uint4*>(dy + (int64_t)(t0 + k) * width + c) : make_uint4(0u, 0u, 0u, 0u);
+      b[k] = row[k] >= 0 ? *reinterpret_cast<const uint4*>(drows + (int64_t)row[k] * width + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float f[K][8];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
       float h[8];
-      unpack8<T>(*reinterpret_cast<const uint4*>(drows + (int64_t)row * width + c), h);
+      unpack8<T>(a[k], f[k]);
+      unpack8<T>(b[k], h);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] += h[i];
+      for (int i = 0; i < 8; ++i) f[k][i] += h[i];
     }
-    // gate = p_top: d logit_e = d gate * p_top * ([e is top] - p_e), with p_e = exp(l_e - l_top) * p_top. No gradient
-    // for a token whose gate was not used.
-    const T* l = logits + (int64_t)t * experts;
-    const float g = gate[t], dg = row >= 0 ? dgate[t] * g : 0.f;
-    if (kRouter) {
-      float lv[E], top = -INFINITY;
-      int at = 0;
 #pragma unroll
-      for (int e = 0; e < E; ++e)
-        if (e < experts) {
-          lv[e] = (float)l[e];
-          if (lv[e] > top || e == 0) {
-            top = lv[e];
-            at = e;
-          }
-        }
+    for (int e = 0; e < E; ++e)
+      if (e < experts) {
+        float w[8];
+        unpack8<T>(__ldg(reinterpret_cast<const uint4*>(router + (int64_t)e * width + c)), w);
 #pragma unroll
-      for (int e = 0; e < E; ++e)
-        if (e < experts) {
-          const T d = (T)(dg * ((e == at ? 1.f : 0.f) - __expf(lv[e] - top) * g));
-          if (c == 0) dlogits[(int64_t)t * experts + e] = d;
-          float w[8];
-          unpack8<T>(s_router[e * cols + col], w);
+        for (int k = 0; k < K; ++k)
 #pragma unroll
-          for (int i = 0; i < 8; ++i) f[i] += (float)d * w[i];
-        }
-    } else if (c == 0) {
-      float top = (float)l[0];
-      int at = 0;
-      for (int e = 1; e < experts; ++e)
-        if ((float)l[e] > top) {
-          top = (float)l[e];
-          at = e;
-        }
-      for (int e = 0; e < experts; ++e)
-        dlogits[(int64_t)t * experts + e] = (T)(dg * ((e == at ? 1.f : 0.f) - __expf((float)l[e] - top) * g));
-    }
-    *reinterpret_cast<uint4*>(dx + (int64_t)t * width + c) = pack8<T>(f);
+          for (int i = 0; i < 8; ++i) f[k][i] += (float)dl[k][e] * w[i];
+      }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (t0 + k < tokens) *reinterpret_cast<uint4*>(dx + (int64_t)(t0 + k) * width + c) = pack8<T>(f[k]);
   }
 }
 
@@ -279,24 +276,21 @@ hlResult_t moeRowGradient(int dt, const void* dy, const float* gate, const void*
   return launched("MoE row gradient");
 }
 
-bool moeRouterFits(int experts, int width) { return experts <= 16 && (size_t)experts * width * 2 <= (48u << 10); }
+bool moeRouterFits(int experts) { return experts <= 16; }
 
-hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const float* gate, const float* dgate,
-                            const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s) {
-  if (width % 8 || width > 2048) return fail(hlInvalidArgument, "MoE gradient: width %d", width);
+hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const int* expert, const float* gate,
+                            const float* dgate, const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s) {
+  if (width % 8) return fail(hlInvalidArgument, "MoE gradient: width %d", width);
   if (tokens == 0) return hlSuccess;
-  const int per = 256 / (width / 8), groups = (tokens + per - 1) / per;
-  const unsigned blocks = (unsigned)(groups < 148 * 6 ? groups : 148 * 6);
-  const bool fits = moeRouterFits(experts, width);
-  const size_t smem = fits ? (size_t)experts * width * 2 : 0;
   HL_HALF_SWITCH(dt, T, {
+    kMoeLogitGradient<T><<<(tokens + 127) / 128, 128, 0, s>>>(row_of, (const T*)logits, expert, gate, dgate, (T*)dlogits, tokens, experts);
     auto go = [&](auto kern) {
-      kern<<<blocks, 256, smem, s>>>((const T*)dy, (const T*)drows, row_of, (const T*)logits, gate, dgate, (const T*)router, (T*)dx, (T*)dlogits, tokens,
-                                     width, experts);
+      constexpr int per = 8 * kTokensPerWarp;
+      kern<<<(tokens + per - 1) / per, 256, 0, s>>>((const T*)dy, (const T*)drows, row_of, (const T*)router, (const T*)dlogits, (T*)dx, tokens, width, experts);
     };
-    if (!fits) go(kMoeTokenGradient<T, 1, false>);
-    else if (experts <= 8) go(kMoeTokenGradient<T, 8, true>);
-    else go(kMoeTokenGradient<T, 16, true>);
+    if (!moeRouterFits(experts)) go(kMoeTokenGradient<T, 0>);
+    else if (experts <= 8) go(kMoeTokenGradient<T, 8>);
+    else go(kMoeTokenGradient<T, 16>);
   });
   return launched("MoE token gradient");
 }

@@ -72,9 +72,9 @@ hlResult_t moeCombine(int dt, const void* x, const float* gate, const void* rows
 hlResult_t moeRowGradient(int dt, const void* dy, const float* gate, const void* rows, const int* token_of, void* drows, float* dgate, int n_rows,
                           int width, cudaStream_t s);
 // Whether moeTokenGradient adds the router's share to dx itself (else the caller adds dlogits * router). dy may be null.
-bool moeRouterFits(int experts, int width);
-hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const float* gate, const float* dgate,
-                            const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s);
+bool moeRouterFits(int experts);
+hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const int* expert, const float* gate,
+                            const float* dgate, const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s);
 
 }  // namespace train
 }  // namespace hl
