@@ -441,6 +441,34 @@ class MoeCombine : public torch::autograd::Function<MoeCombine> {
   }
 };
 
+// One AdamW step on lists of tensors. False (and nothing done) unless all are contiguous CUDA tensors of one type that
+// the kernel takes.
+bool multiAdamW(const std::vector<Tensor>& weights, const std::vector<Tensor>& grads, const std::vector<Tensor>& ms, const std::vector<Tensor>& vs,
+                const std::vector<Tensor>& steps, double lr, double beta1, double beta2, double decay, double eps) {
+  const size_t n = weights.size();
+  if (n == 0 || grads.size() != n || ms.size() != n || vs.size() != n || steps.size() != n) return false;
+  const auto type = weights[0].scalar_type();
+  if (type != at::kBFloat16 && type != at::kHalf && type != at::kFloat) return false;
+  const c10::Device device = weights[0].device();
+  std::vector<train::AdamWTensor> list(n);
+  for (size_t i = 0; i < n; ++i) {
+    for (const Tensor* t : {&weights[i], &grads[i], &ms[i], &vs[i]})
+      if (t->device() != device || !device.is_cuda() || t->scalar_type() != type || t->layout() != at::kStrided || !t->is_contiguous() ||
+          t->numel() != weights[i].numel())
+        return false;
+    if (steps[i].device() != device || steps[i].scalar_type() != at::kFloat || steps[i].numel() != 1) return false;
+    list[i] = {weights[i].data_ptr(), ms[i].data_ptr(), vs[i].data_ptr(), grads[i].data_ptr(), steps[i].data_ptr<float>(), weights[i].numel()};
+  }
+  c10::cuda::CUDAGuard dg(device);
+  at::_foreach_add_(steps, 1);
+  ok(train::multiAdamW(type == at::kFloat ? (int)hlFloat32 : code(weights[0]), list.data(), (int)n, lr, beta1, beta2, decay, eps,
+                       streamOf(weights[0])),
+     "AdamW");
+  for (size_t i = 0; i < n; ++i)   // autograd has to know that these were written
+    for (const Tensor* t : {&weights[i], &ms[i], &vs[i]}) t->unsafeGetTensorImpl()->bump_version();
+  return true;
+}
+
 void shardedAdamW(const Tensor& grad, const Tensor& weight, const std::optional<Tensor>& master, const Tensor& m, const Tensor& v, int64_t ranks,
                   double keep, double beta1, double beta2, double step, double correction2, double eps) {
   c10::cuda::CUDAGuard dg(weight.device());
@@ -513,6 +541,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                          const Tensor& wf, const Tensor& bf, const Tensor& wo, const Tensor& bo, double eps) {
     return BlockPost::apply(x, a, wp, bp, gamma, beta, wf, bf, wo, bo, eps);
   });
+  m.def("moe_layer", [](const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w2, int64_t capacity) {
+    return MoeLayer::apply(x, router, w1, w2, capacity);
+  });
+  m.def("multi_adamw", &multiAdamW);
   m.def("moe_dispatch", [](const Tensor& x, const Tensor& router, int64_t capacity) { return MoeDispatch::apply(x, router, capacity); });
   m.def("moe_experts", [](const Tensor& h, const Tensor& w1, const Tensor& w2) { return MoeExperts::apply(h, w1, w2); });
   m.def("moe_combine", [](const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of, const Tensor& token_of) {
@@ -527,6 +559,3 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("reduce_landing", &reduceLanding);
   m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });
 }
-  m.def("moe_layer", [](const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w2, int64_t capacity) {
-    return MoeLayer::apply(x, router, w1, w2, capacity);
-  });

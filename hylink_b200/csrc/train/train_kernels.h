@@ -64,6 +64,17 @@ struct AdamWArgs {
 hlResult_t shardedAdamW(int dt, const void* grad, void* weight, float* master, float* m, float* v, int64_t count, const AdamWArgs& a,
                         cudaStream_t s);
 
+// One AdamW step on several 16-bit or fp32 tensors at once, moments of the weights' type, arithmetic in fp32. `step` is
+// each tensor's own step count, already advanced.
+struct AdamWTensor {
+  void *weight, *m, *v;
+  const void* grad;
+  const float* step;
+  int64_t count;
+};
+constexpr int kMaxAdamWTensors = 480;
+hlResult_t multiAdamW(int dt, const AdamWTensor* tensors, int n, double lr, double beta1, double beta2, double decay, double eps, cudaStream_t s);
+
 // Mixture of experts (moe.cu). row_of: [tokens], row of the dispatch buffer or -1; token_of: [experts * capacity].
 hlResult_t moeRoute(int dt, const void* logits, int tokens, int experts, int capacity, int* expert, float* gate, int* row_of, int* token_of,
                     cudaStream_t s);

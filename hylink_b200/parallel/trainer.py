@@ -23,6 +23,11 @@ import os
 import torch
 import torch.distributed as dist
 from torch.nn.parallel import DistributedDataParallel as DDP
+from torch.optim import optimizer as _optimizer
+
+from ..ops.extension import ops
+
+_global_hooks = (_optimizer._global_optimizer_pre_hooks, _optimizer._global_optimizer_post_hooks)
 
 
 def init_distributed(backend: str = "hylink"):
@@ -144,6 +149,35 @@ class DDPTrainer:
                             static_graph=False)
         return self._ddp
 
+    def _opt_step(self) -> None:
+        """``self.opt.step()``, through this library's kernel where the optimizer is what the constructor made and nobody
+        watches its steps (a scheduler replaces ``step``, hooks want to be called); its state stays where it is."""
+        opt = self.opt
+        g = opt.param_groups[0]
+        plain = (type(opt) is torch.optim.AdamW and len(opt.param_groups) == 1 and "step" not in opt.__dict__
+                 and not (opt._optimizer_step_pre_hooks or opt._optimizer_step_post_hooks or _global_hooks[0] or _global_hooks[1])
+                 and not (g["amsgrad"] or g["maximize"] or g["differentiable"] or g["capturable"])
+                 and isinstance(g["lr"], float) and isinstance(g["betas"][0], float) and isinstance(g["betas"][1], float)
+                 and getattr(opt, "grad_scale", None) is None and getattr(opt, "found_inf", None) is None)
+        if plain:
+            ps, gs, ms, vs, steps = [], [], [], [], []
+            state = opt.state
+            for p in g["params"]:
+                grad = p.grad
+                if grad is None:
+                    continue
+                st = state.get(p)
+                if not st:                 # the first step: the optimizer sets its state up itself
+                    plain = False
+                    break
+                ps.append(p)
+                gs.append(grad)
+                ms.append(st["exp_avg"])
+                vs.append(st["exp_avg_sq"])
+                steps.append(st["step"])
+        if not plain or not ops().multi_adamw(ps, gs, ms, vs, steps, g["lr"], g["betas"][0], g["betas"][1], g["weight_decay"], g["eps"]):
+            opt.step()
+
     def _replayable(self, idx: torch.Tensor, targets: torch.Tensor) -> bool:
         """Whether this step runs from the graph; captures it when the same step has been run before."""
         signature = getattr(self.model, "step_signature", None)
@@ -189,13 +223,13 @@ class DDPTrainer:
             loss = self._ddp(idx, targets)
         elif self._replayable(idx, targets):
             loss = self._graph.run(idx, targets)
-            self.opt.step()
+            self._opt_step()
             return loss
         else:
             loss = self.model(idx.to(self.device), targets.to(self.device))
         self.opt.zero_grad(set_to_none=True)
         loss.backward()
-        self.opt.step()
+        self._opt_step()
         return loss
 
     def step(self, tokens: torch.Tensor) -> float:

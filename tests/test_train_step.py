@@ -121,3 +121,31 @@ def test_replayed_steps_train_like_eager_ones(name, batch, seq, monkeypatch):
     assert float((weights - want).norm() / want.norm()) < 1e-2
     if fresh:
         dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_multi_tensor_adamw_matches_torch(dtype):
+    """Tensors shorter than a packet, of a ragged length, unaligned, of several chunks; more of them than one launch takes."""
+    from hylink_b200.ops.extension import ops
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    sizes = [1, 7, 8, 8193, 40000] + [5 + i for i in range(500)]
+    ps = [torch.randn(n + 1, generator=g, device="cuda").to(dtype)[1 if i == 3 else 0:n + (1 if i == 3 else 0)] for i, n in enumerate(sizes)]
+    ref = [p.double().clone().requires_grad_() for p in ps]
+    ms, vs = [torch.zeros_like(p) for p in ps], [torch.zeros_like(p) for p in ps]
+    steps = [torch.zeros((), device="cuda") for _ in ps]
+    opt = torch.optim.AdamW(ref, lr=1e-2, betas=(0.9, 0.95), weight_decay=0.1)
+    for _ in range(3):
+        gs = [(0.1 * torch.randn(p.shape, generator=g, device="cuda")).to(dtype) for p in ps]
+        assert ops().multi_adamw(ps, gs, ms, vs, steps, 1e-2, 0.9, 0.95, 0.1, 1e-8)
+        for r, x in zip(ref, gs):
+            r.grad = x.double()
+        opt.step()
+        for p, r, m, v in zip(ps, ref, ms, vs):                 # both go on from the rounded weights and moments
+            tol = {torch.bfloat16: 1e-2, torch.float16: 2e-3, torch.float32: 1e-5}[dtype]
+            torch.testing.assert_close(p.double(), r.detach(), rtol=tol, atol=tol * 1e-1)
+            r.data.copy_(p)
+            opt.state[r]["exp_avg"].copy_(m)
+            opt.state[r]["exp_avg_sq"].copy_(v)
+    assert all(float(s) == 3 for s in steps)
+    assert not ops().multi_adamw(ps[:1], [gs[0].cpu()], ms[:1], vs[:1], steps[:1], 1e-2, 0.9, 0.95, 0.1, 1e-8)
