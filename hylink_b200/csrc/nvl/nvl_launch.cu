@@ -1,6 +1,9 @@
 // Launch side of the dedicated-link kernels (nvl_kernels.cuh): which kernel a call runs and how it is launched.
 #include <cuda_runtime.h>
 
+#include <bitset>
+#include <mutex>
+
 #include "nvl/nvl_device.cuh"
 #include "nvl/nvl_launch.h"
 
@@ -116,6 +119,14 @@ hlResult_t prepareKernels() {
   // Resolve every variant once on the init thread: lazy module loading plus
   // concurrent first launches from several threads can deadlock in the driver
   // (same cure as pcie-ccl-cuda/kernels/wait_kernel.cu:216-234,400-432).
+  // Once per device: the thousand queries take 1.5 ms, which every later group of the process would wait for.
+  static std::mutex mu;
+  static std::bitset<64> done;
+  int device = 0;
+  cudaError_t got = cudaGetDevice(&device);
+  if (got != cudaSuccess) return fail(hlDeviceError, "cudaGetDevice: %s", cudaGetErrorString(got));
+  std::lock_guard<std::mutex> lock(mu);
+  if (device < 64 && done[device]) return hlSuccess;
   static const int kinds[] = {kNvlBarrier, kNvlAllReduceOneShot, kNvlAllReduceTwoShot, kNvlAllReduceNvls,
                               kNvlReduceScatter, kNvlReduceScatterNvls, kNvlAllGather, kNvlBroadcast,
                               kNvlAllToAll, kNvlAllGatherNvls, kNvlBroadcastNvls, kNvlAllReducePipeP2p,
@@ -136,6 +147,7 @@ hlResult_t prepareKernels() {
       }
       if (k == kNvlBarrier) break;
     }
+  if (device < 64) done.set(device);
   return hlSuccess;
 }
 
