@@ -1,6 +1,7 @@
 // Autograd functions of the training step over the kernels of csrc/train: what surrounds the GEMMs and the attention
-// of a transformer block, the language-model head with its loss, the mixture-of-experts layer; and the sharded optimizer. The GEMMs are torch's own (cuBLAS), the
-// attention between the two halves of a block is whatever torch's scaled_dot_product_attention picks.
+// of a transformer block, the language-model head with its loss, the mixture-of-experts layer; the optimizers; and the
+// launches of emulated collectives and of the landing reduce. The GEMMs are torch's own (cuBLAS), the attention between
+// the two halves of a block is whatever torch's scaled_dot_product_attention picks.
 //
 // A block is cut in two around the attention:
 //   blockPre:   x1 = x + y; h = layer norm(x1); q, k, v = h Wqkv^T + b     (y: the branch of the block before)
@@ -10,6 +11,9 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/python.h>
 
 #include "hylink/hylink_ext.h"
@@ -497,36 +501,92 @@ int typeCode(at::ScalarType t) {
     default: TORCH_CHECK(false, "hylink: unsupported dtype ", t);
   }
 }
-using TensorList = std::vector<std::optional<Tensor>>;
-
-// One collective of an emulated group on the current stream; returns the library's result code.
-int emuRun(uintptr_t group, int nranks, int kind, const std::optional<TensorList>& ins, const std::optional<TensorList>& outs, size_t count,
-           size_t in_stride, size_t out_stride, const std::optional<at::ScalarType>& wire, int op, double scale, int root, int algo, int max_blocks) {
-  const void* in[8] = {nullptr};
-  void* out[8] = {nullptr};
-  TORCH_CHECK(nranks <= 8 && (!ins || (int)ins->size() <= nranks) && (!outs || (int)outs->size() <= nranks), "hylink: more buffers than ranks");
-  for (size_t i = 0; ins && i < ins->size(); ++i)
-    if ((*ins)[i]) in[i] = (*ins)[i]->data_ptr();
-  for (size_t i = 0; outs && i < outs->size(); ++i)
-    if ((*outs)[i]) out[i] = (*outs)[i]->data_ptr();
-  const int in_dt = ins ? typeCode((*ins)[0]->scalar_type()) : (int)hlFloat32;
-  const int out_dt = outs ? typeCode((*outs)[0]->scalar_type()) : in_dt;
-  return (int)hlEmuCollective(reinterpret_cast<hlEmu_t>(group), kind, in, out, count, in_stride, out_stride, in_dt, out_dt,
-                              wire ? typeCode(*wire) : in_dt, op, (float)scale, root, algo, max_blocks, c10::cuda::getCurrentCUDAStream().stream());
+// The two calls below are launches of a few microseconds, so their arguments are read by hand: through pybind11's
+// converters (a vector of optional tensors, a dtype) an empty emulated collective of eight ranks took 1.4 us on the
+// host, of two 0.8; read by hand 0.28 and 0.22.
+template <typename F>
+PyObject* native(const char* name, Py_ssize_t want, Py_ssize_t got, F&& body) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_TYPE(want == got, name, " takes ", want, " arguments, not ", got);
+  return PyLong_FromLong(body());
+  END_HANDLE_TH_ERRORS
+}
+long long whole(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+double real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1. && PyErr_Occurred()) throw python_error();
+  return v;
+}
+const Tensor& tensor(PyObject* o) {
+  TORCH_CHECK_TYPE(THPVariable_Check(o), "hylink: expected a tensor, got ", Py_TYPE(o)->tp_name);
+  return THPVariable_Unpack(o);
+}
+// A list or tuple as it is, anything else as a list of its items.
+py::object sequence(PyObject* o) {
+  PyObject* s = PySequence_Fast(o, "hylink: expected a sequence of tensors");
+  if (!s) throw python_error();
+  return py::reinterpret_steal<py::object>(s);
 }
 
-int reduceLanding(const Tensor& dst, const std::vector<Tensor>& srcs, int op, double scale, bool accumulate, int blocks) {
-  TORCH_CHECK_VALUE(dst.is_cuda(), "reduce_landing needs a CUDA destination");
-  std::vector<const void*> p;
-  p.reserve(srcs.size());
-  for (const Tensor& s : srcs) {
-    TORCH_CHECK_VALUE(s.numel() == dst.numel() && s.scalar_type() == dst.scalar_type(), "sources must match the destination's size and dtype");
-    TORCH_CHECK_VALUE(s.is_cuda() || s.is_pinned(), "host sources must be pinned");
-    p.push_back(s.data_ptr());
-  }
-  return (int)hlReduceLanding(dst.data_ptr(), p.data(), (int)p.size(), accumulate, (size_t)dst.numel(), (hlDataType_t)typeCode(dst.scalar_type()),
-                              (hlRedOp_t)op, (float)scale, blocks, c10::cuda::getCurrentCUDAStream().stream());
+// One collective of an emulated group on the current stream; returns the library's result code. Arguments: group, ranks,
+// kind, inputs, outputs, count, segment strides, wire type or None, operator, scale, root, algorithm, CTAs.
+PyObject* emuRun(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  return native("emu_run", 14, nargs, [&]() -> long {
+    const int nranks = (int)whole(args[1]);
+    void* bufs[2][8] = {{nullptr}, {nullptr}};
+    int dt[2] = {-1, -1};
+    for (int k = 0; k < 2; ++k) {
+      if (args[3 + k] == Py_None) continue;
+      const py::object list = sequence(args[3 + k]);
+      const Py_ssize_t n = PySequence_Fast_GET_SIZE(list.ptr());
+      PyObject** items = PySequence_Fast_ITEMS(list.ptr());
+      TORCH_CHECK(nranks <= 8 && n <= nranks, "hylink: more buffers than ranks");
+      TORCH_CHECK(n > 0, "hylink: no buffers");
+      dt[k] = typeCode(tensor(items[0]).scalar_type());
+      for (Py_ssize_t i = 0; i < n; ++i)
+        if (items[i] != Py_None) bufs[k][i] = tensor(items[i]).data_ptr();
+    }
+    if (dt[0] < 0) dt[0] = (int)hlFloat32;
+    if (dt[1] < 0) dt[1] = dt[0];
+    int wire = dt[0];
+    if (args[8] != Py_None) {
+      TORCH_CHECK_TYPE(THPDtype_Check(args[8]), "hylink: the wire type is a torch.dtype");
+      wire = typeCode(reinterpret_cast<THPDtype*>(args[8])->scalar_type);
+    }
+    return (long)hlEmuCollective(reinterpret_cast<hlEmu_t>((uintptr_t)whole(args[0])), (int)whole(args[2]), bufs[0], bufs[1], (size_t)whole(args[5]),
+                                 (size_t)whole(args[6]), (size_t)whole(args[7]), dt[0], dt[1], wire, (int)whole(args[9]), (float)real(args[10]),
+                                 (int)whole(args[11]), (int)whole(args[12]), (int)whole(args[13]), c10::cuda::getCurrentCUDAStream().stream());
+  });
 }
+
+// Destination, sources, operator, scale, accumulate, CTAs.
+PyObject* reduceLanding(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  return native("reduce_landing", 6, nargs, [&]() -> long {
+    const Tensor& dst = tensor(args[0]);
+    TORCH_CHECK_VALUE(dst.is_cuda(), "reduce_landing needs a CUDA destination");
+    const py::object list = sequence(args[1]);
+    const Py_ssize_t n = PySequence_Fast_GET_SIZE(list.ptr());
+    c10::SmallVector<const void*, 8> p;
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      const Tensor& s = tensor(PySequence_Fast_ITEMS(list.ptr())[i]);
+      TORCH_CHECK_VALUE(s.numel() == dst.numel() && s.scalar_type() == dst.scalar_type(), "sources must match the destination's size and dtype");
+      TORCH_CHECK_VALUE(s.is_cuda() || s.is_pinned(), "host sources must be pinned");
+      p.push_back(s.data_ptr());
+    }
+    const int accumulate = PyObject_IsTrue(args[4]);
+    if (accumulate < 0) throw python_error();
+    return (long)hlReduceLanding(dst.data_ptr(), p.data(), (int)p.size(), accumulate != 0, (size_t)dst.numel(),
+                                 (hlDataType_t)typeCode(dst.scalar_type()), (hlRedOp_t)whole(args[2]), (float)real(args[3]), (int)whole(args[5]),
+                                 c10::cuda::getCurrentCUDAStream().stream());
+  });
+}
+PyMethodDef kNativeCalls[] = {{"emu_run", (PyCFunction)(void*)emuRun, METH_FASTCALL, nullptr},
+                              {"reduce_landing", (PyCFunction)(void*)reduceLanding, METH_FASTCALL, nullptr},
+                              {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace
 
@@ -551,11 +611,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return MoeCombine::apply(x, gate, rows, row_of, token_of);
   });
   m.def("sharded_adamw", &shardedAdamW);
-  m.def("emu_run", [](uintptr_t group, int nranks, int kind, const std::optional<TensorList>& ins, const std::optional<TensorList>& outs, size_t count,
-                      size_t in_stride, size_t out_stride, const py::object& wire, int op, double scale, int root, int algo, int max_blocks) {
-    return emuRun(group, nranks, kind, ins, outs, count, in_stride, out_stride,
-                  wire.is_none() ? std::nullopt : std::make_optional(torch::python::detail::py_object_to_dtype(wire)), op, scale, root, algo, max_blocks);
-  });
-  m.def("reduce_landing", &reduceLanding);
+  if (PyModule_AddFunctions(m.ptr(), kNativeCalls)) throw py::error_already_set();
   m.def("head_loss", [](const Tensor& h, const Tensor& w, const Tensor& targets) { return HeadLoss::apply(h, w, targets); });
 }

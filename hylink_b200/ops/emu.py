@@ -26,6 +26,7 @@ class EmuGroup:
     def __init__(self, nranks: int, stage_bytes: int = 64 << 20, timeout_ms: int = 2000, device: int = 0):
         self.nranks = nranks
         self._h = C.c_void_p()
+        self._run = ops().emu_run
         check(lib.hlEmuCreate(nranks, device, stage_bytes, timeout_ms, C.byref(self._h)), "hlEmuCreate")
 
     def close(self):
@@ -42,8 +43,8 @@ class EmuGroup:
     def run(self, kind: str, ins, outs, count: int, *, in_seg_stride: int = 0, out_seg_stride: int = 0,
             wire_dtype=None, op: str = "sum", scale: float = 1.0, root: int = 0, algo: str = "auto",
             max_blocks: int = 0):
-        code = ops().emu_run(self._h.value or 0, self.nranks, KINDS[kind], ins, outs, count, in_seg_stride, out_seg_stride, wire_dtype, OPS[op],
-                             scale, root, ALGOS[algo], max_blocks)
+        code = self._run(self._h.value or 0, self.nranks, KINDS[kind], ins, outs, count, in_seg_stride, out_seg_stride, wire_dtype, OPS[op],
+                         scale, root, ALGOS[algo], max_blocks)
         if code:
             check(code, f"emu {kind}")
 
