@@ -121,6 +121,10 @@ extern "C" hlResult_t hlAllReduceLocalNoAlloc(int nranks, const void* const* ins
     a.in_dt = dtype;
     a.out_dt = dtype;
     a.int_div = op == hlAvg ? nranks : 0;
+    a.abort_word = reinterpret_cast<uint32_t*>(base + kWordsOff + (size_t)i * 128 + 64);
+    a.seq_words = reinterpret_cast<uint64_t*>(base + kWordsOff + (size_t)i * 128 + 80);
+    a.rank = i;
+    a.nranks = nranks;
   }
   // one CTA per 16 KiB, never more than kMaxBlocks per buffer (all rows must be co-resident)
   int blocks = (int)((count * es + (16u << 10) - 1) / (16u << 10));

@@ -221,26 +221,7 @@ __device__ __forceinline__ void timelineStamp(const HlCommDev& c, uint64_t seq, 
 // tile base by `tiles`). Counting at entry instead of at exit keeps the atomic
 // out of the tail of the call; launches of one communicator are stream-ordered,
 // so nobody reads the new values too early.
-__device__ __forceinline__ bool entryOk(const HlCommDev& c, HlCallArgs& a, uint64_t tiles = 0) {
-  __shared__ int s_entry;
-  __shared__ uint64_t s_seq[2];
-  if (threadIdx.x == 0) {
-    s_entry = (*reinterpret_cast<volatile uint32_t*>(c.abort_word) == 0) ? 1 : 0;
-    s_seq[0] = reinterpret_cast<volatile uint64_t*>(c.seq_words)[0];
-    s_seq[1] = reinterpret_cast<volatile uint64_t*>(c.seq_words)[1];
-  }
-  __syncthreads();
-  a.seq = s_seq[0];
-  a.pipe_seq = s_seq[1];
-  if (threadIdx.x == blockDim.x - 1) {
-    const unsigned long long prev = atomicAdd(reinterpret_cast<unsigned long long*>(c.seq_words + 2), 1ull);
-    if (prev + 1 == gridDim.x) {
-      volatile uint64_t* w = c.seq_words;
-      w[2] = 0;
-      w[0] = a.seq + HL_SEQ_STRIDE;
-      w[1] = a.pipe_seq + tiles;
-    }
-  }
+__device__ __forceinline__ void timelineEntry(const HlCommDev& c, const HlCallArgs& a) {
   if (c.timeline != nullptr && threadIdx.x == 0) {
     if (blockIdx.x == 0) {
       uint64_t* meta = c.timeline + (size_t)HL_TL_CALLS * HL_TL_BLOCKS * HL_TL_PHASES + ((a.seq / HL_SEQ_STRIDE) % HL_TL_CALLS) * 4;
@@ -251,6 +232,32 @@ __device__ __forceinline__ bool entryOk(const HlCommDev& c, HlCallArgs& a, uint6
     }
     timelineStamp(c, a.seq, 0);
   }
+}
+// Called by all threads of a CTA once each of them has the words it needs.
+__device__ __forceinline__ void countEntry(const HlCallArgs& a, uint64_t tiles) {
+  if (threadIdx.x == blockDim.x - 1) {
+    const unsigned long long prev = atomicAdd(reinterpret_cast<unsigned long long*>(a.seq_words + 2), 1ull);
+    if (prev + 1 == gridDim.x) {
+      volatile uint64_t* w = a.seq_words;
+      w[2] = 0;
+      w[0] = a.seq + HL_SEQ_STRIDE;
+      if (tiles) w[1] = a.pipe_seq + tiles;
+    }
+  }
+}
+__device__ __forceinline__ bool entryOk(const HlCommDev& c, HlCallArgs& a, uint64_t tiles = 0) {
+  __shared__ int s_entry;
+  __shared__ uint64_t s_seq[2];
+  if (threadIdx.x == 0) {
+    s_entry = (*reinterpret_cast<volatile uint32_t*>(a.abort_word) == 0) ? 1 : 0;
+    s_seq[0] = reinterpret_cast<volatile uint64_t*>(a.seq_words)[0];
+    s_seq[1] = reinterpret_cast<volatile uint64_t*>(a.seq_words)[1];
+  }
+  __syncthreads();
+  a.seq = s_seq[0];
+  a.pipe_seq = s_seq[1];
+  countEntry(a, tiles);
+  timelineEntry(c, a);
   return s_entry != 0;
 }
 

@@ -34,7 +34,9 @@ static const void* pick(int kind, int nranks) {
 
 const void* kernelFor(int kind, int wire_dt, int nranks) {
   if (kind == kNvlBarrier) return (const void*)dev::kBarrier;
-  if (kind == kNvlLlAllReduce || kind == kNvlLlReduceScatter || kind == kNvlLlAllGather || kind == kNvlLlAllToAll) return lowLatencyKernelFor(kind, wire_dt);
+  if (kind == kNvlLlAllReduce || kind == kNvlLlReduceScatter || kind == kNvlLlAllGather || kind == kNvlLlAllToAll ||
+      kind == kNvlLlBroadcast)
+    return lowLatencyKernelFor(kind, wire_dt);
   switch (wire_dt) {
     case hlInt8: return pick<int8_t>(kind, nranks);
     case hlUint8: return pick<uint8_t>(kind, nranks);
@@ -83,6 +85,7 @@ const char* kernelName(int kind) {
     case kNvlLlReduceScatter: return "reducescatter_lowlatency";
     case kNvlLlAllGather: return "allgather_lowlatency";
     case kNvlLlAllToAll: return "alltoall_lowlatency";
+    case kNvlLlBroadcast: return "broadcast_lowlatency";
     case kNvlAllToAllPush: return "alltoall_push";
     case kNvlStreamReduceScatter: return "reducescatter_streamed";
     case kNvlStreamAllGather: return "allgather_streamed";
@@ -134,7 +137,7 @@ hlResult_t prepareKernels() {
                               kNvlReduceScatterPush, kNvlAllGatherPush, kNvlAllGatherLanes, kNvlZcAllReduceNvls,
                               kNvlZcAllReduceP2p, kNvlZcReduceScatterNvls, kNvlZcReduceScatterP2p, kNvlZcAllGatherNvls,
                               kNvlZcAllGatherP2p, kNvlZcBroadcastNvls, kNvlZcBroadcastP2p, kNvlLlAllReduce,
-                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlAllToAllPush,
+                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlLlBroadcast, kNvlAllToAllPush,
                               kNvlStreamReduceScatter, kNvlStreamAllGather, kNvlStreamAllToAll};
   for (int k : kinds)
     for (int dt = 0; dt < hlNumTypes; ++dt) {

@@ -1,5 +1,5 @@
-// Low-latency kernels of the dedicated-link path for small messages: all-reduce, reduce-scatter, all-gather and
-// all-to-all with NO cross-GPU barrier at all.
+// Low-latency kernels of the dedicated-link path for small messages: all-reduce, reduce-scatter, all-gather,
+// all-to-all and broadcast with NO cross-GPU barrier at all.
 //
 // The barrier-based kernels (nvl_kernels.cu) pay two flag round trips per call — about 3 to 8 microseconds each
 // once the stores in front of them have to be acknowledged — which is most of the time of a message of a few MiB.
@@ -15,13 +15,25 @@
 // ago. That reuse is safe without any handshake: in each of these collectives every rank receives from every other
 // rank (directly, or through a shard owner that did), so a rank can only FINISH call k+1 after every peer has
 // STARTED sending in call k+1, i.e. after every peer has left call k (launches of one communicator are
-// stream-ordered); barrier-based kernels in between synchronise all ranks anyway. The tag is the call index + 1 (never 0, the value of cleared memory) and differs from the tag
-// that the same slot held two calls earlier.
+// stream-ordered); barrier-based kernels in between synchronise all ranks anyway. The tag is
+// 2 * call index + 1 (odd: never 0, the value of cleared memory) and differs from the tag that the same slot held two
+// calls earlier.
 //
 // all-to-all:      send segment q to rank q       | receive segment s from rank s into slot s of the output
 // all-gather:      send own segment to every peer | receive the others' segments into the output
 // reduce-scatter:  send segment q to rank q       | receive n-1 contributions, add in rank order, store
 // all-reduce:      reduce-scatter of the n shards (phase 0), then all-gather of the reduced shards (phase 1)
+// broadcast:       the root sends its buffer to every peer; the others send packet 0 alone, as the sign that they have
+//                  started, and everybody waits for all of these (the argument above needs it)
+//
+// All of this is latency. A call is a chain of L2 round trips (0.3 us each and more): the call's words, the caller's
+// data, the packet on its way, the poll that finds it; so whatever a step does not need is out of its way. The first
+// column of data is loaded before the call index is known, the abort word and the call index come at addresses that
+// are launch arguments, and the count of started CTAs is taken after the sends.
+// 8 KiB between ranks of one GPU, us per call before and after: all-gather of 2 ranks 6.1 / 4.1, of 8 6.1 / 4.1;
+// all-reduce of 4 ranks 8.2 / 6.1.
+// The period of a launch that waits for the one before it comes in steps of 2.05 us on this GPU, whatever the kernel:
+// what a call saves shows when it crosses a step.
 //
 // Buffers: any device memory, any alignment, any element count; no type conversion. Sum order is by rank index on every rank: results are bitwise identical
 // across ranks and runs.
@@ -37,7 +49,7 @@
 namespace hl {
 namespace dev {
 
-constexpr int kLlAllReduce = 0, kLlReduceScatter = 1, kLlAllGather = 2, kLlAllToAll = 3;
+constexpr int kLlAllReduce = 0, kLlReduceScatter = 1, kLlAllGather = 2, kLlAllToAll = 3, kLlBroadcast = 4;
 
 __device__ __forceinline__ uint8_t* llSlot(const HlCommDev& c, int owner, int parity, int phase, int src) {
   return c.ll[owner] + ((size_t)((parity * 2 + phase) * HL_MAX_RANKS + src)) * c.ll_slot_bytes;
@@ -146,20 +158,45 @@ template <typename W, int kColl>
 __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
-  if (!entryOk(c, a)) return;
+  const uint32_t aborted = *reinterpret_cast<volatile uint32_t*>(a.abort_word);
+  a.seq = *reinterpret_cast<volatile uint64_t*>(a.seq_words);   // used once the first column has been asked for
   constexpr int N = Packet<W>::N, MR = HL_MAX_RANKS;
-  const int n = c.nranks, r = c.rank;
+  const int n = a.nranks, r = a.rank;
   const uint64_t g0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, gstride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t call = a.seq / HL_SEQ_STRIDE;
-  const uint32_t tag = (uint32_t)(call % 0xfffffffeull) + 1u;
-  const int parity = (int)(call & 1);
   const W* in = reinterpret_cast<const W*>(a.in);
   W* out = reinterpret_cast<W*>(a.out);
   const uint64_t cnt = a.count;
   const uint64_t np = (cnt + N - 1) / N;
+  // shard q of an all-reduce = packets [q * sp, min(np, (q + 1) * sp)) of the whole buffer; rank q reduces it
+  const uint64_t sp = kColl == kLlAllReduce ? (np + n - 1) / n : np;
   // packet j of the segment that starts at element `base` of a buffer
   auto ld = [&](const W* seg, uint64_t j) { return loadUserPacket<W, W>(seg, j * N, cnt, aligned16(seg)); };
   auto st = [&](W* seg, uint64_t j, const uint4& v) { storeUserPacket<W, W>(seg, j * N, cnt, aligned16(seg), v); };
+  const uint32_t peers = ((1u << n) - 1u) & ~(1u << r);
+  uint4 v[MR];   // indexed by compile-time constants only: stays in registers
+  // what this rank has of column j
+  auto column = [&](uint64_t j) {
+    if constexpr (kColl == kLlAllGather) {
+      v[0] = ld(in, j);
+    } else if constexpr (kColl == kLlBroadcast) {
+      v[0] = r == a.root ? ld(in, j) : make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+      for (int q = 0; q < MR; ++q)
+        if (kColl == kLlAllToAll ? q < n : (peers >> q & 1u)) {
+          if constexpr (kColl == kLlAllReduce) {
+            if ((uint64_t)q * sp + j < np) v[q] = ld(in, (uint64_t)q * sp + j);
+          } else {
+            v[q] = ld(in + (uint64_t)q * a.in_seg_stride, j);
+          }
+        }
+    }
+  };
+  if (g0 < sp) column(g0);
+
+  const uint32_t call = (uint32_t)(a.seq / HL_SEQ_STRIDE);
+  const uint32_t tag = 2u * call + 1u;
+  const int parity = (int)(call & 1u);
   // the slot of this rank at every peer, and this rank's own slots, by phase
   uint8_t* to[MR];
 #pragma unroll
@@ -167,51 +204,56 @@ __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* co
     if (q < n) to[q] = llSlot(c, q, parity, 0, r);
   const uint64_t phase2 = (uint64_t)HL_MAX_RANKS * c.ll_slot_bytes;   // from a phase-0 slot to its phase-1 counterpart
   const uint8_t* from = llSlot(c, r, parity, 0, 0);
-  const uint32_t peers = ((1u << n) - 1u) & ~(1u << r);
+  // the columns of this thread; none on a poisoned communicator (a no-op instead of a second hang candidate)
+  const uint64_t end = aborted ? 0 : sp;
   LlWait w;
   w.t0 = 0;
   w.ok = true;
-  uint4 v[MR];   // indexed by compile-time constants only: stays in registers
-  if constexpr (kColl == kLlAllGather) {
-    for (uint64_t j = g0; j < np; j += gstride) {
-      const uint4 own = ld(in, j);
+  for (uint64_t j = g0; j < end;) {
 #pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if (peers >> q & 1u) llSend(to[q], j, own, tag);
-      st(out + (uint64_t)r * a.out_seg_stride, j, own);
-    }
-    for (uint64_t j = g0; j < np && llRecv(c, from, j, tag, peers, w, v); j += gstride) {
-#pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if (peers >> q & 1u) st(out + (uint64_t)q * a.out_seg_stride, j, v[q]);
-    }
-  } else if constexpr (kColl == kLlAllToAll) {
-    for (uint64_t j = g0; j < np; j += gstride) {
-#pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if (q < n) v[q] = ld(in + (uint64_t)q * a.in_seg_stride, j);
-#pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if (peers >> q & 1u) llSend(to[q], j, v[q], tag);
+    for (int q = 0; q < MR; ++q)
+      if (peers >> q & 1u) {
+        if constexpr (kColl == kLlAllGather) llSend(to[q], j, v[0], tag);
+        else if constexpr (kColl == kLlBroadcast) {
+          if (r == a.root || j == 0) llSend(to[q], j, v[0], tag);
+        } else if constexpr (kColl == kLlAllReduce) {
+          if ((uint64_t)q * sp + j < np) llSend(to[q], j, v[q], tag);
+        } else {
+          llSend(to[q], j, v[q], tag);
+        }
+      }
+    if constexpr (kColl == kLlAllGather) st(out + (uint64_t)r * a.out_seg_stride, j, v[0]);
+    if constexpr (kColl == kLlBroadcast)
+      if (r == a.root && in != out) st(out, j, v[0]);
+    if constexpr (kColl == kLlAllToAll) {
 #pragma unroll
       for (int q = 0; q < MR; ++q)   // after every read of this thread's column: in place is safe
         if (q == r) st(out + (uint64_t)r * a.out_seg_stride, j, v[q]);
     }
-    for (uint64_t j = g0; j < np && llRecv(c, from, j, tag, peers, w, v); j += gstride) {
+    j += gstride;
+    if (j < end) column(j);
+  }
+  __syncthreads();                   // every thread has its call index
+  countEntry(a, 0);
+  timelineEntry(c, a);
+
+  if constexpr (kColl == kLlAllGather || kColl == kLlAllToAll) {
+    for (uint64_t j = g0; j < end && llRecv(c, from, j, tag, peers, w, v); j += gstride) {
 #pragma unroll
       for (int q = 0; q < MR; ++q)
         if (peers >> q & 1u) st(out + (uint64_t)q * a.out_seg_stride, j, v[q]);
     }
-  } else if constexpr (kColl == kLlReduceScatter) {
-    for (uint64_t j = g0; j < np; j += gstride) {
+  } else if constexpr (kColl == kLlBroadcast) {
+    const uint32_t root = peers & (1u << a.root);                  // 0 on the root itself
+    for (uint64_t j = g0; j < end; j += gstride) {
+      const uint32_t have = j == 0 ? peers : root;
+      if (!have || !llRecv(c, from, j, tag, have, w, v)) break;    // the root waits with the thread of packet 0 only
 #pragma unroll
       for (int q = 0; q < MR; ++q)
-        if (peers >> q & 1u) v[q] = ld(in + (uint64_t)q * a.in_seg_stride, j);
-#pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if (peers >> q & 1u) llSend(to[q], j, v[q], tag);
+        if (root >> q & 1u) st(out, j, v[q]);
     }
-    for (uint64_t j = g0; j < np; j += gstride) {
+  } else if constexpr (kColl == kLlReduceScatter) {
+    for (uint64_t j = g0; j < end; j += gstride) {
       const uint4 own = ld(in + (uint64_t)r * a.in_seg_stride, j);
       if (!llRecv(c, from, j, tag, peers, w, v)) break;
 #pragma unroll
@@ -220,18 +262,8 @@ __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* co
       st(out, j, llReduce<W>(v, n, a.op, a.scale, a.int_div));
     }
   } else {
-    // shard q = packets [q * sp, min(np, (q + 1) * sp)) of the whole buffer; rank q reduces it
-    const uint64_t sp = (np + n - 1) / n;
     const uint64_t first = (uint64_t)r * sp;
-    const uint64_t mine = first >= np ? 0 : (np - first < sp ? np - first : sp);
-    for (uint64_t j = g0; j < sp; j += gstride) {
-#pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if ((peers >> q & 1u) && (uint64_t)q * sp + j < np) v[q] = ld(in, (uint64_t)q * sp + j);
-#pragma unroll
-      for (int q = 0; q < MR; ++q)
-        if ((peers >> q & 1u) && (uint64_t)q * sp + j < np) llSend(to[q], j, v[q], tag);
-    }
+    const uint64_t mine = first >= np || aborted ? 0 : (np - first < sp ? np - first : sp);
     for (uint64_t j = g0; j < mine; j += gstride) {
       const uint4 own = ld(in, first + j);
       if (!llRecv(c, from, j, tag, peers, w, v)) break;
@@ -244,7 +276,7 @@ __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* co
         if (peers >> q & 1u) llSend(to[q] + phase2, j, red, tag);
       st(out, first + j, red);
     }
-    for (uint64_t j = g0; j < sp && w.ok; j += gstride) {
+    for (uint64_t j = g0; j < end && w.ok; j += gstride) {
       uint32_t have = 0;
 #pragma unroll
       for (int q = 0; q < MR; ++q)
@@ -271,6 +303,7 @@ static const void* pickLl(int kind) {
     case kNvlLlReduceScatter: return (const void*)kLowLatency<W, kLlReduceScatter>;
     case kNvlLlAllGather: return (const void*)kLowLatency<W, kLlAllGather>;
     case kNvlLlAllToAll: return (const void*)kLowLatency<W, kLlAllToAll>;
+    case kNvlLlBroadcast: return (const void*)kLowLatency<W, kLlBroadcast>;
     default: return nullptr;
   }
 }

@@ -417,6 +417,16 @@ bool NvlPath::zeroCopyEligible(const NvlBufs& b, const NvlCall& c, bool in_remot
   return true;
 }
 
+// What a kernel needs of the ranks' tables before anything else.
+void NvlPath::fillEntry(HlEmuCalls* calls) const {
+  for (int i = 0; i < localRanks(); ++i) {
+    calls->c[i].abort_word = host_comm_[i].abort_word;
+    calls->c[i].seq_words = host_comm_[i].seq_words;
+    calls->c[i].rank = host_comm_[i].rank;
+    calls->c[i].nranks = nranks_;
+  }
+}
+
 hlResult_t NvlPath::launchZeroCopy(int kind, const NvlBufs& b, const NvlCall& c, uint64_t in_off, uint64_t out_off, size_t bytes_per_rank,
                                    cudaStream_t s) {
   HL_CUDA(cudaSetDevice(device_));
@@ -424,6 +434,7 @@ hlResult_t NvlPath::launchZeroCopy(int kind, const NvlBufs& b, const NvlCall& c,
   const int nl = localRanks();
   HlEmuCalls calls;
   memset(&calls, 0, sizeof(calls));
+  fillEntry(&calls);
   for (int i = 0; i < nl; ++i) {
     HlCallArgs& a = calls.c[i];
     a.in = b.in[i];
@@ -534,6 +545,7 @@ hlResult_t NvlPath::launchSliced(int kind, const NvlBufs& b, const NvlCall& c, b
     const uint64_t len = std::min<uint64_t>(per_launch, c.count - done);
     HlEmuCalls calls;
     memset(&calls, 0, sizeof(calls));
+    fillEntry(&calls);
     for (int i = 0; i < nl; ++i) {
       HlCallArgs& a = calls.c[i];
       a.in = b.in[i] ? (const char*)b.in[i] + done * is : nullptr;
@@ -609,9 +621,26 @@ int NvlPath::lowLatencyChoice(const NvlBufs& b, const NvlCall& c, int coll, size
     // all-gather 17.1 -> 6.8; 2 MiB 20.1 -> 15.3, 17.4 -> 12.0, 16.9 -> 7.9; 4 MiB 23.2 -> 25.2, 21.5 -> 16.6,
     // 20.4 -> 13.8; 8 MiB reduce-scatter 28.2 -> 23.7, all-gather 23.2 -> 24.3. The two flag rounds of the other
     // kernels cost 10-15 us whatever the size; flagged packets cost half the link rate instead.
-    static const long long ar_max = envInt({"HYLINK_LL_AR_MAX"}, 2LL << 20), rs_max = envInt({"HYLINK_LL_RS_MAX"}, 8LL << 20),
-                           ag_max = envInt({"HYLINK_LL_AG_MAX"}, 4LL << 20), a2a_max = envInt({"HYLINK_LL_A2A_MAX"}, 4LL << 20);
-    const long long lim = coll == 0 ? ar_max : (coll == 1 ? rs_max : (coll == 2 ? ag_max : a2a_max));
+    static const long long asked_max[5] = {envInt({"HYLINK_LL_AR_MAX"}, -1), envInt({"HYLINK_LL_RS_MAX"}, -1), envInt({"HYLINK_LL_AG_MAX"}, -1),
+                                           envInt({"HYLINK_LL_A2A_MAX"}, -1), envInt({"HYLINK_LL_BC_MAX"}, -1)};
+    static const long long link_max[5] = {2LL << 20, 8LL << 20, 4LL << 20, 4LL << 20, 0};
+    // Ranks of one GPU: what counts is the L2 traffic of all ranks together, which flags in the data double, and a barrier
+    // is cheap. Measured, bf16, us this kernel / the staged one, 8 ranks: all-reduce 1 MiB 16.5 / 21.6, 1.5 MiB 22.9 /
+    // 24.0, 2 MiB 31.0 / 24.7; reduce-scatter 1.5 MiB 12.9 / 14.4, 2 MiB 16.6 / 14.5, 4 MiB 38 / 18; all-gather 2 MiB
+    // 16.1 / 16.5, 3 MiB 23.1 / 18.6; all-to-all 1.5 MiB 14.7 / 18.5, 2 MiB 19.0 / 18.5 (the lines of 2 and 4 ranks cross
+    // at the same sizes); broadcast, whose every byte is stored n - 1 times, 2 ranks 512 KiB 6.3 / 8.4, 1 MiB 8.4 / 8.4,
+    // 4 ranks 256 KiB 6.3 / 8.4, 512 KiB 8.4 / 8.4, 8 ranks 64 KiB 6.3 / 8.4, 256 KiB 10.3 / 8.4.
+    static const long long near_max[5] = {3LL << 19, 3LL << 19, 2LL << 20, 3LL << 19, 1LL << 20};
+    const long long own = emu_ ? (coll == 4 ? near_max[4] / nranks_ : near_max[coll]) : link_max[coll];
+    const long long lim = asked_max[coll] >= 0 ? asked_max[coll] : own;
+    if (emu_ && asked_max[coll] < 0 && (long long)wire_bytes <= lim && wire_bytes > (512u << 10) && coll < 3) {
+      // registered buffers take the zero-copy kernel from half a MiB on (us this kernel / that one, 8 ranks, 512 KiB and
+      // 1 MiB: all-reduce 10.4 / 12.4, 16.5 / 12.4; reduce-scatter 7.0 / 10.3, 10.4 / 10.3; all-gather 6.3 / 10.4, 10.4 / 10.4)
+      uint64_t io, oo;
+      const uint64_t reach_in = coll == 1 ? (c.in_seg_stride ? c.in_seg_stride : c.count) * (uint64_t)(nranks_ - 1) + c.count : c.count;
+      const uint64_t reach_out = coll == 2 ? (c.out_seg_stride ? c.out_seg_stride : c.count) * (uint64_t)(nranks_ - 1) + c.count : c.count;
+      if (zeroCopyFlavour(c, coll, wire_bytes) && zeroCopyEligible(b, c, coll != 2, coll != 1, reach_in, reach_out, &io, &oo)) return 0;
+    }
     if ((long long)wire_bytes > lim) return 0;
   }
   if (c.in_dt != c.wire_dt || c.out_dt != c.wire_dt) return no;
@@ -628,9 +657,11 @@ int NvlPath::lowLatencyChoice(const NvlBufs& b, const NvlCall& c, int coll, size
   for (int i = 0; i < localRanks(); ++i) {
     const char* in = (const char*)b.in[i];
     const char* out = (const char*)b.out[i];
-    if (!in || !out) return no;
+    if ((!in && (coll != 4 || i == c.root)) || !out) return no;
     // in place only where every location is read by the thread that later overwrites it
-    if (coll == 0) {
+    if (coll == 4) {
+      if (i == c.root && in != out && !disjoint(in, c.count * ws, out, c.count * ws)) return no;
+    } else if (coll == 0) {
       if (in != out && !disjoint(in, c.count * ws, out, c.count * ws)) return no;
     } else if (coll == 1) {
       const size_t in_bytes = ((n - 1) * istride + c.count) * ws;
@@ -656,6 +687,7 @@ hlResult_t NvlPath::launchLowLatency(int kind, const NvlBufs& b, const NvlCall& 
   const int nl = localRanks();
   HlEmuCalls calls;
   memset(&calls, 0, sizeof(calls));
+  fillEntry(&calls);
   for (int i = 0; i < nl; ++i) {
     HlCallArgs& a = calls.c[i];
     a.in = b.in[i];
@@ -667,6 +699,7 @@ hlResult_t NvlPath::launchLowLatency(int kind, const NvlBufs& b, const NvlCall& 
     a.op = c.op;
     a.in_dt = c.in_dt;
     a.out_dt = c.out_dt;
+    a.root = c.root;
     a.int_div = (c.op == hlAvg) ? nranks_ : 0;
     a.kind = kind;
   }
@@ -794,6 +827,8 @@ hlResult_t NvlPath::allGather(const NvlBufs& b, const NvlCall& c, cudaStream_t s
 hlResult_t NvlPath::broadcast(const NvlBufs& b, const NvlCall& c, cudaStream_t s) {
   if (c.count == 0) return hlSuccess;
   if (c.root < 0 || c.root >= nranks_) return fail(hlInvalidArgument, "broadcast root %d out of range", c.root);
+  const size_t wire_bytes = c.count * hlTypeSize((hlDataType_t)c.wire_dt);
+  if (lowLatencyChoice(b, c, 4, wire_bytes) > 0) return launchLowLatency(kNvlLlBroadcast, b, c, (wire_bytes + 15) / 16, s);
   {
     uint64_t io, oo;
     const int zc = nranks_ > 1 ? zeroCopyFlavour(c, 2, 0) : 0;
@@ -829,3 +864,4 @@ hlResult_t NvlPath::barrier(cudaStream_t s) {
 }
 
 }  // namespace hl
+  fillEntry(&calls);

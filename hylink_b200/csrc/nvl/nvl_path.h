@@ -103,6 +103,7 @@ class NvlPath {
   // Zero-copy kernels: which buffers peers reach in place (and therefore have to be registered, aligned and whole packets).
   bool zeroCopyEligible(const NvlBufs& b, const NvlCall& c, bool in_remote, bool out_remote, uint64_t in_extent, uint64_t out_extent,
                         uint64_t* in_off, uint64_t* out_off) const;
+  void fillEntry(HlEmuCalls* calls) const;
   hlResult_t launchZeroCopy(int kind, const NvlBufs& b, const NvlCall& c, uint64_t in_off, uint64_t out_off, size_t bytes_per_rank,
                             cudaStream_t s);
   int zeroCopyFlavour(const NvlCall& c, int coll, size_t wire_bytes) const;

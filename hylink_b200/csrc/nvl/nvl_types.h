@@ -79,6 +79,11 @@ struct HlCallArgs {
   int lane_parts;           // lane kernels (reduce-scatter, all-gather): HBM-side CTAs per pusher CTA (1..7)
   uint64_t zc_in_off;       // zero-copy kernels: heap offset of `in` (valid when the kernel reads `in` from peers)
   uint64_t zc_out_off;      // zero-copy kernels: heap offset of `out` (valid when the kernel writes peers' `out`)
+  // Of the rank's HlCommDev, so that the first loads of a kernel need not wait for the table (about 0.3 us).
+  uint32_t* abort_word;
+  uint64_t* seq_words;
+  int rank;
+  int nranks;
 };
 
 // One argument block per emulated rank: on a single GPU the N ranks of a test
@@ -128,4 +133,5 @@ enum HlNvlKernel {
   kNvlStreamAllGather = 33,
   kNvlStreamAllToAll = 34,
 };
+  kNvlLlBroadcast = 35,
 #define HL_DEV_ASYMMETRIC 4   // zero-copy call whose buffers do not sit at the same heap offset on every rank

@@ -26,7 +26,8 @@ KINDS = {0: "barrier", 1: "allreduce_oneshot", 2: "allreduce_twoshot", 3: "allre
          22: "zerocopy_reducescatter_p2p", 23: "zerocopy_allgather_nvls", 24: "zerocopy_allgather_p2p",
          25: "zerocopy_broadcast_nvls", 26: "zerocopy_broadcast_p2p",
          27: "lowlatency_allreduce", 28: "lowlatency_reducescatter", 29: "lowlatency_allgather", 30: "lowlatency_alltoall",
-         31: "alltoall_push", 32: "reducescatter_streamed", 33: "allgather_streamed", 34: "alltoall_streamed"}
+         31: "alltoall_push", 32: "reducescatter_streamed", 33: "allgather_streamed", 34: "alltoall_streamed",
+         35: "lowlatency_broadcast"}
 PHASE_NAMES = ["entry", "arrive1", "leave1", "arrive2", "leave2", "arrive3", "leave3", "exit"]
 
 

@@ -228,3 +228,32 @@ def test_missing_rank_runs_into_the_bounded_wait():
     torch.cuda.synchronize()
     assert torch.equal(outs[0], _ordered_sum(ins, torch.float32))
     g.close()
+
+
+# the root's first packet doubles as the sign that a rank has started: one packet, a ragged end, several sweeps of the grid
+@pytest.mark.parametrize("n,count,offset", [(2, 1, 0), (3, 7, 1), (4, 8 * 4099 + 3, 0), (8, 65536, 0), (8, 1000, 3)])
+def test_broadcast(n, count, offset, monkeypatch):
+    monkeypatch.setenv("HYLINK_KERNEL_TIMELINE", "1")
+    g = _group(n, stage_bytes=1 << 20)
+    pad = 8
+    for rep in range(3 * n):                             # roots in turn, each call on the heels of the one before
+        root = rep % n
+        ins = _inputs(n, offset + count, torch.bfloat16, rep)
+        want = ins[root][offset:].clone()
+        outs = [torch.full((offset + count + pad,), 7, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+        bufs = [o[offset:offset + count] for o in outs]
+        if rep % 3 == 1:                                 # in place
+            outs[root][offset:offset + count] = want
+            srcs = bufs
+        else:
+            srcs = [t[offset:] for t in ins]
+        gathered = [torch.empty(n, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+        g.run("broadcast", srcs, bufs, count, root=root)
+        g.run("all_gather", [b[:1] for b in bufs], gathered, 1)
+        g.run("broadcast", gathered, gathered, n, root=(root + 1) % n)
+        for o, e in zip(outs, gathered):
+            assert torch.equal(o[offset:offset + count], want) and bool((o[offset + count:] == 7).all())
+            assert bool((e == want[0]).all())
+    assert g.status(0)[0] == 0
+    assert {launch["kind"] for launch in g.kernel_timeline()} == {"lowlatency_allgather", "lowlatency_broadcast"}
+    g.close()
