@@ -832,8 +832,14 @@ hlResult_t NvlPath::broadcast(const NvlBufs& b, const NvlCall& c, cudaStream_t s
   {
     uint64_t io, oo;
     const int zc = nranks_ > 1 ? zeroCopyFlavour(c, 2, 0) : 0;
-    if (zc && zeroCopyEligible(b, c, false, true, c.count, c.count, &io, &oo))
-      return launchZeroCopy(zc == 1 ? kNvlZcBroadcastNvls : kNvlZcBroadcastP2p, b, c, 0, oo, c.count * hlTypeSize((hlDataType_t)c.wire_dt), s);
+    if (zc && zeroCopyEligible(b, c, false, true, c.count, c.count, &io, &oo)) {
+      // Ranks of one GPU share the stores where the root's input lies in its heap: each takes a slice of it. (Between
+      // GPUs the others do not know where the root's input is.)
+      io = HL_ZC_NOT_SHARED;
+      if (emu_ && !heapOffset(c.root, b.in[c.root], wire_bytes, &io)) io = HL_ZC_NOT_SHARED;
+      const bool shared = io != HL_ZC_NOT_SHARED;
+      return launchZeroCopy(zc == 1 ? kNvlZcBroadcastNvls : kNvlZcBroadcastP2p, b, c, io, oo, shared ? wire_bytes / (size_t)nranks_ : wire_bytes, s);
+    }
     if (wantsZeroCopy(c.algo)) return fail(hlUnsupported, "broadcast: zero-copy needs a registered, 16-byte aligned buffer of whole 16-byte packets");
   }
   const bool nvls = has_mc_ && c.algo != hlAlgoTwoShotP2p && c.algo != hlAlgoOneShot;
@@ -859,9 +865,9 @@ hlResult_t NvlPath::barrier(cudaStream_t s) {
   HL_CHECK(orderAfterPrevious(s));
   HlEmuCalls calls;
   memset(&calls, 0, sizeof(calls));
+  fillEntry(&calls);
   ++launches_;
   return nvl::launch(kNvlBarrier, hlFloat32, dcomm_, calls, emu_ ? emu_active_ : 1, 1, s);
 }
 
 }  // namespace hl
-  fillEntry(&calls);

@@ -85,6 +85,7 @@ struct HlCallArgs {
   int rank;
   int nranks;
 };
+#define HL_ZC_NOT_SHARED (~0ull)   // zc_in_off of a broadcast whose input only the root can read
 
 // One argument block per emulated rank: on a single GPU the N ranks of a test
 // run as ONE cooperative launch with gridDim.y == N (kernels that wait on one
@@ -132,6 +133,6 @@ enum HlNvlKernel {
   kNvlStreamReduceScatter = 32,
   kNvlStreamAllGather = 33,
   kNvlStreamAllToAll = 34,
-};
   kNvlLlBroadcast = 35,
+};
 #define HL_DEV_ASYMMETRIC 4   // zero-copy call whose buffers do not sit at the same heap offset on every rank

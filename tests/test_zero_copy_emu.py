@@ -166,3 +166,26 @@ def test_heap_allocator_reuses_and_merges():
     d = g.alloc_registered(1 << 20)             # both holes merged with the rest
     assert d[0].data_ptr() == pa
     g.close()
+
+
+# slices of the root's input: fewer packets than ranks, a last slice that is short or empty, an input outside the heap
+@pytest.mark.parametrize("n,packets,root,registered", [(8, 3, 5, True), (4, 4097, 3, True), (3, 100001, 1, True), (8, 33, 2, False)])
+def test_broadcast_shared_by_the_ranks(n, packets, root, registered):
+    from hylink_b200.ops import EmuGroup
+
+    g = EmuGroup(n, stage_bytes=1 << 20)
+    count = packets * 8
+    ins = g.alloc_registered(count, torch.bfloat16) if registered else [torch.empty(count, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+    outs = g.alloc_registered(count + 8, torch.bfloat16)
+    for r in range(n):
+        ins[r].copy_(torch.randn(count, device="cuda"))
+        outs[r].fill_(7)
+    want = ins[root].clone()
+    g.run("broadcast", ins, [o[:count] for o in outs], count, root=root, algo="zerocopy_p2p")
+    for o in outs:
+        assert torch.equal(o[:count], want) and bool((o[count:] == 7).all())
+    g.run("broadcast", outs, outs, count, root=root, algo="zerocopy_p2p")     # in place
+    assert all(torch.equal(o[:count], want) for o in outs)
+    assert g.status(0)[0] == 0
+    del ins, outs
+    g.close()
