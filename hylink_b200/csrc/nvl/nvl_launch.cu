@@ -35,7 +35,7 @@ static const void* pick(int kind, int nranks) {
 const void* kernelFor(int kind, int wire_dt, int nranks) {
   if (kind == kNvlBarrier) return (const void*)dev::kBarrier;
   if (kind == kNvlLlAllReduce || kind == kNvlLlReduceScatter || kind == kNvlLlAllGather || kind == kNvlLlAllToAll ||
-      kind == kNvlLlBroadcast)
+      kind == kNvlLlBroadcast || kind == kNvlLlAllReduceOneHop)
     return lowLatencyKernelFor(kind, wire_dt);
   switch (wire_dt) {
     case hlInt8: return pick<int8_t>(kind, nranks);
@@ -85,6 +85,7 @@ const char* kernelName(int kind) {
     case kNvlLlReduceScatter: return "reducescatter_lowlatency";
     case kNvlLlAllGather: return "allgather_lowlatency";
     case kNvlLlAllToAll: return "alltoall_lowlatency";
+    case kNvlLlAllReduceOneHop: return "allreduce_lowlatency_onehop";
     case kNvlLlBroadcast: return "broadcast_lowlatency";
     case kNvlAllToAllPush: return "alltoall_push";
     case kNvlStreamReduceScatter: return "reducescatter_streamed";
@@ -137,7 +138,7 @@ hlResult_t prepareKernels() {
                               kNvlReduceScatterPush, kNvlAllGatherPush, kNvlAllGatherLanes, kNvlZcAllReduceNvls,
                               kNvlZcAllReduceP2p, kNvlZcReduceScatterNvls, kNvlZcReduceScatterP2p, kNvlZcAllGatherNvls,
                               kNvlZcAllGatherP2p, kNvlZcBroadcastNvls, kNvlZcBroadcastP2p, kNvlLlAllReduce,
-                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlLlBroadcast, kNvlAllToAllPush,
+                              kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlLlBroadcast, kNvlLlAllReduceOneHop, kNvlAllToAllPush,
                               kNvlStreamReduceScatter, kNvlStreamAllGather, kNvlStreamAllToAll};
   for (int k : kinds)
     for (int dt = 0; dt < hlNumTypes; ++dt) {

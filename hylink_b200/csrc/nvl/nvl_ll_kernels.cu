@@ -23,6 +23,7 @@
 // all-gather:      send own segment to every peer | receive the others' segments into the output
 // reduce-scatter:  send segment q to rank q       | receive n-1 contributions, add in rank order, store
 // all-reduce:      reduce-scatter of the n shards (phase 0), then all-gather of the reduced shards (phase 1)
+//   in one hop:    all-gather of the whole buffers, added by everybody (the sum order is the same)
 // broadcast:       the root sends its buffer to every peer; the others send packet 0 alone, as the sign that they have
 //                  started, and everybody waits for all of these (the argument above needs it)
 //
@@ -49,7 +50,7 @@
 namespace hl {
 namespace dev {
 
-constexpr int kLlAllReduce = 0, kLlReduceScatter = 1, kLlAllGather = 2, kLlAllToAll = 3, kLlBroadcast = 4;
+constexpr int kLlAllReduce = 0, kLlReduceScatter = 1, kLlAllGather = 2, kLlAllToAll = 3, kLlBroadcast = 4, kLlAllReduceOneHop = 5;
 
 __device__ __forceinline__ uint8_t* llSlot(const HlCommDev& c, int owner, int parity, int phase, int src) {
   return c.ll[owner] + ((size_t)((parity * 2 + phase) * HL_MAX_RANKS + src)) * c.ll_slot_bytes;
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* co
   uint4 v[MR];   // indexed by compile-time constants only: stays in registers
   // what this rank has of column j
   auto column = [&](uint64_t j) {
-    if constexpr (kColl == kLlAllGather) {
+    if constexpr (kColl == kLlAllGather || kColl == kLlAllReduceOneHop) {
       v[0] = ld(in, j);
     } else if constexpr (kColl == kLlBroadcast) {
       v[0] = r == a.root ? ld(in, j) : make_uint4(0u, 0u, 0u, 0u);
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* co
 #pragma unroll
     for (int q = 0; q < MR; ++q)
       if (peers >> q & 1u) {
-        if constexpr (kColl == kLlAllGather) llSend(to[q], j, v[0], tag);
+        if constexpr (kColl == kLlAllGather || kColl == kLlAllReduceOneHop) llSend(to[q], j, v[0], tag);
         else if constexpr (kColl == kLlBroadcast) {
           if (r == a.root || j == 0) llSend(to[q], j, v[0], tag);
         } else if constexpr (kColl == kLlAllReduce) {
@@ -252,9 +253,9 @@ __global__ void __launch_bounds__(HL_LL_THREADS) kLowLatency(const HlCommDev* co
       for (int q = 0; q < MR; ++q)
         if (root >> q & 1u) st(out, j, v[q]);
     }
-  } else if constexpr (kColl == kLlReduceScatter) {
+  } else if constexpr (kColl == kLlReduceScatter || kColl == kLlAllReduceOneHop) {
     for (uint64_t j = g0; j < end; j += gstride) {
-      const uint4 own = ld(in + (uint64_t)r * a.in_seg_stride, j);
+      const uint4 own = ld(kColl == kLlReduceScatter ? in + (uint64_t)r * a.in_seg_stride : in, j);
       if (!llRecv(c, from, j, tag, peers, w, v)) break;
 #pragma unroll
       for (int q = 0; q < MR; ++q)
@@ -304,6 +305,7 @@ static const void* pickLl(int kind) {
     case kNvlLlAllGather: return (const void*)kLowLatency<W, kLlAllGather>;
     case kNvlLlAllToAll: return (const void*)kLowLatency<W, kLlAllToAll>;
     case kNvlLlBroadcast: return (const void*)kLowLatency<W, kLlBroadcast>;
+    case kNvlLlAllReduceOneHop: return (const void*)kLowLatency<W, kLlAllReduceOneHop>;
     default: return nullptr;
   }
 }

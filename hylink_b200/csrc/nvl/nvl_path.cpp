@@ -706,11 +706,13 @@ hlResult_t NvlPath::launchLowLatency(int kind, const NvlBufs& b, const NvlCall& 
   // one thread per packet it sends to (and receives from) every peer; at most one CTA per SM, so that the CTAs
   // with the same index are resident on every rank at the same time (they wait for one another's packets). Small
   // messages spread over more and smaller CTAs: a packet is 2 (n - 1) stores and as many polls of its thread, and an
-  // SM issues them one after the other.
+  // SM issues them one after the other; but every CTA costs its start. (8 ranks, 8 KiB, us with CTAs of 32 / 64 / 128 /
+  // 256 threads: all-reduce in two hops 8.2 / 6.9 / 6.2 / 6.5; 64 KiB 8.2 / 8.2 / 8.2 / 9.5; 2 ranks, 8 KiB
+  // reduce-scatter 5.0 / 4.1 / 4.1.)
   int cap = c.max_blocks > 0 ? std::min(c.max_blocks, 148) : 148;
   if (Config::get().nvl_max_blocks > 0) cap = std::min(cap, Config::get().nvl_max_blocks);
   if (emu_) cap = std::min(cap, std::max(1, 148 / nranks_));
-  int threads = 64;
+  int threads = 128;
   while (threads < HL_LL_THREADS && packets > (uint64_t)cap * threads) threads *= 2;
   const uint64_t want = std::max<uint64_t>(1, (packets + threads - 1) / threads);
   const int blocks = (int)std::min<uint64_t>(want, (uint64_t)cap);
@@ -729,6 +731,12 @@ hlResult_t NvlPath::allReduce(const NvlBufs& b, const NvlCall& c, cudaStream_t s
     if (ll < 0) return fail(hlUnsupported, "all-reduce: the low-latency kernel converts no types and needs a message that fits its slots");
     if (ll > 0) {
       const uint64_t np = (wire_bytes + 15) / 16;
+      // One hop instead of two while what each rank sends, n - 1 times the buffer instead of less than twice, costs less
+      // than the second hop; between two ranks it is no more, and one hop is always the better. Ranks of one GPU, bf16,
+      // us one hop / two: 2 ranks 8 KiB 4.1 / 6.1, 512 KiB 6.1 / 7.7; 4 ranks 8 KiB 4.5 / 6.1, 128 KiB 6.1 / 8.2, 256
+      // KiB 8.2 / 8.2, 512 KiB 10.6 / 8.2; 8 ranks 2 KiB 5.6 / 6.1, 64 KiB 6.1 / 8.2, 96 KiB 8.3 / 8.2, 192 KiB 12.2 / 8.2.
+      if (emu_ && (nranks_ == 2 || wire_bytes * (size_t)nranks_ <= (512u << 10)) && ((np + 31) / 32) * 1024 <= ll_slot_bytes_)
+        return launchLowLatency(kNvlLlAllReduceOneHop, b, c, np, s);
       return launchLowLatency(kNvlLlAllReduce, b, c, (np + (uint64_t)nranks_ - 1) / (uint64_t)nranks_, s);
     }
   }

@@ -134,5 +134,6 @@ enum HlNvlKernel {
   kNvlStreamAllGather = 33,
   kNvlStreamAllToAll = 34,
   kNvlLlBroadcast = 35,
+  kNvlLlAllReduceOneHop = 36,
 };
 #define HL_DEV_ASYMMETRIC 4   // zero-copy call whose buffers do not sit at the same heap offset on every rank

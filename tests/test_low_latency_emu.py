@@ -257,3 +257,22 @@ def test_broadcast(n, count, offset, monkeypatch):
     assert g.status(0)[0] == 0
     assert {launch["kind"] for launch in g.kernel_timeline()} == {"lowlatency_allgather", "lowlatency_broadcast"}
     g.close()
+
+
+# both sides of the size up to which ranks of one GPU reduce in one hop, and counts that are no whole packets
+@pytest.mark.parametrize("n,count", [(8, 5), (8, 32 << 10), (8, (32 << 10) + 1), (3, 87381), (3, 87382), (2, (256 << 10) - 3)])
+def test_allreduce_hops(n, count, monkeypatch):
+    monkeypatch.setenv("HYLINK_KERNEL_TIMELINE", "1")
+    g = _group(n)
+    outs = [torch.full((count + 9,), 7, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+    for rep in range(4):
+        ins = _inputs(n, count, torch.bfloat16, rep)
+        want = _ordered_sum(ins, torch.bfloat16)
+        bufs = [o[rep:rep + count] for o in outs]        # from aligned to not aligned
+        g.run("all_reduce", ins, bufs, count)
+        for o, b in zip(outs, bufs):
+            assert torch.equal(b, want) and bool((o[rep + count:] == 7).all())
+        g.run("all_reduce", ins, ins, count)             # in place
+        assert all(torch.equal(t, want) for t in ins)
+    assert {launch["kind"] for launch in g.kernel_timeline()} == {"lowlatency_allreduce"}
+    g.close()
