@@ -26,7 +26,7 @@ const void* pickKernelT(int kind, int nranks);   // nvl_kernels_*.cu
 template <typename W>
 const void* pickStreamT(int kind, int nranks);   // nvl_stream_*.cu
 
-static bool streamed(int kind) { return kind == kNvlStreamReduceScatter || kind == kNvlStreamAllGather || kind == kNvlStreamAllToAll; }
+static bool streamed(int kind) { return kind == kNvlStreamReduceScatter || kind == kNvlStreamAllGather || kind == kNvlStreamAllToAll || kind == kNvlStreamBroadcast; }
 template <typename W>
 static const void* pick(int kind, int nranks) {
   return streamed(kind) ? pickStreamT<W>(kind, nranks) : pickKernelT<W>(kind, nranks);
@@ -91,6 +91,7 @@ const char* kernelName(int kind) {
     case kNvlStreamReduceScatter: return "reducescatter_streamed";
     case kNvlStreamAllGather: return "allgather_streamed";
     case kNvlStreamAllToAll: return "alltoall_streamed";
+    case kNvlStreamBroadcast: return "broadcast_streamed";
     default: return "?";
   }
 }
@@ -139,7 +140,7 @@ hlResult_t prepareKernels() {
                               kNvlZcAllReduceP2p, kNvlZcReduceScatterNvls, kNvlZcReduceScatterP2p, kNvlZcAllGatherNvls,
                               kNvlZcAllGatherP2p, kNvlZcBroadcastNvls, kNvlZcBroadcastP2p, kNvlLlAllReduce,
                               kNvlLlReduceScatter, kNvlLlAllGather, kNvlLlAllToAll, kNvlLlBroadcast, kNvlLlAllReduceOneHop, kNvlAllToAllPush,
-                              kNvlStreamReduceScatter, kNvlStreamAllGather, kNvlStreamAllToAll};
+                              kNvlStreamReduceScatter, kNvlStreamAllGather, kNvlStreamAllToAll, kNvlStreamBroadcast};
   for (int k : kinds)
     for (int dt = 0; dt < hlNumTypes; ++dt) {
       for (int nr : {2, 4, HL_MAX_RANKS}) {   // rank-count classes (only the pipelined push kernels differ by it)

@@ -487,18 +487,30 @@ int NvlPath::blocksFor(int kind, size_t wire_bytes_per_rank, int max_blocks) con
 // 64 MB 33.2 / 33.0, 33.4 / 34.8; 128 MB 55.5 / 62.5, 57.7 / 67.2. 2 ranks: 64 MB 31.5 / 30.8, 31.6 / 31.6; 128 MB
 // 51.9 / 58.1, 53.9 / 61.0. 8 ranks: 64 MB all-gather 37.2 / 36.6, 128 MB 62.3 / 69.0, all-to-all 76.8 / 85.1; the fold
 // of eight sources leaves the workers of a reduce-scatter too few registers: 74.8 / 67.0, so it stays plain.
-int NvlPath::streamedKind(int kind, const HlEmuCalls& calls, uint64_t sp, size_t elem, int blocks) const {
+int NvlPath::streamedKind(int kind, const HlEmuCalls& calls, uint64_t sp, int wire_dt, int blocks) const {
+  const size_t elem = hlTypeSize((hlDataType_t)wire_dt);
   if (!emu_ || nranks_ < 2) return kind;
   int to;
   switch (kind) {
     case kNvlReduceScatterPush: to = kNvlStreamReduceScatter; break;
     case kNvlAllGatherPush: to = kNvlStreamAllGather; break;
     case kNvlAllToAllPush: to = kNvlStreamAllToAll; break;
+    case kNvlBroadcast: to = kNvlStreamBroadcast; break;
     default: return kind;
   }
-  if (to == kNvlStreamReduceScatter && nranks_ > 4) return kind;
   const uint64_t n = (uint64_t)nranks_;
   constexpr uint64_t kStaysInL2 = 64ull << 20;
+  if (to == kNvlStreamBroadcast) {
+    // us streamed / plain: 2 ranks 16 MB 20.5 / 18.6, 32 MB 33.9 / 40.6; 4 ranks 12 MB 26.8 / 25.7, 16 MB 31.0 / 33.8;
+    // 8 ranks 8 MB 30.8 / 31.1, 64 MB 175 / 249
+    if ((n + 1) * sp * 16 <= kStaysInL2) return kind;
+    for (int i = 0; i < nranks_; ++i) {
+      const HlCallArgs& a = calls.c[i];
+      if (a.in_dt != wire_dt || a.out_dt != wire_dt || ((uintptr_t)a.out & 15) || (i == a.root && ((uintptr_t)a.in & 15))) return kind;
+    }
+    return (uint64_t)blocks * 2 * HL_STREAM_LAG * HL_STREAM_WORKERS * 8 * 16 <= stage_bytes_ ? to : kind;
+  }
+  if (to == kNvlStreamReduceScatter && nranks_ > 4) return kind;
   if (n * n * sp * 16 <= kStaysInL2) return kind;
   for (int i = 0; i < nranks_; ++i) {
     const HlCallArgs& a = calls.c[i];
@@ -589,7 +601,7 @@ hlResult_t NvlPath::launchSliced(int kind, const NvlBufs& b, const NvlCall& c, b
     }
     int run = kind;
     if (emu_) {
-      run = streamedKind(kind, calls, (len + epp - 1) / epp, ws, blocks);
+      run = streamedKind(kind, calls, (len + epp - 1) / epp, c.wire_dt, blocks);
       for (int i = 0; i < nl; ++i) calls.c[i].kind = run;
     }
     const int rows = emu_ ? emu_active_ : 1;

@@ -91,7 +91,7 @@ class NvlPath {
   size_t agLanesMinBytes() const;
   size_t lanesMinBytes() const;   // peer-pointer reduce-scatter: from this size on the lane kernel
   bool nvlsUsable(int wire_dt, int op, bool deterministic) const;
-  int streamedKind(int kind, const HlEmuCalls& calls, uint64_t part_packets, size_t element_bytes, int blocks) const;
+  int streamedKind(int kind, const HlEmuCalls& calls, uint64_t part_packets, int wire_dt, int blocks) const;
   int blocksFor(int kind, size_t wire_bytes_per_rank, int max_blocks) const;
 
  private:

@@ -1,4 +1,4 @@
-// Streamed push kernels: large reduce-scatter, all-gather and all-to-all between ranks of ONE GPU.
+// Streamed kernels: large reduce-scatter, all-gather, all-to-all and broadcast between ranks of ONE GPU.
 //
 // Between GPUs the link is the bound and staging traffic hides behind it. Between ranks of one GPU the staging IS the
 // traffic: a message through slots of its own size moves about 2.2 times the bytes that the caller's buffers hold, all
@@ -16,6 +16,9 @@
 // with 3, 102 with 4, whose ring is too large; with the plain kernel 119).
 // An all-reduce has a second ring (results) and twice the lag, which no longer fits: 230 us against 125. It stays with
 // the plain kernel.
+// Broadcast: the root puts piece t into its own ring and into its output, the others copy piece t - L out of the root's
+// ring. (With the whole message staged first, the others wait for the root's CTAs, an n-th of the GPU: 64 MiB
+// to 8 ranks 249 us, streamed 175; to 4 ranks 132 and 94. The root's CTAs are the bound: they read once and store twice.)
 // Flags are the tile words of the pipelined kernels: [kind 1][CTA][source rank] <- tile base + finished iterations.
 //
 // Roles: worker warps move data; a poller warp watches the peers' flags and opens iterations; a signaller warp waits
@@ -36,7 +39,7 @@
 namespace hl {
 namespace dev {
 
-enum StreamColl { kStreamReduceScatter = 0, kStreamAllGather = 1, kStreamAllToAll = 2 };
+enum StreamColl { kStreamReduceScatter = 0, kStreamAllGather = 1, kStreamAllToAll = 2, kStreamBroadcast = 3 };
 constexpr int kLag = HL_STREAM_LAG, kStreamRing = 2 * kLag;
 constexpr int kWorkWarps = HL_STREAM_WORKERS / 32;
 
@@ -75,7 +78,8 @@ template <typename W, int kColl, int MR>
 __global__ void __launch_bounds__(HL_STREAM_WORKERS + 64, 1) kStream(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
-  constexpr bool kRs = kColl == kStreamReduceScatter, kAg = kColl == kStreamAllGather;
+  constexpr bool kRs = kColl == kStreamReduceScatter, kBc = kColl == kStreamBroadcast;
+  constexpr bool kAg = kColl == kStreamAllGather || kBc;       // one input, not one per peer
   constexpr int N = Packet<W>::N, V = 8 / MR;         // packets of every segment per thread: eight loads in flight
   constexpr uint32_t P = HL_STREAM_WORKERS * V, kStep = HL_STREAM_WORKERS;
   const int n = c.nranks, r = c.rank;
@@ -99,9 +103,9 @@ __global__ void __launch_bounds__(HL_STREAM_WORKERS + 64, 1) kStream(const HlCom
   auto parity = [](int t) { return (uint32_t)(t / kStreamRing) & 1u; };
   const uint64_t limit = 2 * c.timeout_ns + 1000000000ull;      // inside a CTA: the poller gives up first
 
-  const Parts<W> in(a.in, kAg ? 0 : a.in_seg_stride, a.count, 0), out(a.out, kRs ? 0 : a.out_seg_stride, a.count, 0);
+  const Parts<W> in(a.in, kAg ? 0 : a.in_seg_stride, a.count, 0), out(a.out, kRs || kBc ? 0 : a.out_seg_stride, a.count, 0);
   const uint64_t c0 = (uint64_t)blockIdx.x * chunk, c1 = c0 + chunk < sp ? c0 + chunk : sp;
-  const uint64_t ring0 = (uint64_t)blockIdx.x * kStreamRing * n * P;                      // this CTA's ring in a rank's staging
+  const uint64_t ring0 = (uint64_t)blockIdx.x * kStreamRing * (kBc ? 1 : n) * P;                      // this CTA's ring in a rank's staging
   const uint64_t whole = a.count / N, v1 = c1 < whole ? c1 : whole;                       // vector copies end here
   // packets of piece t: how many are full
   auto first = [&](int t) { return c0 + (uint64_t)t * P; };
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(HL_STREAM_WORKERS + 64, 1) kStream(const HlCom
   // the ragged packet of piece t, if it has one: [ragged0, ragged1)
   auto ragged0 = [&](int t) { return first(t) + full(t); };
   auto ragged1 = [&](int t) { return first(t) + P < c1 ? first(t) + P : c1; };
-  const bool own = in.at(kAg ? 0 : r) != out.at(kRs ? 0 : r);
+  const bool own = in.at(kAg ? 0 : r) != out.at(kRs || kBc ? 0 : r);
 
   if (warp == 0) {                                    // ---- poller
     int gave_up = 0;
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(HL_STREAM_WORKERS + 64, 1) kStream(const HlCom
     constexpr int kNext = kAg ? 1 : MR;
     uint4 next[V][kNext];                             // the caller's data of the piece to push
     auto fetch = [&](int t) {
-      if (t >= T) return;
+      if (t >= T || (kBc && r != a.root)) return;
       const uint32_t cnt = full(t);
       if constexpr (kAg) {
         const uint4* src = reinterpret_cast<const uint4*>(in.at(0)) + first(t);
@@ -184,9 +188,47 @@ __global__ void __launch_bounds__(HL_STREAM_WORKERS + 64, 1) kStream(const HlCom
           }
       }
     };
+    const uint4* ring = kBc ? reinterpret_cast<const uint4*>(c.stage[a.root]) + ring0 : nullptr;
     fetch(0);
     for (int t = 0; t < I; ++t) {
       if (!mbWait(&s_open[t % kStreamRing], parity(t), &s_stop, t, limit)) break;
+      if (kBc) {
+        if (r == a.root && t < T) {                   // piece t into the ring and the output
+          const uint32_t cnt = full(t);
+          uint4* slot = reinterpret_cast<uint4*>(c.stage[r]) + ring0 + (uint64_t)(t % kStreamRing) * P;
+          uint4* dst = reinterpret_cast<uint4*>(out.at(0)) + first(t);
+#pragma unroll
+          for (int u = 0; u < V; ++u)
+            if (tid + u * kStep < cnt) slot[tid + u * kStep] = next[u][0];
+          if (own) {
+#pragma unroll
+            for (int u = 0; u < V; ++u)
+              if (tid + u * kStep < cnt) __stcs(dst + tid + u * kStep, next[u][0]);
+          }
+          for (uint64_t j = ragged0(t) + tid; j < ragged1(t); j += kStep) {
+            const uint4 v = ragLoad(in, 0, j);
+            slot[j - first(t)] = v;
+            if (own) ragStore(out, 0, j, v);
+          }
+          fetch(t + 1);
+        } else if (r != a.root && t >= kLag) {        // piece t - L out of it
+          const int w = t - kLag;
+          const uint32_t cnt = full(w);
+          const uint4* landed = ring + (uint64_t)(w % kStreamRing) * P;
+          uint4* dst = reinterpret_cast<uint4*>(out.at(0)) + first(w);
+          uint4 v[V];
+#pragma unroll
+          for (int u = 0; u < V; ++u)
+            if (tid + u * kStep < cnt) v[u] = ldRing(landed + tid + u * kStep);
+#pragma unroll
+          for (int u = 0; u < V; ++u)
+            if (tid + u * kStep < cnt) __stcs(dst + tid + u * kStep, v[u]);
+          for (uint64_t j = ragged0(w) + tid; j < ragged1(w); j += kStep) ragStore(out, 0, j, ldRing(landed + (j - first(w))));
+        }
+        __syncwarp();
+        if (lane == 0) mbArrive(&s_done[t % kStreamRing]);
+        continue;
+      }
       if (t < T) {                                    // push piece t
         const uint64_t slot = ring0 + ((uint64_t)(t % kStreamRing) * n + r) * P;
         const uint32_t cnt = full(t);
@@ -294,6 +336,7 @@ const void* pickStreamT(int kind, int nranks) {
       return nranks <= 2 ? (const void*)kStream<W, kStreamReduceScatter, 2> : (nranks <= 4 ? (const void*)kStream<W, kStreamReduceScatter, 4> : nullptr);
     case kNvlStreamAllGather: return HL_STREAM_PICK(kStreamAllGather);
     case kNvlStreamAllToAll: return HL_STREAM_PICK(kStreamAllToAll);
+    case kNvlStreamBroadcast: return (const void*)kStream<W, kStreamBroadcast, 1>;
     default: return nullptr;
   }
 #undef HL_STREAM_PICK

@@ -135,5 +135,6 @@ enum HlNvlKernel {
   kNvlStreamAllToAll = 34,
   kNvlLlBroadcast = 35,
   kNvlLlAllReduceOneHop = 36,
+  kNvlStreamBroadcast = 37,
 };
 #define HL_DEV_ASYMMETRIC 4   // zero-copy call whose buffers do not sit at the same heap offset on every rank

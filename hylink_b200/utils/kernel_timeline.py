@@ -27,7 +27,7 @@ KINDS = {0: "barrier", 1: "allreduce_oneshot", 2: "allreduce_twoshot", 3: "allre
          25: "zerocopy_broadcast_nvls", 26: "zerocopy_broadcast_p2p",
          27: "lowlatency_allreduce", 28: "lowlatency_reducescatter", 29: "lowlatency_allgather", 30: "lowlatency_alltoall",
          31: "alltoall_push", 32: "reducescatter_streamed", 33: "allgather_streamed", 34: "alltoall_streamed",
-         35: "lowlatency_broadcast", 36: "lowlatency_allreduce"}
+         35: "lowlatency_broadcast", 36: "lowlatency_allreduce", 37: "broadcast_streamed"}
 PHASE_NAMES = ["entry", "arrive1", "leave1", "arrive2", "leave2", "arrive3", "leave3", "exit"]
 
 

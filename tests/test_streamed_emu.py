@@ -94,3 +94,27 @@ def test_streamed_wait_is_bounded():
     assert g.status(0)[0] == 0
     assert all(torch.equal(o, _sum([t[r * seg:(r + 1) * seg] for t in ins], torch.float32)) for r, o in enumerate(outs))
     g.close()
+
+
+# the smallest message that streams, ragged ends, a message of more than one launch, outputs that keep the plain kernel
+@pytest.mark.parametrize("n,count,dtype,offset", [(2, (12 << 20) - 3, torch.bfloat16, 0), (3, (4 << 20) + 9, torch.float32, 0),
+                                                  (8, (4 << 20) + 1, torch.bfloat16, 0), (4, (8 << 20) + 5, torch.bfloat16, 3),
+                                                  (2, (17 << 20) + 2, torch.int32, 0)])
+def test_streamed_broadcast(n, count, dtype, offset, monkeypatch):
+    from hylink_b200.ops import EmuGroup
+
+    monkeypatch.setenv("HYLINK_KERNEL_TIMELINE", "1")
+    g = EmuGroup(n)
+    outs = [torch.full((offset + count + 16,), 7, dtype=dtype, device="cuda") for _ in range(n)]
+    bufs = [o[offset:offset + count] for o in outs]
+    for rep in range(3):                              # back to back, from different roots, in place
+        root = (rep + 1) % n
+        data = _rand(count, dtype, rep)
+        srcs = [data if r == root else bufs[r] for r in range(n)]
+        if rep == 2:
+            bufs[root].copy_(data)
+            srcs = bufs
+        g.run("broadcast", srcs, bufs, count, root=root)
+        assert all(torch.equal(b, data) and bool((o[offset + count:] == 7).all()) for o, b in zip(outs, bufs))
+    assert ("broadcast_streamed" in {launch["kind"] for launch in g.kernel_timeline()}) == (offset == 0)
+    g.close()
