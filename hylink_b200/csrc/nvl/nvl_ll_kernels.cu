@@ -1,7 +1,7 @@
 // Low-latency kernels of the dedicated-link path for small messages: all-reduce, reduce-scatter, all-gather,
 // all-to-all and broadcast with NO cross-GPU barrier at all.
 //
-// The barrier-based kernels (nvl_kernels.cu) pay two flag round trips per call — about 3 to 8 microseconds each
+// The barrier-based kernels (nvl_kernels.cuh) pay two flag round trips per call — about 3 to 8 microseconds each
 // once the stores in front of them have to be acknowledged — which is most of the time of a message of a few MiB.
 // Here every 16-byte store carries its own arrival flag: 8 data bytes and two copies of a 32-bit call tag
 // ({d0, tag, d1, tag}, one st.volatile.v4, so each 8-byte half validates itself), written straight into the
