@@ -27,8 +27,9 @@ constexpr int kRlThreads = 256;
 // These kernels are often launched back to back, and a launch that waits for the one before it to drain costs 3 us and
 // more: 4.3 us from one small fold to the next, in steps of 2.05 however long the kernel is. So a launch may start while
 // its predecessor runs (it lets its own successor do the same at once) and waits here for the predecessor's end, before
-// it touches memory: 2.4 us then, which is the host's share, and 26.0 instead of 27.4 for the
-// fold of four times 32 MiB. All CTAs of the predecessor have started by then, so it never lacks room to finish.
+// it touches memory: 2.4 us then, which is the host's share, and 26.0 instead of 27.4 for the fold of four times 32 MiB.
+// All CTAs of the predecessor have started by then, so it never lacks room to finish. (A CTA must read through the
+// coherent path: what it needs is written while it is already resident.)
 __device__ __forceinline__ void afterPredecessor() {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
