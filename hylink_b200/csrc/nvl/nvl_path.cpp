@@ -638,11 +638,11 @@ int NvlPath::lowLatencyChoice(const NvlBufs& b, const NvlCall& c, int coll, size
     static const long long link_max[5] = {2LL << 20, 8LL << 20, 4LL << 20, 4LL << 20, 0};
     // Ranks of one GPU: what counts is the L2 traffic of all ranks together, which flags in the data double, and a barrier
     // is cheap. Measured, bf16, us this kernel / the staged one, 8 ranks: all-reduce 1 MiB 16.5 / 21.6, 1.5 MiB 22.9 /
-    // 24.0, 2 MiB 31.0 / 24.7; reduce-scatter 1.5 MiB 12.9 / 14.4, 2 MiB 16.6 / 14.5, 4 MiB 38 / 18; all-gather 2 MiB
-    // 16.1 / 16.5, 3 MiB 23.1 / 18.6; all-to-all 1.5 MiB 14.7 / 18.5, 2 MiB 19.0 / 18.5 (the lines of 2 and 4 ranks cross
-    // at the same sizes); broadcast, whose every byte is stored n - 1 times, 2 ranks 512 KiB 6.3 / 8.4, 1 MiB 8.4 / 8.4,
-    // 4 ranks 256 KiB 6.3 / 8.4, 512 KiB 8.4 / 8.4, 8 ranks 64 KiB 6.3 / 8.4, 256 KiB 10.3 / 8.4.
-    static const long long near_max[5] = {3LL << 19, 3LL << 19, 2LL << 20, 3LL << 19, 1LL << 20};
+    // 24.0, 2 MiB 31.0 / 24.7; reduce-scatter 1.5 MiB 12.9 / 14.4, 2 MiB 16.6 / 14.5, 4 MiB 38 / 18; all-gather 1.5 MiB
+    // 12.4 / 16.5, 2 MiB 16.1 / 16.5 (in odd segments 34.8 / 31.0); all-to-all 1.5 MiB 14.7 / 18.5, 2 MiB 19.0 / 18.5 (the
+    // lines of 2 and 4 ranks cross at the same sizes); broadcast, whose every byte is stored n - 1 times, 2 ranks 512 KiB
+    // 6.3 / 8.4, 1 MiB 8.4 / 8.4, 4 ranks 256 KiB 6.3 / 8.4, 512 KiB 8.4 / 8.4, 8 ranks 64 KiB 6.3 / 8.4, 256 KiB 10.3 / 8.4.
+    static const long long near_max[5] = {3LL << 19, 3LL << 19, 3LL << 19, 3LL << 19, 1LL << 20};
     const long long own = emu_ ? (coll == 4 ? near_max[4] / nranks_ : near_max[coll]) : link_max[coll];
     const long long lim = asked_max[coll] >= 0 ? asked_max[coll] : own;
     if (emu_ && asked_max[coll] < 0 && (long long)wire_bytes <= lim && wire_bytes > (512u << 10) && coll < 3) {
