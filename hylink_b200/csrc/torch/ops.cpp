@@ -217,33 +217,21 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
 // logits = h W^T and their mean cross entropy. The vocabulary is padded to a multiple of 64: an odd leading dimension
 // keeps cuBLAS off the tensor-memory kernels (8192 x 50257 x 1024 in bf16 on B200: 7.43 ms against 0.60 for the logits,
 // 4.71 against 0.55 for the weight gradient); padding the weight is a copy of 0.04 ms.
-// The input gradient sums over the vocabulary. Given the odd size cuBLAS takes a kernel that cuts the sum into parts and
-// carries it from part to part in 16 bits, as long as torch allows reduced-precision reductions, which is its default.
-// That shows: behind a token's target entry the tiny probabilities of the rest are lost, the same way for every token.
-// The number of parts is 5 from 192 tiles of 256 x 128 on (6144 rows of 1024, 8192 of 768), and 6 to 24 in no simple
-// order below. From there on the parts are computed here as products over the padded size on the fast kernels, into
-// fp32, and the carried sum is kept as it was, so that a training run goes on as it would have: 99.6 % of the elements
-// are the same bits. (In one pass, or in another number of parts, the gradients of a 24-layer model move by 2 to 3 % in
-// the second step, where the noise between two runs is 0.6 %.) 8192 x 50257 x 1024: 5.6 ms -> 0.7.
-// With reduced-precision reductions switched off the sum is one pass in fp32.
-constexpr int64_t kHeadParts = 5, kHeadPartTiles = 192;
+// The input gradient sums over the vocabulary. While torch allows reduced-precision reductions (its default) and the
+// vocabulary is no multiple of eight, that sum is the library's product over exactly the vocabulary, as the plain modules
+// call it: its rounding is part of what a training run with them gives. Switched off, or with an even vocabulary, it is
+// one pass over the padded operands (zero behind the vocabulary on both sides), summed in fp32 and rounded once.
+// 8192 x 50257 x 1024: 5.6 ms against 0.56. The padded pass everywhere would be nearer to fp32 (first-step gradients of
+// the 24-layer model 1.37e-2 from an fp32 model, 1.71e-2 with the plain modules), but from the second step on its
+// gradients are 3 % away from those of the plain modules, where two runs of these differ by 0.8 %.
 bool reducedPrecisionSums(at::ScalarType t) {
   const auto& ctx = at::globalContext();
   return (t == at::kBFloat16 ? ctx.allowBF16ReductionCuBLAS() : ctx.allowFP16ReductionCuBLAS()) == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK;
 }
 // d [rows][padded], zero behind `vocab`; w [padded][width].
 Tensor headInputGradient(const Tensor& d, const Tensor& w, int64_t vocab) {
-  const int64_t padded = d.size(1), tiles = (d.size(0) + 255) / 256 * ((w.size(1) + 127) / 128);
   if (vocab % 8 == 0 || !reducedPrecisionSums(d.scalar_type())) return at::mm(d, w);
-  if (tiles < kHeadPartTiles) return at::mm(d.narrow(1, 0, vocab), w.narrow(0, 0, vocab));
-  const int64_t part = ((vocab + kHeadParts - 1) / kHeadParts + 7) / 8 * 8;
-  Tensor out = at::mm(d.narrow(1, 0, std::min(part, padded)), w.narrow(0, 0, std::min(part, padded)));
-  for (int64_t at = part; at < vocab; at += part) {
-    const int64_t k = std::min(part, padded - at);
-    const Tensor sum = at::mm(d.narrow(1, at, k), w.narrow(0, at, k), at::kFloat);
-    ok(train::carrySum(code(out), sum.data_ptr<float>(), out.data_ptr(), out.numel(), streamOf(out)), "head gradient");
-  }
-  return out;
+  return at::mm(d.narrow(1, 0, vocab), w.narrow(0, 0, vocab));
 }
 
 class HeadLoss : public torch::autograd::Function<HeadLoss> {

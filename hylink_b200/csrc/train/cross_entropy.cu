@@ -138,25 +138,6 @@ __global__ void __launch_bounds__(kCeThreads) kCrossEntropyBackward(const T* __r
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) kCarrySum(const float4* __restrict__ part, uint4* __restrict__ out, int64_t packets) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= packets) return;
-  const float4 a = part[2 * i], b = part[2 * i + 1];
-  float f[8];
-  unpack8<T>(out[i], f);
-  f[0] += a.x, f[1] += a.y, f[2] += a.z, f[3] += a.w, f[4] += b.x, f[5] += b.y, f[6] += b.z, f[7] += b.w;
-  out[i] = pack8<T>(f);
-}
-
-hlResult_t carrySum(int dt, const float* part, void* out, int64_t count, cudaStream_t s) {
-  if (count % 8) return fail(hlInvalidArgument, "carried sum: %lld elements", (long long)count);
-  if (count == 0) return hlSuccess;
-  const int64_t packets = count / 8;
-  HL_HALF_SWITCH(dt, T, { kCarrySum<T><<<(unsigned)((packets + 255) / 256), 256, 0, s>>>((const float4*)part, (uint4*)out, packets); });
-  return launched("carried sum");
-}
-
 hlResult_t crossEntropyForward(int dt, const void* logits, int64_t stride, const int64_t* targets, int64_t rows, int vocab, int64_t ignore_index,
                                float* lse, float* row_loss, float* loss, cudaStream_t s) {
   if (stride % 8 || stride < vocab || vocab < 1) return fail(hlInvalidArgument, "cross entropy: stride %lld, vocabulary %d", (long long)stride, vocab);

@@ -52,9 +52,6 @@ hlResult_t crossEntropyForward(int dt, const void* logits, int64_t stride, const
 hlResult_t crossEntropyBackward(int dt, const void* logits, int64_t stride, const int64_t* targets, int64_t rows, int vocab, int64_t ignore_index,
                                 const float* lse, const float* loss, const float* grad, void* dlogits, cudaStream_t s);
 
-// out += part, element by element, rounded to the 16-bit type. count a multiple of 8.
-hlResult_t carrySum(int dt, const float* part, void* out, int64_t count, cudaStream_t s);
-
 // One AdamW update of `count` elements (a multiple of 8). The gradient is a sum over `ranks`; `keep` = 1 - lr * decay,
 // `rest1` = 1 - beta1 and `rest2` = 1 - beta2 (not to be taken in fp32: 1 - 0.999f is 5e-5 off), `step` =
 // lr / (1 - beta1^t), `correction2` = 1 - beta2^t. master: fp32 copy of 16-bit weights, or null.
