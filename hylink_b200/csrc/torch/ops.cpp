@@ -39,9 +39,15 @@ int code(const Tensor& t) {
 }
 cudaStream_t streamOf(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 Tensor floats(const Tensor& like, at::IntArrayRef sizes) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+bool aligned(const Tensor& t) { return ((uintptr_t)t.data_ptr() & 15) == 0; }
+// What the kernels' 16-byte packets need of whatever comes from outside (tokens, weights, incoming gradients, what saved-tensor
+// hooks give back): contiguous, and on a 16-byte boundary. Parameters that are views into one flat buffer start anywhere.
+Tensor dense(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return aligned(c) ? c : c.clone();
+}
 // Rows of a [..., width] tensor as one matrix.
-Tensor rowsOf(const Tensor& t) { return t.is_contiguous() ? t.view({-1, t.size(-1)}) : t.reshape({-1, t.size(-1)}); }
-Tensor dense(const Tensor& t) { return t.contiguous(); }
+Tensor rowsOf(const Tensor& t) { return dense(t).view({-1, t.size(-1)}); }
 
 // The gradients below are computed by kernels that autograd does not see into.
 void onceOnly() { TORCH_CHECK(!at::GradMode::is_enabled(), "hylink: the fused training step is differentiable once"); }
@@ -75,8 +81,9 @@ Normed normForward(const Tensor& x, const Tensor& y, const Tensor& gamma, const 
   return r;
 }
 // Returns dx; `partials` becomes [3][parts][width].
-Tensor normBackward(const Tensor& dh, const Tensor& x, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, const Tensor& residual,
+Tensor normBackward(const Tensor& dh, const Tensor& x_, const Tensor& mean, const Tensor& rstd, const Tensor& gamma_, const Tensor& residual,
                     bool dx_sums, Tensor* partials, int* parts) {
+  const Tensor x = dense(x_), gamma = dense(gamma_);
   const int64_t width = x.size(-1), rows = x.numel() / width;
   *parts = train::layerNormPartials(rows);
   *partials = floats(x, {3, *parts, width});
@@ -184,7 +191,8 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &a = s[0], &wp = s[1], &x2 = s[2], &gamma = s[5], &h = s[6], &wf = s[7], &u = s[8], &act = s[9], &wo = s[10];
+    const Tensor &a = s[0], &wp = s[1], &x2 = s[2], &gamma = s[5], &h = s[6], &wf = s[7], &act = s[9], &wo = s[10];
+    const Tensor u = dense(s[8]);
     c10::cuda::CUDAGuard dg(x2.device());
     const int64_t width = x2.size(-1), rows = x2.numel() / width, hidden = u.size(1);
     const int dt = code(x2), sp = train::stripPartials(rows);
@@ -259,7 +267,8 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &h = s[0], &wpad = s[1], &targets = s[2], &logits = s[3], &lse = s[4], &loss = s[5];
+    const Tensor &h = s[0], &wpad = s[1], &targets = s[2], &lse = s[4], &loss = s[5];
+    const Tensor logits = dense(s[3]);
     c10::cuda::CUDAGuard dg(h.device());
     const int64_t vocab = ctx->saved_data["vocab"].toInt();
     const Tensor grad = g[0].to(at::kFloat).contiguous();
@@ -294,8 +303,9 @@ Routed moeRouted(const Tensor& x, const Tensor& router, int64_t capacity) {
   return r;
 }
 // {dx, drouter}; dres may be undefined.
-std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& router, const Tensor& logits, const Tensor& expert, const Tensor& gate,
+std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& router_, const Tensor& logits, const Tensor& expert, const Tensor& gate,
                                             const Tensor& row_of, const Tensor& dres, const Tensor& dsend, const Tensor& dgate) {
+  const Tensor router = dense(router_);
   const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
   Tensor dx = at::empty_like(x), dlogits = at::empty_like(logits);
   ok(train::moeTokenGradient(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
@@ -317,9 +327,10 @@ Expert moeExpert(const Tensor& h, const Tensor& w1, const Tensor& w2) {
   return e;
 }
 // {dh, dw1, dw2}
-variable_list moeExpertBackward(const Tensor& h, const Tensor& w1, const Tensor& w2, const Tensor& u, const Tensor& act, const Tensor& dout) {
+variable_list moeExpertBackward(const Tensor& h, const Tensor& w1, const Tensor& w2, const Tensor& u_, const Tensor& act, const Tensor& dout) {
   Tensor dact = at::bmm(dout, w2.transpose(1, 2));
   Tensor dw2 = at::bmm(act.transpose(1, 2), dout);
+  const Tensor u = dense(u_);
   Tensor du = at::empty_like(u);
   ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
      "gelu backward");
@@ -359,7 +370,8 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &x = s[0], &router = s[1], &w1 = s[2], &w2 = s[3], &h = s[9], &rows = s[12];
+    const Tensor &router = s[1], &w1 = s[2], &w2 = s[3], &h = s[9];
+    const Tensor x = dense(s[0]), rows = dense(s[12]);
     c10::cuda::CUDAGuard dg(x.device());
     const Tensor dy = dense(g[0]);
     const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8]);
@@ -386,7 +398,7 @@ class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &x = s[0], &gate = s[4];
+    const Tensor x = dense(s[0]), &gate = s[4];
     c10::cuda::CUDAGuard dg(x.device());
     const Tensor dres = g[0].defined() ? dense(g[0]) : Tensor();
     const Tensor dsend = g[1].defined() ? dense(g[1]) : at::zeros({ctx->saved_data["rows"].toInt(), x.size(1)}, x.options());
@@ -416,10 +428,10 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
 // y = x + gate * rows[row_of] for the tokens that have a row.
 class MoeCombine : public torch::autograd::Function<MoeCombine> {
  public:
-  static Variable forward(AutogradContext* ctx, const Variable& x, const Variable& gate, const Variable& rows_, const Variable& row_of,
+  static Variable forward(AutogradContext* ctx, const Variable& x_, const Variable& gate, const Variable& rows_, const Variable& row_of,
                           const Variable& token_of) {
-    c10::cuda::CUDAGuard dg(x.device());
-    const Tensor rows = dense(rows_);
+    c10::cuda::CUDAGuard dg(x_.device());
+    const Tensor x = dense(x_), rows = dense(rows_);
     ctx->save_for_backward({gate, rows, token_of});
     return moeCombined(x, gate, rows, row_of);
   }
@@ -428,7 +440,7 @@ class MoeCombine : public torch::autograd::Function<MoeCombine> {
     const auto s = ctx->get_saved_variables();
     c10::cuda::CUDAGuard dg(s[1].device());
     const Tensor dy = dense(g[0]);
-    const auto [drows, dgate] = moeCombinedBackward(dy, s[0], s[1], s[2]);
+    const auto [drows, dgate] = moeCombinedBackward(dy, s[0], dense(s[1]), s[2]);
     return {dy, dgate, drows, Tensor(), Tensor()};
   }
 };
@@ -461,18 +473,24 @@ bool multiAdamW(const std::vector<Tensor>& weights, const std::vector<Tensor>& g
   return true;
 }
 
-void shardedAdamW(const Tensor& grad, const Tensor& weight, const std::optional<Tensor>& master, const Tensor& m, const Tensor& v, int64_t ranks,
+// False (and nothing done) for a shard that the kernel does not take: it wants packets of contiguous CUDA tensors.
+bool shardedAdamW(const Tensor& grad, const Tensor& weight, const std::optional<Tensor>& master, const Tensor& m, const Tensor& v, int64_t ranks,
                   double keep, double beta1, double beta2, double step, double correction2, double eps) {
-  c10::cuda::CUDAGuard dg(weight.device());
   const int64_t n = weight.numel();
-  TORCH_CHECK(grad.is_contiguous() && weight.is_contiguous() && m.is_contiguous() && v.is_contiguous() && grad.numel() == n && m.numel() == n &&
-                  v.numel() == n && (!master || (master->is_contiguous() && master->numel() == n)),
-              "hylink: sharded AdamW needs contiguous tensors of one size");
+  const auto type = weight.scalar_type();
+  const auto fits = [&](const Tensor& t, at::ScalarType want) {
+    return t.scalar_type() == want && t.device() == weight.device() && t.layout() == at::kStrided && t.is_contiguous() && t.numel() == n && aligned(t);
+  };
+  if (!weight.is_cuda() || n % 8 || (type != at::kBFloat16 && type != at::kHalf && type != at::kFloat) || !fits(weight, type) || !fits(grad, type) ||
+      !fits(m, at::kFloat) || !fits(v, at::kFloat) || (master && (type == at::kFloat || !fits(*master, at::kFloat))))
+    return false;
+  c10::cuda::CUDAGuard dg(weight.device());
   const train::AdamWArgs a = {(float)ranks, (float)keep, (float)beta1, (float)(1 - beta1), (float)beta2, (float)(1 - beta2), (float)step, (float)correction2, (float)eps};
   const int dt = weight.scalar_type() == at::kFloat ? (int)hlFloat32 : code(weight);
   ok(train::shardedAdamW(dt, grad.data_ptr(), weight.data_ptr(), master ? master->data_ptr<float>() : nullptr, m.data_ptr<float>(),
                          v.data_ptr<float>(), n, a, streamOf(weight)),
      "sharded AdamW");
+  return true;
 }
 
 // ---- calls whose cost on the host is most of a small one: argument lists are taken apart here, not in Python

@@ -62,9 +62,8 @@ class ShardedAdamW:
         b1, b2 = self.betas
         keep, step, correction2 = 1 - self.lr * self.wd, self.lr / (1 - b1 ** self.t), 1 - b2 ** self.t
         mine = self.flat[self.r * self.shard:(self.r + 1) * self.shard]
-        if mine.is_cuda and mine.dtype in (torch.bfloat16, torch.float16, torch.float32):
-            ops().sharded_adamw(self.grad_shard, mine, self.master, self.m, self.v, self.n, keep, b1, b2, step, correction2, self.eps)
-        else:
+        if not (mine.is_cuda and ops().sharded_adamw(self.grad_shard, mine, self.master, self.m, self.v, self.n, keep, b1, b2, step, correction2,
+                                                     self.eps)):
             g = self.grad_shard.float() / self.n
             w = self.master if self.master is not None else mine.float()
             w.mul_(keep)

@@ -41,6 +41,28 @@ def test_fused_step_matches_fp32(width, heads, vocab, batch, seq, dtype):
         assert err <= max(1.3 * base, 1e-3), (n, float(err), float(base))
 
 
+def test_fused_step_takes_parameters_off_the_packet_boundary():
+    """As views into one flat buffer, behind a parameter of three elements."""
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+
+    torch.manual_seed(4)
+    plain = GPT2(GPT2Config(n_layer=2, n_head=3, d_model=264, vocab_size=1024, n_ctx=64)).cuda().to(torch.bfloat16)
+    model = copy.deepcopy(plain)
+    flat = torch.empty(3 + sum(p.numel() for p in model.parameters()), device="cuda", dtype=torch.bfloat16)
+    at = 3
+    for p in model.parameters():
+        p.data = flat[at:at + p.numel()].view(p.shape).copy_(p.data)
+        at += p.numel()
+        assert p.data_ptr() % 16
+    idx, targets = (torch.randint(0, 1024, (2, 37), device="cuda") for _ in range(2))
+    assert model._fusable(torch.empty(1, device="cuda", dtype=torch.bfloat16), targets)
+    want_loss, want = _grads(plain, idx, targets)
+    loss, got = _grads(model, idx, targets)
+    assert abs(loss - want_loss) <= 2e-3 * abs(want_loss)
+    for n, w in want.items():                        # other places are other kernels of the library for the products
+        assert float((got[n] - w).norm() / w.norm()) < 2e-2, n
+
+
 def _head_case(rows, width, vocab):
     g = torch.Generator(device="cuda").manual_seed(1)
     h = torch.randn(rows, width, generator=g, device="cuda").to(torch.bfloat16).requires_grad_()

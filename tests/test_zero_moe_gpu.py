@@ -88,3 +88,57 @@ def test_moe_matches_the_dense_layer(tokens, width, experts, capacity):
     for (n, p), q in zip(layer.named_parameters(), ref.parameters()):
         if float(q.grad.norm()) > 1e-6:
             assert rel(p.grad, q.grad) < 2e-2, n
+
+
+def _off_boundary(t):
+    """A contiguous copy of `t` that starts inside a 16-byte packet."""
+    out = torch.empty(t.numel() + 3, dtype=t.dtype, device=t.device)[3:].view(t.shape)
+    assert out.is_contiguous() and out.data_ptr() % 16
+    return out.copy_(t)
+
+
+# experts whose gradients a warp holds in registers, and more
+@pytest.mark.parametrize("tokens,width,experts,capacity", [(37, 64, 4, 11), (300, 264, 20, 17)])
+@pytest.mark.parametrize("pieces", [False, True])
+def test_moe_takes_tensors_off_the_packet_boundary(tokens, width, experts, capacity, pieces):
+    """Weights that a parameter of three elements shifts in ShardedAdamW's flat buffer; tokens and gradients that are views."""
+    import copy
+
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+    from hylink_b200.parallel.zero import ShardedAdamW
+
+    torch.manual_seed(tokens)
+    plain = ExpertParallelMLP(width, 4 * width, experts_per_rank=experts, capacity=capacity).cuda().to(torch.bfloat16)
+    layer = copy.deepcopy(plain)
+    lead = torch.nn.Parameter(torch.zeros(3, device="cuda", dtype=torch.bfloat16))
+    ShardedAdamW([lead, *layer.parameters()])
+    assert layer.router.weight.data_ptr() % 16
+    if pieces:                                       # the form in which tokens travel: weights of another type take it on one rank too
+        for m in (plain, layer):
+            m.w1.data = m.w1.data.float()
+            m.w1.grad = None
+    x, dy = (torch.randn(tokens, width, device="cuda").to(torch.bfloat16) for _ in range(2))
+    results = []
+    for m, place in ((plain, lambda t: t.clone()), (layer, _off_boundary)):
+        xi = place(x).requires_grad_()
+        assert m._fusable(xi)
+        y = m(xi)
+        y.backward(place(dy))
+        results.append([y.detach(), xi.grad, *(p.grad for p in m.parameters())])
+    for a, b in zip(*results):
+        assert float((a.float() - b.float()).norm()) <= 1e-2 * float(a.float().norm()) + 1e-6
+
+
+def test_sharded_adamw_takes_a_gradient_off_the_packet_boundary():
+    from hylink_b200.parallel.zero import ShardedAdamW
+
+    torch.manual_seed(1)
+    start, grad = torch.randn(1003, device="cuda").to(torch.bfloat16), torch.randn(1003, device="cuda").to(torch.bfloat16)
+    weights = []
+    for place in (lambda t: t.clone(), _off_boundary):
+        opt = ShardedAdamW([torch.nn.Parameter(start.clone())], lr=1e-2)
+        opt.flat_grad[:1003].copy_(grad)
+        opt.flat_grad = opt.grad_shard = place(opt.flat_grad)
+        opt.step()
+        weights.append(opt.master.clone())
+    torch.testing.assert_close(*weights, rtol=1e-5, atol=1e-6)
