@@ -148,11 +148,11 @@ __global__ void __launch_bounds__(HL_STREAM_WORKERS + 64, 1) kStream(const HlCom
         }
         gave_up = __any_sync(0xffffffffu, gave_up);
       }
+      __syncwarp();                                   // every lane's acquire, before lane 0 lets the workers on (a vote orders no memory)
       if (lane == 0) {
         if (gave_up) s_stop = t;
         else if (t < I) mbArrive(&s_open[t % kStreamRing]);
       }
-      __syncwarp();
     }
   } else if (warp == 1) {                             // ---- signaller
     for (int t = 0; t < I; ++t) {
