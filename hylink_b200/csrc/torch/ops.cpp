@@ -248,6 +248,8 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
     c10::cuda::CUDAGuard dg(h_.device());
     const Tensor h = rowsOf(h_), targets = targets_.reshape({-1}).contiguous();
     const int64_t vocab = w.size(0), padded = (vocab + 63) / 64 * 64, rows = h.size(0);
+    TORCH_CHECK_VALUE(targets.scalar_type() == at::kLong && targets.device() == h.device() && targets.numel() == rows, "hylink: ", rows,
+                      " rows and ", targets.numel(), " targets");
     Tensor wpad = w;
     if (padded != vocab || !w.is_contiguous()) {
       wpad = at::empty({padded, w.size(1)}, w.options());
@@ -598,6 +600,7 @@ PyMethodDef kNativeCalls[] = {{"emu_run", (PyCFunction)(void*)emuRun, METH_FASTC
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("max_norm_width") = train::kMaxNormWidth;
+  m.attr("max_rows") = train::kMaxRows;
   m.def("add_norm", [](const Tensor& x, const std::optional<Tensor>& y, const Tensor& gamma, const Tensor& beta, double eps) {
     return AddNorm::apply(x, y, gamma, beta, eps);
   });

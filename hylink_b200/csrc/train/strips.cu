@@ -176,7 +176,8 @@ static hlResult_t strip(int dt, const Op& op, float* partials, int64_t rows, int
   if (width % 8) return fail(hlUnsupported, "strip kernels: width %d", width);
   if (rows == 0) return hlSuccess;
   const dim3 grid((unsigned)((width + 255) / 256), (unsigned)stripPartials(rows));
-  if (grid.y > 65535) return fail(hlUnsupported, "strip kernels: %lld rows", (long long)rows);
+  static_assert(kMaxRows == 65535LL * kStripRows, "one CTA per range of rows");
+  if (rows > kMaxRows) return fail(hlUnsupported, "strip kernels: %lld rows", (long long)rows);
   HL_HALF_SWITCH(dt, T, { kStrip<T, Op><<<grid, kStripThreads, 0, s>>>(op, partials, rows, width); });
   return launched("strip");
 }

@@ -8,7 +8,8 @@
 namespace hl {
 namespace train {
 
-constexpr int kMaxNormWidth = 1024;   // a warp holds a whole row and three column sums in registers
+constexpr int kMaxNormWidth = 1024;   // the ring of the backward pass holds whole rows, a lane the sums of its columns
+constexpr int64_t kMaxRows = 65535 * 128;   // of the strip kernels: their row ranges are the grid's second dimension
 
 // Column sums end in two steps: the kernels that walk the rows write one fp32 partial per CTA and column, one later
 // launch adds up the partials of several of them. `src` is [rows][width], `dst` has the element type of the call.

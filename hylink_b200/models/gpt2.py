@@ -95,7 +95,7 @@ class GPT2(nn.Module):
         b, t = idx.shape
         pos = torch.arange(t, device=idx.device)
         x = self.wte(idx) + self.wpe(pos)
-        if targets is not None and self._fusable(x, targets):
+        if targets is not None and self._sizes_fit(idx, targets) and self._fusable(x, targets):
             return self._fused_loss(x, targets)
         for blk in self.blocks:
             x = blk(x)
@@ -104,6 +104,12 @@ class GPT2(nn.Module):
         if targets is None:
             return logits
         return F.cross_entropy(logits.float().view(-1, logits.size(-1)), targets.reshape(-1))
+
+    @staticmethod
+    def _sizes_fit(idx: torch.Tensor, targets: torch.Tensor) -> bool:
+        """A target per token, where the tokens are (anything else is an error that the plain loss reports), and no more rows
+        than the fused operators take."""
+        return targets.numel() == idx.numel() and targets.device == idx.device and (not idx.is_cuda or idx.numel() <= ops().max_rows)
 
     def _fusable(self, x: torch.Tensor, targets: torch.Tensor) -> bool:
         """Whether the loss can go through the fused operators: a 16-bit model on a GPU, made of the plain modules
@@ -130,7 +136,7 @@ class GPT2(nn.Module):
     def step_signature(self, idx: torch.Tensor, targets: torch.Tensor):
         """What a recorded training step depends on besides its inputs' values: equal signatures may share a recording.
         None when a step has effects that a recording would not repeat (hooks) or does not take the fused operators."""
-        if not self._fusable(self.wte.weight, targets) or _hooked(self) or not torch.is_grad_enabled():
+        if not self._sizes_fit(idx, targets) or not self._fusable(self.wte.weight, targets) or _hooked(self) or not torch.is_grad_enabled():
             return None
         ps = list(self.parameters())
         if any(p._backward_hooks or p._post_accumulate_grad_hooks for p in ps):

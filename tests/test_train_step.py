@@ -108,6 +108,22 @@ def test_head_gradient_is_one_product_of_the_library():
     assert torch.equal(got, d[:, :vocab] @ w.detach())
 
 
+@pytest.mark.parametrize("targets", [(2, 7), (1, 8), (2, 9)])
+def test_as_many_targets_as_tokens(targets):
+    """Another number of targets is the plain loss's error, and the operator's own."""
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.ops.extension import ops
+
+    model = GPT2(GPT2Config(n_layer=1, n_head=2, d_model=64, vocab_size=100, n_ctx=16)).cuda().to(torch.bfloat16)
+    idx, t = torch.zeros(2, 8, dtype=torch.int64, device="cuda"), torch.zeros(targets, dtype=torch.int64, device="cuda")
+    with pytest.raises(ValueError):
+        model(idx, t)
+    with pytest.raises(ValueError):
+        ops().head_loss(torch.zeros(2, 8, 64, device="cuda", dtype=torch.bfloat16), model.wte.weight, t)
+    assert model.step_signature(idx, t) is None
+    assert model.step_signature(idx, idx) is not None and bool(model(idx, idx.reshape(-1)).isfinite())
+
+
 def test_out_of_range_target_gives_nan_and_large_logits_stay_finite():
     from hylink_b200.ops.extension import ops
 
