@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.extension import ops
+from ..ops.extension import ops, overridden
 
 
 @dataclass
@@ -40,10 +40,6 @@ class GPT2Config:
     def by_name(name: str) -> "GPT2Config":
         return {"gpt2-medium": GPT2Config.medium, "medium": GPT2Config.medium, "tiny": GPT2Config.tiny,
                 "gpt2-small": lambda: GPT2Config(n_layer=12, n_head=12, d_model=768)}[name]()
-
-
-def _hooked(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
 
 
 def _any_global_hook() -> bool:
@@ -113,7 +109,7 @@ class GPT2(nn.Module):
 
     def _fusable(self, x: torch.Tensor, targets: torch.Tensor) -> bool:
         """Whether the loss can go through the fused operators: a 16-bit model on a GPU, made of the plain modules
-        above (no hooks, nothing replaced), at widths whose rows a warp can hold."""
+        above (no hooks, nothing replaced, no `forward` of an instance's own), at widths whose rows a warp can hold."""
         c = self.config
         if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.numel() and targets.is_cuda and targets.dtype == torch.int64):
             return False
@@ -123,11 +119,11 @@ class GPT2(nn.Module):
             return False
         mods = [self.ln_f, self.wte]
         for blk in self.blocks:
-            if type(blk) is not Block or _hooked(blk):
+            if type(blk) is not Block or overridden(blk):
                 return False
             mods += (blk.ln1, blk.qkv, blk.proj, blk.ln2, blk.fc, blk.out)
         for m in mods:
-            if type(m) not in (nn.LayerNorm, nn.Linear, nn.Embedding) or _hooked(m) or m.weight.dtype != x.dtype:
+            if type(m) not in (nn.LayerNorm, nn.Linear, nn.Embedding) or overridden(m) or m.weight.dtype != x.dtype:
                 return False
             if type(m) is not nn.Embedding and m.bias is None:
                 return False
@@ -136,7 +132,9 @@ class GPT2(nn.Module):
     def step_signature(self, idx: torch.Tensor, targets: torch.Tensor):
         """What a recorded training step depends on besides its inputs' values: equal signatures may share a recording.
         None when a step has effects that a recording would not repeat (hooks) or does not take the fused operators."""
-        if not self._sizes_fit(idx, targets) or not self._fusable(self.wte.weight, targets) or _hooked(self) or not torch.is_grad_enabled():
+        if not self._sizes_fit(idx, targets) or not self._fusable(self.wte.weight, targets) or not torch.is_grad_enabled():
+            return None
+        if type(self) is not GPT2 or type(self.wpe) is not nn.Embedding or overridden(self) or overridden(self.wpe):
             return None
         ps = list(self.parameters())
         if any(p._backward_hooks or p._post_accumulate_grad_hooks for p in ps):

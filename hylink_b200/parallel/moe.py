@@ -17,7 +17,7 @@ import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.extension import ops
+from ..ops.extension import ops, overridden
 
 
 class _AllToAll(torch.autograd.Function):
@@ -82,11 +82,11 @@ class ExpertParallelMLP(nn.Module):
         return y
 
     def _fusable(self, x) -> bool:
-        """16-bit tokens on a GPU, a plain router of the same type, rows of whole 16-byte packets."""
+        """16-bit tokens on a GPU, a plain router of the same type (its own `forward`, no hooks), rows of whole 16-byte packets."""
         r = self.router
         return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.shape[0] > 0 and x.shape[1] % 8 == 0
                 and self.w1.shape[2] % 8 == 0 and type(r) is nn.Linear and r.bias is None and r.weight.dtype == x.dtype
-                and not (r._forward_hooks or r._forward_pre_hooks or r._backward_hooks or r._backward_pre_hooks)
+                and not overridden(r)
                 and not torch.is_autocast_enabled("cuda"))
 
     def _fused(self, x):

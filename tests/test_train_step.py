@@ -183,6 +183,64 @@ def test_replayed_steps_train_like_eager_ones(name, batch, seq, monkeypatch):
         dist.destroy_process_group()
 
 
+def _counted(module, seen):
+    plain = module.forward
+    module.forward = lambda *a: (seen.append(1), plain(*a))[1]
+
+
+@pytest.mark.parametrize("where", ["blocks.1", "blocks.0.fc", "blocks.0.ln2", "ln_f", "wte", "wpe", ""])
+def test_a_forward_of_an_instance_is_called(where):
+    """On the model, its blocks and their layers: in every step, recorded ones included."""
+    import torch.distributed as dist
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.parallel.trainer import DDPTrainer, init_distributed
+
+    fresh = not dist.is_initialized()
+    if fresh:
+        init_distributed("hylink")
+    model, seen = GPT2(GPT2Config.tiny()), []
+    t = DDPTrainer(model, torch.device("cuda", 0))
+    _counted(model.get_submodule(where), seen)
+    tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
+    for _ in range(4):
+        t.step(tokens)
+    assert len(seen) == 4
+    t.close()
+    if fresh:
+        dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("what", ["hook on wpe", "subclass"])
+def test_a_step_with_effects_is_not_replayed(what):
+    import torch.distributed as dist
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.parallel.trainer import DDPTrainer, init_distributed
+
+    seen = []
+
+    class Counting(GPT2):
+        def forward(self, *a):
+            seen.append(1)
+            return super().forward(*a)
+
+    fresh = not dist.is_initialized()
+    if fresh:
+        init_distributed("hylink")
+    model = (Counting if what == "subclass" else GPT2)(GPT2Config.tiny())
+    if what != "subclass":
+        model.wpe.register_forward_hook(lambda *a: seen.append(1))
+    t = DDPTrainer(model, torch.device("cuda", 0))
+    tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
+    for _ in range(4):
+        t.step(tokens)
+    assert len(seen) == 4
+    t.close()
+    if fresh:
+        dist.destroy_process_group()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_multi_tensor_adamw_matches_torch(dtype):
     """Tensors shorter than a packet, of a ragged length, unaligned, of several chunks; more of them than one launch takes."""

@@ -142,3 +142,13 @@ def test_sharded_adamw_takes_a_gradient_off_the_packet_boundary():
         opt.step()
         weights.append(opt.master.clone())
     torch.testing.assert_close(*weights, rtol=1e-5, atol=1e-6)
+
+
+def test_the_routers_own_forward_is_called():
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+
+    layer, seen = ExpertParallelMLP(64, 128, experts_per_rank=4, capacity=16).cuda().to(torch.bfloat16), []
+    plain = layer.router.forward
+    layer.router.forward = lambda x: (seen.append(1), plain(x))[1]
+    layer(torch.randn(10, 64, device="cuda", dtype=torch.bfloat16))
+    assert len(seen) == 1
