@@ -113,21 +113,26 @@ class GPT2(nn.Module):
         c = self.config
         if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.numel() and targets.is_cuda and targets.dtype == torch.int64):
             return False
-        if c.d_model > ops().max_norm_width or c.d_model % 8 or (c.d_model // c.n_head) % 8 or torch.is_autocast_enabled("cuda"):
+        d = c.d_model
+        if d > ops().max_norm_width or d % 8 or torch.is_autocast_enabled("cuda"):
             return False
         if _any_global_hook():
             return False
-        mods = [self.ln_f, self.wte]
+        mods = [(self.ln_f, nn.LayerNorm, d, 0), (self.wte, nn.Embedding, 0, d)]
         for blk in self.blocks:
-            if type(blk) is not Block or overridden(blk):
+            if type(blk) is not Block or overridden(blk) or d % blk.n_head or (d // blk.n_head) % 8:
                 return False
-            mods += (blk.ln1, blk.qkv, blk.proj, blk.ln2, blk.fc, blk.out)
-        for m in mods:
-            if type(m) not in (nn.LayerNorm, nn.Linear, nn.Embedding) or overridden(m) or m.weight.dtype != x.dtype:
+            mods += ((blk.ln1, nn.LayerNorm, d, 0), (blk.qkv, nn.Linear, 3 * d, d), (blk.proj, nn.Linear, d, d), (blk.ln2, nn.LayerNorm, d, 0),
+                     (blk.fc, nn.Linear, 0, d), (blk.out, nn.Linear, d, 0))
+        for m, kind, rows, cols in mods:     # 0: any number
+            if type(m) is not kind or overridden(m):
                 return False
-            if type(m) is not nn.Embedding and m.bias is None:
+            w = m.weight
+            if w is None or w.dtype != x.dtype or w.dim() != (1 if kind is nn.LayerNorm else 2):
                 return False
-        return True
+            if (rows and w.shape[0] != rows) or (cols and w.shape[1] != cols) or (kind is not nn.Embedding and m.bias is None):
+                return False
+        return all(blk.fc.weight.shape[0] % 8 == 0 for blk in self.blocks)
 
     def step_signature(self, idx: torch.Tensor, targets: torch.Tensor):
         """What a recorded training step depends on besides its inputs' values: equal signatures may share a recording.

@@ -183,6 +183,36 @@ def test_replayed_steps_train_like_eager_ones(name, batch, seq, monkeypatch):
         dist.destroy_process_group()
 
 
+@pytest.mark.parametrize("change", ["no affine", "no bias", "wide norm", "odd hidden", "heads"])
+def test_other_layers_run_as_modules(change):
+    """Layers of the plain classes that the fused operators do not take."""
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+
+    torch.manual_seed(7)
+    ref = GPT2(GPT2Config(n_layer=2, n_head=4, d_model=64, vocab_size=100, n_ctx=16)).cuda()
+    b = ref.blocks[1]
+    nn = torch.nn
+    with torch.device("cuda"):
+        if change == "no affine":
+            b.ln1, ref.ln_f = nn.LayerNorm(64, elementwise_affine=False), nn.LayerNorm(64, elementwise_affine=False)
+        elif change == "no bias":
+            b.ln2 = nn.LayerNorm(64, bias=False)
+        elif change == "wide norm":
+            b.ln1 = nn.LayerNorm((8, 64))
+        elif change == "odd hidden":
+            b.fc, b.out = nn.Linear(64, 101), nn.Linear(101, 64)
+        else:
+            b.n_head = 16
+    model = copy.deepcopy(ref).to(torch.bfloat16)
+    ref = copy.deepcopy(model).float()
+    idx = torch.randint(0, 100, (2, 8), device="cuda")
+    loss, got = _grads(model, idx, idx)
+    want_loss, want = _grads(ref, idx, idx)
+    assert abs(loss - want_loss) <= 5e-3 * abs(want_loss)
+    for n, w in want.items():                        # two layers of 16-bit modules
+        assert float((got[n] - w).norm()) <= 3e-2 * float(w.norm()) + 1e-6, n
+
+
 def _counted(module, seen):
     plain = module.forward
     module.forward = lambda *a: (seen.append(1), plain(*a))[1]
