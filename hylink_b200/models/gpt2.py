@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.extension import ops, overridden
+from ..ops.extension import global_module_hooks, ops, overridden, plain_eager, traced
 
 
 @dataclass
@@ -40,12 +40,6 @@ class GPT2Config:
     def by_name(name: str) -> "GPT2Config":
         return {"gpt2-medium": GPT2Config.medium, "medium": GPT2Config.medium, "tiny": GPT2Config.tiny,
                 "gpt2-small": lambda: GPT2Config(n_layer=12, n_head=12, d_model=768)}[name]()
-
-
-def _any_global_hook() -> bool:
-    from torch.nn.modules import module as g
-
-    return bool(g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)
 
 
 class Block(nn.Module):
@@ -91,7 +85,7 @@ class GPT2(nn.Module):
         b, t = idx.shape
         pos = torch.arange(t, device=idx.device)
         x = self.wte(idx) + self.wpe(pos)
-        if targets is not None and self._sizes_fit(idx, targets) and self._fusable(x, targets):
+        if targets is not None and not traced() and self._sizes_fit(idx, targets) and self._fusable(x, targets):
             return self._fused_loss(x, targets)
         for blk in self.blocks:
             x = blk(x)
@@ -116,7 +110,7 @@ class GPT2(nn.Module):
         d = c.d_model
         if d > ops().max_norm_width or d % 8 or torch.is_autocast_enabled("cuda"):
             return False
-        if _any_global_hook():
+        if global_module_hooks() or not plain_eager(x, targets):
             return False
         mods = [(self.ln_f, nn.LayerNorm, d, 0), (self.wte, nn.Embedding, 0, d)]
         for blk in self.blocks:
@@ -128,7 +122,7 @@ class GPT2(nn.Module):
             if type(m) is not kind or overridden(m):
                 return False
             w = m.weight
-            if w is None or w.dtype != x.dtype or w.dim() != (1 if kind is nn.LayerNorm else 2):
+            if type(w) not in (nn.Parameter, torch.Tensor) or type(m.bias if kind is not nn.Embedding else w) not in (nn.Parameter, torch.Tensor) or w.dtype != x.dtype or w.dim() != (1 if kind is nn.LayerNorm else 2):
                 return False
             if (rows and w.shape[0] != rows) or (cols and w.shape[1] != cols) or (kind is not nn.Embedding and m.bias is None):
                 return False

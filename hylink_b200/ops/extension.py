@@ -5,6 +5,11 @@ import importlib.machinery
 import importlib.util
 from pathlib import Path
 
+import torch
+from torch.autograd import forward_ad
+from torch.nn.modules import module as _modules
+from torch.utils._device import DeviceContext
+
 _module = None
 
 
@@ -12,8 +17,6 @@ def ops():
     """The extension module. It is built in-tree; a missing one is built now, and a broken one is an error."""
     global _module
     if _module is None:
-        import torch  # noqa: F401  (the extension links against it)
-
         from .. import _native  # noqa: F401  (loads libhylink_b200.so first)
 
         path = Path(__file__).resolve().parent.parent / "lib" / "_hylink_ops.so"
@@ -30,8 +33,6 @@ def ops():
 
 def is_half_cuda(*tensors) -> bool:
     """Whether all tensors are CUDA tensors of one 16-bit float type."""
-    import torch
-
     dt = tensors[0].dtype
     return dt in (torch.bfloat16, torch.float16) and all(t.is_cuda and t.dtype == dt for t in tensors)
 
@@ -39,3 +40,27 @@ def is_half_cuda(*tensors) -> bool:
 def overridden(m) -> bool:
     """Whether calling module ``m`` does anything besides its class's ``forward``: hooks, or a ``forward`` of its own."""
     return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__)
+
+
+def traced() -> bool:
+    return torch.compiler.is_compiling() or torch.jit.is_tracing()
+
+
+def plain_eager(*tensors) -> bool:
+    """Whether ordinary eager autograd is all that looks at a call on these tensors. The operators work on addresses and have
+    one backward: under tracing and compilation, function transforms (vmap, torch.func), forward-mode differentiation and
+    modes that watch every call, and for tensor subclasses, the plain modules run."""
+    if any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter for t in tensors):
+        return False
+    if traced() or forward_ad._current_level >= 0:
+        return False
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack():
+        return False
+    # a default device is a mode too, one that the operators need not see
+    return all(type(torch._C._get_function_stack_at(i)) is DeviceContext for i in range(torch._C._len_torch_function_stack()))
+
+
+def global_module_hooks() -> bool:
+    """Whether hooks on every module's calls are registered."""
+    g = _modules
+    return bool(g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)

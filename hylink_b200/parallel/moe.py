@@ -17,7 +17,7 @@ import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.extension import ops, overridden
+from ..ops.extension import global_module_hooks, ops, overridden, plain_eager, traced
 
 
 class _AllToAll(torch.autograd.Function):
@@ -60,7 +60,7 @@ class ExpertParallelMLP(nn.Module):
     def forward(self, x):
         """x: [tokens, d_model] (this rank's tokens). Returns the same shape."""
         t, d = x.shape
-        if self._fusable(x):
+        if not traced() and self._fusable(x):
             return self._fused(x)
         probs = F.softmax(self.router(x).float(), dim=-1)
         gate, expert = probs.max(dim=-1)                                   # top-1
@@ -86,7 +86,7 @@ class ExpertParallelMLP(nn.Module):
         r = self.router
         return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.shape[0] > 0 and x.shape[1] % 8 == 0
                 and self.w1.shape[2] % 8 == 0 and type(r) is nn.Linear and r.bias is None and r.weight.dtype == x.dtype
-                and not overridden(r)
+                and not overridden(r) and not global_module_hooks() and plain_eager(x, r.weight, self.w1, self.w2)
                 and not torch.is_autocast_enabled("cuda"))
 
     def _fused(self, x):

@@ -213,6 +213,58 @@ def test_other_layers_run_as_modules(change):
         assert float((got[n] - w).norm()) <= 3e-2 * float(w.norm()) + 1e-6, n
 
 
+def _small(dtype=torch.bfloat16):
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+
+    torch.manual_seed(9)
+    model = GPT2(GPT2Config(n_layer=2, n_head=2, d_model=64, vocab_size=100, n_ctx=16)).cuda().to(dtype)
+    return model, torch.randint(0, 100, (2, 8), device="cuda"), torch.randint(0, 100, (2, 8), device="cuda")
+
+
+def test_tracing_and_compilation_see_the_modules():
+    model, idx, targets = _small()
+    want = model(idx, targets)
+    traced = torch.jit.trace(model, (targets, idx), check_trace=False)
+    torch.testing.assert_close(traced(idx, targets), want, rtol=2e-3, atol=0)
+    torch.testing.assert_close(torch.compile(model, backend="eager", fullgraph=True)(idx, targets), want, rtol=2e-3, atol=0)
+
+
+def test_transforms_and_modes_see_the_modules():
+    import torch.autograd.forward_ad as fwd
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchDispatchMode):
+        names = set()
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.add(str(func))
+            return func(*args, **(kwargs or {}))
+
+    model, idx, targets = _small()
+    want_loss, want = _grads(model, idx, targets)
+    params = dict(model.named_parameters())
+    got = torch.func.grad(lambda p: torch.func.functional_call(model, p, (idx, targets)))(params)
+    for n, w in want.items():
+        assert float((got[n].float() - w).norm() / w.norm()) < 2e-2, n
+    # the derivative along the gradient is its squared norm
+    with sdpa_kernel(SDPBackend.MATH), fwd.dual_level():
+        dual = {n: fwd.make_dual(p.detach(), want[n].to(p.dtype)) for n, p in params.items()}
+        slope = fwd.unpack_dual(torch.func.functional_call(model, dual, (idx, targets))).tangent
+    squared = sum(float(w.double().square().sum()) for w in want.values())
+    assert abs(float(slope) - squared) < 2e-2 * squared
+    with Seen() as seen:
+        model(idx, targets)
+    assert any("gelu" in n for n in seen.names)
+    fake = FakeTensorMode()
+    stand_ins, *tokens = [{n: fake.from_tensor(p.detach()) for n, p in params.items()}, fake.from_tensor(idx), fake.from_tensor(targets)]
+    with fake:
+        assert torch.func.functional_call(model, stand_ins, tuple(tokens)).shape == ()
+    with torch.device("cuda"):                       # a default device is no reason
+        assert model._fusable(torch.empty(1, dtype=torch.bfloat16), targets)
+
+
 def _counted(module, seen):
     plain = module.forward
     module.forward = lambda *a: (seen.append(1), plain(*a))[1]

@@ -152,3 +152,30 @@ def test_the_routers_own_forward_is_called():
     layer.router.forward = lambda x: (seen.append(1), plain(x))[1]
     layer(torch.randn(10, 64, device="cuda", dtype=torch.bfloat16))
     assert len(seen) == 1
+
+
+def test_moe_under_modes_and_hooks_runs_as_modules():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+
+    class Seen(TorchDispatchMode):
+        names = set()
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.add(str(func))
+            return func(*args, **(kwargs or {}))
+
+    torch.manual_seed(2)
+    layer = ExpertParallelMLP(64, 128, experts_per_rank=4, capacity=16).cuda().to(torch.bfloat16)
+    x = torch.randn(10, 64, device="cuda", dtype=torch.bfloat16)
+    with Seen() as seen:
+        layer(x)
+    assert any("gelu" in n for n in seen.names)
+    calls = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda m, a, o: calls.append(m))
+    try:
+        layer(x)
+    finally:
+        handle.remove()
+    assert layer.router in calls
