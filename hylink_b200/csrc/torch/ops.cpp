@@ -10,6 +10,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
@@ -49,8 +50,29 @@ Tensor dense(const Tensor& t) {
 // Rows of a [..., width] tensor as one matrix.
 Tensor rowsOf(const Tensor& t) { return dense(t).view({-1, t.size(-1)}); }
 
-// The gradients below are computed by kernels that autograd does not see into.
-void onceOnly() { TORCH_CHECK(!at::GradMode::is_enabled(), "hylink: the fused training step is differentiable once"); }
+// The gradients below are computed by kernels that autograd does not see into. Where a caller asks for a backward pass that
+// can be differentiated again (create_graph; gradient mode is on inside it then), a node runs its forward once more as plain
+// operations on aliases of its inputs, and lets autograd write that backward pass. Aliases, because an input may depend on
+// another one (the head's weight is also the embedding), and the gradients wanted here are those of the node alone.
+bool wantsGraph() { return at::GradMode::is_enabled(); }
+Tensor viewOf(const Tensor& t) { return t.defined() ? t.view_as(t) : t; }
+// d(outs)/d(inputs) applied to `grads`; undefined for inputs that need no gradient.
+variable_list recorded(const variable_list& outs, const variable_list& grads, const variable_list& inputs) {
+  variable_list o, g, wanted, result(inputs.size());
+  for (size_t i = 0; i < outs.size(); ++i)
+    if (outs[i].requires_grad() && grads[i].defined()) {
+      o.push_back(outs[i]);
+      g.push_back(grads[i]);
+    }
+  for (const Tensor& t : inputs)
+    if (t.defined() && t.requires_grad()) wanted.push_back(t);
+  if (o.empty() || wanted.empty()) return result;
+  const variable_list got = torch::autograd::grad(o, wanted, g, true, true, true);
+  for (size_t i = 0, k = 0; i < inputs.size(); ++i)
+    if (inputs[i].defined() && inputs[i].requires_grad()) result[i] = got[k++];
+  return result;
+}
+Tensor plus(const Tensor& a, const Tensor& b) { return a.defined() ? (b.defined() ? a + b : a) : b; }
 
 // Column-sum partials collected over a backward pass and added up in one launch.
 class Columns {
@@ -101,14 +123,20 @@ class AddNorm : public torch::autograd::Function<AddNorm> {
     c10::cuda::CUDAGuard dg(x_.device());
     const Tensor x = dense(x_), y = y_ ? dense(*y_) : Tensor();
     Normed n = normForward(x, y, gamma, beta, eps);
-    ctx->save_for_backward({n.sum, n.mean, n.rstd, gamma});
+    ctx->save_for_backward({n.sum, n.mean, n.rstd, gamma, x_, y_ ? *y_ : Tensor(), beta});
     ctx->saved_data["y"] = y.defined();
+    ctx->saved_data["eps"] = eps;
     return n.out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
     c10::cuda::CUDAGuard dg(s[0].device());
+    if (wantsGraph()) {
+      const Tensor gamma = viewOf(s[3]), x = viewOf(s[4]), y = viewOf(s[5]), beta = viewOf(s[6]);
+      variable_list r = recorded({at::layer_norm(plus(x, y), {x.size(-1)}, gamma, beta, ctx->saved_data["eps"].toDouble())}, g, {x, y, gamma, beta});
+      r.emplace_back();
+      return r;
+    }
     Tensor parts;
     int np;
     const int64_t w = s[0].size(-1);
@@ -131,17 +159,25 @@ class BlockPre : public torch::autograd::Function<BlockPre> {
     Normed n = normForward(x, y, gamma, beta, eps);
     const Tensor h = n.out.view({-1, width});
     const Tensor qkv = at::addmm(b, h, w.t()).view({batch, seq, 3, heads, hd}).permute({2, 0, 3, 1, 4});
-    ctx->save_for_backward({n.sum, n.mean, n.rstd, gamma, h, w});
+    ctx->save_for_backward({n.sum, n.mean, n.rstd, gamma, h, w, beta, b});
     ctx->saved_data["y"] = y.defined();
+    ctx->saved_data["eps"] = eps;
     return {n.sum, qkv[0], qkv[1], qkv[2]};   // without y the sum is the input itself
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
     const Tensor &x = s[0], &gamma = s[3], &h = s[4], &w = s[5];
     c10::cuda::CUDAGuard dg(x.device());
     const int64_t batch = x.size(0), seq = x.size(1), width = x.size(2);
     const int64_t heads = g[1].size(1), hd = g[1].size(3), rows = batch * seq, n3 = 3 * heads * hd;
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(x), viewOf(gamma), viewOf(s[6]), viewOf(w), viewOf(s[7])};
+      const Tensor n = at::layer_norm(in[0], {width}, in[1], in[2], ctx->saved_data["eps"].toDouble());
+      const Tensor qkv = at::linear(n, in[3], in[4]).view({batch, seq, 3, heads, hd}).permute({2, 0, 3, 1, 4});
+      const variable_list r = recorded({qkv[0], qkv[1], qkv[2]}, {g[1], g[2], g[3]}, in);
+      const Tensor dx = plus(g[0], r[0]);
+      return {dx, ctx->saved_data["y"].toBool() ? dx : Tensor(), r[1], r[2], r[3], r[4], Tensor(), Tensor()};
+    }
     Tensor dqkv = at::empty({rows, n3}, x.options());
     const int sp = train::stripPartials(rows);
     Tensor bias_parts = floats(x, {sp, n3});
@@ -184,17 +220,24 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     Tensor act = at::empty_like(u);
     ok(train::geluForward(code(u), u.data_ptr(), act.data_ptr(), u.numel(), streamOf(u)), "gelu");
     const Tensor y = at::addmm(bo, act, wo.t()).view(x.sizes());
-    ctx->save_for_backward({a, wp, n.sum, n.mean, n.rstd, gamma, h, wf, u, act, wo});
-    ctx->saved_data["a"] = a_.sizes().vec();
+    ctx->save_for_backward({a_, wp, n.sum, n.mean, n.rstd, gamma, h, wf, u, act, wo, beta, bf, bo});
+    ctx->saved_data["eps"] = eps;
     return {n.sum, y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &a = s[0], &wp = s[1], &x2 = s[2], &gamma = s[5], &h = s[6], &wf = s[7], &act = s[9], &wo = s[10];
-    const Tensor u = dense(s[8]);
+    const Tensor &wp = s[1], &x2 = s[2], &gamma = s[5], &h = s[6], &wf = s[7], &act = s[9], &wo = s[10];
     c10::cuda::CUDAGuard dg(x2.device());
-    const int64_t width = x2.size(-1), rows = x2.numel() / width, hidden = u.size(1);
+    const int64_t width = x2.size(-1), rows = x2.numel() / width;
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(x2), viewOf(gamma), viewOf(s[11]), viewOf(wf), viewOf(s[12]), viewOf(wo), viewOf(s[13])};
+      const Tensor n = at::layer_norm(in[0], {width}, in[1], in[2], ctx->saved_data["eps"].toDouble());
+      const variable_list r = recorded({at::linear(at::gelu(at::linear(n, in[3], in[4]), "tanh"), in[5], in[6])}, {g[1]}, in);
+      const Tensor dx = plus(g[0], r[0]), d = dx.reshape({rows, width}), a = s[0].reshape({rows, -1});
+      return {dx, at::mm(d, wp).view(s[0].sizes()), at::mm(d.t(), a), d.sum(0), r[1], r[2], r[3], r[4], r[5], r[6], Tensor()};
+    }
+    const Tensor a = rowsOf(s[0]), u = dense(s[8]);
+    const int64_t hidden = u.size(1);
     const int dt = code(x2), sp = train::stripPartials(rows);
     cudaStream_t st = streamOf(x2);
     TORCH_CHECK(g[1].defined(), "hylink: the block's branch has no gradient");
@@ -212,7 +255,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     Tensor dx = normBackward(dh, x2, s[3], s[4], gamma, dense(g[0]), true, &parts, &np);
     const Tensor dxr = dx.view({rows, width});
     Tensor dwp = at::mm(dxr.t(), a);
-    Tensor da = at::mm(dxr, wp).view(ctx->saved_data["a"].toIntVector());
+    Tensor da = at::mm(dxr, wp).view(s[0].sizes());
     Columns cols(gamma);
     const float* p = parts.data_ptr<float>();
     Tensor dgamma = cols.add(p, np, width), dbeta = cols.add(p + np * width, np, width), dbp = cols.add(p + 2 * np * width, np, width);
@@ -261,25 +304,29 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
     ok(train::crossEntropyForward(code(h), logits.data_ptr(), padded, targets.data_ptr<int64_t>(), rows, (int)vocab, -100, lse.data_ptr<float>(),
                                   row_loss.data_ptr<float>(), loss.data_ptr<float>(), streamOf(h)),
        "cross entropy");
-    ctx->save_for_backward({h, wpad, targets, logits, lse, loss});
-    ctx->saved_data["vocab"] = vocab;
-    ctx->saved_data["h"] = h_.sizes().vec();
+    ctx->save_for_backward({h_, wpad, targets, logits, lse, loss, w});
     return loss.select(0, 0).clone();
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
-    const Tensor &h = s[0], &wpad = s[1], &targets = s[2], &lse = s[4], &loss = s[5];
-    const Tensor logits = dense(s[3]);
-    c10::cuda::CUDAGuard dg(h.device());
-    const int64_t vocab = ctx->saved_data["vocab"].toInt();
+    const Tensor &wpad = s[1], &targets = s[2], &lse = s[4], &loss = s[5];
+    c10::cuda::CUDAGuard dg(s[0].device());
+    const int64_t vocab = s[6].size(0);
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(s[0]), viewOf(s[6])};
+      const Tensor z = at::linear(in[0], in[1]).to(at::kFloat).reshape({-1, vocab});
+      variable_list r = recorded({at::cross_entropy_loss(z, targets, {}, at::Reduction::Mean, -100)}, g, in);
+      r.emplace_back();
+      return r;
+    }
+    const Tensor h = rowsOf(s[0]), logits = dense(s[3]);
     const Tensor grad = g[0].to(at::kFloat).contiguous();
     Tensor dlogits = at::empty_like(logits);
     ok(train::crossEntropyBackward(code(h), logits.data_ptr(), logits.size(1), targets.data_ptr<int64_t>(), h.size(0), (int)vocab, -100,
                                    lse.data_ptr<float>(), loss.data_ptr<float>(), grad.data_ptr<float>(), dlogits.data_ptr(), streamOf(h)),
        "cross entropy backward");
     Tensor dw = at::mm(dlogits.narrow(1, 0, vocab).t(), h);
-    Tensor dh = headInputGradient(dlogits, wpad, vocab).view(ctx->saved_data["h"].toIntVector());
+    Tensor dh = headInputGradient(dlogits, wpad, vocab).view(s[0].sizes());
     return {dh, dw, Tensor()};
   }
 };
@@ -356,6 +403,19 @@ std::pair<Tensor, Tensor> moeCombinedBackward(const Tensor& dy, const Tensor& ga
   return {drows, dgate};
 }
 
+// The same as plain operations, for a recorded backward pass: with the routing as it was chosen.
+Tensor plainGate(const Tensor& x, const Tensor& router, const Tensor& expert) {
+  return at::softmax(at::linear(x, router).to(at::kFloat), -1).gather(1, expert.to(at::kLong).unsqueeze(1)).squeeze(1);
+}
+Tensor plainRows(const Tensor& from, const Tensor& index) {
+  const Tensor i = index.to(at::kLong);
+  return from.index_select(0, i.clamp_min(0)).masked_fill((i < 0).unsqueeze(1), 0);
+}
+Tensor plainExperts(const Tensor& h, const Tensor& w1, const Tensor& w2) { return at::bmm(at::gelu(at::bmm(h, w1), "tanh"), w2); }
+Tensor plainCombined(const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of) {
+  return x + gate.unsqueeze(1).to(x.scalar_type()) * plainRows(rows.reshape({-1, x.size(1)}), row_of);
+}
+
 // The whole layer where the experts are all here: one node instead of a dozen. (Host time of a layer of 1072 tokens,
 // forward and backward: 300 us in pieces, 210 in one.)
 class MoeLayer : public torch::autograd::Function<MoeLayer> {
@@ -366,15 +426,21 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const Routed r = moeRouted(x, router, capacity);
     const Tensor h = r.send.view({router.size(0), capacity, x.size(1)});
     const Expert e = moeExpert(h, w1, w2);
-    ctx->save_for_backward({x, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out});
+    ctx->save_for_backward({x_, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out});
     return moeCombined(x, r.gate, e.out, r.row_of);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
     const Tensor &router = s[1], &w1 = s[2], &w2 = s[3], &h = s[9];
+    c10::cuda::CUDAGuard dg(s[0].device());
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(s[0]), viewOf(router), viewOf(w1), viewOf(w2)};
+      const Tensor out = plainExperts(plainRows(in[0], s[8]).view(h.sizes()), in[2], in[3]);
+      variable_list r = recorded({plainCombined(in[0], plainGate(in[0], in[1], s[5]), out, s[7])}, g, in);
+      r.emplace_back();
+      return r;
+    }
     const Tensor x = dense(s[0]), rows = dense(s[12]);
-    c10::cuda::CUDAGuard dg(x.device());
     const Tensor dy = dense(g[0]);
     const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8]);
     const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows);
@@ -391,17 +457,21 @@ class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
     c10::cuda::CUDAGuard dg(x_.device());
     const Tensor x = dense(x_);
     const Routed r = moeRouted(x, router, capacity);
-    ctx->save_for_backward({x, router, r.logits, r.expert, r.gate, r.row_of});
+    ctx->save_for_backward({x_, router, r.logits, r.expert, r.gate, r.row_of, r.token_of});
     ctx->saved_data["rows"] = router.size(0) * capacity;
     ctx->mark_non_differentiable({r.row_of, r.token_of});
     ctx->set_materialize_grads(false);
     return {x, r.send, r.gate, r.row_of, r.token_of};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
+    c10::cuda::CUDAGuard dg(s[0].device());
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(s[0]), viewOf(s[1])};
+      const variable_list r = recorded({plainRows(in[0], s[6]), plainGate(in[0], in[1], s[3])}, {g[1], g[2]}, in);
+      return {plus(g[0], r[0]), r[1], Tensor()};
+    }
     const Tensor x = dense(s[0]), &gate = s[4];
-    c10::cuda::CUDAGuard dg(x.device());
     const Tensor dres = g[0].defined() ? dense(g[0]) : Tensor();
     const Tensor dsend = g[1].defined() ? dense(g[1]) : at::zeros({ctx->saved_data["rows"].toInt(), x.size(1)}, x.options());
     const Tensor dgate = g[2].defined() ? dense(g[2]) : at::zeros_like(gate);
@@ -420,9 +490,12 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
     return e.out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
     c10::cuda::CUDAGuard dg(s[0].device());
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(s[0]), viewOf(s[1]), viewOf(s[2])};
+      return recorded({plainExperts(in[0], in[1], in[2])}, g, in);
+    }
     return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]));
   }
 };
@@ -434,13 +507,17 @@ class MoeCombine : public torch::autograd::Function<MoeCombine> {
                           const Variable& token_of) {
     c10::cuda::CUDAGuard dg(x_.device());
     const Tensor x = dense(x_), rows = dense(rows_);
-    ctx->save_for_backward({gate, rows, token_of});
+    ctx->save_for_backward({gate, rows_, token_of, row_of});
     return moeCombined(x, gate, rows, row_of);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    onceOnly();
     const auto s = ctx->get_saved_variables();
     c10::cuda::CUDAGuard dg(s[1].device());
+    if (wantsGraph()) {
+      const variable_list in = {viewOf(s[0]), viewOf(s[1])};
+      const variable_list r = recorded({plainCombined(at::zeros_like(g[0]), in[0], in[1], s[3])}, g, in);
+      return {g[0], r[0], r[1], Tensor(), Tensor()};
+    }
     const Tensor dy = dense(g[0]);
     const auto [drows, dgate] = moeCombinedBackward(dy, s[0], dense(s[1]), s[2]);
     return {dy, dgate, drows, Tensor(), Tensor()};

@@ -265,6 +265,26 @@ def test_transforms_and_modes_see_the_modules():
         assert model._fusable(torch.empty(1, dtype=torch.bfloat16), targets)
 
 
+def test_a_step_can_be_differentiated_again():
+    """The gradient of the squared length of the gradient; the same gradients with a graph behind them."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+
+    def penalty(model, idx, targets):
+        model.zero_grad(set_to_none=True)
+        with sdpa_kernel(SDPBackend.MATH):
+            loss = model(idx, targets)
+            grads = torch.autograd.grad(loss, list(model.parameters()), create_graph=True)
+            sum(g.float().square().sum() for g in grads).backward()
+        return [g.detach().float() for g in grads], [p.grad.float() for p in model.parameters()]
+
+    model, idx, targets = _small()
+    ref = copy.deepcopy(model).float()
+    names = [n for n, _ in model.named_parameters()]
+    for tol, got, want in zip((2e-2, 5e-2), penalty(model, idx, targets), penalty(ref, idx, targets)):
+        for n, a, b in zip(names, got, want):
+            assert float((a - b).norm()) <= tol * float(b.norm()) + 1e-4, n
+
+
 def _counted(module, seen):
     plain = module.forward
     module.forward = lambda *a: (seen.append(1), plain(*a))[1]

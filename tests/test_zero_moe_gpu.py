@@ -179,3 +179,33 @@ def test_moe_under_modes_and_hooks_runs_as_modules():
     finally:
         handle.remove()
     assert layer.router in calls
+
+
+@pytest.mark.parametrize("pieces", [False, True])
+def test_moe_can_be_differentiated_again(pieces):
+    """A gradient penalty, against the same layer as modules; the third expert overflows."""
+    import copy
+
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+
+    torch.manual_seed(3)
+    layer = ExpertParallelMLP(64, 128, experts_per_rank=4, capacity=9).cuda().to(torch.bfloat16)
+    with torch.no_grad():
+        layer.router.weight.mul_(4)
+        layer.w1.mul_(5)
+        layer.w2.mul_(5)
+    if pieces:
+        layer.w1.data = layer.w1.data.float()
+    plain = copy.deepcopy(layer)
+    plain._fusable = lambda x: False
+    x0, dy = (torch.randn(40, 64, device="cuda").to(torch.bfloat16) for _ in range(2))
+    results = []
+    for m in (layer, plain):
+        x = x0.clone().requires_grad_()
+        assert m is plain or m._fusable(x)
+        y = m(x * 1)                                 # not a leaf
+        grads = torch.autograd.grad(y, [x, *m.parameters()], dy, create_graph=True)
+        sum(g.float().square().sum() for g in grads).backward()
+        results.append([*(g.detach().float() for g in grads), x.grad.float(), *(p.grad.float() for p in m.parameters())])
+    for i, (a, b) in enumerate(zip(*results)):       # the plain layer rounds every step to 16 bits, the dot products of the gate among them
+        assert float((a - b).norm()) <= 3e-2 * float(b.norm()) + 1e-6, i
