@@ -74,6 +74,15 @@ variable_list recorded(const variable_list& outs, const variable_list& grads, co
 }
 Tensor plus(const Tensor& a, const Tensor& b) { return a.defined() ? (b.defined() ? a + b : a) : b; }
 
+// Whether any of the inputs [from, to] of a node (its tensors in order, absent ones not counted) is to get a gradient: the
+// products of frozen weights are left out.
+bool needed(AutogradContext* ctx, size_t from, size_t to) {
+  for (size_t i = from; i <= to; ++i)
+    if (ctx->needs_input_grad(i)) return true;
+  return false;
+}
+bool needed(AutogradContext* ctx, size_t i) { return needed(ctx, i, i); }
+
 // Column-sum partials collected over a backward pass and added up in one launch.
 class Columns {
  public:
@@ -191,14 +200,17 @@ class BlockPre : public torch::autograd::Function<BlockPre> {
     }
     ok(train::packQkvGradient(code(x), gs, dqkv.data_ptr(), bias_parts.data_ptr<float>(), batch, seq, (int)heads, (int)hd, streamOf(x)),
        "attention gradient");
-    Tensor dw = at::mm(dqkv.t(), h);
-    Tensor dh = at::mm(dqkv, w);
-    Tensor parts;
-    int np;
-    Tensor dx = normBackward(dh, x, s[1], s[2], gamma, dense(g[0]), false, &parts, &np);
+    const size_t y = ctx->saved_data["y"].toBool();
+    Tensor dw, dx, dgamma, dbeta, parts;
+    if (needed(ctx, 3 + y)) dw = at::mm(dqkv.t(), h);
     Columns cols(gamma);
-    const float* p = parts.data_ptr<float>();
-    Tensor dgamma = cols.add(p, np, width), dbeta = cols.add(p + np * width, np, width);
+    if (needed(ctx, 0, 2 + y)) {
+      int np;
+      dx = normBackward(at::mm(dqkv, w), x, s[1], s[2], gamma, dense(g[0]), false, &parts, &np);
+      const float* p = parts.data_ptr<float>();
+      dgamma = cols.add(p, np, width);
+      dbeta = cols.add(p + np * width, np, width);
+    }
     Tensor db = cols.add(bias_parts.data_ptr<float>(), sp, n3);
     cols.finish();
     return {dx, ctx->saved_data["y"].toBool() ? dx : Tensor(), dgamma, dbeta, dw, db, Tensor(), Tensor()};
@@ -242,24 +254,30 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     cudaStream_t st = streamOf(x2);
     TORCH_CHECK(g[1].defined(), "hylink: the block's branch has no gradient");
     const Tensor gy = rowsOf(g[1]);
-    Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {sp, hidden});
-    ok(train::columnSums(dt, gy.data_ptr(), out_parts.data_ptr<float>(), rows, (int)width, st), "bias gradient");
-    Tensor dact = at::mm(gy, wo);
-    Tensor dwo = at::mm(gy.t(), act);
-    Tensor du = at::empty_like(u);
-    ok(train::geluBackward(dt, dact.data_ptr(), u.data_ptr(), du.data_ptr(), fc_parts.data_ptr<float>(), rows, (int)hidden, st), "gelu backward");
-    Tensor dwf = at::mm(du.t(), h);
-    Tensor dh = at::mm(du, wf);
-    Tensor parts;
-    int np;
-    Tensor dx = normBackward(dh, x2, s[3], s[4], gamma, dense(g[0]), true, &parts, &np);
-    const Tensor dxr = dx.view({rows, width});
-    Tensor dwp = at::mm(dxr.t(), a);
-    Tensor da = at::mm(dxr, wp).view(s[0].sizes());
+    Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {sp, hidden}), parts;
+    Tensor dwo, dwf, dwp, da, dx, dgamma, dbeta, dbp, dbf;
     Columns cols(gamma);
-    const float* p = parts.data_ptr<float>();
-    Tensor dgamma = cols.add(p, np, width), dbeta = cols.add(p + np * width, np, width), dbp = cols.add(p + 2 * np * width, np, width);
-    Tensor dbf = cols.add(fc_parts.data_ptr<float>(), sp, hidden), dbo = cols.add(out_parts.data_ptr<float>(), sp, width);
+    ok(train::columnSums(dt, gy.data_ptr(), out_parts.data_ptr<float>(), rows, (int)width, st), "bias gradient");
+    Tensor dbo = cols.add(out_parts.data_ptr<float>(), sp, width);
+    if (needed(ctx, 8)) dwo = at::mm(gy.t(), act);
+    if (needed(ctx, 0, 7)) {
+      Tensor dact = at::mm(gy, wo);
+      Tensor du = at::empty_like(u);
+      ok(train::geluBackward(dt, dact.data_ptr(), u.data_ptr(), du.data_ptr(), fc_parts.data_ptr<float>(), rows, (int)hidden, st), "gelu backward");
+      dbf = cols.add(fc_parts.data_ptr<float>(), sp, hidden);
+      if (needed(ctx, 6)) dwf = at::mm(du.t(), h);
+      if (needed(ctx, 0, 5)) {
+        int np;
+        dx = normBackward(at::mm(du, wf), x2, s[3], s[4], gamma, dense(g[0]), true, &parts, &np);
+        const Tensor dxr = dx.view({rows, width});
+        if (needed(ctx, 2)) dwp = at::mm(dxr.t(), a);
+        if (needed(ctx, 1)) da = at::mm(dxr, wp).view(s[0].sizes());
+        const float* p = parts.data_ptr<float>();
+        dgamma = cols.add(p, np, width);
+        dbeta = cols.add(p + np * width, np, width);
+        dbp = cols.add(p + 2 * np * width, np, width);
+      }
+    }
     cols.finish();
     return {dx, da, dwp, dbp, dgamma, dbeta, dwf, dbf, dwo, dbo, Tensor()};
   }
@@ -325,8 +343,9 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
     ok(train::crossEntropyBackward(code(h), logits.data_ptr(), logits.size(1), targets.data_ptr<int64_t>(), h.size(0), (int)vocab, -100,
                                    lse.data_ptr<float>(), loss.data_ptr<float>(), grad.data_ptr<float>(), dlogits.data_ptr(), streamOf(h)),
        "cross entropy backward");
-    Tensor dw = at::mm(dlogits.narrow(1, 0, vocab).t(), h);
-    Tensor dh = headInputGradient(dlogits, wpad, vocab).view(s[0].sizes());
+    Tensor dw, dh;
+    if (needed(ctx, 1)) dw = at::mm(dlogits.narrow(1, 0, vocab).t(), h);
+    if (needed(ctx, 0)) dh = headInputGradient(dlogits, wpad, vocab).view(s[0].sizes());
     return {dh, dw, Tensor()};
   }
 };
@@ -351,9 +370,9 @@ Routed moeRouted(const Tensor& x, const Tensor& router, int64_t capacity) {
   ok(train::moeGather(x.data_ptr(), r.token_of.data_ptr<int>(), r.send.data_ptr(), (int)(experts * capacity), (int)width, streamOf(x)), "MoE dispatch");
   return r;
 }
-// {dx, drouter}; dres may be undefined.
+// {dx, drouter (where it is needed)}; dres may be undefined.
 std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& router_, const Tensor& logits, const Tensor& expert, const Tensor& gate,
-                                            const Tensor& row_of, const Tensor& dres, const Tensor& dsend, const Tensor& dgate) {
+                                            const Tensor& row_of, const Tensor& dres, const Tensor& dsend, const Tensor& dgate, bool router_needed) {
   const Tensor router = dense(router_);
   const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
   Tensor dx = at::empty_like(x), dlogits = at::empty_like(logits);
@@ -362,7 +381,7 @@ std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& route
                              dlogits.data_ptr(), (int)tokens, (int)width, (int)experts, streamOf(x)),
      "MoE token gradient");
   if (!train::moeRouterFits((int)experts)) dx.addmm_(dlogits, router);
-  return {dx, at::mm(dlogits.t(), x)};
+  return {dx, router_needed ? at::mm(dlogits.t(), x) : Tensor()};
 }
 struct Expert {
   Tensor u, act, out;
@@ -375,16 +394,21 @@ Expert moeExpert(const Tensor& h, const Tensor& w1, const Tensor& w2) {
   e.out = at::bmm(e.act, w2);
   return e;
 }
-// {dh, dw1, dw2}
-variable_list moeExpertBackward(const Tensor& h, const Tensor& w1, const Tensor& w2, const Tensor& u_, const Tensor& act, const Tensor& dout) {
-  Tensor dact = at::bmm(dout, w2.transpose(1, 2));
-  Tensor dw2 = at::bmm(act.transpose(1, 2), dout);
-  const Tensor u = dense(u_);
-  Tensor du = at::empty_like(u);
-  ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
-     "gelu backward");
-  Tensor dw1 = at::bmm(h.transpose(1, 2), du);
-  return {at::bmm(du, w1.transpose(1, 2)), dw1, dw2};
+// {dh, dw1, dw2}, those that are needed
+variable_list moeExpertBackward(const Tensor& h, const Tensor& w1, const Tensor& w2, const Tensor& u_, const Tensor& act, const Tensor& dout, bool h_needed,
+                                bool w1_needed, bool w2_needed) {
+  Tensor dh, dw1, dw2;
+  if (w2_needed) dw2 = at::bmm(act.transpose(1, 2), dout);
+  if (h_needed || w1_needed) {
+    Tensor dact = at::bmm(dout, w2.transpose(1, 2));
+    const Tensor u = dense(u_);
+    Tensor du = at::empty_like(u);
+    ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
+       "gelu backward");
+    if (w1_needed) dw1 = at::bmm(h.transpose(1, 2), du);
+    if (h_needed) dh = at::bmm(du, w1.transpose(1, 2));
+  }
+  return {dh, dw1, dw2};
 }
 Tensor moeCombined(const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of) {
   Tensor y = at::empty_like(x);
@@ -443,8 +467,10 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const Tensor x = dense(s[0]), rows = dense(s[12]);
     const Tensor dy = dense(g[0]);
     const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8]);
-    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows);
-    const auto [dx, drouter] = moeRoutedBackward(x, router, s[4], s[5], s[6], s[7], dy, e[0], dgate);
+    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, needed(ctx, 0), needed(ctx, 2), needed(ctx, 3));
+    if (!needed(ctx, 0, 1)) return {Tensor(), Tensor(), e[1], e[2], Tensor()};
+    const Tensor dsend = e[0].defined() ? e[0] : at::zeros_like(h);   // the router alone
+    const auto [dx, drouter] = moeRoutedBackward(x, router, s[4], s[5], s[6], s[7], dy, dsend, dgate, needed(ctx, 1));
     return {dx, drouter, e[1], e[2], Tensor()};
   }
 };
@@ -475,7 +501,7 @@ class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
     const Tensor dres = g[0].defined() ? dense(g[0]) : Tensor();
     const Tensor dsend = g[1].defined() ? dense(g[1]) : at::zeros({ctx->saved_data["rows"].toInt(), x.size(1)}, x.options());
     const Tensor dgate = g[2].defined() ? dense(g[2]) : at::zeros_like(gate);
-    const auto [dx, drouter] = moeRoutedBackward(x, s[1], s[2], s[3], gate, s[5], dres, dsend, dgate);
+    const auto [dx, drouter] = moeRoutedBackward(x, s[1], s[2], s[3], gate, s[5], dres, dsend, dgate, needed(ctx, 1));
     return {dx, drouter, Tensor()};
   }
 };
@@ -496,7 +522,7 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
       const variable_list in = {viewOf(s[0]), viewOf(s[1]), viewOf(s[2])};
       return recorded({plainExperts(in[0], in[1], in[2])}, g, in);
     }
-    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]));
+    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), needed(ctx, 0), needed(ctx, 1), needed(ctx, 2));
   }
 };
 

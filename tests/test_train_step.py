@@ -285,6 +285,36 @@ def test_a_step_can_be_differentiated_again():
             assert float((a - b).norm()) <= tol * float(b.norm()) + 1e-4, n
 
 
+# frozen parameters by the end of their name, and how many of the step's products for gradients remain: 2 blocks x 8 and the head's 2
+@pytest.mark.parametrize("frozen,products", [([], 18), (["fc.weight", "out.weight", "qkv.weight", "proj.weight"], 10), (["wte.weight", "wpe.weight"], 17),
+                                             (["blocks."], 10), (["wte.weight", "wpe.weight", "blocks."], 1)])
+def test_products_of_frozen_weights_are_left_out(frozen, products):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Products(TorchDispatchMode):
+        count = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.count += func is torch.ops.aten.mm.default
+            return func(*args, **(kwargs or {}))
+
+    model, idx, targets = _small()
+    _, want = _grads(model, idx, targets)
+    model.zero_grad(set_to_none=True)
+    left = []
+    for n, p in model.named_parameters():
+        p.requires_grad_(not any(f in n for f in frozen))
+        left += [n] * p.requires_grad
+    loss = model(idx, targets)
+    with Products() as seen:
+        loss.backward()
+    assert seen.count == products
+    for n, p in model.named_parameters():
+        assert (p.grad is None) == (n not in left)
+        if n in left and n != "wte.weight":
+            assert torch.equal(p.grad.float(), want[n]), n
+
+
 def _counted(module, seen):
     plain = module.forward
     module.forward = lambda *a: (seen.append(1), plain(*a))[1]

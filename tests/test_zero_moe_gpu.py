@@ -209,3 +209,34 @@ def test_moe_can_be_differentiated_again(pieces):
         results.append([*(g.detach().float() for g in grads), x.grad.float(), *(p.grad.float() for p in m.parameters())])
     for i, (a, b) in enumerate(zip(*results)):       # the plain layer rounds every step to 16 bits, the dot products of the gate among them
         assert float((a - b).norm()) <= 3e-2 * float(b.norm()) + 1e-6, i
+
+
+@pytest.mark.parametrize("frozen,products", [([], 4), (["w1", "w2"], 2), (["x"], 3), (["x", "router.weight"], 3), (["x", "router.weight", "w1"], 1),
+                                             (["x", "w1", "w2"], 0)])
+def test_moe_leaves_the_products_of_frozen_weights_out(frozen, products):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+
+    class Products(TorchDispatchMode):
+        count = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.count += func is torch.ops.aten.bmm.default
+            return func(*args, **(kwargs or {}))
+
+    torch.manual_seed(5)
+    layer = ExpertParallelMLP(64, 128, experts_per_rank=4, capacity=12).cuda().to(torch.bfloat16)
+    x, dy = (torch.randn(40, 64, device="cuda").to(torch.bfloat16) for _ in range(2))
+    leaves = {"x": x, **dict(layer.named_parameters())}
+    for t in leaves.values():
+        t.requires_grad_(True)
+    want = dict(zip(leaves, torch.autograd.grad(layer(x), list(leaves.values()), dy)))
+    for n, t in leaves.items():
+        t.requires_grad_(n not in frozen)
+    y = layer(x)
+    with Products() as seen:
+        y.backward(dy)
+    assert seen.count == products
+    for n, t in leaves.items():
+        assert t.grad is None if n in frozen else torch.equal(t.grad, want[n]), n
