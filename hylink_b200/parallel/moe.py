@@ -79,9 +79,12 @@ class ExpertParallelMLP(nn.Module):
         return y
 
     def _fusable(self, x) -> bool:
-        """16-bit tokens on a GPU, a plain router of the same type (its own `forward`, no hooks), rows of whole 16-byte packets."""
+        """16-bit tokens on a GPU, a plain router of the same type (its class's `forward`, no hooks), rows of whole 16-byte
+        packets, no more tokens and slots than the kernels take."""
         r = self.router
+        slots = self.n_experts * self.cap
         return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.shape[0] > 0 and x.shape[1] % 8 == 0
+                and 0 < slots <= ops().max_rows and x.shape[0] <= ops().max_rows and r.weight.shape[0] == self.n_experts
                 and self.w1.shape[2] % 8 == 0 and type(r) is nn.Linear and r.bias is None and r.weight.dtype == x.dtype
                 and not overridden(r) and not global_module_hooks() and plain_eager(x, r.weight, self.w1, self.w2)
                 and not torch.is_autocast_enabled("cuda"))

@@ -240,3 +240,16 @@ def test_moe_leaves_the_products_of_frozen_weights_out(frozen, products):
     assert seen.count == products
     for n, t in leaves.items():
         assert t.grad is None if n in frozen else torch.equal(t.grad, want[n]), n
+
+
+def test_sizes_beyond_the_moe_kernels_run_as_modules():
+    from hylink_b200.ops.extension import ops
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+
+    layer = ExpertParallelMLP(64, 128, experts_per_rank=4, capacity=5).cuda().to(torch.bfloat16)
+    x = torch.randn(10, 64, device="cuda", dtype=torch.bfloat16)
+    for capacity, fits in ((0, False), (5, True), (ops().max_rows // 4, True), (ops().max_rows // 4 + 1, False)):
+        layer.cap = capacity
+        assert layer._fusable(x) == fits
+    layer.cap, layer.n_experts = 5, 3
+    assert not layer._fusable(x)
