@@ -485,7 +485,10 @@ class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
     const Routed r = moeRouted(x, router, capacity);
     ctx->save_for_backward({x_, router, r.logits, r.expert, r.gate, r.row_of, r.token_of});
     ctx->saved_data["rows"] = router.size(0) * capacity;
-    ctx->mark_non_differentiable({r.row_of, r.token_of});
+    // Without a gradient for the tokens the exchange of the rows needs none either, and a rank that takes the plain path (one
+    // without tokens) must find its peers in as many exchanges as it has itself.
+    if (x_.requires_grad()) ctx->mark_non_differentiable({r.row_of, r.token_of});
+    else ctx->mark_non_differentiable({r.row_of, r.token_of, r.send});
     ctx->set_materialize_grads(false);
     return {x, r.send, r.gate, r.row_of, r.token_of};
   }

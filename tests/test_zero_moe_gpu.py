@@ -253,3 +253,16 @@ def test_sizes_beyond_the_moe_kernels_run_as_modules():
         assert layer._fusable(x) == fits
     layer.cap, layer.n_experts = 5, 3
     assert not layer._fusable(x)
+
+
+@pytest.mark.parametrize("wanted", [False, True])
+def test_dispatched_rows_want_a_gradient_when_the_tokens_do(wanted):
+    """As on the plain path: every rank then takes part in the same number of exchanges, whichever path it is on."""
+    from hylink_b200.ops.extension import ops
+
+    x = torch.randn(10, 64, device="cuda", dtype=torch.bfloat16).requires_grad_(wanted)
+    router = torch.randn(4, 64, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    _, send, gate, row_of, token_of = ops().moe_dispatch(x, router, 5)
+    assert send.requires_grad == wanted and gate.requires_grad and not row_of.requires_grad and not token_of.requires_grad
+    gate.sum().backward()
+    assert bool(router.grad.isfinite().all()) and (x.grad is not None) == wanted
