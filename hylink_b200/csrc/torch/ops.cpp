@@ -417,9 +417,9 @@ Tensor moeCombined(const Tensor& x, const Tensor& gate, const Tensor& rows, cons
      "MoE combine");
   return y;
 }
-// {drows, dgate}; dgate: only tokens with a row are written, and read
+// {drows, dgate}; dgate is zero for tokens without a row: autograd's anomaly check and hooks read all of it
 std::pair<Tensor, Tensor> moeCombinedBackward(const Tensor& dy, const Tensor& gate, const Tensor& rows, const Tensor& token_of) {
-  Tensor drows = at::empty_like(rows), dgate = at::empty_like(gate);
+  Tensor drows = at::empty_like(rows), dgate = at::zeros_like(gate);
   const int width = (int)rows.size(-1);
   ok(train::moeRowGradient(code(rows), dy.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), token_of.data_ptr<int>(), drows.data_ptr(),
                            dgate.data_ptr<float>(), (int)(rows.numel() / width), width, streamOf(rows)),

@@ -266,3 +266,18 @@ def test_dispatched_rows_want_a_gradient_when_the_tokens_do(wanted):
     assert send.requires_grad == wanted and gate.requires_grad and not row_of.requires_grad and not token_of.requires_grad
     gate.sum().backward()
     assert bool(router.grad.isfinite().all()) and (x.grad is not None) == wanted
+
+
+def test_the_gates_gradient_is_whole():
+    """Zero for a token beyond the capacity, whatever the memory held before."""
+    from hylink_b200.ops.extension import ops
+
+    x = torch.randn(40, 64, device="cuda", dtype=torch.bfloat16)
+    router = torch.randn(1, 64, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    x1, send, gate, row_of, token_of = ops().moe_dispatch(x, router, 5)
+    for _ in range(3):
+        trash = [torch.full((40,), float("nan"), device="cuda") for _ in range(8)]
+        del trash
+        y = ops().moe_combine(x1, gate, send, row_of, token_of)
+        dgate, = torch.autograd.grad(y, gate, torch.ones_like(y), retain_graph=True)
+        assert bool((dgate[row_of < 0] == 0).all()) and bool(dgate[row_of >= 0].isfinite().all())
