@@ -1,6 +1,6 @@
 // Routing, dispatch and combine of a top-1 mixture-of-experts layer with a fixed capacity per expert.
 //
-// moeRoute       a thread per token: the expert with the largest logit and its softmax probability (the gate)
+// moeRoute       a thread per token: the expert with the largest softmax probability, which is the gate
 // moeAssign      a CTA per expert: walks the tokens in order, numbers the expert's own by a scan over the CTA; a token's row is expert * capacity + number, or none beyond the capacity. The CTA also writes
 //                the inverse map (row -> token), so that everything after it can go by rows: every row of the dispatch
 //                buffer is then written exactly once, empty ones with zeros, and nothing needs clearing or atomics.
@@ -24,18 +24,22 @@ __global__ void __launch_bounds__(128) kMoeRoute(const T* __restrict__ logits, i
   if (t >= tokens) return;
   const T* p = logits + (int64_t)t * experts;
   float best = (float)p[0];
+  for (int e = 1; e < experts; ++e) best = fmaxf(best, (float)p[e]);
+  float sum = 0.f;
+  for (int e = 0; e < experts; ++e) sum += expf((float)p[e] - best);
+  // The maximum of the probabilities, as a softmax and a maximum give it: the first of equal ones (logits may differ and
+  // their probabilities not), and the first that is NaN (with a NaN or an infinite logit all of them are).
+  float top = expf((float)p[0] - best) / sum;
   int at = 0;
   for (int e = 1; e < experts; ++e) {
-    const float l = (float)p[e];
-    if (l > best) {   // the first of equal ones
-      best = l;
+    const float q = expf((float)p[e] - best) / sum;
+    if (q > top) {
+      top = q;
       at = e;
     }
   }
-  float sum = 0.f;
-  for (int e = 0; e < experts; ++e) sum += expf((float)p[e] - best);
   expert[t] = at;
-  gate[t] = 1.f / sum;
+  gate[t] = top;
 }
 
 constexpr int kAssignThreads = 1024, kAssignTokens = 4;   // four consecutive tokens per thread and sweep

@@ -281,3 +281,24 @@ def test_the_gates_gradient_is_whole():
         y = ops().moe_combine(x1, gate, send, row_of, token_of)
         dgate, = torch.autograd.grad(y, gate, torch.ones_like(y), retain_graph=True)
         assert bool((dgate[row_of < 0] == 0).all()) and bool(dgate[row_of >= 0].isfinite().all())
+
+
+def test_routing_of_equal_infinite_and_nan_logits():
+    """Expert and gate of every token are the maximum of the softmax, as torch finds it."""
+    from hylink_b200.ops.extension import ops
+
+    torch.manual_seed(6)
+    router, x = (torch.randn(n, 64, device="cuda") for n in (8, 40))
+    router[5] = router[2]                            # equal logits
+    x[:8] *= 1e-9                                    # different logits, one probability
+    x[8:16] *= 1e38                                  # infinite ones of either sign
+    x[16, 3], x[17, 9] = float("nan"), float("inf")
+    x[18] = 0
+    broken = router.clone()
+    broken[3, 0] = float("nan")                      # one expert's logits are NaN for every token
+    x = x.to(torch.bfloat16)
+    for w in (router.to(torch.bfloat16), broken.to(torch.bfloat16)):
+        want, expert = torch.softmax((x @ w.t()).float(), -1).max(-1)
+        _, _, gate, row_of, _ = ops().moe_dispatch(x, w, 40)
+        assert torch.equal(row_of.long() // 40, expert)
+        torch.testing.assert_close(gate, want, rtol=1e-6, atol=0, equal_nan=True)
