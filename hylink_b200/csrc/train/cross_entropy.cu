@@ -27,6 +27,12 @@ __global__ void __launch_bounds__(kCeThreads) kCrossEntropyForward(const T* __re
 #pragma unroll
     for (int i = 1; i < 8; ++i)
       if (i < n) top = fmaxf(top, f[i]);
+    if (top == -INFINITY) {   // nothing to add, unless one of them is NaN (exp(-inf - -inf) would be, in every case)
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < n && f[i] != -INFINITY) s = NAN;
+      return;
+    }
     if (top > m) {
       s *= __expf(m - top);
       m = top;
@@ -54,8 +60,8 @@ __global__ void __launch_bounds__(kCeThreads) kCrossEntropyForward(const T* __re
     take(f, 1);
   }
   const float wm = warpMax(m);
-  // a thread without logits, or one with only -inf, contributes nothing (and no NaN from inf - inf)
-  s = warpSum(m == -INFINITY ? 0.f : s * __expf(m - wm));
+  // under a maximum of -inf (no logits, or only -inf and NaN) the sum is zero or NaN already, and inf - inf not to be formed
+  s = warpSum(m == -INFINITY ? s : s * __expf(m - wm));
   if ((threadIdx.x & 31) == 0) {
     s_max[threadIdx.x >> 5] = wm;
     s_sum[threadIdx.x >> 5] = s;
@@ -65,7 +71,7 @@ __global__ void __launch_bounds__(kCeThreads) kCrossEntropyForward(const T* __re
     const bool in = threadIdx.x < kCeThreads / 32;
     const float wm2 = in ? s_max[threadIdx.x] : -INFINITY;
     const float top = warpMax(wm2);
-    const float total = warpSum(in && wm2 != -INFINITY ? s_sum[threadIdx.x] * __expf(wm2 - top) : 0.f);
+    const float total = warpSum(!in ? 0.f : (wm2 == -INFINITY ? s_sum[threadIdx.x] : s_sum[threadIdx.x] * __expf(wm2 - top)));
     if (threadIdx.x == 0) {
       const float z = top + logf(total);
       const int64_t t = targets[row];

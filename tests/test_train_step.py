@@ -136,6 +136,33 @@ def test_out_of_range_target_gives_nan_and_large_logits_stay_finite():
     assert bool(ops().head_loss(h, w, t).isnan())
 
 
+# all packets of a thread, or the first of several, a warp, a row; a value among others, a packet of them
+@pytest.mark.parametrize("value", [float("-inf"), float("nan"), float("inf")])
+@pytest.mark.parametrize("vocab", [13, 4000, 4104 + 3])
+def test_infinite_and_nan_logits(value, vocab):
+    """Loss and gradient as the plain loss has them. With a unit vector for h the logits are the weight's first column."""
+    from hylink_b200.ops.extension import ops
+
+    torch.manual_seed(vocab)
+    base = torch.randn(vocab, device="cuda").to(torch.bfloat16)
+    h = torch.zeros(2, 8, device="cuda", dtype=torch.bfloat16)
+    h[:, 0] = 1
+    for lo, hi in ((0, 8), (0, 256), (3, 4), (8, 13), (0, vocab), (vocab - 1, vocab)):
+        w = torch.zeros(vocab, 8, device="cuda", dtype=torch.bfloat16)
+        w[:, 0] = base
+        w[lo:min(hi, vocab), 0] = value
+        for targets in ((1, vocab - 2), (lo, 9)):
+            t = torch.tensor(targets, device="cuda")
+            z = w[:, 0].float().expand(2, vocab).clone().requires_grad_()
+            want = torch.nn.functional.cross_entropy(z, t)
+            dz, = torch.autograd.grad(want, z)
+            wg = w.clone().requires_grad_()
+            got = ops().head_loss(h, wg, t)
+            dw, = torch.autograd.grad(got, wg)
+            torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5, equal_nan=True)
+            torch.testing.assert_close(dw[:, 0].float(), dz.to(torch.bfloat16).float().sum(0), rtol=2e-2, atol=1e-5, equal_nan=True)
+
+
 @pytest.mark.parametrize("name,batch,seq", [("tiny", 3, 64), ("gpt2-small", 2, 100)])
 def test_replayed_steps_train_like_eager_ones(name, batch, seq, monkeypatch):
     """Forward and backward from a graph from the second step on, against the same steps run eagerly: with a learning rate
