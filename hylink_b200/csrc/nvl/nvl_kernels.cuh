@@ -1330,9 +1330,6 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kZeroCopy(const HlCommDev* com
         }
       }
     } else {
-      // about eight packets per thread in flight; more of them means fewer warps or longer stalls between loading and
-      // storing (4 x 25 MiB emulated on one GPU: 37 us with eight, 39 with twelve)
-      constexpr int U = MR <= 2 ? 4 : (MR <= 4 ? 2 : 1);
       const uint4* pi[MR];
       uint4* po[MR];
 #pragma unroll
@@ -1341,32 +1338,40 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kZeroCopy(const HlCommDev* com
           pi[q] = reinterpret_cast<const uint4*>(c.heap[q] + a.zc_in_off) + first;
           po[q] = reinterpret_cast<uint4*>(c.heap[(r + q) % n] + a.zc_out_off) + first;
         }
-      for (uint64_t i = x.g0; i < cnt; i += x.gstride * U) {
-        uint4 v[U][MR];
+      auto fold = [&](auto unroll) {
+        constexpr int U = decltype(unroll)::value;
+        for (uint64_t i = x.g0; i < cnt; i += x.gstride * U) {
+          uint4 v[U][MR];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint64_t j = i + (uint64_t)u * x.gstride;
-          if (j < cnt) {
-#pragma unroll
-            for (int q = 0; q < MR; ++q)
-              if (q < n) v[u][q] = pi[q][j];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint64_t j = i + (uint64_t)u * x.gstride;
-          if (j < cnt) {
-            const uint4 red = reducePackets<W, MR>(v[u], n, a.op, a.scale, a.int_div);
-            if constexpr (kColl == kZcAllReduce) {
+          for (int u = 0; u < U; ++u) {
+            const uint64_t j = i + (uint64_t)u * x.gstride;
+            if (j < cnt) {
 #pragma unroll
               for (int q = 0; q < MR; ++q)
-                if (q < n) po[q][j] = red;
-            } else {
-              out_local[j] = red;
+                if (q < n) v[u][q] = pi[q][j];
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint64_t j = i + (uint64_t)u * x.gstride;
+            if (j < cnt) {
+              const uint4 red = reducePackets<W, MR>(v[u], n, a.op, a.scale, a.int_div);
+              if constexpr (kColl == kZcAllReduce) {
+#pragma unroll
+                for (int q = 0; q < MR; ++q)
+                  if (q < n) po[q][j] = red;
+              } else {
+                out_local[j] = red;
+              }
             }
           }
         }
-      }
+      };
+      // Ranks of one GPU: about eight packets per thread in flight; more of them means fewer warps or longer stalls between
+      // loading and storing (4 x 25 MiB: 37 us with eight, 39 with twelve). Between GPUs about a dozen: a load from a peer
+      // takes several times as long, and the kernel's figures there were taken with that.
+      if (c.one_device) fold(std::integral_constant<int, MR <= 2 ? 4 : (MR <= 4 ? 2 : 1)>());
+      else fold(std::integral_constant<int, MR <= 2 ? 6 : (MR <= 4 ? 3 : 2)>());
     }
   } else {
     // All-gather: this rank's input goes to segment r of every output. Broadcast: the root's input to every output; where

@@ -720,11 +720,12 @@ hlResult_t NvlPath::launchLowLatency(int kind, const NvlBufs& b, const NvlCall& 
   // messages spread over more and smaller CTAs: a packet is 2 (n - 1) stores and as many polls of its thread, and an
   // SM issues them one after the other; but every CTA costs its start. (8 ranks, 8 KiB, us with CTAs of 32 / 64 / 128 /
   // 256 threads: all-reduce in two hops 8.2 / 6.9 / 6.2 / 6.5; 64 KiB 8.2 / 8.2 / 8.2 / 9.5; 2 ranks, 8 KiB
-  // reduce-scatter 5.0 / 4.1 / 4.1.)
+  // reduce-scatter 5.0 / 4.1 / 4.1. Ranks of one GPU all of them; between GPUs, where this has not been timed, CTAs keep
+  // the most threads they can have.)
   int cap = c.max_blocks > 0 ? std::min(c.max_blocks, 148) : 148;
   if (Config::get().nvl_max_blocks > 0) cap = std::min(cap, Config::get().nvl_max_blocks);
   if (emu_) cap = std::min(cap, std::max(1, 148 / nranks_));
-  int threads = 128;
+  int threads = emu_ ? 128 : HL_LL_THREADS;
   while (threads < HL_LL_THREADS && packets > (uint64_t)cap * threads) threads *= 2;
   const uint64_t want = std::max<uint64_t>(1, (packets + threads - 1) / threads);
   const int blocks = (int)std::min<uint64_t>(want, (uint64_t)cap);
@@ -874,9 +875,11 @@ hlResult_t NvlPath::allToAll(const NvlBufs& b, const NvlCall& c, cudaStream_t s)
     if (ll < 0) return fail(hlUnsupported, "all-to-all: the low-latency kernel converts no types and needs a message that fits its slots");
     if (ll > 0) return launchLowLatency(kNvlLlAllToAll, b, c, (seg_wire + 15) / 16, s);
   }
-  // stores straight from the caller's buffer into the peers' staging, unless the call converts types or asks for the
-  // pull kernel by name; the own segment never touches the staging
-  const bool push = c.in_dt == c.wire_dt && c.out_dt == c.wire_dt && c.algo != hlAlgoTwoShotP2p;
+  // Between ranks of one GPU: stores straight from the caller's buffer into the peers' staging, unless the call converts
+  // types or asks for the pull kernel by name; the own segment never touches the staging. Between GPUs, where the two
+  // have not been timed against each other, only by name.
+  const bool same = c.in_dt == c.wire_dt && c.out_dt == c.wire_dt;
+  const bool push = same && (c.algo == hlAlgoPush || (emu_ && c.algo != hlAlgoTwoShotP2p));
   return launchSliced(push ? kNvlAllToAllPush : kNvlAllToAll, b, c, true, s);
 }
 
