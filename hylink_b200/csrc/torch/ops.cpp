@@ -671,9 +671,13 @@ PyObject* emuRun(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       TORCH_CHECK_TYPE(THPDtype_Check(args[8]), "hylink: the wire type is a torch.dtype");
       wire = typeCode(reinterpret_cast<THPDtype*>(args[8])->scalar_type);
     }
-    return (long)hlEmuCollective(reinterpret_cast<hlEmu_t>((uintptr_t)whole(args[0])), (int)whole(args[2]), bufs[0], bufs[1], (size_t)whole(args[5]),
-                                 (size_t)whole(args[6]), (size_t)whole(args[7]), dt[0], dt[1], wire, (int)whole(args[9]), (float)real(args[10]),
-                                 (int)whole(args[11]), (int)whole(args[12]), (int)whole(args[13]), c10::cuda::getCurrentCUDAStream().stream());
+    const hlEmu_t group = reinterpret_cast<hlEmu_t>((uintptr_t)whole(args[0]));
+    const int kind = (int)whole(args[2]), op = (int)whole(args[9]), root = (int)whole(args[11]), algo = (int)whole(args[12]), ctas = (int)whole(args[13]);
+    const size_t count = (size_t)whole(args[5]), in_stride = (size_t)whole(args[6]), out_stride = (size_t)whole(args[7]);
+    const float scale = (float)real(args[10]);
+    py::gil_scoped_release others;   // a launch waits while the stream's queue is full
+    return (long)hlEmuCollective(group, kind, bufs[0], bufs[1], count, in_stride, out_stride, dt[0], dt[1], wire, op, scale, root, algo, ctas,
+                                 c10::cuda::getCurrentCUDAStream().stream());
   });
 }
 
@@ -693,9 +697,14 @@ PyObject* reduceLanding(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
     const int accumulate = PyObject_IsTrue(args[4]);
     if (accumulate < 0) throw python_error();
-    return (long)hlReduceLanding(dst.data_ptr(), p.data(), (int)p.size(), accumulate != 0, (size_t)dst.numel(),
-                                 (hlDataType_t)typeCode(dst.scalar_type()), (hlRedOp_t)whole(args[2]), (float)real(args[3]), (int)whole(args[5]),
-                                 c10::cuda::getCurrentCUDAStream().stream());
+    void* const to = dst.data_ptr();
+    const size_t count = (size_t)dst.numel();
+    const auto type = (hlDataType_t)typeCode(dst.scalar_type());
+    const auto op = (hlRedOp_t)whole(args[2]);
+    const float scale = (float)real(args[3]);
+    const int ctas = (int)whole(args[5]);
+    py::gil_scoped_release others;
+    return (long)hlReduceLanding(to, p.data(), (int)p.size(), accumulate != 0, count, type, op, scale, ctas, c10::cuda::getCurrentCUDAStream().stream());
   });
 }
 PyMethodDef kNativeCalls[] = {{"emu_run", (PyCFunction)(void*)emuRun, METH_FASTCALL, nullptr},

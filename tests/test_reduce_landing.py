@@ -63,3 +63,62 @@ def test_pinned_host_source_and_unaligned():
     reduce_landing(dst2[:count], [host[:count]], accumulate=True)  # aligned: vector path over PCIe
     torch.cuda.synchronize()
     assert torch.equal(dst2[:count], dev[:count] + host[:count].cuda())
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """A stream whose queue is full makes the next launch wait; the interpreter must not wait with it."""
+    import threading
+    import time
+
+    from hylink_b200.ops import reduce_landing
+
+    src, dst = (torch.ones(16, device="cuda") for _ in range(2))
+    reduce_landing(dst, [src])
+    torch.cuda.synchronize()
+
+    def fill():
+        torch.cuda._sleep(1_000_000_000)                 # about half a second
+        for _ in range(4000):
+            reduce_landing(dst, [src])
+
+    t = threading.Thread(target=fill)
+    t.start()
+    worst, last = 0.0, time.perf_counter()
+    while t.is_alive():
+        now = time.perf_counter()
+        worst, last = max(worst, now - last), now
+    t.join()
+    torch.cuda.synchronize()
+    assert worst < 0.2, worst
+
+
+def test_folds_captured_in_a_graph():
+    """A chain of folds whose launches overlap, with an ordinary kernel and a copy between them."""
+    from hylink_b200.ops import reduce_landing
+
+    a, b = (torch.zeros(1 << 18, device="cuda") for _ in range(2))
+    x = torch.ones(1 << 18, device="cuda")
+
+    def chain():
+        reduce_landing(a, [x, b])
+        reduce_landing(b, [a], accumulate=True, scale=0.5)
+        a.mul_(2)
+        reduce_landing(b, [a])
+        x.copy_(b)
+        reduce_landing(a, [x], accumulate=True)
+
+    chain()
+    torch.cuda.synchronize()
+    for t, v in ((a, 0), (b, 0), (x, 1)):
+        t.fill_(v)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    va, vb, vx = 0.0, 0.0, 1.0
+    for _ in range(6):
+        graph.replay()
+        va = vx + vb
+        va *= 2
+        vb = vx = va
+        va += vx
+        assert bool((a == va).all()) and bool((b == vb).all()) and bool((x == vx).all())
