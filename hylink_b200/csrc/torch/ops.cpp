@@ -553,6 +553,15 @@ class MoeCombine : public torch::autograd::Function<MoeCombine> {
   }
 };
 
+// Whether anything hangs on the nodes that accumulate these parameters' gradients (a recorded step would not call it).
+bool accumulationHooks(const std::vector<Tensor>& params) {
+  for (const Tensor& p : params) {
+    const auto node = torch::autograd::impl::try_get_grad_accumulator(p);
+    if (node && !(node->pre_hooks().empty() && node->post_hooks().empty() && node->tensor_pre_hooks().empty())) return true;
+  }
+  return false;
+}
+
 // One AdamW step on lists of tensors. False (and nothing done) unless all are contiguous CUDA tensors of one type that
 // the kernel takes.
 bool multiAdamW(const std::vector<Tensor>& weights, const std::vector<Tensor>& grads, const std::vector<Tensor>& ms, const std::vector<Tensor>& vs,
@@ -729,6 +738,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return MoeLayer::apply(x, router, w1, w2, capacity);
   });
   m.def("multi_adamw", &multiAdamW);
+  m.def("accumulation_hooks", &accumulationHooks);
   m.def("moe_dispatch", [](const Tensor& x, const Tensor& router, int64_t capacity) { return MoeDispatch::apply(x, router, capacity); });
   m.def("moe_experts", [](const Tensor& h, const Tensor& w1, const Tensor& w2) { return MoeExperts::apply(h, w1, w2); });
   m.def("moe_combine", [](const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of, const Tensor& token_of) {

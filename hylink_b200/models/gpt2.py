@@ -130,17 +130,21 @@ class GPT2(nn.Module):
 
     def step_signature(self, idx: torch.Tensor, targets: torch.Tensor):
         """What a recorded training step depends on besides its inputs' values: equal signatures may share a recording.
-        None when a step has effects that a recording would not repeat (hooks) or does not take the fused operators."""
+        None when a step has effects that a recording would not repeat (hooks of any kind) or does not take the fused operators."""
         if not self._sizes_fit(idx, targets) or not self._fusable(self.wte.weight, targets) or not torch.is_grad_enabled():
             return None
         if type(self) is not GPT2 or type(self.wpe) is not nn.Embedding or overridden(self) or overridden(self.wpe):
             return None
         ps = list(self.parameters())
-        if any(p._backward_hooks or p._post_accumulate_grad_hooks for p in ps):
+        if any(p._backward_hooks or p._post_accumulate_grad_hooks for p in ps) or ops().accumulation_hooks(ps):
+            return None
+        if torch._C._autograd._top_saved_tensors_default_hooks(False) is not None:
             return None
         cuda = torch.backends.cuda
         flags = (torch.are_deterministic_algorithms_enabled(), cuda.flash_sdp_enabled(), cuda.mem_efficient_sdp_enabled(), cuda.cudnn_sdp_enabled(),
-                 cuda.math_sdp_enabled(), cuda.matmul.allow_bf16_reduced_precision_reduction, cuda.matmul.allow_fp16_reduced_precision_reduction)
+                 cuda.math_sdp_enabled(), cuda.fp16_bf16_reduction_math_sdp_allowed(), tuple(torch._C._get_sdp_priority_order()),
+                 torch._C._get_cublas_allow_bf16_reduced_precision_reduction(), torch._C._get_cublas_allow_fp16_reduced_precision_reduction(),
+                 cuda.matmul.allow_fp16_accumulation, torch._C._get_blas_preferred_backend())
         eps = tuple(m.eps for blk in self.blocks for m in (blk.ln1, blk.ln2)) + (self.ln_f.eps,)
         heads = tuple(blk.n_head for blk in self.blocks)
         return tuple((p.data_ptr(), p.requires_grad, p.shape) for p in ps), eps, heads, flags

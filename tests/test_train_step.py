@@ -1,4 +1,5 @@
 """The fused training-step operators against the same model in fp32 through plain PyTorch modules."""
+import contextlib
 import copy
 
 import pytest
@@ -370,7 +371,7 @@ def test_a_forward_of_an_instance_is_called(where):
         dist.destroy_process_group()
 
 
-@pytest.mark.parametrize("what", ["hook on wpe", "subclass"])
+@pytest.mark.parametrize("what", ["hook on wpe", "subclass", "accumulation", "accumulation, before", "saved tensors"])
 def test_a_step_with_effects_is_not_replayed(what):
     import torch.distributed as dist
 
@@ -388,13 +389,25 @@ def test_a_step_with_effects_is_not_replayed(what):
     if fresh:
         init_distributed("hylink")
     model = (Counting if what == "subclass" else GPT2)(GPT2Config.tiny())
-    if what != "subclass":
+    if what == "hook on wpe":
         model.wpe.register_forward_hook(lambda *a: seen.append(1))
     t = DDPTrainer(model, torch.device("cuda", 0))
+    if what.startswith("accumulation"):
+        p = model.blocks[1].fc.weight
+        node = p.expand_as(p).grad_fn.next_functions[0][0]
+        (node.register_prehook if what.endswith("before") else node.register_hook)(lambda *a: seen.append(1))
     tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
-    for _ in range(4):
-        t.step(tokens)
-    assert len(seen) == 4
+    context = contextlib.nullcontext()
+    if what == "saved tensors":
+        first = []
+        context = torch.autograd.graph.saved_tensors_hooks(lambda x: (first.append(1), x)[1], lambda x: x)
+    with context:
+        for _ in range(4):
+            t.step(tokens)
+            if what == "saved tensors":
+                seen += [1] * bool(first)
+                first.clear()
+    assert len(seen) == 4 and t._graph is None
     t.close()
     if fresh:
         dist.destroy_process_group()
