@@ -6,7 +6,8 @@ stores-only all-reduce: push of the shards, wait for the peers' pushes, fold and
 peers' results, copy-out. They show where a multi-GPU launch spends its time without a profiler attached (kernels of
 several ranks that wait on one another cannot be replayed under one).
 
-``decode(words)`` returns one dict per recorded launch, oldest first; ``summarise`` turns the per-CTA stamps into
+``decode(words)`` returns one dict per recorded launch, oldest first (``code``: the kernel's number, which also tells the
+low-latency all-reduce in one hop, 36, from the one in two, 27); ``summarise`` turns the per-CTA stamps into
 per-phase medians. ``python -m hylink_b200.utils.kernel_timeline`` under torchrun runs a few collectives and prints
 the summary of each rank-0 launch.
 """
@@ -45,7 +46,7 @@ def decode(words):
         for b in range(n):
             base = (slot * TL_BLOCKS + b) * TL_PHASES
             per_block.append(words[base: base + TL_PHASES])
-        out.append({"seq": seq, "kind": KINDS.get(kb >> 32, str(kb >> 32)), "blocks": blocks, "count": count, "stamps": per_block})
+        out.append({"seq": seq, "kind": KINDS.get(kb >> 32, str(kb >> 32)), "code": kb >> 32, "blocks": blocks, "count": count, "stamps": per_block})
     out.sort(key=lambda d: d["seq"])
     return out
 

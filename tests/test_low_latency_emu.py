@@ -260,8 +260,8 @@ def test_broadcast(n, count, offset, monkeypatch):
 
 
 # both sides of the size up to which ranks of one GPU reduce in one hop, and counts that are no whole packets
-@pytest.mark.parametrize("n,count", [(8, 5), (8, 32 << 10), (8, (32 << 10) + 1), (3, 87381), (3, 87382), (2, (256 << 10) - 3)])
-def test_allreduce_hops(n, count, monkeypatch):
+@pytest.mark.parametrize("n,count,hops", [(8, 5, 1), (8, 32 << 10, 1), (8, (32 << 10) + 1, 2), (3, 87381, 1), (3, 87382, 2), (2, (256 << 10) - 3, 1)])
+def test_allreduce_hops(n, count, hops, monkeypatch):
     monkeypatch.setenv("HYLINK_KERNEL_TIMELINE", "1")
     g = _group(n)
     outs = [torch.full((count + 9,), 7, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
@@ -275,4 +275,5 @@ def test_allreduce_hops(n, count, monkeypatch):
         g.run("all_reduce", ins, ins, count)             # in place
         assert all(torch.equal(t, want) for t in ins)
     assert {launch["kind"] for launch in g.kernel_timeline()} == {"lowlatency_allreduce"}
+    assert {launch["code"] for launch in g.kernel_timeline()} == {36 if hops == 1 else 27}
     g.close()
