@@ -413,6 +413,53 @@ def test_a_step_with_effects_is_not_replayed(what):
         dist.destroy_process_group()
 
 
+@pytest.mark.parametrize("where", ["before", "inside"])
+def test_a_failed_capture_leaves_eager_steps(where, monkeypatch, capsys):
+    """Raised on the host, before the capture begins and in the middle of the recorded forward pass: one message, the steps go on."""
+    import torch.distributed as dist
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.parallel import trainer
+    from hylink_b200.parallel.trainer import DDPTrainer, init_distributed
+
+    fresh = not dist.is_initialized()
+    if fresh:
+        init_distributed("hylink")
+    torch.manual_seed(8)
+    first = GPT2(GPT2Config.tiny())
+    tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
+    plain = GPT2._fused_loss
+
+    def fails(self, x, targets):
+        loss = plain(self, x, targets)
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("no room")
+        return loss
+
+    def train(broken):
+        with monkeypatch.context() as m:
+            m.setenv("HYLINK_TRAIN_GRAPH", "1" if broken else "0")
+            if broken and where == "before":
+                m.setattr(trainer._StepGraph, "_capture", lambda self, model: (_ for _ in ()).throw(RuntimeError("no room")))
+            elif broken:
+                m.setattr(GPT2, "_fused_loss", fails)
+            t = DDPTrainer(copy.deepcopy(first), torch.device("cuda", 0))
+            losses = [t.step(tokens) for _ in range(4)]
+            assert t._graph is None and not t._use_graph
+            grads = [p.grad for p in t.model.parameters()]
+            t.close()
+            return losses, grads
+
+    losses, grads = train(True)
+    assert capsys.readouterr().out.count("not replayed") == 1
+    want, want_grads = train(False)
+    torch.testing.assert_close(torch.tensor(losses), torch.tensor(want), rtol=5e-3, atol=0)
+    for a, b in zip(grads, want_grads):
+        assert float((a.float() - b.float()).norm()) <= 3e-2 * float(b.float().norm()) + 1e-6
+    if fresh:
+        dist.destroy_process_group()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_multi_tensor_adamw_matches_torch(dtype):
     """Tensors shorter than a packet, of a ragged length, unaligned, of several chunks; more of them than one launch takes."""
