@@ -149,6 +149,11 @@ class DDPTrainer:
                             static_graph=False)
         return self._ddp
 
+    @ddp.setter
+    def ddp(self, wrapper) -> None:
+        """A wrapper of the caller's own, which every step goes through from now on."""
+        self._graph, self._ddp = None, wrapper
+
     def _opt_step(self) -> None:
         """``self.opt.step()``, through this library's kernel where the optimizer is what the constructor made and nobody
         watches its steps (a scheduler replaces ``step``, hooks want to be called); its state stays where it is."""

@@ -413,6 +413,29 @@ def test_a_step_with_effects_is_not_replayed(what):
         dist.destroy_process_group()
 
 
+def test_a_wrapper_of_the_callers_own():
+    import torch.distributed as dist
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.parallel.trainer import DDPTrainer, init_distributed
+
+    fresh = not dist.is_initialized()
+    if fresh:
+        init_distributed("hylink")
+    model, seen = GPT2(GPT2Config.tiny()), []
+    t = DDPTrainer(model, torch.device("cuda", 0))
+    tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
+    for _ in range(3):
+        t.step(tokens)
+    t.ddp = lambda idx, targets: (seen.append(1), model(idx, targets))[1]
+    for _ in range(3):
+        t.step(tokens)
+    assert len(seen) == 3
+    t.close()
+    if fresh:
+        dist.destroy_process_group()
+
+
 @pytest.mark.parametrize("where", ["before", "inside"])
 def test_a_failed_capture_leaves_eager_steps(where, monkeypatch, capsys):
     """Raised on the host, before the capture begins and in the middle of the recorded forward pass: one message, the steps go on."""
