@@ -302,3 +302,16 @@ def test_routing_of_equal_infinite_and_nan_logits():
         _, _, gate, row_of, _ = ops().moe_dispatch(x, w, 40)
         assert torch.equal(row_of.long() // 40, expert)
         torch.testing.assert_close(gate, want, rtol=1e-6, atol=0, equal_nan=True)
+
+
+def test_gelu_over_all_16_bit_values():
+    """Every finite bf16 value, through experts whose two products are the identity: the bits of torch's own kernel."""
+    from hylink_b200.ops.extension import ops
+
+    x = torch.arange(1 << 16, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = x[x.isfinite()]
+    x = x[:x.numel() // 8 * 8].view(1, -1, 8)
+    eye = torch.eye(8, device="cuda", dtype=torch.bfloat16)[None]
+    got = ops().moe_experts(x, eye, eye)
+    want = torch.nn.functional.gelu(x, approximate="tanh")
+    assert torch.equal(got, want), [(float(a), float(b), float(c)) for a, b, c in zip(x[got != want], got[got != want], want[got != want])][:20]
