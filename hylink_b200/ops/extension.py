@@ -31,12 +31,6 @@ def ops():
     return _module
 
 
-def is_half_cuda(*tensors) -> bool:
-    """Whether all tensors are CUDA tensors of one 16-bit float type."""
-    dt = tensors[0].dtype
-    return dt in (torch.bfloat16, torch.float16) and all(t.is_cuda and t.dtype == dt for t in tensors)
-
-
 def overridden(m) -> bool:
     """Whether calling module ``m`` does anything besides its class's ``forward``: hooks, or a ``forward`` of its own."""
     return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__)
