@@ -35,6 +35,21 @@ __device__ __forceinline__ void afterPredecessor() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// One choice of operator per packet.
+template <int N, typename A>
+__device__ __forceinline__ void foldPacket(int op, A* acc, const A* b) {
+  auto each = [&](auto f) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) acc[e] = f(acc[e], b[e]);
+  };
+  switch (op) {
+    case hlProd: each([](A x, A y) { return applyOp((int)hlProd, x, y); }); break;
+    case hlMax: each([](A x, A y) { return applyOp((int)hlMax, x, y); }); break;
+    case hlMin: each([](A x, A y) { return applyOp((int)hlMin, x, y); }); break;
+    default: each([](A x, A y) { return applyOp((int)hlSum, x, y); }); break;
+  }
+}
+
 // Bound by memory. A thread folds U packets: it has the loads of all their operands in flight at once (the operand
 // count is compiled in, in classes), adds in a fixed order and stores. The grid covers the message; CTAs that retire
 // and start keep more loads in flight than a resident grid whose threads alternate between loading and storing
@@ -42,9 +57,12 @@ __device__ __forceinline__ void afterPredecessor() {
 // four packets deep and the operator chosen per element, 38.9). With one or two operands a thread that folds a single
 // packet is gone before its CTA has cost less than it moved: U is four there, while the CTAs still fill the SMs (28 MB
 // copied: 16.3 us with one packet, 12.3 with four). A caller's own block count makes it loop.
-// kSum: the operator is known to be an addition; otherwise it is looked up per element.
+// kSum: the operator is known to be an addition; otherwise it is looked up per packet (per element a fold of two 32 MiB
+// sources of bf16 took 42.9 us, 12.7 now). The widest class gives up registers for a fourth CTA per SM (five operands of
+// 32 MiB, bf16: 51.2 us with two CTAs, 33.7 with four).
 template <typename T, int MR, int U, bool kSum>
-__global__ void __launch_bounds__(kRlThreads) kReduceLanding(const __grid_constant__ nvl::ReduceLandingArgs a, const void* const first, int n) {
+__global__ void __launch_bounds__(kRlThreads, MR <= 4 ? 0 : (sizeof(T) == 1 ? 3 : 4)) kReduceLanding(const __grid_constant__ nvl::ReduceLandingArgs a,
+                                                                                                              const void* const first, int n) {
   afterPredecessor();
   constexpr int N = Packet<T>::N;
   using Acc = typename Wire<T>::Acc;
@@ -74,8 +92,7 @@ __global__ void __launch_bounds__(kRlThreads) kReduceLanding(const __grid_consta
         for (int q = 1; q < MR; ++q)
           if (q < n) {
             Packet<T>::unpack(v[u][q], b);
-#pragma unroll
-            for (int e = 0; e < N; ++e) acc[e] = kSum ? (Acc)(acc[e] + b[e]) : applyOp(a.op, acc[e], b[e]);
+            foldPacket<N>(kSum ? (int)hlSum : a.op, acc, b);
           }
         finish<T>(acc, a.scale, 0);
         reinterpret_cast<uint4*>(dst)[i0 + u * kRlThreads] = Packet<T>::pack(acc);
@@ -155,16 +172,18 @@ static cudaError_t launchEarly(const void* fn, unsigned blocks, unsigned threads
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-// Operand classes: 2 (one source into an accumulator), 4, 9; operators other than the sum share the widest. `packets`
-// of a thread: 1, or what reduceLandingUnroll says.
-static int reduceLandingUnroll(int operands, bool sum) { return !sum || operands > 2 ? 1 : 4; }
+// Operand classes: 2 (one source into an accumulator), 4, 9. `packets` of a thread: 1, or what reduceLandingUnroll says.
+static int reduceLandingUnroll(int operands) { return operands > 2 ? 1 : 4; }
+template <typename T, bool kSum>
+static const void* reduceLandingClass(int operands, int packets) {
+  using namespace dev;
+  if (operands <= 2) return packets == 1 ? (const void*)kReduceLanding<T, 2, 1, kSum> : (const void*)kReduceLanding<T, 2, 4, kSum>;
+  if (operands <= 4) return (const void*)kReduceLanding<T, 4, 1, kSum>;
+  return (const void*)kReduceLanding<T, 9, 1, kSum>;
+}
 template <typename T>
 static const void* reduceLandingFor(int operands, bool sum, int packets) {
-  using namespace dev;
-  if (!sum) return (const void*)kReduceLanding<T, 9, 1, false>;
-  if (operands <= 2) return packets == 1 ? (const void*)kReduceLanding<T, 2, 1, true> : (const void*)kReduceLanding<T, 2, 4, true>;
-  if (operands <= 4) return (const void*)kReduceLanding<T, 4, 1, true>;
-  return (const void*)kReduceLanding<T, 9, 1, true>;
+  return sum ? reduceLandingClass<T, true>(operands, packets) : reduceLandingClass<T, false>(operands, packets);
 }
 static const void* reduceLandingFn(int dt, int operands, bool sum, int packets) {
   switch (dt) {
@@ -185,9 +204,9 @@ static const void* reduceLandingFn(int dt, int operands, bool sum, int packets) 
 hlResult_t launchReduceLanding(const ReduceLandingArgs& a, int blocks, cudaStream_t stream) {
   if (a.nsrc < 1 || a.nsrc > 8) return fail(hlInvalidArgument, "reduce landing: nsrc %d out of [1,8]", a.nsrc);
   int operands = a.nsrc + (a.accumulate ? 1 : 0);
-  const bool sum = a.op == hlSum || a.op == hlAvg;
+  const bool sum = a.op == hlSum || a.op == hlAvg || operands == 1;   // one operand: nothing to choose
   const uint64_t packets = (a.count * hlTypeSize((hlDataType_t)a.dtype) + 15) / 16;
-  int unroll = reduceLandingUnroll(operands, sum);
+  int unroll = reduceLandingUnroll(operands);
   if (packets < (uint64_t)148 * 8 * dev::kRlThreads * unroll) unroll = 1;   // fewer than eight CTAs per SM
   const void* fn = reduceLandingFn(a.dtype, operands, sum, unroll);
   if (!fn) return fail(hlUnsupported, "reduce landing: unsupported dtype %d", a.dtype);
@@ -218,7 +237,7 @@ hlResult_t prepareReduceLanding() {
   for (int dt = 0; dt < hlNumTypes; ++dt)
     for (int operands : {2, 4, 9})
       for (bool sum : {false, true})
-        for (int packets : {1, reduceLandingUnroll(operands, sum)}) {
+        for (int packets : {1, reduceLandingUnroll(operands)}) {
           cudaFuncAttributes at;
           cudaError_t e = cudaFuncGetAttributes(&at, reduceLandingFn(dt, operands, sum, packets));
           if (e != cudaSuccess) return fail(hlDeviceError, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));

@@ -49,6 +49,24 @@ def test_k_way_three_address(op, k):
     assert torch.equal(dst, acc.to(torch.bfloat16))
 
 
+# one, two, up to four and up to nine operands; one packet per thread and four, whole packets and a rest, off the boundary
+@pytest.mark.parametrize("op", ["max", "min", "prod"])
+@pytest.mark.parametrize("k,accumulate", [(1, False), (1, True), (2, False), (3, True), (4, True), (8, False)])
+@pytest.mark.parametrize("dtype,count,off", [(torch.bfloat16, 4097, 0), (torch.float16, 9_700_003, 0), (torch.int8, 100_003, 0), (torch.float32, 3001, 1)])
+def test_operators_in_every_operand_class(op, k, accumulate, dtype, count, off):
+    from hylink_b200.ops import reduce_landing
+
+    srcs = [_rand(count + off, dtype, 20 + i)[off:] for i in range(k)]
+    dst = _rand(count + off, dtype, 5)[off:]
+    up = (lambda t: t.float()) if dtype in (torch.bfloat16, torch.float16) else (lambda t: t)
+    parts = ([up(dst)] if accumulate else []) + [up(s) for s in srcs]
+    want = parts[0].clone()
+    for p in parts[1:]:
+        want = {"max": torch.maximum, "min": torch.minimum, "prod": torch.mul}[op](want, p)
+    reduce_landing(dst, srcs, op=op, accumulate=accumulate)
+    assert torch.equal(dst, want.to(dtype))
+
+
 def test_pinned_host_source_and_unaligned():
     from hylink_b200.ops import reduce_landing
 
