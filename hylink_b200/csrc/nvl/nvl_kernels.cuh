@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
 // All-gather and all-to-all: nothing to fold, a segment goes from the sender's buffer through the receiver's slot into
 // the receiver's output.
 template <typename W, bool kGather>
-__global__ void __launch_bounds__(HL_NVL_THREADS) kExchangePush(const HlCommDev* comms, HlEmuCalls calls) {
+__global__ void __launch_bounds__(HL_NVL_THREADS, 1) kExchangePush(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
   if (!entryOk(c, a)) return;
@@ -1174,8 +1174,10 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kAllGatherLanes(const HlCom
 }
 
 // ------------------------------------------------------------------ broadcast
+// One CTA per SM (NvlPath::blocksFor): with the registers of two a thread's packets got in one another's way (fp32 outputs
+// that start inside a packet, 64 MiB to 4 ranks of one GPU: 144 us instead of 225).
 template <typename W, bool kNvls>
-__global__ void __launch_bounds__(HL_NVL_THREADS) kBroadcast(const HlCommDev* comms, HlEmuCalls calls) {
+__global__ void __launch_bounds__(HL_NVL_THREADS, 1) kBroadcast(const HlCommDev* comms, HlEmuCalls calls) {
   const HlCommDev& c = comms[blockIdx.y];
   HlCallArgs a = calls.c[blockIdx.y];
   if (!entryOk(c, a)) return;

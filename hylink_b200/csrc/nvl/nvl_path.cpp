@@ -474,6 +474,7 @@ int NvlPath::blocksFor(int kind, size_t wire_bytes_per_rank, int max_blocks) con
   // The push all-reduce pays two grid-wide flag rounds whose cost grows with the CTA count: below 16 MiB a
   // smaller grid is faster (8 MiB on 2 GPUs: 207 GB/s with 96 CTAs, 164 GB/s with 148).
   if (kind == kNvlAllReducePush && wire_bytes_per_rank < (16u << 20)) cap = std::min(cap, 96);
+  if (kind == kNvlBroadcast || kind == kNvlBroadcastNvls) cap = std::min(cap, 148);   // one per SM is resident, whatever was asked for
   const size_t per_cta = kind == kNvlAllReduceOneShot ? (8u << 10) : (16u << 10);
   size_t want = (wire_bytes_per_rank + per_cta - 1) / per_cta;
   if (want < 1) want = 1;
