@@ -503,7 +503,7 @@ int NvlPath::streamedKind(int kind, const HlEmuCalls& calls, uint64_t sp, int wi
   constexpr uint64_t kStaysInL2 = 64ull << 20;
   if (to == kNvlStreamBroadcast) {
     // us streamed / plain: 2 ranks 16 MB 20.5 / 18.6, 32 MB 33.9 / 40.6; 4 ranks 12 MB 26.8 / 25.7, 16 MB 31.0 / 33.8;
-    // 8 ranks 8 MB 30.8 / 31.1, 64 MB 175 / 249
+    // 8 ranks 8 MB 30.8 / 31.1, 64 MB 180 to 200 / 249
     if ((n + 1) * sp * 16 <= kStaysInL2) return kind;
     for (int i = 0; i < nranks_; ++i) {
       const HlCallArgs& a = calls.c[i];

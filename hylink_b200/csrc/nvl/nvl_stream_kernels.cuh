@@ -18,7 +18,7 @@
 // the plain kernel.
 // Broadcast: the root puts piece t into its own ring and into its output, the others copy piece t - L out of the root's
 // ring. (With the whole message staged first, the others wait for the root's CTAs, an n-th of the GPU: 64 MiB
-// to 8 ranks 249 us, streamed 175; to 4 ranks 132 and 94. The root's CTAs are the bound: they read once and store twice.)
+// to 8 ranks 249 us, streamed 180 to 200; to 4 ranks 132 and 96. The root's CTAs are the bound: they read once and store twice.)
 // Flags are the tile words of the pipelined kernels: [kind 1][CTA][source rank] <- tile base + finished iterations.
 //
 // Roles: worker warps move data; a poller warp watches the peers' flags and opens iterations; a signaller warp waits

@@ -103,7 +103,8 @@ class GPT2(nn.Module):
 
     def _fusable(self, x: torch.Tensor, targets: torch.Tensor) -> bool:
         """Whether the loss can go through the fused operators: a 16-bit model on a GPU, made of the plain modules
-        above (no hooks, nothing replaced, no `forward` of an instance's own), at widths whose rows a warp can hold."""
+        above (no hooks, nothing replaced, no `forward` of an instance's own), of the shapes they have here, at
+        widths that the layer norm's backward kernel takes."""
         c = self.config
         if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.numel() and targets.is_cuda and targets.dtype == torch.int64):
             return False
@@ -121,10 +122,11 @@ class GPT2(nn.Module):
         for m, kind, rows, cols in mods:     # 0: any number
             if type(m) is not kind or overridden(m):
                 return False
-            w = m.weight
-            if type(w) not in (nn.Parameter, torch.Tensor) or type(m.bias if kind is not nn.Embedding else w) not in (nn.Parameter, torch.Tensor) or w.dtype != x.dtype or w.dim() != (1 if kind is nn.LayerNorm else 2):
+            tensors = (m.weight,) if kind is nn.Embedding else (m.weight, m.bias)
+            if any(type(t) not in (nn.Parameter, torch.Tensor) or t.dtype != x.dtype for t in tensors):
                 return False
-            if (rows and w.shape[0] != rows) or (cols and w.shape[1] != cols) or (kind is not nn.Embedding and m.bias is None):
+            shape = m.weight.shape
+            if len(shape) != (1 if kind is nn.LayerNorm else 2) or (rows and shape[0] != rows) or (cols and shape[1] != cols):
                 return False
         return all(blk.fc.weight.shape[0] % 8 == 0 for blk in self.blocks)
 
