@@ -371,7 +371,7 @@ def test_a_forward_of_an_instance_is_called(where):
         dist.destroy_process_group()
 
 
-@pytest.mark.parametrize("what", ["hook on wpe", "subclass", "accumulation", "accumulation, before", "saved tensors"])
+@pytest.mark.parametrize("what", ["hook on wpe", "subclass", "accumulation", "accumulation, before", "accumulation, later", "saved tensors"])
 def test_a_step_with_effects_is_not_replayed(what):
     import torch.distributed as dist
 
@@ -392,11 +392,15 @@ def test_a_step_with_effects_is_not_replayed(what):
     if what == "hook on wpe":
         model.wpe.register_forward_hook(lambda *a: seen.append(1))
     t = DDPTrainer(model, torch.device("cuda", 0))
+    tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
+    if what.endswith("later"):
+        for _ in range(3):
+            t.step(tokens)
+        assert t._graph is not None
     if what.startswith("accumulation"):
         p = model.blocks[1].fc.weight
         node = p.expand_as(p).grad_fn.next_functions[0][0]
         (node.register_prehook if what.endswith("before") else node.register_hook)(lambda *a: seen.append(1))
-    tokens = torch.randint(0, 1024, (2, 33)).pin_memory()
     context = contextlib.nullcontext()
     if what == "saved tensors":
         first = []
