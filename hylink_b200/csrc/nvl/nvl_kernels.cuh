@@ -719,7 +719,9 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* c
 //   all-reduce      stream shard s of the input straight from the caller's buffer into slot `rank` of its owner | barrier |
 //                   fold the own shard (read from the caller's buffer) and the landed slots in ascending rank order,
 //                   store the result to the caller's output and into every peer's result area | barrier | copy the
-//                   peers' results out of the local result area | barrier
+//                   peers' results out of the local result area | barrier. Ranks of one GPU store a result once, in the
+//                   owner's result area, and copy it out of there: it stays in L2, where n - 1 copies of it do not (8 ranks x
+//                   16 MiB of fp32 123 us with a copy per peer, 97 with one; 4 ranks 59 and 51, 2 ranks 26.7 and 26.6)
 //   reduce-scatter  push the peers' segments | barrier | fold | barrier
 //   all-gather      store the own segment into every peer's slot and into the own output | barrier | copy out | barrier
 //   all-to-all      push the peers' segments, copy the own one | barrier | copy out | barrier
@@ -825,6 +827,9 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
   const Parts<W> in(a.in, kAllReduce ? sp * N : a.in_seg_stride, a.count, kAllReduce ? a.count : 0);
   const Parts<W> out(a.out, sp * N, a.count, kAllReduce ? a.count : 0);   // reduce-scatter: part 0 alone
   const uint64_t res_off = sp * (uint64_t)n;                              // results live behind the slots
+  // Ranks of one GPU: a result is stored once, in its owner's result area, and the peers read it there.
+  const bool near = c.one_device != 0;
+  const int copies = near ? 1 : n - 1;
   for (int k = 1; k < n; ++k) {
     const int q = peerOf(r, k, n);
     pushPart<W>(reinterpret_cast<uint4*>(c.stage[q]) + (uint64_t)r * sp, in.at(q), in.elems(q), x);
@@ -843,7 +848,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
     if constexpr (kAllReduce) {
 #pragma unroll
       for (int k = 1; k < MR; ++k)
-        if (k < n) dst[k] = reinterpret_cast<uint4*>(c.stage[peerOf(r, k, n)]) + res_off + (uint64_t)r * sp;
+        if (k <= copies) dst[k] = reinterpret_cast<uint4*>(c.stage[near ? r : peerOf(r, k, n)]) + res_off + (uint64_t)r * sp;
     }
     for (uint32_t i = (uint32_t)x.g0; i < whole; i += g * U) {
       uint4 v[U][MR];
@@ -860,7 +865,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
           if constexpr (kAllReduce) {
 #pragma unroll
             for (int k = 1; k < MR; ++k)
-              if (k < n) dst[k][i + u * g] = red;
+              if (k <= copies) dst[k][i + u * g] = red;
           }
         }
     }
@@ -887,7 +892,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
           if constexpr (kAllReduce) {
 #pragma unroll
             for (int k = 1; k < MR; ++k)
-              if (k < n) dst[k][i] = red;
+              if (k <= copies) dst[k][i] = red;
           }
         }
       }
@@ -897,7 +902,7 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
   if constexpr (kAllReduce) {
     for (int k = 1; k < n; ++k) {
       const int q = peerOf(r, k, n);
-      pullPart<W>(out.at(q), reinterpret_cast<const uint4*>(c.stage[r]) + res_off + (uint64_t)q * sp, out.elems(q), x);
+      pullPart<W>(out.at(q), reinterpret_cast<const uint4*>(c.stage[near ? q : r]) + res_off + (uint64_t)q * sp, out.elems(q), x);
     }
     // rule A: the result areas just read are where a peer's next (larger) call pushes its slots
     blockBarrier(c, a, 3, 3);
