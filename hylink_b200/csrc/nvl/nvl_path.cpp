@@ -484,10 +484,12 @@ int NvlPath::blocksFor(int kind, size_t wire_bytes_per_rank, int max_blocks) con
 // Between ranks of one GPU: the streamed form of a push kernel when the staging of the plain one (all ranks together)
 // would not stay in L2, every segment starts on a 16-byte boundary and the ring fits the staging region; else the kind
 // itself. (All ranks' buffers are at hand here; between GPUs a choice must not depend on a pointer.)
-// Measured, bf16, us streamed / plain by staging bytes. 4 ranks: 32 MB reduce-scatter 21.7 / 19.4, all-gather 21.5 / 19.8;
-// 64 MB 33.2 / 33.0, 33.4 / 34.8; 128 MB 55.5 / 62.5, 57.7 / 67.2. 2 ranks: 64 MB 31.5 / 30.8, 31.6 / 31.6; 128 MB
-// 51.9 / 58.1, 53.9 / 61.0. 8 ranks: 64 MB all-gather 37.2 / 36.6, 128 MB 62.3 / 69.0, all-to-all 76.8 / 85.1; the fold
+// Measured, bf16, us streamed / plain by staging bytes. 4 ranks: reduce-scatter 32 MB 21.7 / 19.4, 64 MB 33.2 / 33.0, 128 MB
+// 55.5 / 62.5. 2 ranks: 64 MB 31.5 / 30.8, 128 MB 51.9 / 58.1. 8 ranks: all-to-all 128 MB 76.8 / 85.1; the fold
 // of eight sources leaves the workers of a reduce-scatter too few registers: 74.8 / 67.0, so it stays plain.
+// All-gather, whose ring holds a piece once for all peers and pays from a quarter of that: 4 ranks 16 MB 12.5 / 12.9, 24 MB 14.5 /
+// 16.5, 64 MB 24.3 / 33.0; 8 ranks 24 MB 17.6 / 18.0, 32 MB 20.8 / 20.7, 64 MB 30.5 / 35.2; 2 ranks 16 MB 13.0 / 12.4, 32 MB
+// 18.4 / 17.6, 48 MB 22.6 / 23.0, 64 MB 28.5 / 30.9.
 int NvlPath::streamedKind(int kind, const HlEmuCalls& calls, uint64_t sp, int wire_dt, int blocks) const {
   const size_t elem = hlTypeSize((hlDataType_t)wire_dt);
   if (!emu_ || nranks_ < 2) return kind;
@@ -512,15 +514,16 @@ int NvlPath::streamedKind(int kind, const HlEmuCalls& calls, uint64_t sp, int wi
     return (uint64_t)blocks * 2 * HL_STREAM_LAG * HL_STREAM_WORKERS * 8 * 16 <= stage_bytes_ ? to : kind;
   }
   if (to == kNvlStreamReduceScatter && nranks_ > 4) return kind;
-  if (n * n * sp * 16 <= kStaysInL2) return kind;
+  const uint64_t plain = n * n * sp * 16;
+  if (plain <= (to == kNvlStreamAllGather ? (n > 2 ? kStaysInL2 / 4 : kStaysInL2 / 2) : kStaysInL2)) return kind;
   for (int i = 0; i < nranks_; ++i) {
     const HlCallArgs& a = calls.c[i];
     if (((uintptr_t)a.in | (uintptr_t)a.out) & 15) return kind;
     if (kind != kNvlAllGatherPush && (a.in_seg_stride * elem) % 16) return kind;
     if (kind != kNvlReduceScatterPush && (a.out_seg_stride * elem) % 16) return kind;
   }
-  const uint64_t piece = (uint64_t)HL_STREAM_WORKERS * 8 / (nranks_ <= 2 ? 2 : (nranks_ <= 4 ? 4 : 8));
-  const uint64_t ring = (uint64_t)blocks * 2 * HL_STREAM_LAG * n * piece * 16;
+  const uint64_t piece = (uint64_t)HL_STREAM_WORKERS * (to == kNvlStreamAllGather ? 16 : 8) / (nranks_ <= 2 ? 2 : (nranks_ <= 4 ? 4 : 8));
+  const uint64_t ring = (uint64_t)blocks * 2 * HL_STREAM_LAG * (to == kNvlStreamAllGather ? 1 : n) * piece * 16;   // a slot per sender, or one
   return ring <= stage_bytes_ ? to : kind;
 }
 
@@ -842,7 +845,7 @@ hlResult_t NvlPath::allGather(const NvlBufs& b, const NvlCall& c, cudaStream_t s
   static const bool ag_push = envBool({"HYLINK_AG_PUSH"}, true);
   const bool push = same && c.algo != hlAlgoTwoShotP2p && ag_push;
   const size_t seg_bytes = c.count * hlTypeSize((hlDataType_t)c.wire_dt);
-  const bool lanes = push && (c.algo == hlAlgoPipelined || (c.algo == hlAlgoAuto && seg_bytes * (size_t)nranks_ >= agLanesMinBytes()));
+  const bool lanes = push && (c.algo == hlAlgoPipelined || (c.algo == hlAlgoAuto && !emu_ && seg_bytes * (size_t)nranks_ >= agLanesMinBytes()));
   return launchSliced(lanes ? kNvlAllGatherLanes : (push ? kNvlAllGatherPush : kNvlAllGather), b, c, true, s);
 }
 

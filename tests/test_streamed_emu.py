@@ -75,6 +75,25 @@ def test_streamed_collectives(n, seg, dtype, offset, monkeypatch):
     g.close()
 
 
+# two whole pieces for every CTA (a piece: 448 threads of eight, four or two packets), one packet more or less, ragged ends
+@pytest.mark.parametrize("n,extra", [(2, 0), (2, 5), (3, 1), (4, -8), (4, 0), (4, 8), (8, -1), (8, 0), (8, 9)])
+def test_streamed_all_gather_at_the_edges_of_its_pieces(n, extra, monkeypatch):
+    from hylink_b200.ops import EmuGroup
+
+    monkeypatch.setenv("HYLINK_KERNEL_TIMELINE", "1")
+    g = EmuGroup(n)
+    seg = 148 // n * 448 * (8 if n <= 2 else 4 if n <= 4 else 2) * 2 * 8 + extra
+    stride = (seg + 7) // 8 * 8
+    for rep in range(3):                              # back to back: a slow reader of one call, a fast writer of the next
+        ins = [_rand(seg, torch.bfloat16, 10 * rep + r) for r in range(n)]
+        outs = [torch.full((n * stride + 8,), 7, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+        g.run("all_gather", ins, outs, seg, out_seg_stride=stride)
+        for o in outs:
+            assert all(torch.equal(o[q * stride:q * stride + seg], ins[q]) and bool((o[q * stride + seg:(q + 1) * stride] == 7).all()) for q in range(n))
+    assert "allgather_streamed" in {launch["kind"] for launch in g.kernel_timeline()}
+    g.close()
+
+
 def test_streamed_wait_is_bounded():
     from hylink_b200.ops import EmuGroup
 
