@@ -56,6 +56,7 @@ const CudaDriver* CudaDriver::get() {
     resolve("cuMulticastBindMem", &d.cuMulticastBindMem);
     resolve("cuMulticastUnbind", &d.cuMulticastUnbind);
     resolve("cuMulticastGetGranularity", &d.cuMulticastGetGranularity);
+    resolve("cuTensorMapEncodeTiled", &d.cuTensorMapEncodeTiled);
     d.ok = ok;
   });
   return d.ok ? &d : nullptr;

@@ -217,6 +217,27 @@ class BlockPre : public torch::autograd::Function<BlockPre> {
   }
 };
 
+// Products with gelu, or its gradient, in the own kernel's epilogue. `out` [groups][n][m] or [n][m]; see GemmSpec.
+train::GemmSpec product(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, const Tensor& out, int64_t k, int ragged = train::kGemmWhole,
+                        int epilogue = train::kGemmStore, const Tensor& aux = Tensor()) {
+  return {a.data_ptr(), b.data_ptr(), out.data_ptr(), aux.defined() ? aux.data_ptr() : nullptr, (int)out.size(-1), (int)out.size(-2), (int)k,
+          a_mn, b_mn, ragged, epilogue};
+}
+void products(const train::GemmSpec* specs, int n, const Tensor& like, const Tensor& count = Tensor()) {
+  ok(train::expertGemm(code(like), specs, n, like.dim() == 3 ? (int)like.size(0) : 1, count.defined() ? count.data_ptr<int>() : nullptr, streamOf(like)),
+     "grouped product");
+}
+// What the own kernel takes of an operand besides its place: anything else is left to the library, errors among it.
+bool operand(const Tensor& t, const Tensor& like, at::IntArrayRef sizes) {
+  return t.sizes() == sizes && t.scalar_type() == like.scalar_type() && t.device() == like.device() && t.layout() == at::kStrided;
+}
+bool ownExperts(const Tensor& h, const Tensor& w1, const Tensor& w2) {
+  if (h.dim() != 3 || w1.dim() != 3 || !h.is_cuda() || (h.scalar_type() != at::kBFloat16 && h.scalar_type() != at::kHalf)) return false;
+  const int64_t experts = h.size(0), width = h.size(2), hidden = w1.size(2);
+  return operand(w1, h, {experts, width, hidden}) && operand(w2, h, {experts, hidden, width}) &&
+         train::expertGemmPays(experts * h.size(1), width, hidden);
+}
+
 class BlockPost : public torch::autograd::Function<BlockPost> {
  public:
   static variable_list forward(AutogradContext* ctx, const Variable& x_, const Variable& a_, const Variable& wp, const Variable& bp,
@@ -352,7 +373,7 @@ class HeadLoss : public torch::autograd::Function<HeadLoss> {
 
 // ---- top-1 mixture of experts
 struct Routed {
-  Tensor logits, expert, gate, row_of, token_of, send;
+  Tensor logits, expert, gate, row_of, token_of, count, send;
 };
 Routed moeRouted(const Tensor& x, const Tensor& router, int64_t capacity) {
   const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
@@ -362,10 +383,11 @@ Routed moeRouted(const Tensor& x, const Tensor& router, int64_t capacity) {
   r.expert = at::empty({tokens}, ints);
   r.row_of = at::empty({tokens}, ints);
   r.token_of = at::empty({experts * capacity}, ints);
+  r.count = at::empty({experts}, ints);
   r.gate = floats(x, {tokens});
   r.send = at::empty({experts * capacity, width}, x.options());
   ok(train::moeRoute(code(x), r.logits.data_ptr(), (int)tokens, (int)experts, (int)capacity, r.expert.data_ptr<int>(), r.gate.data_ptr<float>(),
-                     r.row_of.data_ptr<int>(), r.token_of.data_ptr<int>(), streamOf(x)),
+                     r.row_of.data_ptr<int>(), r.token_of.data_ptr<int>(), r.count.data_ptr<int>(), streamOf(x)),
      "MoE routing");
   ok(train::moeGather(x.data_ptr(), r.token_of.data_ptr<int>(), r.send.data_ptr(), (int)(experts * capacity), (int)width, streamOf(x)), "MoE dispatch");
   return r;
@@ -375,7 +397,8 @@ std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& route
                                             const Tensor& row_of, const Tensor& dres, const Tensor& dsend, const Tensor& dgate, bool router_needed) {
   const Tensor router = dense(router_);
   const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
-  Tensor dx = at::empty_like(x), dlogits = at::empty_like(logits);
+  Tensor dx = at::empty_like(x);
+  Tensor dlogits = at::empty_like(logits);
   ok(train::moeTokenGradient(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
                              expert.data_ptr<int>(), gate.data_ptr<float>(), dgate.data_ptr<float>(), router.data_ptr(), dx.data_ptr(),
                              dlogits.data_ptr(), (int)tokens, (int)width, (int)experts, streamOf(x)),
@@ -386,27 +409,67 @@ std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& route
 struct Expert {
   Tensor u, act, out;
 };
-Expert moeExpert(const Tensor& h, const Tensor& w1, const Tensor& w2) {
+// h: [experts][rows][width]. `count`: rows of each expert in use (the others are zeros), undefined where that is not known; results
+// of rows out of use may be anything then.
+Expert moeExpert(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const Tensor& count) {
   Expert e;
-  e.u = at::bmm(h, w1);
+  if (ownExperts(h_, w1_, w2_)) {
+    const Tensor h = dense(h_), w1 = dense(w1_), w2 = dense(w2_);
+    e.u = at::empty({h.size(0), h.size(1), w1.size(2)}, h.options());
+    e.act = at::empty_like(e.u);
+    e.out = at::empty_like(h);
+    const train::GemmSpec first = product(w1, true, h, false, e.u, h.size(2), train::kGemmRaggedN, train::kGemmGelu, e.act);
+    products(&first, 1, h, count);
+    const train::GemmSpec second = product(w2, true, e.act, false, e.out, w1.size(2), train::kGemmRaggedN);
+    products(&second, 1, h, count);
+    return e;
+  }
+  e.u = at::bmm(h_, w1_);
   e.act = at::empty_like(e.u);
   ok(train::geluForward(code(e.u), e.u.data_ptr(), e.act.data_ptr(), e.u.numel(), streamOf(e.u)), "gelu");
-  e.out = at::bmm(e.act, w2);
+  e.out = at::bmm(e.act, w2_);
   return e;
 }
 // {dh, dw1, dw2}, those that are needed
-variable_list moeExpertBackward(const Tensor& h, const Tensor& w1, const Tensor& w2, const Tensor& u_, const Tensor& act, const Tensor& dout, bool h_needed,
-                                bool w1_needed, bool w2_needed) {
+variable_list moeExpertBackward(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const Tensor& u_, const Tensor& act_, const Tensor& dout_,
+                                const Tensor& count, bool h_needed, bool w1_needed, bool w2_needed) {
   Tensor dh, dw1, dw2;
-  if (w2_needed) dw2 = at::bmm(act.transpose(1, 2), dout);
+  if (ownExperts(h_, w1_, w2_)) {
+    const Tensor h = dense(h_), w1 = dense(w1_), w2 = dense(w2_), u = dense(u_), act = dense(act_), dout = dense(dout_);
+    const int64_t rows = h.size(1), width = h.size(2), hidden = w1.size(2);
+    train::GemmSpec specs[2];
+    int n = 0;
+    Tensor du;
+    if (h_needed || w1_needed) {
+      du = at::empty_like(u);
+      specs[n++] = product(w2, false, dout, false, du, width, train::kGemmRaggedN, train::kGemmGeluGradient, u);
+    }
+    if (w2_needed) {
+      dw2 = at::empty_like(w2);
+      specs[n++] = product(dout, true, act, true, dw2, rows, train::kGemmRaggedK);
+    }
+    if (n) products(specs, n, h, count);
+    n = 0;
+    if (h_needed) {                                  // the longer tiles first
+      dh = at::empty_like(h);
+      specs[n++] = product(w1, false, du, false, dh, hidden, train::kGemmRaggedN);
+    }
+    if (w1_needed) {
+      dw1 = at::empty_like(w1);
+      specs[n++] = product(du, true, h, true, dw1, rows, train::kGemmRaggedK);
+    }
+    if (n) products(specs, n, h, count);
+    return {dh, dw1, dw2};
+  }
+  if (w2_needed) dw2 = at::bmm(act_.transpose(1, 2), dout_);
   if (h_needed || w1_needed) {
-    Tensor dact = at::bmm(dout, w2.transpose(1, 2));
+    Tensor dact = at::bmm(dout_, w2_.transpose(1, 2));
     const Tensor u = dense(u_);
     Tensor du = at::empty_like(u);
     ok(train::geluBackward(code(u), dact.data_ptr(), u.data_ptr(), du.data_ptr(), nullptr, u.size(0) * u.size(1), (int)u.size(2), streamOf(u)),
        "gelu backward");
-    if (w1_needed) dw1 = at::bmm(h.transpose(1, 2), du);
-    if (h_needed) dh = at::bmm(du, w1.transpose(1, 2));
+    if (w1_needed) dw1 = at::bmm(h_.transpose(1, 2), du);
+    if (h_needed) dh = at::bmm(du, w1_.transpose(1, 2));
   }
   return {dh, dw1, dw2};
 }
@@ -449,8 +512,8 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const Tensor x = dense(x_);
     const Routed r = moeRouted(x, router, capacity);
     const Tensor h = r.send.view({router.size(0), capacity, x.size(1)});
-    const Expert e = moeExpert(h, w1, w2);
-    ctx->save_for_backward({x_, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out});
+    const Expert e = moeExpert(h, w1, w2, r.count);
+    ctx->save_for_backward({x_, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out, r.count});
     return moeCombined(x, r.gate, e.out, r.row_of);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -467,7 +530,7 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const Tensor x = dense(s[0]), rows = dense(s[12]);
     const Tensor dy = dense(g[0]);
     const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8]);
-    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, needed(ctx, 0), needed(ctx, 2), needed(ctx, 3));
+    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, s[13], needed(ctx, 0), needed(ctx, 2), needed(ctx, 3));
     if (!needed(ctx, 0, 1)) return {Tensor(), Tensor(), e[1], e[2], Tensor()};
     const Tensor dsend = e[0].defined() ? e[0] : at::zeros_like(h);   // the router alone
     const auto [dx, drouter] = moeRoutedBackward(x, router, s[4], s[5], s[6], s[7], dy, dsend, dgate, needed(ctx, 1));
@@ -514,7 +577,7 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
  public:
   static Variable forward(AutogradContext* ctx, const Variable& h, const Variable& w1, const Variable& w2) {
     c10::cuda::CUDAGuard dg(h.device());
-    const Expert e = moeExpert(h, w1, w2);
+    const Expert e = moeExpert(h, w1, w2, Tensor());
     ctx->save_for_backward({h, w1, w2, e.u, e.act});
     return e.out;
   }
@@ -525,7 +588,7 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
       const variable_list in = {viewOf(s[0]), viewOf(s[1]), viewOf(s[2])};
       return recorded({plainExperts(in[0], in[1], in[2])}, g, in);
     }
-    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), needed(ctx, 0), needed(ctx, 1), needed(ctx, 2));
+    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), Tensor(), needed(ctx, 0), needed(ctx, 1), needed(ctx, 2));
   }
 };
 

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(128) kMoeRoute(const T* __restrict__ logits, i
 
 constexpr int kAssignThreads = 1024, kAssignTokens = 4;   // four consecutive tokens per thread and sweep
 __global__ void __launch_bounds__(kAssignThreads) kMoeAssign(const int* __restrict__ expert, int tokens, int capacity, int* __restrict__ row_of,
-                                                             int* __restrict__ token_of) {
+                                                             int* __restrict__ token_of, int* __restrict__ count) {
   __shared__ int s_count[kAssignThreads / 32];
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = 0;   // tokens of this expert so far
@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kAssignThreads) kMoeAssign(const int* __restri
     __syncthreads();
   }
   for (int k = base + threadIdx.x; k < capacity; k += kAssignThreads) token_of[e * capacity + k] = -1;
+  if (threadIdx.x == 0) count[e] = base < capacity ? base : capacity;
 }
 
 // A warp per row: dst[row] = src[index[row]], zeros where there is none.
@@ -247,13 +248,13 @@ __global__ void __launch_bounds__(256, 4) kMoeTokenGradient(const T* __restrict_
 }
 
 hlResult_t moeRoute(int dt, const void* logits, int tokens, int experts, int capacity, int* expert, float* gate, int* row_of, int* token_of,
-                    cudaStream_t s) {
+                    int* count, cudaStream_t s) {
   if (experts < 1 || capacity < 1 || (int64_t)experts * capacity > 0x7fffffff)
     return fail(hlInvalidArgument, "MoE routing: %d experts of capacity %d", experts, capacity);
   if (tokens > 0) {
     HL_HALF_SWITCH(dt, T, { kMoeRoute<T><<<(tokens + 127) / 128, 128, 0, s>>>((const T*)logits, tokens, experts, expert, gate); });
   }
-  kMoeAssign<<<experts, kAssignThreads, 0, s>>>(expert, tokens, capacity, row_of, token_of);
+  kMoeAssign<<<experts, kAssignThreads, 0, s>>>(expert, tokens, capacity, row_of, token_of, count);
   return launched("MoE routing");
 }
 

@@ -14,24 +14,6 @@ namespace train {
 constexpr int kStripThreads = 256, kStripWarps = kStripThreads / 32, kStripUnroll = 4;
 constexpr int kStripRows = 128;   // rows of one CTA: 16 per warp; 8192 x 4096 makes 1024 CTAs, 8192 x 1024 256
 
-// 0.5 (1 + tanh z) = 1 / (1 + exp(-2 z)) =: s, and 1 - s = exp(-2 z) s: two special-function operations and no
-// cancellation. (tanhf costs more issue slots than the kernels have at memory speed: 8 x 1280 x 4096 in bf16, forward
-// 37.7 us with it and 32.3 without, backward 60.4 and 50.4.) The exponent is capped where s no longer matters, so that exp(-2 z) s stays finite.
-struct GeluGate {
-  float s, rest;
-};
-__device__ __forceinline__ GeluGate geluGate(float u) {
-  const float e = __expf(fminf(-1.5957691216057308f * (u + 0.044715f * u * u * u), 80.f));
-  const float s = __fdividef(1.f, 1.f + e);
-  return {s, e * s};
-}
-__device__ __forceinline__ float gelu(float u) {
-  // far below zero the sum 1 + tanh z cancels in fp32; there the plain formula is kept, so that results stay those of
-  // torch's own kernel bit for bit in bf16 (checked over all values)
-  if (u < -2.5f) return 0.5f * u * (1.f + tanhf(0.7978845608028654f * (u + 0.044715f * u * u * u)));
-  return u * geluGate(u).s;
-}
-
 struct SumOp {   // column sums alone
   const void* src;
 };
@@ -95,12 +77,7 @@ __global__ void __launch_bounds__(kStripThreads, 4) kStrip(const __grid_constant
           if constexpr (std::is_same<Op, GeluOp>::value) {
             float u[8];
             unpack8<T>(b[k], u);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const GeluGate q = geluGate(u[i]);
-              const float dz = 1.5957691216057308f * (1.f + 3.f * 0.044715f * u[i] * u[i]);
-              f[i] *= q.s + u[i] * q.s * q.rest * dz;
-            }
+            timesGeluSlope<8>(f, u);
             const uint4 p = pack8<T>(f);
             *reinterpret_cast<uint4*>(reinterpret_cast<T*>(op.du) + row * width + col) = p;
             unpack8<T>(p, f);   // the bias gradient is the sum of what the GEMMs see
@@ -139,8 +116,7 @@ __global__ void __launch_bounds__(256) kGeluForward(const uint4* __restrict__ u,
     if (i0 + k * 256 < packets) {
       float f[8];
       unpack8<T>(v[k], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = gelu(f[i]);
+      geluAll<8>(f);
       out[i0 + k * 256] = pack8<T>(f);
     }
 }

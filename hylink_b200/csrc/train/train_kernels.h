@@ -73,9 +73,9 @@ struct AdamWTensor {
 constexpr int kMaxAdamWTensors = 480;
 hlResult_t multiAdamW(int dt, const AdamWTensor* tensors, int n, double lr, double beta1, double beta2, double decay, double eps, cudaStream_t s);
 
-// Mixture of experts (moe.cu). row_of: [tokens], row of the dispatch buffer or -1; token_of: [experts * capacity].
+// Mixture of experts (moe.cu). row_of: [tokens], row of the dispatch buffer or -1; token_of: [experts * capacity]; count: [experts], rows in use.
 hlResult_t moeRoute(int dt, const void* logits, int tokens, int experts, int capacity, int* expert, float* gate, int* row_of, int* token_of,
-                    cudaStream_t s);
+                    int* count, cudaStream_t s);
 hlResult_t moeGather(const void* src, const int* index, void* dst, int rows, int width, cudaStream_t s);
 hlResult_t moeCombine(int dt, const void* x, const float* gate, const void* rows, const int* row_of, void* y, int tokens, int width, cudaStream_t s);
 hlResult_t moeRowGradient(int dt, const void* dy, const float* gate, const void* rows, const int* token_of, void* drows, float* dgate, int n_rows,
@@ -84,6 +84,28 @@ hlResult_t moeRowGradient(int dt, const void* dy, const float* gate, const void*
 bool moeRouterFits(int experts);
 hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const int* expert, const float* gate,
                             const float* dgate, const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s);
+
+// Products of groups of matrices (expert_gemm.cu): out[g][n][m] = sum over k of A[g][m][k] B[g][n][k]. a_mn / b_mn: the operand is
+// stored [g][k][m] / [g][k][n] instead. All are contiguous and start on 16-byte boundaries, inner dimensions are multiples of 8.
+// With `counts`, a group's n (kGemmRaggedN) or k (kGemmRaggedK) ends at counts[g], rounded up to 32 rows, one at least;
+// operand rows between the two are zeros, and rows of `out` behind them are not written.
+enum GemmRagged { kGemmWhole = 0, kGemmRaggedN = 1, kGemmRaggedK = 2 };
+// What follows: nothing; aux = gelu(out); out = product * gelu'(aux). The product is rounded before it goes on.
+enum GemmEpilogue { kGemmStore = 0, kGemmGelu = 1, kGemmGeluGradient = 2 };
+struct GemmSpec {
+  const void *a, *b;
+  void *out, *aux;
+  int m, n, k;
+  bool a_mn, b_mn;
+  int ragged, epilogue;
+  const void* bias = nullptr;    // [m], added before the product is rounded; not with kGemmGeluGradient
+  float* columns = nullptr;      // kGemmGeluGradient: partials of the sums of `out` over n: [gemmPartials(n)][m]; one group, without counts
+};
+inline int gemmPartials(int64_t n) { return 2 * (int)((n + 255) / 256); }
+// Whether experts of this width and hidden width, with this many rows in all, go through it.
+bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden);
+// One launch of `n` products, two at most.
+hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s);
 
 }  // namespace train
 }  // namespace hl

@@ -315,3 +315,75 @@ def test_gelu_over_all_16_bit_values():
     got = ops().moe_experts(x, eye, eye)
     want = torch.nn.functional.gelu(x, approximate="tanh")
     assert torch.equal(got, want), [(float(a), float(b), float(c)) for a, b, c in zip(x[got != want], got[got != want], want[got != want])][:20]
+
+
+def _plain_experts(h, w1, w2, dy):
+    """Forward and gradients in fp64, rounded where the layer stores a 16-bit tensor."""
+    r = [t.detach().double() for t in (h, w1, w2, dy)]
+    at = lambda t: t.to(h.dtype).double()                                   # noqa: E731
+    u = at(torch.bmm(r[0], r[1])).requires_grad_()
+    act = torch.nn.functional.gelu(u, approximate="tanh")
+    a = at(act.detach())
+    dact = at(torch.bmm(r[3], r[2].transpose(1, 2)))
+    du = at(torch.autograd.grad(act, u, dact)[0])
+    return torch.bmm(a, r[2]), torch.bmm(du, r[1].transpose(1, 2)), torch.bmm(r[0].transpose(1, 2), du), torch.bmm(a.transpose(1, 2), r[3])
+
+
+# tiles are 256 x 256, an operand's box 64, k goes in blocks of 64 and steps of 16, rows in steps of 32
+@pytest.mark.parametrize("experts,rows,width,hidden", [(1, 512, 256, 1024), (3, 257, 264, 1032), (2, 31, 512, 2048), (40, 33, 136, 520), (2, 320, 1000, 72),
+                                                       (1, 1, 4096, 4096), (5, 129, 320, 1288)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["dense", "off the boundary", "transposed", "strided"])
+def test_expert_products_at_the_edges_of_their_tiles(experts, rows, width, hidden, dtype, form):
+    from hylink_b200.ops.extension import ops
+
+    assert experts * rows * width * hidden >= 1 << 24                       # these go through the own kernel
+    torch.manual_seed(rows)
+    place = {"dense": lambda t: t, "off the boundary": _off_boundary, "transposed": lambda t: t.transpose(1, 2).contiguous().transpose(1, 2),
+             "strided": lambda t: torch.cat([t, t], 2)[:, :, :t.shape[2]]}[form]
+    h, dy = (torch.randn(experts, rows, width, device="cuda").to(dtype) for _ in range(2))
+    w1 = (torch.randn(experts, width, hidden, device="cuda") * width ** -0.5).to(dtype)
+    w2 = (torch.randn(experts, hidden, width, device="cuda") * hidden ** -0.5).to(dtype)
+    want = _plain_experts(h, w1, w2, dy)
+    leaves = [place(t).requires_grad_() for t in (h, w1, w2)]
+    y = ops().moe_experts(*leaves)
+    got = (y.detach(), *torch.autograd.grad(y, leaves, place(dy)))
+    # a result is rounded once, and where an fp32 sum falls on the other side of a tie an intermediate is one step off: under one
+    # step (2^-8 or 2^-11 of the value) in all, in the mean; a single entry is off by sums of such steps
+    step = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for name, a, b in zip(("y", "dh", "dw1", "dw2"), got, want):
+        diff = (a.double() - b).abs()
+        assert float(diff.norm() / b.norm()) < step, name
+        assert float((diff / (b.abs() + b.square().mean().sqrt())).max()) < 8 * step, name
+
+
+# an expert without tokens, with one, with a full and with an overflowing queue; capacities off every step
+@pytest.mark.parametrize("capacity", [1, 31, 300, 513])
+def test_experts_of_any_load(capacity):
+    """Rows beyond an expert's tokens are not computed: whatever memory held there must not be seen."""
+    from hylink_b200.ops.extension import ops
+
+    torch.manual_seed(capacity)
+    experts, width, hidden = 5, 256, 1 << 14
+    load = torch.tensor([0, 1, min(capacity, 40), capacity, capacity + 70])
+    expert = torch.repeat_interleave(torch.arange(experts), load)[torch.randperm(int(load.sum()))].cuda()
+    router = torch.zeros(experts, width, device="cuda")
+    router[:, :experts] = 30 * torch.eye(experts, device="cuda")
+    x = torch.randn(expert.numel(), width, device="cuda")
+    x[:, :experts] = torch.nn.functional.one_hot(expert, experts).float()
+    w1, w2 = (torch.randn(experts, *s, device="cuda") * s[0] ** -0.5 for s in ((width, hidden), (hidden, width)))
+    leaves = [t.to(torch.bfloat16).requires_grad_() for t in (x, router, w1, w2)]
+    dy = torch.randn_like(leaves[0])
+    trash = [torch.full((experts, capacity, hidden), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(6)]
+    del trash
+    y = ops().moe_layer(*leaves, capacity)
+    got = (y.detach(), *torch.autograd.grad(y, (leaves[0], leaves[2], leaves[3]), dy))
+    fx, fw1, fw2 = (t.detach().double().requires_grad_() for t in (leaves[0], leaves[2], leaves[3]))
+    out = fx.clone()
+    for e in range(experts):
+        mine = (expert == e).nonzero().squeeze(1)[:capacity]
+        out[mine] = fx[mine] + torch.nn.functional.gelu(fx[mine] @ fw1[e], approximate="tanh") @ fw2[e]     # the gate is one
+    want = (out, *torch.autograd.grad(out, (fx, fw1, fw2), dy.double()))
+    for name, a, b in zip(("y", "dx", "dw1", "dw2"), got, want):
+        assert bool(a.isfinite().all()), name
+        assert float((a.double() - b).norm()) < 3 * 2.0 ** -8 * float(b.norm()), name      # three roundings on the way
