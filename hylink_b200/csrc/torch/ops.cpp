@@ -249,9 +249,19 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     const Tensor p = at::addmm(bp, a, wp.t());
     Normed n = normForward(x, p.view(x.sizes()), gamma, beta, eps);
     const Tensor h = n.out.view({-1, width});
-    const Tensor u = at::addmm(bf, h, wf.t());
-    Tensor act = at::empty_like(u);
-    ok(train::geluForward(code(u), u.data_ptr(), act.data_ptr(), u.numel(), streamOf(u)), "gelu");
+    Tensor u, act;
+    if (wf.dim() == 2 && operand(wf, h, {wf.size(0), width}) && operand(bf, h, {wf.size(0)}) && train::mlpGemmPays(h.size(0), width, wf.size(0))) {
+      u = at::empty({h.size(0), wf.size(0)}, h.options());
+      act = at::empty_like(u);
+      const Tensor w = dense(wf), bias = bf.contiguous();
+      train::GemmSpec p = product(w, false, h, false, u, width, train::kGemmWhole, train::kGemmGelu, act);
+      p.bias = bias.data_ptr();
+      products(&p, 1, h);
+    } else {
+      u = at::addmm(bf, h, wf.t());
+      act = at::empty_like(u);
+      ok(train::geluForward(code(u), u.data_ptr(), act.data_ptr(), u.numel(), streamOf(u)), "gelu");
+    }
     const Tensor y = at::addmm(bo, act, wo.t()).view(x.sizes());
     ctx->save_for_backward({a_, wp, n.sum, n.mean, n.rstd, gamma, h, wf, u, act, wo, beta, bf, bo});
     ctx->saved_data["eps"] = eps;
@@ -275,17 +285,26 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     cudaStream_t st = streamOf(x2);
     TORCH_CHECK(g[1].defined(), "hylink: the block's branch has no gradient");
     const Tensor gy = rowsOf(g[1]);
-    Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {sp, hidden}), parts;
+    const bool own = operand(wo, gy, {width, hidden}) && operand(u, gy, {rows, hidden}) && train::mlpGemmPays(rows, width, hidden);
+    const int fcp = own ? train::gemmPartials(rows) : sp;
+    Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {fcp, hidden}), parts;
     Tensor dwo, dwf, dwp, da, dx, dgamma, dbeta, dbp, dbf;
     Columns cols(gamma);
     ok(train::columnSums(dt, gy.data_ptr(), out_parts.data_ptr<float>(), rows, (int)width, st), "bias gradient");
     Tensor dbo = cols.add(out_parts.data_ptr<float>(), sp, width);
     if (needed(ctx, 8)) dwo = at::mm(gy.t(), act);
     if (needed(ctx, 0, 7)) {
-      Tensor dact = at::mm(gy, wo);
       Tensor du = at::empty_like(u);
-      ok(train::geluBackward(dt, dact.data_ptr(), u.data_ptr(), du.data_ptr(), fc_parts.data_ptr<float>(), rows, (int)hidden, st), "gelu backward");
-      dbf = cols.add(fc_parts.data_ptr<float>(), sp, hidden);
+      if (own) {
+        const Tensor w = dense(wo);
+        train::GemmSpec p = product(w, true, gy, false, du, width, train::kGemmWhole, train::kGemmGeluGradient, u);
+        p.columns = fc_parts.data_ptr<float>();
+        products(&p, 1, gy);
+      } else {
+        const Tensor dact = at::mm(gy, wo);
+        ok(train::geluBackward(dt, dact.data_ptr(), u.data_ptr(), du.data_ptr(), fc_parts.data_ptr<float>(), rows, (int)hidden, st), "gelu backward");
+      }
+      dbf = cols.add(fc_parts.data_ptr<float>(), fcp, hidden);
       if (needed(ctx, 6)) dwf = at::mm(du.t(), h);
       if (needed(ctx, 0, 5)) {
         int np;

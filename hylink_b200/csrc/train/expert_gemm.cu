@@ -408,6 +408,12 @@ CUresult encode(const CudaDriver* d, CUtensorMap* m, int dt, const void* p, int6
 bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden) {
   return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (1 << 24);
 }
+// One product with a bias, which the library's kernels take too: what is gained is the element-wise pass alone, and that once the tiles fill
+// the GPU. Training steps, ms own / library: 4096 rows of 768 x 3072 8.49 / 8.56, 3072 of 1024 x 4096 14.51 / 14.62, 8192
+// 29.5 / 30.4; 1024 rows 9.11 / 9.06, 512 7.71 / 7.53, 256 7.47 / 7.02.
+bool mlpGemmPays(int64_t rows, int64_t width, int64_t hidden) {
+  return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (1LL << 33);
+}
 
 hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s) {
   const CudaDriver* d = CudaDriver::get();

@@ -104,6 +104,8 @@ struct GemmSpec {
 inline int gemmPartials(int64_t n) { return 2 * (int)((n + 255) / 256); }
 // Whether experts of this width and hidden width, with this many rows in all, go through it.
 bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden);
+// The same for the first product of a transformer block's MLP, and the gradient of what follows it.
+bool mlpGemmPays(int64_t rows, int64_t width, int64_t hidden);
 // One launch of `n` products, two at most.
 hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s);
 
