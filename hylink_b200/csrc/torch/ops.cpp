@@ -417,6 +417,18 @@ std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& route
   const Tensor router = dense(router_);
   const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
   Tensor dx = at::empty_like(x);
+  if (router_needed && train::moeTokensAndRouterFits((int)experts)) {
+    const int parts = train::moeRouterPartials((int)tokens);
+    Tensor partials = floats(x, {parts, experts * width});
+    ok(train::moeTokensAndRouter(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
+                                 expert.data_ptr<int>(), gate.data_ptr<float>(), dgate.data_ptr<float>(), router.data_ptr(), x.data_ptr(), dx.data_ptr(),
+                                 partials.data_ptr<float>(), (int)tokens, (int)width, (int)experts, streamOf(x)),
+       "MoE token gradient");
+    Columns cols(x);
+    Tensor drouter = cols.add(partials.data_ptr<float>(), parts, experts * width).view({experts, width});
+    cols.finish();
+    return {dx, drouter};
+  }
   Tensor dlogits = at::empty_like(logits);
   ok(train::moeTokenGradient(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),
                              expert.data_ptr<int>(), gate.data_ptr<float>(), dgate.data_ptr<float>(), router.data_ptr(), dx.data_ptr(),
@@ -499,9 +511,10 @@ Tensor moeCombined(const Tensor& x, const Tensor& gate, const Tensor& rows, cons
      "MoE combine");
   return y;
 }
-// {drows, dgate}; dgate is zero for tokens without a row: autograd's anomaly check and hooks read all of it
-std::pair<Tensor, Tensor> moeCombinedBackward(const Tensor& dy, const Tensor& gate, const Tensor& rows, const Tensor& token_of) {
-  Tensor drows = at::empty_like(rows), dgate = at::zeros_like(gate);
+// {drows, dgate}; with `whole`, dgate is zero for tokens without a row, which matters where it leaves this file: autograd's anomaly
+// check and hooks read all of it
+std::pair<Tensor, Tensor> moeCombinedBackward(const Tensor& dy, const Tensor& gate, const Tensor& rows, const Tensor& token_of, bool whole = true) {
+  Tensor drows = at::empty_like(rows), dgate = whole ? at::zeros_like(gate) : at::empty_like(gate);
   const int width = (int)rows.size(-1);
   ok(train::moeRowGradient(code(rows), dy.data_ptr(), gate.data_ptr<float>(), rows.data_ptr(), token_of.data_ptr<int>(), drows.data_ptr(),
                            dgate.data_ptr<float>(), (int)(rows.numel() / width), width, streamOf(rows)),
@@ -548,7 +561,7 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     }
     const Tensor x = dense(s[0]), rows = dense(s[12]);
     const Tensor dy = dense(g[0]);
-    const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8]);
+    const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8], false);
     const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, s[13], needed(ctx, 0), needed(ctx, 2), needed(ctx, 3));
     if (!needed(ctx, 0, 1)) return {Tensor(), Tensor(), e[1], e[2], Tensor()};
     const Tensor dsend = e[0].defined() ? e[0] : at::zeros_like(h);   // the router alone

@@ -8,6 +8,7 @@
 // moeCombine     y = x + gate * row
 // moeRowGradient d row = gate * dy; d gate = <dy, row>
 // moeTokenGradient  d logits of the gate's softmax; dx = dy + d row + d logits * router
+// moeTokensAndRouter  the same, and the router's gradient with it
 // All of them are bound by memory (16-byte packets, a warp or more per row). As tensor operations the same layer took
 // a one-hot matrix, a scan of it along the tokens in 64-bit integers (1.7 ms for 8192 tokens), sorted index updates
 // and eleven host round trips for the sizes of boolean selections.
@@ -247,6 +248,115 @@ __global__ void __launch_bounds__(256, 4) kMoeTokenGradient(const T* __restrict_
   }
 }
 
+// The last three steps of a layer's backward pass in one walk over the tokens, for up to eight experts: the logits' gradients
+// (as above), dx = dy + d row + d logits * router, and the sums over the tokens of d logits * x, which are the router's gradient.
+// Bound by memory: dy, the rows and x in, dx out. A CTA first works out its tokens' rows and logits' gradients, a thread per token, and
+// leaves them in shared memory (each warp for itself, between its loads, took 46 us: a chain of three loads per token). Then a
+// warp keeps 256 columns of the router and of the sums in registers and walks tokens, four at a time: twelve packets per
+// lane in flight. (128 columns and twice the warps: 37 us.) The warps share out up to 1024 columns and, where the rows are narrower,
+// the tokens. Sums go out as one partial per CTA. 8192 x 1024, eight experts: 33 us, and 3.4 to add the partials up; the kernels above 24.3
+// + 3.2 and a GEMM over eight rows 15.3, with the gaps between them 50. (What the products before have written leaves L2 meanwhile: 84 MB
+// beside the 67 that are moved here.)
+constexpr int kSumExperts = 8, kSumThreads = 256, kSumBlock = 1024, kSumTokens = 4;
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads, 1) kMoeTokensAndRouter(const T* __restrict__ dy, const T* __restrict__ drows, const int* __restrict__ row_of,
+                                                                      const T* __restrict__ logits, const int* __restrict__ expert,
+                                                                      const float* __restrict__ gate, const float* __restrict__ dgate,
+                                                                      const T* __restrict__ router, const T* __restrict__ x, T* __restrict__ dx,
+                                                                      float* __restrict__ partials, int tokens, int width, int experts, int shares) {
+  constexpr int E = kSumExperts, K = kSumTokens;
+  extern __shared__ float s_sums[];                    // [warps][E][256]
+  __shared__ __align__(16) float s_dl[kSumThreads][E];
+  __shared__ int s_row[kSumThreads];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int share = warp % shares, group = warp / shares, groups = kSumThreads / 32 / shares;   // of the columns, of the tokens
+  const int col = blockIdx.y * kSumBlock + share * 256 + lane * 8;
+  const bool live = group < groups && col < width;
+  uint64_t w[E][4], acc[E][4];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    float f[8];
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (live && e < experts) v = *reinterpret_cast<const uint4*>(router + (int64_t)e * width + col);
+    unpack8<T>(v, f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[e][i] = pair(f[2 * i], f[2 * i + 1]);
+      acc[e][i] = 0;
+    }
+  }
+  const int per = (tokens + gridDim.x - 1) / gridDim.x, t0 = blockIdx.x * per, t1 = min(tokens, t0 + per);
+  for (int base = t0; base < t1; base += kSumThreads) {
+    const int many = min(kSumThreads, t1 - base);
+    __syncthreads();
+    if ((int)threadIdx.x < many) {
+      const int t = base + threadIdx.x, at = expert[t], row = row_of[t];
+      const T* l = logits + (int64_t)t * experts;
+      const float g = gate[t], dg = row >= 0 ? dgate[t] * g : 0.f, top = (float)l[at];
+      s_row[threadIdx.x] = row;
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        s_dl[threadIdx.x][e] = e < experts ? (float)(T)(dg * ((e == at ? 1.f : 0.f) - __expf((float)l[e] - top) * g)) : 0.f;
+    }
+    __syncthreads();
+    for (int i = group; live && i < many; i += K * groups) {
+      uint4 a[K], b[K], c[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const bool here = i + k * groups < many;
+        const int row = here ? s_row[i + k * groups] : -1;
+        const int64_t at = (int64_t)(base + i + k * groups) * width + col;
+        a[k] = here && dy ? *reinterpret_cast<const uint4*>(dy + at) : make_uint4(0u, 0u, 0u, 0u);
+        b[k] = row >= 0 ? *reinterpret_cast<const uint4*>(drows + (int64_t)row * width + col) : make_uint4(0u, 0u, 0u, 0u);
+        c[k] = here ? *reinterpret_cast<const uint4*>(x + at) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (i + k * groups < many) {
+          float f[8], h[8];
+          uint64_t sum[4], in[4];
+          unpack8<T>(a[k], f);
+          unpack8<T>(b[k], h);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) sum[j] = add2(pair(f[2 * j], f[2 * j + 1]), pair(h[2 * j], h[2 * j + 1]));
+          unpack8<T>(c[k], h);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) in[j] = pair(h[2 * j], h[2 * j + 1]);
+#pragma unroll
+          for (int q = 0; q < E; q += 4) {
+            const float4 d4 = *reinterpret_cast<const float4*>(&s_dl[i + k * groups][q]);
+            const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (q + e < experts) {
+                const uint64_t d2 = pair(d[e], d[e]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  sum[j] = fma2(d2, w[q + e][j], sum[j]);
+                  acc[q + e][j] = fma2(d2, in[j], acc[q + e][j]);
+                }
+              }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) unpair(sum[j], f[2 * j], f[2 * j + 1]);
+          *reinterpret_cast<uint4*>(dx + (int64_t)(base + i + k * groups) * width + col) = pack8<T>(f);
+        }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint64_t*>(s_sums + (warp * E + e) * 256 + lane * 8 + 2 * i) = acc[e][i];
+  __syncthreads();
+  const int columns = min(kSumBlock, width - (int)blockIdx.y * kSumBlock);
+  for (int i = threadIdx.x; i < experts * columns; i += kSumThreads) {
+    const int e = i / columns, c = i - e * columns;
+    float sum = 0.f;
+    for (int g = 0; g < groups; ++g) sum += s_sums[((g * shares + (c >> 8)) * E + e) * 256 + (c & 255)];
+    partials[((int64_t)blockIdx.x * experts + e) * width + blockIdx.y * kSumBlock + c] = sum;
+  }
+}
+
 hlResult_t moeRoute(int dt, const void* logits, int tokens, int experts, int capacity, int* expert, float* gate, int* row_of, int* token_of,
                     int* count, cudaStream_t s) {
   if (experts < 1 || capacity < 1 || (int64_t)experts * capacity > 0x7fffffff)
@@ -296,6 +406,24 @@ hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int
     if (!moeRouterFits(experts)) go(kMoeTokenGradient<T, 0>);
     else if (experts <= 8) go(kMoeTokenGradient<T, 8>);
     else go(kMoeTokenGradient<T, 16>);
+  });
+  return launched("MoE token gradient");
+}
+
+bool moeTokensAndRouterFits(int experts) { return experts <= kSumExperts; }
+int moeRouterPartials(int tokens) { return tokens < 148 ? tokens : 148; }
+
+hlResult_t moeTokensAndRouter(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const int* expert, const float* gate,
+                              const float* dgate, const void* router, const void* x, void* dx, float* partials, int tokens, int width, int experts,
+                              cudaStream_t s) {
+  if (width % 8 || experts < 1 || experts > kSumExperts || tokens < 1) return fail(hlInvalidArgument, "MoE gradient: %d x %d, %d experts", tokens, width, experts);
+  const int blocks = (width + kSumBlock - 1) / kSumBlock, shares = blocks > 1 ? kSumBlock / 256 : (width + 255) / 256;
+  const size_t smem = (size_t)(kSumThreads / 32) * kSumExperts * 256 * sizeof(float);
+  HL_HALF_SWITCH(dt, T, {
+    cudaFuncSetAttribute((const void*)kMoeTokensAndRouter<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kMoeTokensAndRouter<T><<<dim3((unsigned)moeRouterPartials(tokens), (unsigned)blocks), kSumThreads, smem, s>>>(
+        (const T*)dy, (const T*)drows, row_of, (const T*)logits, expert, gate, dgate, (const T*)router, (const T*)x, (T*)dx, partials, tokens, width,
+        experts, shares);
   });
   return launched("MoE token gradient");
 }

@@ -85,6 +85,14 @@ bool moeRouterFits(int experts);
 hlResult_t moeTokenGradient(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const int* expert, const float* gate,
                             const float* dgate, const void* router, void* dx, void* dlogits, int tokens, int width, int experts, cudaStream_t s);
 
+// The same, and partials of the router's gradient ([moeRouterPartials(tokens)][experts * width], to be finished by finishColumns), in
+// one pass; for as many experts as fit.
+bool moeTokensAndRouterFits(int experts);
+int moeRouterPartials(int tokens);
+hlResult_t moeTokensAndRouter(int dt, const void* dy, const void* drows, const int* row_of, const void* logits, const int* expert, const float* gate,
+                              const float* dgate, const void* router, const void* x, void* dx, float* partials, int tokens, int width, int experts,
+                              cudaStream_t s);
+
 // Products of groups of matrices (expert_gemm.cu): out[g][n][m] = sum over k of A[g][m][k] B[g][n][k]. a_mn / b_mn: the operand is
 // stored [g][k][m] / [g][k][n] instead. All are contiguous and start on 16-byte boundaries, inner dimensions are multiples of 8.
 // With `counts`, a group's n (kGemmRaggedN) or k (kGemmRaggedK) ends at counts[g], rounded up to 32 rows, one at least;

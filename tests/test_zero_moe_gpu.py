@@ -387,3 +387,35 @@ def test_experts_of_any_load(capacity):
     for name, a, b in zip(("y", "dx", "dw1", "dw2"), got, want):
         assert bool(a.isfinite().all()), name
         assert float((a.double() - b).norm()) < 3 * 2.0 ** -8 * float(b.norm()), name      # three roundings on the way
+
+
+# a warp's 256 columns, a CTA's 1024, rows that leave warps without work; fewer tokens than CTAs, more than a CTA's threads; one to all experts
+@pytest.mark.parametrize("tokens,width,experts", [(1, 8, 1), (147, 264, 8), (149, 768, 3), (600, 1032, 8), (40000, 256, 2), (1200, 2048, 5)])
+def test_the_routers_gradient_at_the_edges_of_its_blocks(tokens, width, experts):
+    from hylink_b200.ops.extension import ops
+
+    torch.manual_seed(tokens)
+    capacity = max(1, tokens // experts)             # some tokens have no row
+    x, dy = (torch.randn(tokens, width, device="cuda").to(torch.bfloat16) for _ in range(2))
+    router = (torch.randn(experts, width, device="cuda") * width ** -0.5).to(torch.bfloat16)
+    w1, w2 = (torch.randn(experts, *s, device="cuda").mul(s[0] ** -0.5).to(torch.bfloat16) for s in ((width, 64), (64, width)))
+    leaves = [t.clone().requires_grad_() for t in (x, router)]
+    y = ops().moe_layer(*leaves, w1, w2, capacity)
+    dx, drouter = torch.autograd.grad(y, leaves, dy)
+    # the same pieces, with the router's share left to a product and the sums to fp64
+    alone = [x.clone().requires_grad_(), router]
+    plain = torch.autograd.grad(ops().moe_layer(*alone, w1, w2, capacity), alone[0], dy)[0]
+    assert torch.equal(dx, plain)                    # without the router's gradient the tokens' comes from the kernel of its own
+    x1, send, gate, row_of, _ = ops().moe_dispatch(x, router, capacity)
+    p = torch.softmax((x @ router.t()).double(), -1)
+    expert = p.argmax(-1)
+    h = torch.bmm(torch.nn.functional.gelu(torch.bmm(send.view(experts, capacity, width).double(), w1.double()), approximate="tanh"), w2.double())
+    dgate = torch.where(row_of >= 0, (dy.double() * h.view(-1, width)[row_of.long().clamp_min(0)]).sum(1), 0.)
+    onehot = torch.nn.functional.one_hot(expert, experts)
+    dlogits = (dgate * p.gather(1, expert[:, None]).squeeze(1))[:, None] * (onehot - p)
+    want = dlogits.t() @ x.double()
+    # 16-bit logits' gradients from rows that were rounded three times: two steps of 2^-8 in the mean
+    if float(want.norm()) > 0:
+        assert float((drouter.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8
+    else:
+        assert not drouter.any()
