@@ -237,10 +237,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
       const int rows = j.n - t.n0;                     // of the tile that exist
       auto row = [&](int c, int i) { return c * kChunk + 8 * i + (lane >> 2); };
       uint4 pre[4];                                    // pre-activations of the next chunk
-      auto fetch = [&](int c) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (live && row(c, i) < rows) pre[i] = __ldcs(reinterpret_cast<const uint4*>(aux + (int64_t)row(c, i) * j.m));
+      auto fetch = [&](int c, int i) {
+        if (live && row(c, i) < rows) pre[i] = __ldcs(reinterpret_cast<const uint4*>(aux + (int64_t)row(c, i) * j.m));
       };
       float bias[4], sums[8];
 #pragma unroll
@@ -250,7 +248,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) sums[i] = 0.f;
-      if (epilogue == kGemmGeluGradient && group < chunks) fetch(group);
+      if (epilogue == kGemmGeluGradient && group < chunks) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fetch(group, i);
+      }
       if (!__all_sync(0xffffffffu, tc::barWait(tc::smem(&s_acc_full[acc]), n >> 1 & 1, stop, kGemmLimitNs))) break;
       tc::fenceAfter();
       // Chunk c to one of the two places in shared memory; the accumulator is free with the last of them.
@@ -287,6 +288,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
             for (int k = 0; k < 2; ++k) {
               unpack8<T>(v[i + k], f + 8 * k);
               unpack8<T>(pre[i + k], u + 8 * k);
+              if (c + 2 < chunks) fetch(c + 2, i + k);
             }
             timesGeluSlope<16>(f, u);
 #pragma unroll
@@ -300,7 +302,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
               }
             }
           }
-          if (c + 2 < chunks) fetch(c + 2);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)

@@ -513,3 +513,29 @@ def test_multi_tensor_adamw_matches_torch(dtype):
             opt.state[r]["exp_avg_sq"].copy_(v)
     assert all(float(s) == 3 for s in steps)
     assert not ops().multi_adamw(ps[:1], [gs[0].cpu()], ms[:1], vs[:1], steps[:1], 1e-2, 0.9, 0.95, 0.1, 1e-8)
+
+
+# the smallest MLP whose products carry gelu themselves (2^33 multiplications), rows off the steps of 32 and of a tile's 256, fp16
+@pytest.mark.parametrize("rows,width,hidden,dtype", [(2048, 1024, 4096, torch.bfloat16), (2049, 1024, 4096, torch.bfloat16), (4100, 520, 4104, torch.bfloat16),
+                                                     (2300, 1024, 4096, torch.float16)])
+def test_gelu_inside_the_products_of_an_mlp(rows, width, hidden, dtype):
+    from hylink_b200.ops.extension import ops
+
+    assert rows * width * hidden >= 1 << 33
+    torch.manual_seed(rows)
+    make = lambda *s, scale=1.0: (torch.randn(*s, device="cuda") * scale).to(dtype)            # noqa: E731
+    x, a, dx2, dy2 = (make(1, rows, width) for _ in range(4))
+    wp, bp, gamma, beta = make(width, width, scale=width ** -0.5), make(width, scale=0.1), 1 + make(width, scale=0.1), make(width, scale=0.1)
+    wf, bf = make(hidden, width, scale=width ** -0.5), make(hidden, scale=0.1)
+    wo, bo = make(width, hidden, scale=hidden ** -0.5), make(width, scale=0.1)
+    leaves = [t.requires_grad_() for t in (x, a, wp, bp, gamma, beta, wf, bf, wo, bo)]
+    x2, y2 = ops().block_post(*leaves, 1e-5)
+    got = (x2.detach(), y2.detach(), *torch.autograd.grad((x2, y2), leaves, (dx2, dy2)))
+    r = [t.detach().double().requires_grad_() for t in leaves]
+    F = torch.nn.functional
+    rx2 = r[0] + F.linear(r[1], r[2], r[3])
+    ry2 = F.linear(F.gelu(F.linear(F.layer_norm(rx2, (width,), r[4], r[5], 1e-5), r[6], r[7]), approximate="tanh"), r[8], r[9])
+    want = (rx2, ry2, *torch.autograd.grad((rx2, ry2), r, (dx2.double(), dy2.double())))
+    step = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for i, (g, w) in enumerate(zip(got, want)):      # up to six roundings one after the other, each half a step at most
+        assert float((g.double() - w).norm() / w.norm()) < 3 * step, i
