@@ -8,8 +8,8 @@
 // the other half belongs to the tile before, which the epilogue warps empty meanwhile. Persistent, one pair per two SMs.
 //   warp 0      TMA loads, six stages of 64 of k (32 KB per CTA; 8 x 1024 x 1024 x 4096 in bf16: four stages 60 us, five 56.2, six 55.6)
 //   warp 1      products, in the pair's first CTA alone
-//   warps 4-11  epilogue: chunks of 32 x 32, rounded, transposed by stmatrix through 2 KB of the warp's own, and stored as rows
-//               of 64 bytes; no warp waits for another. (Chunks of 128 x 32 that leave by TMA, with barriers of 128 threads: 75 us
+//   warps 4-11  epilogue: chunks of 32 x 32, rounded, transposed by stmatrix through shared memory of the warp's own (two
+//               places of 2 KB in turn), and stored as rows of 64 bytes; no warp waits for another. (Chunks of 128 x 32 that leave by TMA, with barriers of 128 threads: 75 us
 //               where this takes 67.)
 // Loads and products run in all lanes of their warps up to the instruction itself, so that its operands are in uniform
 // registers: in a branch of one lane the same loops took 86 us instead of 57.
@@ -19,11 +19,12 @@
 // and k end at the `counts` that routing found, rounded up to 32. Rows between a count and the rounding are zeros.
 //
 // 8 x 1024 x 1024 x 4096 in bf16, 69 GFLOP, back to back for a second, under the power cap: 62 to 64 us without an epilogue (the library 61.5 to
-// 67), 77 with gelu (library and gelu kernel 86), 88 with gelu's gradient (97); in short runs 54, 67 and 76. Bound by power
+// 67), 77 to 80 with gelu (the library's product 65, gelu alone 21), 88 with its gradient (67 and 30); in short runs 54, 67 and 74. Bound by power
 // without an epilogue, with one by its warps. Tried: pairs of 512 x 256 with one set of accumulators, which read a quarter less (55 us, 75
 // with gelu: the epilogue then has half the time), also with sixteen epilogue warps (58, 72).
 // The sums go up k in the order of the library's own kernels: results are theirs, bit for bit, where this was compared.
-// Every wait is bounded; one that runs out sets the status word, which the next launch reports.
+// Every wait is bounded; one that runs out sets the status word, which the process's next launch reports as
+// an error.
 #include <cuda.h>
 
 #include <atomic>
