@@ -719,9 +719,9 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* c
 //   all-reduce      stream shard s of the input straight from the caller's buffer into slot `rank` of its owner | barrier |
 //                   fold the own shard (read from the caller's buffer) and the landed slots in ascending rank order,
 //                   store the result to the caller's output and into every peer's result area | barrier | copy the
-//                   peers' results out of the local result area | barrier. Ranks of one GPU store a result once, in the
+//                   peers' results out of the local result area | barrier. Three or more ranks of one GPU store a result once, in the
 //                   owner's result area, and copy it out of there: it stays in L2, where n - 1 copies of it do not (8 ranks x
-//                   16 MiB of fp32 123 us with a copy per peer, 97 with one; 4 ranks 59 and 51, 2 ranks 26.7 and 26.6)
+//                   16 MiB of fp32 123 us with a copy per peer, 97 with one; 4 ranks 59 and 51)
 //   reduce-scatter  push the peers' segments | barrier | fold | barrier
 //   all-gather      store the own segment into every peer's slot and into the own output | barrier | copy out | barrier
 //   all-to-all      push the peers' segments, copy the own one | barrier | copy out | barrier
@@ -827,8 +827,9 @@ __global__ void __launch_bounds__(HL_NVL_THREADS) kPush(const HlCommDev* comms, 
   const Parts<W> in(a.in, kAllReduce ? sp * N : a.in_seg_stride, a.count, kAllReduce ? a.count : 0);
   const Parts<W> out(a.out, sp * N, a.count, kAllReduce ? a.count : 0);   // reduce-scatter: part 0 alone
   const uint64_t res_off = sp * (uint64_t)n;                              // results live behind the slots
-  // Ranks of one GPU: a result is stored once, in its owner's result area, and the peers read it there.
-  const bool near = c.one_device != 0;
+  // Ranks of one GPU: a result is stored once, in its owner's result area, and the peers read it there. Of two ranks one copy is all there is,
+  // and the reader's own area the better place (1.9 million elements of fp16 12.6 us, in the owner's 13.1).
+  const bool near = MR > 2 && c.one_device != 0;
   const int copies = near ? 1 : n - 1;
   for (int k = 1; k < n; ++k) {
     const int q = peerOf(r, k, n);
