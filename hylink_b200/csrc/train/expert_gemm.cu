@@ -291,7 +291,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
               unpack8<T>(pre[i + k], u + 8 * k);
               if (c + 2 < chunks) fetch(c + 2, i + k);
             }
-            timesGeluSlope<16>(f, u);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) f[k] *= geluSlope(u[k]);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               v[i + k] = pack8<T>(f + 8 * k);

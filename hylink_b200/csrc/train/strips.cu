@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(kStripThreads, 4) kStrip(const __grid_constant
           if constexpr (std::is_same<Op, GeluOp>::value) {
             float u[8];
             unpack8<T>(b[k], u);
-            timesGeluSlope<8>(f, u);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] *= geluSlope(u[i]);
             const uint4 p = pack8<T>(f);
             *reinterpret_cast<uint4*>(reinterpret_cast<T*>(op.du) + row * width + col) = p;
             unpack8<T>(p, f);   // the bias gradient is the sum of what the GEMMs see
@@ -116,7 +117,8 @@ __global__ void __launch_bounds__(256) kGeluForward(const uint4* __restrict__ u,
     if (i0 + k * 256 < packets) {
       float f[8];
       unpack8<T>(v[k], f);
-      geluAll<8>(f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = gelu(f[i]);
       out[i0 + k * 256] = pack8<T>(f);
     }
 }

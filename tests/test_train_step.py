@@ -539,3 +539,42 @@ def test_gelu_inside_the_products_of_an_mlp(rows, width, hidden, dtype):
     step = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     for i, (g, w) in enumerate(zip(got, want)):      # up to six roundings one after the other, each half a step at most
         assert float((g.double() - w).norm() / w.norm()) < 3 * step, i
+
+
+# every 16-bit pattern in some order, in the element-wise kernels (one row) and in the products' epilogues (2^33 multiplications)
+@pytest.mark.parametrize("rows,width", [(1, 64), (512, 256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gelu_of_a_value_beside_any_others(rows, width, dtype):
+    """gelu has torch's bits in bf16, and it and its slope are those of the value alone: infinities, NaN and far values beside it change nothing."""
+    from hylink_b200.ops.extension import ops
+
+    hidden = 1 << 16
+    zeros = lambda *s: torch.zeros(*s, device="cuda", dtype=dtype)             # noqa: E731
+    values = torch.arange(hidden, device="cuda").to(torch.int16).view(dtype)
+
+    def through(u):                                                            # pre-activations are the bias, the outputs' gradient picks row 0
+        x, a, wp, bp, gamma, beta, wf, wo, bo = (zeros(1, rows, width), zeros(1, rows, width), zeros(width, width), zeros(width), 1 + zeros(width),
+                                                 zeros(width), zeros(hidden, width), zeros(width, hidden), zeros(width))
+        wo[0], bf, dy = 1, u.clone().requires_grad_(), zeros(1, rows, width)
+        dy[0, 0, 0] = 1
+        x2, y2 = ops().block_post(x, a, wp, bp, gamma, beta, wf, bf, wo.requires_grad_(), bo, 1e-5)
+        act, slope = torch.autograd.grad(y2, (wo, bf), dy)
+        return act[0], slope
+
+    act, slope = through(values)
+    want = torch.nn.functional.gelu(values, approximate="tanh")
+    fin, step, least = want.isfinite(), *((2.0 ** -8, 0.0) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -25))    # half a step of the type, of its least
+    if dtype == torch.bfloat16:
+        assert torch.equal(act[fin], want[fin])
+    else:                                                                      # rounded to the other side of a tie
+        assert bool(((act - want).abs()[fin].double() <= 2 * step * want.abs()[fin].double() + 2 * least).all())
+    u = values.double().requires_grad_()
+    (exact,) = torch.autograd.grad(torch.nn.functional.gelu(u, approximate="tanh").sum(), u)
+    near = values.abs() < 1e4                                                  # further out u^3 leaves fp32's range, in torch's kernel too
+    # one rounding to the type, and the fp32 operations before it: some 2^-22 of terms up to 2
+    assert bool(((slope.double() - exact).abs()[near] <= step * exact.abs()[near] + 2.0 ** -21 + least).all())
+    for seed in range(6):
+        order = torch.randperm(hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+        a, s = through(values[order])
+        for got, one in ((a, act[order]), (s, slope[order])):
+            assert torch.equal(got[one.isfinite()], one[one.isfinite()])
