@@ -817,6 +817,15 @@ PyMethodDef kNativeCalls[] = {{"emu_run", (PyCFunction)(void*)emuRun, METH_FASTC
 
 }  // namespace
 
+// A product whose operands never arrive, and whose waits end after this time: for tests of what is reported then.
+void productWithoutOperands(const Tensor& a, double limit_ms) {
+  TORCH_CHECK(a.dim() == 2 && a.is_cuda() && a.is_contiguous() && a.size(1) % 8 == 0 && a.size(0) % 8 == 0, "hylink: a matrix of whole packets");
+  c10::cuda::CUDAGuard dg(a.device());
+  const Tensor out = at::empty({a.size(0), a.size(0)}, a.options());
+  const train::GemmSpec p = product(a, false, a, false, out, a.size(1));
+  ok(train::expertGemm(code(a), &p, 1, 1, nullptr, streamOf(a), (uint64_t)(limit_ms * 1e6), false), "grouped product");
+}
+
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("max_norm_width") = train::kMaxNormWidth;
   m.attr("max_rows") = train::kMaxRows;
@@ -832,6 +841,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_layer", [](const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w2, int64_t capacity) {
     return MoeLayer::apply(x, router, w1, w2, capacity);
   });
+  m.def("check_products", [](int device) { ok(train::gemmStatus(device, true), "products"); });
+  m.def("product_without_operands", &productWithoutOperands);
   m.def("multi_adamw", &multiAdamW);
   m.def("accumulation_hooks", &accumulationHooks);
   m.def("moe_dispatch", [](const Tensor& x, const Tensor& router, int64_t capacity) { return MoeDispatch::apply(x, router, capacity); });

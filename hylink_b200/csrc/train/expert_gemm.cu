@@ -23,8 +23,8 @@
 // without an epilogue, with one by its warps. Tried: pairs of 512 x 256 with one set of accumulators, which read a quarter less (55 us, 75
 // with gelu: the epilogue then has half the time), also with sixteen epilogue warps (58, 72).
 // The sums go up k in the order of the library's own kernels: results are theirs, bit for bit, where this was compared.
-// Every wait is bounded; one that runs out sets the status word, which the process's next launch reports as
-// an error.
+// Every wait is bounded; one that runs out sets the device's status word, which stays set until gemmStatus has reported it: to whoever
+// waits for the results (a trainer after its step, replayed from a graph or not), and to every launch until then.
 #include <cuda.h>
 
 #include <atomic>
@@ -42,7 +42,7 @@ constexpr int kGemmStages = 6, kTile = 256, kKBlock = 64, kStageBytes = 32768, k
 constexpr int kGemmThreads = 384, kEpilogueWarps = 8, kChunkStaging = 2048, kWarpStaging = 2 * kChunkStaging;
 constexpr int kGemmShared = kGemmStages * kStageBytes + kEpilogueWarps * kWarpStaging + 1024;
 constexpr int kTmemColumns = 512;
-constexpr uint64_t kGemmLimitNs = 2000000000ull;
+constexpr uint64_t kGemmLimitNs = 2000000000ull, kSettleNs = 1000000ull;
 
 struct GemmJob {
   CUtensorMap a, b;
@@ -57,6 +57,8 @@ struct GemmArgs {
   int jobs, groups;
   const int* counts;
   volatile unsigned* status;
+  uint64_t limit_ns;              // of every wait
+  int loads;                      // 0: operands never arrive, for tests of the limit
 };
 
 struct Tile {
@@ -122,7 +124,7 @@ __device__ __forceinline__ void transposeChunk(const float* r, const float* bias
 template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kExpertGemm(const __grid_constant__ GemmArgs args) {
   extern __shared__ uint8_t s_raw[];
-  __shared__ __align__(8) uint64_t s_full[kGemmStages], s_empty[kGemmStages], s_acc_full[2], s_acc_empty[2];
+  __shared__ __align__(8) uint64_t s_full[kGemmStages], s_empty[kGemmStages], s_acc_full[2], s_acc_empty[2], s_done;
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_stop;
   const uint32_t stages = (tc::smem(s_raw) + 1023) & ~1023u, staging = stages + kGemmStages * kStageBytes;
@@ -139,6 +141,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
       tc::barInit(tc::smem(&s_acc_full[i]), 1);
       tc::barInit(tc::smem(&s_acc_empty[i]), 2 * kEpilogueWarps);
     }
+    tc::barInit(tc::smem(&s_done), 1);
     tc::barInitFence();
   }
   if (warp == 1 && lane == 0)
@@ -157,9 +160,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
   Tile t;
 
   if (warp == 0) {                                     // ---- loads
-    int s = 0;
+    int s = 0, rounds = 0;
     uint32_t phase = 1;                                // of the wait for a free stage: the first round finds all of them free
-    bool go = true;
+    bool go = args.loads != 0;
     const uint32_t full0 = tc::mapToRank(tc::smem(&s_full[0]), 0);
     for (int at = pair; go && walk.seek(args, at, &t); at += pairs) {
       const GemmJob& j = *t.job;
@@ -169,7 +172,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
       const uint32_t bytes = two ? 8 * kBoxBytes : 6 * kBoxBytes;
       const bool a_mn = j.a_mn != 0, b_mn = j.b_mn != 0;
       for (int k = 0; k < t.k_blocks * kKBlock; k += kKBlock) {
-        go = tc::barWait(tc::smem(&s_empty[s]), phase, stop, kGemmLimitNs);
+        go = tc::barWait(tc::smem(&s_empty[s]), phase, stop, args.limit_ns);
         if (!(go = __all_sync(0xffffffffu, go))) break;
         if (tc::elected()) {
           if (rank == 0) tc::barExpect(tc::smem(&s_full[s]), bytes);
@@ -183,9 +186,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
         if (++s == kGemmStages) {
           s = 0;
           phase ^= 1;
+          rounds = 1;
         }
       }
     }
+    if (!go && rank == 0)                              // given up: the pair's copies are counted here, those that both have asked for land first
+      for (int i = rounds ? 0 : kGemmStages - s; i < kGemmStages; ++i) {
+        const int at = (s + i) % kGemmStages;          // oldest first; stages from s on were filled in the round before
+        tc::barWait(tc::smem(&s_full[at]), at < s ? phase ^ 1 : phase, nullptr, kSettleNs);
+      }
   } else if (warp == 1 && rank == 0) {                 // ---- products
     const uint32_t kind = 1u << 4 | (std::is_same<T, __nv_bfloat16>::value ? 1u << 7 | 1u << 10 : 0u) | (uint32_t)(kTile >> 4) << 24;
     int s = 0, n = 0;
@@ -194,7 +203,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
     for (int at = pair; go && walk.seek(args, at, &t); at += pairs, ++n) {
       const GemmJob& j = *t.job;
       const int acc = n & 1;
-      go = tc::barWait<true>(tc::smem(&s_acc_empty[acc]), (n >> 1 & 1) ^ 1, stop, kGemmLimitNs);
+      go = tc::barWait<true>(tc::smem(&s_acc_empty[acc]), (n >> 1 & 1) ^ 1, stop, args.limit_ns);
       if (!(go = __all_sync(0xffffffffu, go))) break;
       tc::fenceAfter();
       const bool a_mn = j.a_mn != 0, b_mn = j.b_mn != 0;
@@ -203,7 +212,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
       const uint64_t a_step = a_mn ? 2048 >> 4 : 32 >> 4, b_step = b_mn ? 2048 >> 4 : 32 >> 4;   // 16 of k
       const uint64_t a0 = tc::operand(stages, a_mn, kBoxBytes), b0 = tc::operand(stages + 2 * kBoxBytes, b_mn, kBoxBytes);
       for (int kb = 0; kb < t.k_blocks; ++kb) {
-        go = tc::barWait(tc::smem(&s_full[s]), phase, stop, kGemmLimitNs);
+        go = tc::barWait(tc::smem(&s_full[s]), phase, stop, args.limit_ns);
         if (!(go = __all_sync(0xffffffffu, go))) break;
         tc::fenceAfter();
         const int steps = kb + 1 < t.k_blocks ? kKBlock / 16 : t.last_steps;
@@ -221,6 +230,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
           phase ^= 1;
         }
       }
+    }
+    if (!go) {                                         // given up: the products that were issued read shared memory until they are done
+      if (tc::elected()) tc::commitPair(tc::smem(&s_done));
+      __syncwarp();
+      tc::barWait(tc::smem(&s_done), 0, nullptr, kSettleNs);
     }
   } else if (warp >= 4) {                              // ---- epilogue
     const int group = (warp - 4) >> 2, q = warp & 3;   // a warp reads the 32 lanes of its place in a group of four
@@ -253,7 +267,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
 #pragma unroll
         for (int i = 0; i < 4; ++i) fetch(group, i);
       }
-      if (!__all_sync(0xffffffffu, tc::barWait(tc::smem(&s_acc_full[acc]), n >> 1 & 1, stop, kGemmLimitNs))) break;
+      if (!__all_sync(0xffffffffu, tc::barWait(tc::smem(&s_acc_full[acc]), n >> 1 & 1, stop, args.limit_ns))) break;
       tc::fenceAfter();
       // Chunk c to one of the two places in shared memory; the accumulator is free with the last of them.
       auto stage = [&](int c) {
@@ -329,10 +343,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
     }
   }
   __syncwarp();
-  if (*stop) {                                         // given up: tell, and let the copies in flight land
+  if (*stop) {                                         // given up: tell. A copy that one CTA alone has asked for ends no phase: it gets the time of many
     *args.status = 1;
     __threadfence_system();
-    for (const uint64_t t0 = tc::nowNs(); tc::nowNs() - t0 < 200000;) {
+    for (const uint64_t t0 = tc::nowNs(); tc::nowNs() - t0 < kSettleNs;) {
     }
   }
   __syncwarp();
@@ -344,29 +358,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) kEx
 
 namespace {
 
-// Set by a kernel whose wait ran out; null where page-locked memory could not be had.
-unsigned* gaveUp() {
-  static unsigned* word = nullptr;
+// A word per device in page-locked memory, set by a kernel whose wait ran out; null where that memory could not be had.
+constexpr int kDevices = 64;
+std::atomic<unsigned*> g_words{nullptr};
+unsigned* statusWords() {
   static std::once_flag once;
   std::call_once(once, [] {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // the caller's stream may be recording
     cudaThreadExchangeStreamCaptureMode(&mode);
     void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-      word = (unsigned*)p;
-      *(volatile unsigned*)word = 0;
+    if (cudaHostAlloc(&p, kDevices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      for (int i = 0; i < kDevices; ++i) ((volatile unsigned*)p)[i] = 0;
+      g_words.store((unsigned*)p, std::memory_order_release);
     } else {
       cudaGetLastError();
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
   });
-  return word;
+  return g_words.load(std::memory_order_acquire);
 }
 
 // Pairs of CTAs that run at once on the current device; 0 where the kernel does not run.
 template <typename T>
 int residentPairs() {
-  constexpr int kDevices = 64;
   static std::atomic<int> known[kDevices];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) return 0;
@@ -418,24 +432,35 @@ bool mlpGemmPays(int64_t rows, int64_t width, int64_t hidden) {
   return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (1LL << 33);
 }
 
-hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s) {
+hlResult_t gemmStatus(int device, bool clear) {
+  unsigned* const words = g_words.load(std::memory_order_acquire);
+  if (device < 0 && cudaGetDevice(&device) != cudaSuccess) {
+    cudaGetLastError();
+    return hlSuccess;                                  // no device, no products
+  }
+  if (!words || device >= kDevices || !((volatile unsigned*)words)[device]) return hlSuccess;
+  if (clear) ((volatile unsigned*)words)[device] = 0;
+  return fail(hlTimeout, "grouped product: a wait on device %d ran out, results since then are not valid", device);
+}
+
+hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s, uint64_t limit_ns, bool loads) {
   const CudaDriver* d = CudaDriver::get();
   if (!d || !d->cuTensorMapEncodeTiled) return fail(hlUnsupported, "grouped product: no driver for tensor maps");
   if (n < 1 || n > 2 || groups < 1) return fail(hlInvalidArgument, "grouped product: %d products of %d groups", n, groups);
   int dev = 0;
   HL_CUDA(cudaGetDevice(&dev));
   HL_CUDA(cudaSetDevice(dev));   // a thread that has made no runtime call yet has no context, which the driver's encoder wants
-  unsigned* const status = gaveUp();
-  if (!status) return fail(hlDeviceError, "grouped product: no page-locked memory");
-  if (*(volatile unsigned*)status) {
-    *(volatile unsigned*)status = 0;
-    return fail(hlDeviceError, "grouped product: a wait in an earlier launch ran out, its results are not valid");
-  }
+  unsigned* const words = statusWords();
+  if (!words) return fail(hlDeviceError, "grouped product: no page-locked memory");
+  if (dev >= kDevices) return fail(hlUnsupported, "grouped product: device %d", dev);
+  if (const hlResult_t e = gemmStatus(dev, false)) return e;
   GemmArgs g;
   g.jobs = n;
   g.groups = groups;
   g.counts = counts;
-  g.status = status;
+  g.status = words + dev;
+  g.limit_ns = limit_ns ? limit_ns : kGemmLimitNs;
+  g.loads = loads;
   int64_t tiles = 0;
   for (int i = 0; i < n; ++i) {
     const GemmSpec& x = specs[i];

@@ -75,18 +75,18 @@ __device__ __forceinline__ bool barTest(uint32_t bar, uint32_t parity) {
   return done != 0;
 }
 // Waits for the phase of this parity. False once *stop is set, by this wait when `limit_ns` have gone by or by another
-// thread of the CTA: then nobody waits any longer.
+// thread of the CTA: then nobody waits any longer. Without `stop` the time alone ends it.
 template <bool kCluster = false>
 __device__ __forceinline__ bool barWait(uint32_t bar, uint32_t parity, volatile int* stop, uint64_t limit_ns) {
   uint64_t t0 = 0;
   for (uint32_t spins = 0;; ++spins) {
     if (barTest<kCluster>(bar, parity)) return true;
     if ((spins & 63u) == 63u) {
-      if (*stop) return false;
+      if (stop && *stop) return false;
       const uint64_t now = nowNs();
       if (t0 == 0) t0 = now;
       if (now - t0 > limit_ns) {
-        *stop = 1;
+        if (stop) *stop = 1;
         return false;
       }
     }

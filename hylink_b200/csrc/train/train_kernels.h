@@ -114,8 +114,12 @@ inline int gemmPartials(int64_t n) { return 2 * (int)((n + 255) / 256); }
 bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden);
 // The same for the first product of a transformer block's MLP, and the gradient of what follows it.
 bool mlpGemmPays(int64_t rows, int64_t width, int64_t hidden);
-// One launch of `n` products, two at most.
-hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s);
+// One launch of `n` products, two at most. `limit_ns` ends every wait inside it (0: two seconds); without `loads` operands never
+// arrive, for tests of that.
+hlResult_t expertGemm(int dt, const GemmSpec* specs, int n, int groups, const int* counts, cudaStream_t s, uint64_t limit_ns = 0, bool loads = true);
+// An error once a wait inside a product on `device` (-1: the current one) has run out, until it is asked with `clear`. Launches ask
+// without. The results of that product and of what came after it are not valid; to be asked where the host has waited for them.
+hlResult_t gemmStatus(int device, bool clear);
 
 }  // namespace train
 }  // namespace hl

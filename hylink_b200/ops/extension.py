@@ -31,6 +31,13 @@ def ops():
     return _module
 
 
+def check_products(device: int | None = None) -> None:
+    """Raises, once, if a wait inside one of this library's matrix products on ``device`` (default: the current one) has run out
+    since the last call: results that came after it are not valid. To be called where the host has waited for results;
+    ``DDPTrainer.step`` does. Launches of further products raise too until then."""
+    ops().check_products(-1 if device is None else device)
+
+
 def overridden(m) -> bool:
     """Whether calling module ``m`` does anything besides its class's ``forward``: hooks, or a ``forward`` of its own."""
     return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__)

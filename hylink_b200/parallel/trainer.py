@@ -25,7 +25,7 @@ import torch.distributed as dist
 from torch.nn.parallel import DistributedDataParallel as DDP
 from torch.optim import optimizer as _optimizer
 
-from ..ops.extension import ops
+from ..ops.extension import check_products, ops
 
 _global_hooks = (_optimizer._global_optimizer_pre_hooks, _optimizer._global_optimizer_post_hooks)
 
@@ -224,6 +224,7 @@ class DDPTrainer:
                 if self._ddp.reducer._rebuild_buckets():
                     self._ddp._has_rebuilt_buckets = True
         self._steps += 1
+        check_products(self.device.index)     # of steps that nobody has waited for
         if self._ddp is not None:
             loss = self._ddp(idx, targets)
         elif self._replayable(idx, targets):
@@ -238,11 +239,13 @@ class DDPTrainer:
         return loss
 
     def step(self, tokens: torch.Tensor) -> float:
-        """``tokens``: pinned host tensor [batch, seq + 1] of token ids. Returns the loss."""
+        """``tokens``: pinned host tensor [batch, seq + 1] of token ids. Returns the loss. An error of a kernel in this step is raised
+        here; the weights have been updated by then."""
         if self._dev_batch is None or self._dev_batch.shape != tokens.shape:
             self._dev_batch = torch.empty(tokens.shape, dtype=tokens.dtype, device=self.device)
         self._dev_batch.copy_(tokens, non_blocking=True)
         loss = self.step_device(self._dev_batch[:, :-1], self._dev_batch[:, 1:])
         self._loss_host.copy_(loss.detach().float().reshape(1), non_blocking=True)
         torch.cuda.current_stream().synchronize()
+        check_products(self.device.index)     # a replayed graph reports nothing by itself
         return float(self._loss_host[0])

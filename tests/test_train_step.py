@@ -578,3 +578,64 @@ def test_gelu_of_a_value_beside_any_others(rows, width, dtype):
         a, s = through(values[order])
         for got, one in ((a, act[order]), (s, slope[order])):
             assert torch.equal(got[one.isfinite()], one[one.isfinite()])
+
+
+def test_a_product_that_gives_up_is_reported(monkeypatch):
+    """A wait inside a product that runs out (its operands never arrive) is an error for whoever waits for the results: in the step that
+    it happens in, replayed from a graph or not, once; and for launches until then."""
+    import math
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.ops import check_products
+    from hylink_b200.ops.extension import ops
+    from hylink_b200.parallel.trainer import DDPTrainer, init_distributed
+
+    monkeypatch.setenv("MASTER_PORT", "29575")
+    init_distributed("hylink")
+    a = torch.randn(264, 136, device="cuda").to(torch.bfloat16)
+    h, w1, w2 = (torch.randn(2, *s, device="cuda").to(torch.bfloat16) for s in ((256, 256), (256, 512), (512, 256)))     # 2^26: the own products
+
+    def gives_up():
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="ran out"):
+            check_products()
+        check_products()                             # reported once
+
+    check_products()
+    ops().product_without_operands(a, 20.0)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="ran out"):
+        ops().moe_experts(h, w1, w2)
+    gives_up()
+    ops().moe_experts(h, w1, w2)                     # and the next one works
+    # recorded: the host enters no launch function when the graph runs
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        ops().product_without_operands(a, 20.0)
+    torch.cuda.synchronize()
+    check_products()
+    graph.replay()
+    gives_up()
+    # a trainer's step, eager and replayed
+    torch.manual_seed(0)
+    trainer = DDPTrainer(GPT2(GPT2Config.tiny()), torch.device("cuda", 0))
+    tokens = torch.randint(0, 1024, (2, 65)).pin_memory()
+    for step in range(5):
+        trainer.step(tokens)
+        real = trainer._opt_step
+
+        def after_a_product(real=real):
+            ops().product_without_operands(a, 20.0)
+            real()
+
+        trainer._opt_step = after_a_product
+        with pytest.raises(RuntimeError, match="ran out"):
+            trainer.step(tokens)
+        trainer._opt_step = real
+        assert math.isfinite(trainer.step(tokens))
+    assert trainer._graph is not None                # the later ones were replayed
+    ops().product_without_operands(a, 20.0)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="ran out"):
+        trainer.step_device(tokens[:, :-1].cuda(), tokens[:, 1:].cuda())
+    trainer.close()
