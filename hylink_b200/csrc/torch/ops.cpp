@@ -235,7 +235,11 @@ bool ownExperts(const Tensor& h, const Tensor& w1, const Tensor& w2) {
   if (h.dim() != 3 || w1.dim() != 3 || !h.is_cuda() || (h.scalar_type() != at::kBFloat16 && h.scalar_type() != at::kHalf)) return false;
   const int64_t experts = h.size(0), width = h.size(2), hidden = w1.size(2);
   return operand(w1, h, {experts, width, hidden}) && operand(w2, h, {experts, hidden, width}) &&
-         train::expertGemmPays(experts * h.size(1), width, hidden);
+         train::expertGemmPays(experts * h.size(1), width, hidden) && train::gemmRuns(code(h));
+}
+// The first product of a block's MLP, or gelu's gradient with the product before it: `weight` and `matrix` are its operands, the result [rows][hidden].
+bool ownMlp(const Tensor& matrix, const Tensor& weight, at::IntArrayRef sizes, int64_t rows, int64_t width, int64_t hidden) {
+  return matrix.is_cuda() && operand(weight, matrix, sizes) && train::mlpGemmPays(rows, width, hidden) && train::gemmRuns(code(matrix));
 }
 
 class BlockPost : public torch::autograd::Function<BlockPost> {
@@ -250,7 +254,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     Normed n = normForward(x, p.view(x.sizes()), gamma, beta, eps);
     const Tensor h = n.out.view({-1, width});
     Tensor u, act;
-    if (wf.dim() == 2 && operand(wf, h, {wf.size(0), width}) && operand(bf, h, {wf.size(0)}) && train::mlpGemmPays(h.size(0), width, wf.size(0))) {
+    if (wf.dim() == 2 && operand(bf, h, {wf.size(0)}) && ownMlp(h, wf, {wf.size(0), width}, h.size(0), width, wf.size(0))) {
       u = at::empty({h.size(0), wf.size(0)}, h.options());
       act = at::empty_like(u);
       const Tensor w = dense(wf), bias = bf.contiguous();
@@ -285,7 +289,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     cudaStream_t st = streamOf(x2);
     TORCH_CHECK(g[1].defined(), "hylink: the block's branch has no gradient");
     const Tensor gy = rowsOf(g[1]);
-    const bool own = operand(wo, gy, {width, hidden}) && operand(u, gy, {rows, hidden}) && train::mlpGemmPays(rows, width, hidden);
+    const bool own = operand(u, gy, {rows, hidden}) && ownMlp(gy, wo, {width, hidden}, rows, width, hidden);
     const int fcp = own ? train::gemmPartials(rows) : sp;
     Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {fcp, hidden}), parts;
     Tensor dwo, dwf, dwp, da, dx, dgamma, dbeta, dbp, dbf;

@@ -419,6 +419,14 @@ CUresult encode(const CudaDriver* d, CUtensorMap* m, int dt, const void* p, int6
 
 }  // namespace
 
+bool gemmRuns(int dt) {
+  static const bool wanted = envBool({"HYLINK_OWN_PRODUCTS"}, true);
+  const CudaDriver* d = wanted ? CudaDriver::get() : nullptr;
+  int dev = 0;
+  if (!d || !d->cuTensorMapEncodeTiled || cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices || !statusWords()) return false;
+  return dt == hlBfloat16 ? residentPairs<__nv_bfloat16>() > 0 : dt == hlFloat16 && residentPairs<__half>() > 0;
+}
+
 // Small ones are bound by the host, which issues four launches here and eight to the library: whole layers, us own / library,
 // 64 tokens of 256 x 1024 201 / 241, 500 of 1024 x 4096 194 / 237, 2500 235 / 272. (The kernels alone, of which the library's are the faster
 // there: 2^24 37 / 30, 2^28 53 / 36; from some 2500 tokens of 1024 x 4096 on the own ones are.) Below 2^24 nothing is left to win: 31 / 30.

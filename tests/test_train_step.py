@@ -639,3 +639,59 @@ def test_a_product_that_gives_up_is_reported(monkeypatch):
     with pytest.raises(RuntimeError, match="ran out"):
         trainer.step_device(tokens[:, :-1].cuda(), tokens[:, 1:].cuda())
     trainer.close()
+
+
+_PRODUCTS = """
+import sys, torch
+from hylink_b200.ops.extension import ops
+out, dtype = {}, torch.bfloat16
+g = torch.Generator("cuda").manual_seed(5)
+make = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=g) * scale).to(dtype)
+for rows, width, hidden in ((8192, 1024, 4096), (4096, 768, 3072)):       # MLPs of the two larger models
+    x, a, dx2, dy2 = (make(1, rows, width) for _ in range(4))
+    wp, bp, gamma, beta = make(width, width, scale=width ** -0.5), make(width, scale=0.1), 1 + make(width, scale=0.1), make(width, scale=0.1)
+    wf, bf = make(hidden, width, scale=width ** -0.5), make(hidden, scale=0.1)
+    wo, bo = make(width, hidden, scale=hidden ** -0.5), make(width, scale=0.1)
+    leaves = [t.requires_grad_() for t in (x, a, wp, bp, gamma, beta, wf, bf, wo, bo)]
+    def go():
+        x2, y2 = ops().block_post(*leaves, 1e-5)
+        return (x2.detach(), y2.detach(), *torch.autograd.grad((x2, y2), leaves, (dx2, dy2)))
+    for name, t in zip("x2 y2 dx da dwp dbp dgamma dbeta dwf dbf dwo dbo".split(), go()):
+        out[f"mlp {rows} {name}"] = t.cpu()
+for tokens, width, experts in ((8192, 1024, 8), (500, 512, 2)):
+    capacity = tokens * 5 // 4 // experts
+    leaves = [t.requires_grad_() for t in (make(tokens, width), make(experts, width, scale=width ** -0.5), make(experts, width, 4 * width, scale=width ** -0.5),
+                                           make(experts, 4 * width, width, scale=0.5 * width ** -0.5))]
+    dy = make(tokens, width)
+    def go():
+        y = ops().moe_layer(*leaves, capacity)
+        return (y.detach(), *torch.autograd.grad(y, leaves, dy))
+    for name, t in zip("y dx drouter dw1 dw2".split(), go()):
+        out[f"moe {tokens} {name}"] = t.cpu()
+with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+    go()
+    torch.cuda.synchronize()
+out["own"] = any("kExpertGemm" in e.name for e in p.events())
+torch.save(out, sys.argv[1])
+"""
+
+
+def test_the_products_bits_are_the_librarys(tmp_path):
+    """Without the own products, switched off or not available, the same calls give the same results: the training step's forward
+    pass rests on that."""
+    import os
+    import subprocess
+    import sys
+
+    got = []
+    for own in ("1", "0"):
+        path = tmp_path / own
+        subprocess.run([sys.executable, "-c", _PRODUCTS, str(path)], check=True, timeout=300, env={**os.environ, "HYLINK_OWN_PRODUCTS": own})
+        got.append(torch.load(path))
+    assert got[0].pop("own") and not got[1].pop("own")
+    for name, a in got[0].items():
+        b = got[1][name]
+        if name.endswith("dbf"):                     # fp32 partials, added up in another order: a step of the result at most
+            assert bool(((a - b).abs().double() <= 2.0 ** -7 * b.abs().double() + 2.0 ** -16).all()), name
+        else:
+            assert torch.equal(a, b), name
