@@ -8,6 +8,7 @@
 //   blockPost:  x2 = x1 + a Wproj^T + b; h = layer norm(x2); y2 = gelu(h Wfc^T + b) Wout^T + b;  returns x2, y2
 // The add of y2 is left to the next block's (or the final) layer norm, which reads x2 anyway.
 #include <ATen/ATen.h>
+#include <ATen/SavedTensorHooks.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/autograd.h>
@@ -443,12 +444,13 @@ std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& route
 }
 struct Expert {
   Tensor u, act, out;
+  bool own = false;   // by the own products: the backward pass follows, whatever it would choose itself
 };
 // h: [experts][rows][width]. `count`: rows of each expert in use (the others are zeros), undefined where that is not known; results
 // of rows out of use may be anything then.
 Expert moeExpert(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const Tensor& count) {
   Expert e;
-  if (ownExperts(h_, w1_, w2_)) {
+  if ((e.own = ownExperts(h_, w1_, w2_))) {
     const Tensor h = dense(h_), w1 = dense(w1_), w2 = dense(w2_);
     e.u = at::empty({h.size(0), h.size(1), w1.size(2)}, h.options());
     e.act = at::empty_like(e.u);
@@ -467,9 +469,15 @@ Expert moeExpert(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const T
 }
 // {dh, dw1, dw2}, those that are needed
 variable_list moeExpertBackward(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const Tensor& u_, const Tensor& act_, const Tensor& dout_,
-                                const Tensor& count, bool h_needed, bool w1_needed, bool w2_needed) {
+                                bool own, const Tensor& count, bool h_needed, bool w1_needed, bool w2_needed) {
   Tensor dh, dw1, dw2;
-  if (ownExperts(h_, w1_, w2_)) {
+  if (own) {
+    // nothing else looks at these between the hooks that gave them back and the kernel
+    const bool fit = h_.dim() == 3 && w1_.dim() == 3 && operand(h_, dout_, dout_.sizes()) && operand(w1_, h_, {h_.size(0), h_.size(2), w1_.size(2)}) &&
+                     operand(w2_, h_, {h_.size(0), w1_.size(2), h_.size(2)}) && operand(u_, h_, {h_.size(0), h_.size(1), w1_.size(2)}) &&
+                     operand(act_, h_, u_.sizes()) &&
+                     (!count.defined() || (count.scalar_type() == at::kInt && count.device() == h_.device() && count.numel() == h_.size(0) && count.is_contiguous()));
+    TORCH_CHECK(fit, "hylink: the experts' saved tensors have come back with other sizes, types or places");
     const Tensor h = dense(h_), w1 = dense(w1_), w2 = dense(w2_), u = dense(u_), act = dense(act_), dout = dense(dout_);
     const int64_t rows = h.size(1), width = h.size(2), hidden = w1.size(2);
     train::GemmSpec specs[2];
@@ -548,8 +556,11 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const Tensor x = dense(x_);
     const Routed r = moeRouted(x, router, capacity);
     const Tensor h = r.send.view({router.size(0), capacity, x.size(1)});
-    const Expert e = moeExpert(h, w1, w2, r.count);
-    ctx->save_for_backward({x_, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out, r.count});
+    // Hooks on saved tensors see all of them, and may scale what they keep by its largest value: rows out of use are computed then (zeros).
+    const Tensor count = at::SavedTensorDefaultHooks::get_hooks() ? Tensor() : r.count;
+    const Expert e = moeExpert(h, w1, w2, count);
+    ctx->save_for_backward({x_, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out, count});
+    ctx->saved_data["own"] = e.own;
     return moeCombined(x, r.gate, e.out, r.row_of);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -566,7 +577,8 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const Tensor x = dense(s[0]), rows = dense(s[12]);
     const Tensor dy = dense(g[0]);
     const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8], false);
-    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, s[13], needed(ctx, 0), needed(ctx, 2), needed(ctx, 3));
+    const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, ctx->saved_data["own"].toBool(), s[13], needed(ctx, 0), needed(ctx, 2),
+                                              needed(ctx, 3));
     if (!needed(ctx, 0, 1)) return {Tensor(), Tensor(), e[1], e[2], Tensor()};
     const Tensor dsend = e[0].defined() ? e[0] : at::zeros_like(h);   // the router alone
     const auto [dx, drouter] = moeRoutedBackward(x, router, s[4], s[5], s[6], s[7], dy, dsend, dgate, needed(ctx, 1));
@@ -615,6 +627,7 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
     c10::cuda::CUDAGuard dg(h.device());
     const Expert e = moeExpert(h, w1, w2, Tensor());
     ctx->save_for_backward({h, w1, w2, e.u, e.act});
+    ctx->saved_data["own"] = e.own;
     return e.out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -624,7 +637,8 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
       const variable_list in = {viewOf(s[0]), viewOf(s[1]), viewOf(s[2])};
       return recorded({plainExperts(in[0], in[1], in[2])}, g, in);
     }
-    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), Tensor(), needed(ctx, 0), needed(ctx, 1), needed(ctx, 2));
+    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), ctx->saved_data["own"].toBool(), Tensor(), needed(ctx, 0), needed(ctx, 1),
+                             needed(ctx, 2));
   }
 };
 

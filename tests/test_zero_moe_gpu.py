@@ -419,3 +419,47 @@ def test_the_routers_gradient_at_the_edges_of_its_blocks(tokens, width, experts)
         assert float((drouter.double() - want).norm() / want.norm()) < 2 * 2.0 ** -8
     else:
         assert not drouter.any()
+
+
+def test_hooks_on_the_experts_saved_tensors():
+    """Hooks see rows out of use too, and may keep a tensor in any form: what they see is finite, what one that scales by the largest value gives
+    back is good for the gradients, and a tensor that comes back in another type is an error."""
+    from hylink_b200.ops.extension import ops
+
+    torch.manual_seed(3)
+    tokens, width, hidden, experts, capacity = 300, 256, 1024, 4, 500           # most rows are out of use; 2^29
+    leaves = [(torch.randn(*s, device="cuda") * scale).to(torch.bfloat16).requires_grad_()
+              for s, scale in (((tokens, width), 1.0), ((experts, width), width ** -0.5), ((experts, width, hidden), width ** -0.5),
+                               ((experts, hidden, width), hidden ** -0.5))]
+    dy = torch.randn(tokens, width, device="cuda").to(torch.bfloat16)
+
+    def spoil():                                                                # memory that the next tensors will get
+        trash = [torch.full((experts, capacity, n), float("nan"), device="cuda", dtype=torch.bfloat16) for n in (hidden, width) for _ in range(4)]
+        del trash
+
+    def through(pack, unpack):
+        spoil()
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            y = ops().moe_layer(*leaves, capacity)
+        spoil()
+        return torch.autograd.grad(y, leaves, dy)
+
+    want = torch.autograd.grad(ops().moe_layer(*leaves, capacity), leaves, dy)
+    seen = []
+
+    def scaled(t):
+        if not t.is_floating_point():
+            return t
+        seen.append(bool(t.isfinite().all()))
+        top = t.abs().max().float().clamp_min(1e-30)
+        return (t.float() / top * 32767).round().to(torch.int16), top, t.dtype
+
+    got = through(scaled, lambda k: k if isinstance(k, torch.Tensor) else (k[0].float() * (k[1] / 32767)).to(k[2]))
+    assert len(seen) >= 9 and all(seen)
+    for name, a, b in zip(("dx", "drouter", "dw1", "dw2"), got, want):
+        assert bool(a.isfinite().all()), name
+        # kept to 2^-16 of the largest value, which is some eight times the mean: under two steps of bf16 on the way
+        assert float((a.double() - b.double()).norm()) < 2 * 2.0 ** -8 * float(b.double().norm()), name
+    big = experts * capacity * hidden
+    with pytest.raises(RuntimeError, match="hylink"):
+        through(lambda t: t, lambda t: t.float() if t.numel() == big and t.dim() == 3 else t)
