@@ -232,11 +232,15 @@ void products(const train::GemmSpec* specs, int n, const Tensor& like, const Ten
 bool operand(const Tensor& t, const Tensor& like, at::IntArrayRef sizes) {
   return t.sizes() == sizes && t.scalar_type() == like.scalar_type() && t.device() == like.device() && t.layout() == at::kStrided;
 }
+bool captured(const Tensor& t) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(streamOf(t), &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+}
 bool ownExperts(const Tensor& h, const Tensor& w1, const Tensor& w2) {
   if (h.dim() != 3 || w1.dim() != 3 || !h.is_cuda() || (h.scalar_type() != at::kBFloat16 && h.scalar_type() != at::kHalf)) return false;
   const int64_t experts = h.size(0), width = h.size(2), hidden = w1.size(2);
   return operand(w1, h, {experts, width, hidden}) && operand(w2, h, {experts, hidden, width}) &&
-         train::expertGemmPays(experts * h.size(1), width, hidden) && train::gemmRuns(code(h));
+         train::expertGemmPays(experts * h.size(1), width, hidden, captured(h)) && train::gemmRuns(code(h));
 }
 // The first product of a block's MLP, or gelu's gradient with the product before it: `weight` and `matrix` are its operands, the result [rows][hidden].
 bool ownMlp(const Tensor& matrix, const Tensor& weight, at::IntArrayRef sizes, int64_t rows, int64_t width, int64_t hidden) {

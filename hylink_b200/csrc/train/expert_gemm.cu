@@ -427,11 +427,14 @@ bool gemmRuns(int dt) {
   return dt == hlBfloat16 ? residentPairs<__nv_bfloat16>() > 0 : dt == hlFloat16 && residentPairs<__half>() > 0;
 }
 
-// Small ones are bound by the host, which issues four launches here and eight to the library: whole layers, us own / library,
-// 64 tokens of 256 x 1024 201 / 241, 500 of 1024 x 4096 194 / 237, 2500 235 / 272. (The kernels alone, of which the library's are the faster
-// there: 2^24 37 / 30, 2^28 53 / 36; from some 2500 tokens of 1024 x 4096 on the own ones are.) Below 2^24 nothing is left to win: 31 / 30.
-bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden) {
-  return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (1 << 24);
+// From 2^33 multiplications on the tiles fill the GPU, and the kernels are the faster ones. Smaller layers take the host longer than the GPU,
+// and the host has four launches to issue here and eight with the library. Recorded into a graph they take the GPU alone. Whole layers, forward
+// and backward, us own / library, issued and (recorded): 64 tokens of 256 x 1024, eight experts 206 / 294 (57 / 51); 200 of 1024 x 4096, eight
+// 208 / 262 (170 / 142); 1072 of 768 x 3072, eight 243 / 298 (149 / 136); 2500 of 512 x 2048, eight 207 / 263 (133 / 115); from 2^33 on 2500 of
+// 1024 x 4096, four 225 / 266 (205 / 232), 5000 353 / 390 (317 / 338). Below 2^24 nothing is left to win: 31 / 30 for the products.
+// (A small layer that is issued behind work that keeps the GPU busy loses those 6 to 20 % too; the host does not know of that.)
+bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden, bool captured) {
+  return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (captured ? 1LL << 33 : 1LL << 24);
 }
 // One product with a bias, which the library's kernels take too: what is gained is the element-wise pass alone, and that once the tiles fill
 // the GPU. Training steps, ms own / library: 4096 rows of 768 x 3072 8.49 / 8.56, 3072 of 1024 x 4096 14.51 / 14.62, 8192

@@ -113,8 +113,8 @@ inline int gemmPartials(int64_t n) { return 2 * (int)((n + 255) / 256); }
 // Whether it runs on the current device: a GPU and a driver that it is made for, page-locked memory for its status, and not switched
 // off (HYLINK_OWN_PRODUCTS=0). Where it does not, the library's products are taken.
 bool gemmRuns(int dt);
-// Whether experts of this width and hidden width, with this many rows in all, go through it.
-bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden);
+// Whether experts of this width and hidden width, with this many rows in all, go through it; `captured`: into a CUDA graph.
+bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden, bool captured);
 // The same for the first product of a transformer block's MLP, and the gradient of what follows it.
 bool mlpGemmPays(int64_t rows, int64_t width, int64_t hidden);
 // One launch of `n` products, two at most. `limit_ns` ends every wait inside it (0: two seconds); without `loads` operands never

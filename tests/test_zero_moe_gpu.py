@@ -463,3 +463,34 @@ def test_hooks_on_the_experts_saved_tensors():
     big = experts * capacity * hidden
     with pytest.raises(RuntimeError, match="hylink"):
         through(lambda t: t, lambda t: t.float() if t.numel() == big and t.dim() == 3 else t)
+
+
+# below and from the 2^33 multiplications on from which the own products are the faster ones on the GPU
+@pytest.mark.parametrize("rows,own", [(2000, False), (2048, True)])
+def test_recorded_experts_take_the_faster_products(rows, own):
+    """Recorded into a graph, a layer costs the GPU's time alone. An eager layer of the same size is issued faster by the own products,
+    whatever its size, and its backward pass goes the way of its forward pass, recorded or not."""
+    from hylink_b200.ops.extension import ops
+
+    torch.manual_seed(rows)
+    h, w1, w2, dy = ((torch.randn(1, *s, device="cuda") * 0.03).to(torch.bfloat16).requires_grad_(i < 3)
+                     for i, s in enumerate(((rows, 1024), (1024, 4096), (4096, 1024), (rows, 1024))))
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):                    # a backward pass runs where its forward pass did
+        eager = ops().moe_experts(h, w1, w2)
+        want = torch.autograd.grad(eager, (h, w1, w2), dy, retain_graph=True)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        y = ops().moe_experts(h, w1, w2)
+        got = torch.autograd.grad(y, (h, w1, w2), dy)
+        mixed = torch.autograd.grad(eager, (h, w1, w2), dy)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        graph.replay()
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events()]
+    # a layer: two launches forward and two backward; `mixed` is the backward pass of an eager one
+    assert sum("kExpertGemm" in n for n in names) == (6 if own else 2), names
+    assert torch.equal(y, eager)
+    for a, b, c in zip(got, mixed, want):
+        assert torch.equal(a, c) and torch.equal(b, c)
