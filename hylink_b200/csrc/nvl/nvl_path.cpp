@@ -779,10 +779,12 @@ hlResult_t NvlPath::allReduce(const NvlBufs& b, const NvlCall& c, cudaStream_t s
 }
 
 // Gathered bytes from which the peer-pointer all-gather uses the lane kernel (2 GPUs, bf16: 550 against 462 GB/s at
-// 256 MiB, 622 against 486 GB/s at 1 GiB, 375 against 390 GB/s at 64 MiB).
+// 256 MiB, 622 against 486 GB/s at 1 GiB, 375 against 390 GB/s at 64 MiB). Ranks of one GPU use it where the variable asks for it: the streamed
+// and the plain push kernel are faster there at any size. Lanes / push, us: 128 MiB of bf16 in segments that start inside a packet,
+// 2 ranks 353 / 239, 4 901 / 490, 8 2019 / 1119, aligned 4 ranks 378 / 155; 256 MiB through 1 MiB of staging, 4 ranks 7867 / 2991.
 size_t NvlPath::agLanesMinBytes() const {
-  static const size_t v = (size_t)envInt({"HYLINK_AG_LANES_MIN_BYTES"}, 128LL << 20);  // read once: this sits on the launch path
-  return v;
+  static const long long v = envInt({"HYLINK_AG_LANES_MIN_BYTES"}, -1);  // read once: this sits on the launch path
+  return v >= 0 ? (size_t)v : (emu_ ? SIZE_MAX : (size_t)128 << 20);
 }
 size_t NvlPath::lanesMinBytes() const {
   static const size_t v = (size_t)envInt({"HYLINK_RS_LANES_MIN_BYTES"}, 128LL << 20);
@@ -845,7 +847,7 @@ hlResult_t NvlPath::allGather(const NvlBufs& b, const NvlCall& c, cudaStream_t s
   static const bool ag_push = envBool({"HYLINK_AG_PUSH"}, true);
   const bool push = same && c.algo != hlAlgoTwoShotP2p && ag_push;
   const size_t seg_bytes = c.count * hlTypeSize((hlDataType_t)c.wire_dt);
-  const bool lanes = push && (c.algo == hlAlgoPipelined || (c.algo == hlAlgoAuto && !emu_ && seg_bytes * (size_t)nranks_ >= agLanesMinBytes()));
+  const bool lanes = push && (c.algo == hlAlgoPipelined || (c.algo == hlAlgoAuto && seg_bytes * (size_t)nranks_ >= agLanesMinBytes()));
   return launchSliced(lanes ? kNvlAllGatherLanes : (push ? kNvlAllGatherPush : kNvlAllGather), b, c, true, s);
 }
 

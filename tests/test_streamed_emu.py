@@ -137,3 +137,30 @@ def test_streamed_broadcast(n, count, dtype, offset, monkeypatch):
         assert all(torch.equal(b, data) and bool((o[offset + count:] == 7).all()) for o, b in zip(outs, bufs))
     assert ("broadcast_streamed" in {launch["kind"] for launch in g.kernel_timeline()}) == (offset == 0)
     g.close()
+
+
+@pytest.mark.parametrize("least,kind", [(None, "allgather_streamed"), (str(192 << 20), "allgather_streamed"), (str(160 << 20), "allgather_lanes")])
+def test_the_lane_kernel_can_be_asked_for(least, kind):
+    """HYLINK_AG_LANES_MIN_BYTES counts between ranks of one GPU too, where it is set; without it they stream, at any size."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from hylink_b200.ops import EmuGroup
+g = EmuGroup(2)
+seg = 40 << 20
+ins = [torch.arange(seg, device="cuda").add(r).to(torch.bfloat16) for r in range(2)]
+outs = [torch.zeros(2 * seg, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+g.run("all_gather", ins, outs, seg, out_seg_stride=seg)
+torch.cuda.synchronize()
+assert all(torch.equal(o, torch.cat(ins)) for o in outs)
+print("kinds", *{launch["kind"] for launch in g.kernel_timeline()})
+"""
+    env = {**os.environ, "HYLINK_KERNEL_TIMELINE": "1"}
+    env.pop("HYLINK_AG_LANES_MIN_BYTES", None)
+    if least:
+        env["HYLINK_AG_LANES_MIN_BYTES"] = least
+    out = subprocess.run([sys.executable, "-c", code], check=True, timeout=120, env=env, capture_output=True, text=True).stdout
+    assert f"kinds {kind}" in out
