@@ -715,7 +715,8 @@ __global__ void __launch_bounds__(HL_NVL_THREADS, 1) kPipeCta(const HlCommDev* c
 }
 
 // ------------------------------------------------------------------ push kernels over peer pointers
-// Every access to a peer is a posted store and every load is local:
+// Every access to a peer is a posted store and every load is local (between ranks of one GPU, where nothing is far, an all-reduce reads its
+// results from the peers' areas):
 //   all-reduce      stream shard s of the input straight from the caller's buffer into slot `rank` of its owner | barrier |
 //                   fold the own shard (read from the caller's buffer) and the landed slots in ascending rank order,
 //                   store the result to the caller's output and into every peer's result area | barrier | copy the

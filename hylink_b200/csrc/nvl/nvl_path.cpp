@@ -59,12 +59,13 @@ hlResult_t NvlPath::finishInit(int timeout_ms) {
   }
   HlCommDev h[HL_MAX_RANKS];
   memset(h, 0, sizeof(h));
+  const bool near = envBool({"HYLINK_EMU_NEAR"}, true);   // off: emulated ranks run the kernels as ranks of different GPUs do
   for (int i = 0; i < nl; ++i) {
     HlCommDev& c = h[i];
     c.rank = emu_ ? i : rank_;
     c.nranks = nranks_;
     c.max_blocks = HL_MAX_BLOCKS;
-    c.one_device = emu_ ? 1 : 0;
+    c.one_device = emu_ && near ? 1 : 0;
     for (int q = 0; q < nranks_; ++q) {
       uint8_t* base = (uint8_t*)(emu_ ? emu_mem_[q] : region_.ptr[q]);
       c.stage[q] = base;

@@ -33,7 +33,7 @@ struct HlCommDev {
   int rank;
   int nranks;
   int max_blocks;
-  int one_device;                  // all ranks share this GPU: flags are exchanged at GPU scope
+  int one_device;                  // all ranks share this GPU: flags are exchanged at GPU scope, a result may stay where it was made
   uint8_t* stage[HL_MAX_RANKS];    // symmetric staging region
   uint64_t* flags[HL_MAX_RANKS];   // [HL_FLAG_KINDS][HL_MAX_BLOCKS][HL_MAX_RANKS] monotonically increasing words
   uint8_t* mc_stage;               // NVSwitch multicast alias of stage (null without NVLS)

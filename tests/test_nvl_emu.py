@@ -393,3 +393,34 @@ def test_all_gather_kernels_agree(n, algo):
             assert torch.all(bufs[r][q * seg + prefix:(q + 1) * seg] == 3)
     assert g.status(0)[0] == 0
     g.close()
+
+
+@pytest.mark.parametrize("near", ["1", "0"])
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_staged_collectives_in_both_forms(n, dtype, near, monkeypatch):
+    """As ranks of one GPU run them, and as ranks of different GPUs do: counts that end inside a packet and inside a shard, buffers that
+    start inside a packet, in place, in several launches, back to back."""
+    monkeypatch.setenv("HYLINK_EMU_NEAR", near)
+    g = _group(n, stage_bytes=4 << 20)
+    for rep, (count, offset) in enumerate([(1, 0), (4099, 1), (65536, 0), (300001, 0), (300001, 3), ((1 << 20) + 7, 0), (1 << 20, 5)]):
+        ins = [_rand(count + offset, dtype, 13 * r + rep)[offset:] for r in range(n)]
+        ref = _ordered_sum(ins, torch.float32)
+        outs = [torch.full((count + offset + 8,), 3, dtype=dtype, device="cuda") for _ in range(n)]
+        for again in range(3):                       # a fast rank's next call beside a slow one's last reads
+            g.run("all_reduce", ins, [o[offset:offset + count] for o in outs], count, algo="push")
+        for o in outs:
+            assert torch.equal(o[offset:offset + count], ref.to(dtype)), (count, offset)
+            assert bool((o[:offset] == 3).all()) and bool((o[offset + count:] == 3).all())
+        bufs = [t.clone() for t in ins]
+        g.run("all_reduce", bufs, bufs, count, algo="push")
+        assert all(torch.equal(b, ref.to(dtype)) for b in bufs)
+        seg = count // n
+        if seg:
+            g.run("reduce_scatter", ins, [o[offset:] for o in outs], seg, in_seg_stride=seg, algo="push")
+            assert all(torch.equal(o[offset:offset + seg], ref[r * seg:(r + 1) * seg].to(dtype)) for r, o in enumerate(outs))
+            g.run("all_gather", ins, [o[offset:] for o in outs], seg, out_seg_stride=seg, algo="push")
+            assert all(torch.equal(o[offset + q * seg:offset + (q + 1) * seg], ins[q][:seg]) for o in outs for q in range(n))
+            g.run("all_to_all", ins, [o[offset:] for o in outs], seg, in_seg_stride=seg, out_seg_stride=seg)
+            assert all(torch.equal(o[offset + q * seg:offset + (q + 1) * seg], ins[q][r * seg:(r + 1) * seg]) for r, o in enumerate(outs) for q in range(n))
+    g.close()
