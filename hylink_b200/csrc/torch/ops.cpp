@@ -426,7 +426,7 @@ std::pair<Tensor, Tensor> moeRoutedBackward(const Tensor& x, const Tensor& route
   const Tensor router = dense(router_);
   const int64_t tokens = x.size(0), width = x.size(1), experts = router.size(0);
   Tensor dx = at::empty_like(x);
-  if (router_needed && train::moeTokensAndRouterFits((int)experts)) {
+  if (router_needed && tokens > 0 && train::moeTokensAndRouterFits((int)experts)) {   // (no tokens: a gradient of zeros, by the product below)
     const int parts = train::moeRouterPartials((int)tokens);
     Tensor partials = floats(x, {parts, experts * width});
     ok(train::moeTokensAndRouter(code(x), dres.defined() ? dres.data_ptr() : nullptr, dsend.data_ptr(), row_of.data_ptr<int>(), logits.data_ptr(),

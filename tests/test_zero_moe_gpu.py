@@ -494,3 +494,19 @@ def test_recorded_experts_take_the_faster_products(rows, own):
     assert torch.equal(y, eager)
     for a, b, c in zip(got, mixed, want):
         assert torch.equal(a, c) and torch.equal(b, c)
+
+
+@pytest.mark.parametrize("experts", [1, 4, 12])
+def test_operators_without_tokens(experts):
+    """A rank may have no tokens: outputs are empty, the weights' gradients zero."""
+    from hylink_b200.ops.extension import ops
+
+    make = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16).requires_grad_()      # noqa: E731
+    x, router, w1, w2 = make(0, 64), make(experts, 64), make(experts, 64, 128), make(experts, 128, 64)
+    y = ops().moe_layer(x, router, w1, w2, 8)
+    grads = torch.autograd.grad(y, (x, router, w1, w2), torch.zeros_like(y))
+    x1, send, gate, row_of, token_of = ops().moe_dispatch(x, router, 8)
+    grads += torch.autograd.grad((x1, send, gate), (x, router), (torch.zeros_like(x1), torch.randn_like(send), torch.zeros_like(gate)))
+    assert y.shape == x1.shape == (0, 64) and not send.any() and bool((token_of == -1).all())
+    for g, t in zip(grads, (x, router, w1, w2, x, router)):
+        assert g.shape == t.shape and not g.any()
