@@ -236,22 +236,27 @@ bool captured(const Tensor& t) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(streamOf(t), &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
-bool ownExperts(const Tensor& h, const Tensor& w1, const Tensor& w2) {
-  if (h.dim() != 3 || w1.dim() != 3 || !h.is_cuda() || (h.scalar_type() != at::kBFloat16 && h.scalar_type() != at::kHalf)) return false;
+// `alone`: nothing else holds multiprocessors for long while the call runs. A product's tiles are dealt out beforehand to as many CTAs as
+// an empty GPU holds, one per multiprocessor; those that find theirs taken start when the others are done. Beside a kernel on 16 (32) of
+// them, us own / library: a block's second half forward 241 / 204 (294 / 280), backward 388 / 343 (521 / 499), experts of 8 x 1024 x 1024 x 4096
+// forward 198 / 146 (216 / 206), backward 347 / 280 (372 / 382); alone 179 / 194, 304 / 323, 134 / 140, 220 / 267. Gradient
+// all-reduces of a job of several ranks are such kernels.
+bool ownExperts(const Tensor& h, const Tensor& w1, const Tensor& w2, bool alone) {
+  if (!alone || h.dim() != 3 || w1.dim() != 3 || !h.is_cuda() || (h.scalar_type() != at::kBFloat16 && h.scalar_type() != at::kHalf)) return false;
   const int64_t experts = h.size(0), width = h.size(2), hidden = w1.size(2);
   return operand(w1, h, {experts, width, hidden}) && operand(w2, h, {experts, hidden, width}) &&
          train::expertGemmPays(experts * h.size(1), width, hidden, captured(h)) && train::gemmRuns(code(h));
 }
 // The first product of a block's MLP, or gelu's gradient with the product before it: `weight` and `matrix` are its operands, the result [rows][hidden].
-bool ownMlp(const Tensor& matrix, const Tensor& weight, at::IntArrayRef sizes, int64_t rows, int64_t width, int64_t hidden) {
-  return matrix.is_cuda() && operand(weight, matrix, sizes) && train::mlpGemmPays(rows, width, hidden) && train::gemmRuns(code(matrix));
+bool ownMlp(const Tensor& matrix, const Tensor& weight, at::IntArrayRef sizes, int64_t rows, int64_t width, int64_t hidden, bool alone) {
+  return alone && matrix.is_cuda() && operand(weight, matrix, sizes) && train::mlpGemmPays(rows, width, hidden) && train::gemmRuns(code(matrix));
 }
 
 class BlockPost : public torch::autograd::Function<BlockPost> {
  public:
   static variable_list forward(AutogradContext* ctx, const Variable& x_, const Variable& a_, const Variable& wp, const Variable& bp,
                                const Variable& gamma, const Variable& beta, const Variable& wf, const Variable& bf, const Variable& wo,
-                               const Variable& bo, double eps) {
+                               const Variable& bo, double eps, bool alone) {
     c10::cuda::CUDAGuard dg(x_.device());
     const Tensor x = dense(x_), a = rowsOf(a_);
     const int64_t width = x.size(-1);
@@ -259,7 +264,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     Normed n = normForward(x, p.view(x.sizes()), gamma, beta, eps);
     const Tensor h = n.out.view({-1, width});
     Tensor u, act;
-    if (wf.dim() == 2 && operand(bf, h, {wf.size(0)}) && ownMlp(h, wf, {wf.size(0), width}, h.size(0), width, wf.size(0))) {
+    if (wf.dim() == 2 && operand(bf, h, {wf.size(0)}) && ownMlp(h, wf, {wf.size(0), width}, h.size(0), width, wf.size(0), alone)) {
       u = at::empty({h.size(0), wf.size(0)}, h.options());
       act = at::empty_like(u);
       const Tensor w = dense(wf), bias = bf.contiguous();
@@ -274,6 +279,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     const Tensor y = at::addmm(bo, act, wo.t()).view(x.sizes());
     ctx->save_for_backward({a_, wp, n.sum, n.mean, n.rstd, gamma, h, wf, u, act, wo, beta, bf, bo});
     ctx->saved_data["eps"] = eps;
+    ctx->saved_data["alone"] = alone;
     return {n.sum, y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -286,7 +292,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
       const Tensor n = at::layer_norm(in[0], {width}, in[1], in[2], ctx->saved_data["eps"].toDouble());
       const variable_list r = recorded({at::linear(at::gelu(at::linear(n, in[3], in[4]), "tanh"), in[5], in[6])}, {g[1]}, in);
       const Tensor dx = plus(g[0], r[0]), d = dx.reshape({rows, width}), a = s[0].reshape({rows, -1});
-      return {dx, at::mm(d, wp).view(s[0].sizes()), at::mm(d.t(), a), d.sum(0), r[1], r[2], r[3], r[4], r[5], r[6], Tensor()};
+      return {dx, at::mm(d, wp).view(s[0].sizes()), at::mm(d.t(), a), d.sum(0), r[1], r[2], r[3], r[4], r[5], r[6], Tensor(), Tensor()};
     }
     const Tensor a = rowsOf(s[0]), u = dense(s[8]);
     const int64_t hidden = u.size(1);
@@ -294,7 +300,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
     cudaStream_t st = streamOf(x2);
     TORCH_CHECK(g[1].defined(), "hylink: the block's branch has no gradient");
     const Tensor gy = rowsOf(g[1]);
-    const bool own = operand(u, gy, {rows, hidden}) && ownMlp(gy, wo, {width, hidden}, rows, width, hidden);
+    const bool own = operand(u, gy, {rows, hidden}) && ownMlp(gy, wo, {width, hidden}, rows, width, hidden, ctx->saved_data["alone"].toBool());
     const int fcp = own ? train::gemmPartials(rows) : sp;
     Tensor out_parts = floats(x2, {sp, width}), fc_parts = floats(x2, {fcp, hidden}), parts;
     Tensor dwo, dwf, dwp, da, dx, dgamma, dbeta, dbp, dbf;
@@ -328,7 +334,7 @@ class BlockPost : public torch::autograd::Function<BlockPost> {
       }
     }
     cols.finish();
-    return {dx, da, dwp, dbp, dgamma, dbeta, dwf, dbf, dwo, dbo, Tensor()};
+    return {dx, da, dwp, dbp, dgamma, dbeta, dwf, dbf, dwo, dbo, Tensor(), Tensor()};
   }
 };
 
@@ -452,9 +458,9 @@ struct Expert {
 };
 // h: [experts][rows][width]. `count`: rows of each expert in use (the others are zeros), undefined where that is not known; results
 // of rows out of use may be anything then.
-Expert moeExpert(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const Tensor& count) {
+Expert moeExpert(const Tensor& h_, const Tensor& w1_, const Tensor& w2_, const Tensor& count, bool alone) {
   Expert e;
-  if ((e.own = ownExperts(h_, w1_, w2_))) {
+  if ((e.own = ownExperts(h_, w1_, w2_, alone))) {
     const Tensor h = dense(h_), w1 = dense(w1_), w2 = dense(w2_);
     e.u = at::empty({h.size(0), h.size(1), w1.size(2)}, h.options());
     e.act = at::empty_like(e.u);
@@ -555,14 +561,15 @@ Tensor plainCombined(const Tensor& x, const Tensor& gate, const Tensor& rows, co
 // forward and backward: 300 us in pieces, 210 in one.)
 class MoeLayer : public torch::autograd::Function<MoeLayer> {
  public:
-  static Variable forward(AutogradContext* ctx, const Variable& x_, const Variable& router, const Variable& w1, const Variable& w2, int64_t capacity) {
+  static Variable forward(AutogradContext* ctx, const Variable& x_, const Variable& router, const Variable& w1, const Variable& w2, int64_t capacity,
+                          bool alone) {
     c10::cuda::CUDAGuard dg(x_.device());
     const Tensor x = dense(x_);
     const Routed r = moeRouted(x, router, capacity);
     const Tensor h = r.send.view({router.size(0), capacity, x.size(1)});
     // Hooks on saved tensors see all of them, and may scale what they keep by its largest value: rows out of use are computed then (zeros).
     const Tensor count = at::SavedTensorDefaultHooks::get_hooks() ? Tensor() : r.count;
-    const Expert e = moeExpert(h, w1, w2, count);
+    const Expert e = moeExpert(h, w1, w2, count, alone);
     ctx->save_for_backward({x_, router, w1, w2, r.logits, r.expert, r.gate, r.row_of, r.token_of, h, e.u, e.act, e.out, count});
     ctx->saved_data["own"] = e.own;
     return moeCombined(x, r.gate, e.out, r.row_of);
@@ -575,7 +582,7 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
       const variable_list in = {viewOf(s[0]), viewOf(router), viewOf(w1), viewOf(w2)};
       const Tensor out = plainExperts(plainRows(in[0], s[8]).view(h.sizes()), in[2], in[3]);
       variable_list r = recorded({plainCombined(in[0], plainGate(in[0], in[1], s[5]), out, s[7])}, g, in);
-      r.emplace_back();
+      r.resize(6);
       return r;
     }
     const Tensor x = dense(s[0]), rows = dense(s[12]);
@@ -583,10 +590,10 @@ class MoeLayer : public torch::autograd::Function<MoeLayer> {
     const auto [drows, dgate] = moeCombinedBackward(dy, s[6], rows, s[8], false);
     const variable_list e = moeExpertBackward(h, w1, w2, s[10], s[11], drows, ctx->saved_data["own"].toBool(), s[13], needed(ctx, 0), needed(ctx, 2),
                                               needed(ctx, 3));
-    if (!needed(ctx, 0, 1)) return {Tensor(), Tensor(), e[1], e[2], Tensor()};
+    if (!needed(ctx, 0, 1)) return {Tensor(), Tensor(), e[1], e[2], Tensor(), Tensor()};
     const Tensor dsend = e[0].defined() ? e[0] : at::zeros_like(h);   // the router alone
     const auto [dx, drouter] = moeRoutedBackward(x, router, s[4], s[5], s[6], s[7], dy, dsend, dgate, needed(ctx, 1));
-    return {dx, drouter, e[1], e[2], Tensor()};
+    return {dx, drouter, e[1], e[2], Tensor(), Tensor()};
   }
 };
 
@@ -627,9 +634,9 @@ class MoeDispatch : public torch::autograd::Function<MoeDispatch> {
 // out = gelu(h W1) W2, per expert.
 class MoeExperts : public torch::autograd::Function<MoeExperts> {
  public:
-  static Variable forward(AutogradContext* ctx, const Variable& h, const Variable& w1, const Variable& w2) {
+  static Variable forward(AutogradContext* ctx, const Variable& h, const Variable& w1, const Variable& w2, bool alone) {
     c10::cuda::CUDAGuard dg(h.device());
-    const Expert e = moeExpert(h, w1, w2, Tensor());
+    const Expert e = moeExpert(h, w1, w2, Tensor(), alone);
     ctx->save_for_backward({h, w1, w2, e.u, e.act});
     ctx->saved_data["own"] = e.own;
     return e.out;
@@ -639,10 +646,14 @@ class MoeExperts : public torch::autograd::Function<MoeExperts> {
     c10::cuda::CUDAGuard dg(s[0].device());
     if (wantsGraph()) {
       const variable_list in = {viewOf(s[0]), viewOf(s[1]), viewOf(s[2])};
-      return recorded({plainExperts(in[0], in[1], in[2])}, g, in);
+      variable_list r = recorded({plainExperts(in[0], in[1], in[2])}, g, in);
+      r.emplace_back();
+      return r;
     }
-    return moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), ctx->saved_data["own"].toBool(), Tensor(), needed(ctx, 0), needed(ctx, 1),
-                             needed(ctx, 2));
+    variable_list r = moeExpertBackward(s[0], s[1], s[2], s[3], s[4], dense(g[0]), ctx->saved_data["own"].toBool(), Tensor(), needed(ctx, 0),
+                                        needed(ctx, 1), needed(ctx, 2));
+    r.emplace_back();
+    return r;
   }
 };
 
@@ -856,19 +867,22 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("block_pre", [](const Tensor& x, const std::optional<Tensor>& y, const Tensor& gamma, const Tensor& beta, const Tensor& w, const Tensor& b,
                         int64_t heads, double eps) { return BlockPre::apply(x, y, gamma, beta, w, b, heads, eps); });
+  // `alone`: see ownExperts
+  using py::arg;
   m.def("block_post", [](const Tensor& x, const Tensor& a, const Tensor& wp, const Tensor& bp, const Tensor& gamma, const Tensor& beta,
-                         const Tensor& wf, const Tensor& bf, const Tensor& wo, const Tensor& bo, double eps) {
-    return BlockPost::apply(x, a, wp, bp, gamma, beta, wf, bf, wo, bo, eps);
-  });
-  m.def("moe_layer", [](const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w2, int64_t capacity) {
-    return MoeLayer::apply(x, router, w1, w2, capacity);
-  });
+                         const Tensor& wf, const Tensor& bf, const Tensor& wo, const Tensor& bo, double eps, bool alone) {
+    return BlockPost::apply(x, a, wp, bp, gamma, beta, wf, bf, wo, bo, eps, alone);
+  }, arg(), arg(), arg(), arg(), arg(), arg(), arg(), arg(), arg(), arg(), arg(), arg("alone") = true);
+  m.def("moe_layer", [](const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w2, int64_t capacity, bool alone) {
+    return MoeLayer::apply(x, router, w1, w2, capacity, alone);
+  }, arg(), arg(), arg(), arg(), arg(), arg("alone") = true);
   m.def("check_products", [](int device) { ok(train::gemmStatus(device, true), "products"); });
   m.def("product_without_operands", &productWithoutOperands);
   m.def("multi_adamw", &multiAdamW);
   m.def("accumulation_hooks", &accumulationHooks);
   m.def("moe_dispatch", [](const Tensor& x, const Tensor& router, int64_t capacity) { return MoeDispatch::apply(x, router, capacity); });
-  m.def("moe_experts", [](const Tensor& h, const Tensor& w1, const Tensor& w2) { return MoeExperts::apply(h, w1, w2); });
+  m.def("moe_experts", [](const Tensor& h, const Tensor& w1, const Tensor& w2, bool alone) { return MoeExperts::apply(h, w1, w2, alone); }, arg(), arg(),
+        arg(), arg("alone") = true);
   m.def("moe_combine", [](const Tensor& x, const Tensor& gate, const Tensor& rows, const Tensor& row_of, const Tensor& token_of) {
     return MoeCombine::apply(x, gate, rows, row_of, token_of);
   });

@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.extension import global_module_hooks, ops, overridden, plain_eager, traced
+from ..ops.extension import alone, global_module_hooks, ops, overridden, plain_eager, traced
 
 
 @dataclass
@@ -143,7 +143,7 @@ class GPT2(nn.Module):
         if torch._C._autograd._top_saved_tensors_default_hooks(False) is not None:
             return None
         cuda = torch.backends.cuda
-        flags = (torch.are_deterministic_algorithms_enabled(), cuda.flash_sdp_enabled(), cuda.mem_efficient_sdp_enabled(), cuda.cudnn_sdp_enabled(),
+        flags = (alone(), torch.are_deterministic_algorithms_enabled(), cuda.flash_sdp_enabled(), cuda.mem_efficient_sdp_enabled(), cuda.cudnn_sdp_enabled(),
                  cuda.math_sdp_enabled(), cuda.fp16_bf16_reduction_math_sdp_allowed(), tuple(torch._C._get_sdp_priority_order()),
                  torch._C._get_cublas_allow_bf16_reduced_precision_reduction(), torch._C._get_cublas_allow_fp16_reduced_precision_reduction(),
                  cuda.matmul.allow_fp16_accumulation, torch._C._get_blas_preferred_backend())
@@ -154,12 +154,13 @@ class GPT2(nn.Module):
     def _fused_loss(self, x: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
         f = ops()
         b, t, d = x.shape
+        by_itself = alone()
         branch = None      # what the block before adds to the residual stream: the next layer norm reads both
         for blk in self.blocks:
             x, q, k, v = f.block_pre(x, branch, blk.ln1.weight, blk.ln1.bias, blk.qkv.weight, blk.qkv.bias, blk.n_head, blk.ln1.eps)
             a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
             x, branch = f.block_post(x, a.transpose(1, 2).reshape(b, t, d), blk.proj.weight, blk.proj.bias, blk.ln2.weight, blk.ln2.bias,
-                                     blk.fc.weight, blk.fc.bias, blk.out.weight, blk.out.bias, blk.ln2.eps)
+                                     blk.fc.weight, blk.fc.bias, blk.out.weight, blk.out.bias, blk.ln2.eps, by_itself)
         h = f.add_norm(x, branch, self.ln_f.weight, self.ln_f.bias, self.ln_f.eps)
         return f.head_loss(h, self.wte.weight, targets)
 

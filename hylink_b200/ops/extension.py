@@ -6,6 +6,7 @@ import importlib.util
 from pathlib import Path
 
 import torch
+import torch.distributed as dist
 from torch.autograd import forward_ad
 from torch.nn.modules import module as _modules
 from torch.utils._device import DeviceContext
@@ -36,6 +37,11 @@ def check_products(device: int | None = None) -> None:
     since the last call: results that came after it are not valid. To be called where the host has waited for results;
     ``DDPTrainer.step`` does. Launches of further products raise too until then."""
     ops().check_products(-1 if device is None else device)
+
+
+def alone() -> bool:
+    """Whether this process is a job by itself: with several ranks, collectives hold multiprocessors beside the products."""
+    return not (dist.is_available() and dist.is_initialized() and dist.get_world_size() > 1)
 
 
 def overridden(m) -> bool:

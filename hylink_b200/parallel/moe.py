@@ -17,7 +17,7 @@ import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.extension import global_module_hooks, ops, overridden, plain_eager, traced
+from ..ops.extension import alone, global_module_hooks, ops, overridden, plain_eager, traced
 
 
 class _AllToAll(torch.autograd.Function):
@@ -92,12 +92,12 @@ class ExpertParallelMLP(nn.Module):
     def _fused(self, x):
         f, d = ops(), x.shape[1]
         if self.n == 1 and self.w1.dtype == x.dtype and self.w2.dtype == x.dtype:
-            return f.moe_layer(x, self.router.weight, self.w1, self.w2, self.cap)
+            return f.moe_layer(x, self.router.weight, self.w1, self.w2, self.cap, alone())
         x, send, gate, row_of, token_of = f.moe_dispatch(x, self.router.weight, self.cap)
         # rows are ordered (destination rank, local expert, slot); with one rank they are where they belong
         recv = all_to_all(send, self.group) if self.n > 1 else send
         h = recv.view(self.n, self.epr, self.cap, d).transpose(0, 1).reshape(self.epr, self.n * self.cap, d)
-        h = f.moe_experts(h, self.w1.to(h.dtype), self.w2.to(h.dtype))
+        h = f.moe_experts(h, self.w1.to(h.dtype), self.w2.to(h.dtype), alone())
         back = h.view(self.epr, self.n, self.cap, d).transpose(0, 1).reshape(self.n_experts * self.cap, d)
         got = all_to_all(back, self.group) if self.n > 1 else back
         return f.moe_combine(x, gate, got, row_of, token_of)

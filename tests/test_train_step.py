@@ -695,3 +695,41 @@ def test_the_products_bits_are_the_librarys(tmp_path):
             assert bool(((a - b).abs().double() <= 2.0 ** -7 * b.abs().double() + 2.0 ** -16).all()), name
         else:
             assert torch.equal(a, b), name
+
+
+def test_products_of_a_job_of_several_ranks_are_the_librarys(monkeypatch):
+    """The own products deal their tiles out to an empty GPU's multiprocessors; gradient all-reduces of other ranks hold some of them."""
+    import torch.distributed as dist
+
+    from hylink_b200.models.gpt2 import GPT2, GPT2Config
+    from hylink_b200.parallel.moe import ExpertParallelMLP
+    from hylink_b200.parallel.trainer import init_distributed
+
+    monkeypatch.setenv("MASTER_PORT", "29576")
+    init_distributed("hylink")
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        model = GPT2(GPT2Config(n_layer=1, vocab_size=1024)).to(torch.bfloat16)                              # 2048 tokens: 2^33
+        layer = ExpertParallelMLP(512, 2048, experts_per_rank=2, capacity=128).to(torch.bfloat16)            # 2^28
+    idx = torch.randint(0, 1024, (2, 1024), device="cuda")
+    x = torch.randn(200, 512, device="cuda").to(torch.bfloat16)
+
+    def step():
+        model.zero_grad(set_to_none=True)
+        layer.zero_grad(set_to_none=True)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+            loss = model(idx, idx)
+            loss.backward()
+            y = layer(x)
+            y.sum().backward()
+            torch.cuda.synchronize()
+        return (loss.detach(), y.detach(), *(q.grad for m in (layer, model.blocks) for q in m.parameters())), sum("kExpertGemm" in e.name for e in p.events())
+
+    one, launches = step()
+    assert launches > 3                              # MLP: one each way; experts: two each way
+    monkeypatch.setattr(dist, "get_world_size", lambda group=None: 2)
+    two, launches = step()
+    assert launches == 0
+    assert torch.equal(one[0], two[0]) and torch.equal(one[1], two[1])
+    for a, b in zip(one[2:], two[2:]):               # attention's own backward pass adds up in any order
+        assert float((a - b).float().norm()) <= 2.0 ** -7 * float(b.float().norm())
