@@ -1,7 +1,8 @@
 // Autograd functions of the training step over the kernels of csrc/train: what surrounds the GEMMs and the attention
 // of a transformer block, the language-model head with its loss, the mixture-of-experts layer; the optimizers; and the
-// launches of emulated collectives and of the landing reduce. The GEMMs are torch's own (cuBLAS), the attention between
-// the two halves of a block is whatever torch's scaled_dot_product_attention picks.
+// launches of emulated collectives and of the landing reduce. Products that gelu or its gradient follows go through the kernel of
+// train/expert_gemm.cu where that pays, and so do an expert layer's others; the rest of the GEMMs are torch's own (cuBLAS), the
+// attention between the two halves of a block is whatever torch's scaled_dot_product_attention picks.
 //
 // A block is cut in two around the attention:
 //   blockPre:   x1 = x + y; h = layer norm(x1); q, k, v = h Wqkv^T + b     (y: the branch of the block before)

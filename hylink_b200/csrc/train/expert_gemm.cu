@@ -10,19 +10,21 @@
 //   warp 1      products, in the pair's first CTA alone
 //   warps 4-11  epilogue: chunks of 32 x 32, rounded, transposed by stmatrix through shared memory of the warp's own (two
 //               places of 2 KB in turn), and stored as rows of 64 bytes; no warp waits for another. (Chunks of 128 x 32 that leave by TMA, with barriers of 128 threads: 75 us
-//               where this takes 67.)
+//               where this takes 67; both with a reciprocal for four of gelu's values.)
 // Loads and products run in all lanes of their warps up to the instruction itself, so that its operands are in uniform
 // registers: in a branch of one lane the same loops took 86 us instead of 57.
 //
 // The tokens are n, the weights' rows are m: an expert's last tile is as wide as its tokens need, in steps of 32, where rows of
-// tokens as m would come in steps of 256. The layer's capacity (1.25 times the average in use) costs nothing then: tiles
-// and k end at the `counts` that routing found, rounded up to 32. Rows between a count and the rounding are zeros.
+// tokens as m would come in steps of 256. Where routing is part of the call, the layer's capacity (1.25 times the average in use) costs
+// nothing then: tiles and k end at the `counts` that it found, rounded up to 32. Rows between a count and the rounding are zeros.
 //
-// 8 x 1024 x 1024 x 4096 in bf16, 69 GFLOP, back to back for a second, under the power cap: 62 to 64 us without an epilogue (the library 61.5 to
-// 67), 77 to 80 with gelu (the library's product 65, gelu alone 21), 88 with its gradient (67 and 30); in short runs 54, 67 and 74. Bound by power
-// without an epilogue, with one by its warps. Tried: pairs of 512 x 256 with one set of accumulators, which read a quarter less (55 us, 75
-// with gelu: the epilogue then has half the time), also with sixteen epilogue warps (58, 72).
-// The sums go up k in the order of the library's own kernels: results are theirs, bit for bit, where this was compared.
+// 8 x 1024 x 1024 x 4096 in bf16, 69 GFLOP a product, every row in use, us here / the library with gelu's passes. Short runs: with gelu 71 / 55 + 26,
+// k = 4096 54.6 / 48, gelu's gradient 82 / 55 + 41, the product behind it 52.5 / 48, the gradient with dW2 124 / 55 + 41 + 55, dW1 with dh 99 / 55 + 47.
+// Back to back for a second, under the power cap, forward and backward: 95 + 67 + 156 + 119 here, 447 there in eight. So with every row in use
+// the two are even; a layer gains by the rows that are not (8192 tokens, 622 -> 510). Bound by power without an epilogue, with one by its
+// warps. Tried: pairs of 512 x 256 with one set of accumulators, which read a quarter less (55 us for k = 4096; slower with gelu, whose
+// epilogue then has half the time), also with sixteen epilogue warps (58).
+// The sums go up k in the order of the library's own kernels: results are theirs, bit for bit (the tests compare the two).
 // Every wait is bounded; one that runs out sets the device's status word, which stays set until gemmStatus has reported it: to whoever
 // waits for the results (a trainer after its step, replayed from a graph or not), and to every launch until then.
 #include <cuda.h>
@@ -437,8 +439,8 @@ bool expertGemmPays(int64_t rows, int64_t width, int64_t hidden, bool captured) 
   return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (captured ? 1LL << 33 : 1LL << 24);
 }
 // One product with a bias, which the library's kernels take too: what is gained is the element-wise pass alone, and that once the tiles fill
-// the GPU. Training steps, ms own / library: 4096 rows of 768 x 3072 8.49 / 8.56, 3072 of 1024 x 4096 14.51 / 14.62, 8192
-// 29.5 / 30.4; 1024 rows 9.11 / 9.06, 512 7.71 / 7.53, 256 7.47 / 7.02.
+// the GPU. Training steps, ms own / library: 8192 rows of 1024 x 4096 27.65 / 27.94 (four runs each in turn, which differ by 0.1), 3072 12.93 /
+// 12.94, 4096 of 768 x 3072 7.68 / 7.68, 8192 13.36 / 13.36; below the line 1024 rows of 1024 x 4096 9.11 / 9.06, 512 7.71 / 7.53, 256 7.47 / 7.02.
 bool mlpGemmPays(int64_t rows, int64_t width, int64_t hidden) {
   return width % 8 == 0 && hidden % 8 == 0 && rows * width * hidden >= (1LL << 33);
 }
